@@ -28,6 +28,7 @@
 #include "urgent.cuh"
 #include "stream_step.cuh"
 #include "tiled.cuh"
+#include "record.cuh"
 
 #include <cub/device/device_scan.cuh>
 
@@ -57,6 +58,7 @@ int fail(int code, const char *fmt, ...)
         }                                                                                        \
     } while(0)
 
+constexpr size_t STAGE_BYTES = 256 * 1024;  // page-locked buffer of a runner through which small arrays reach pageable memory
 constexpr size_t ARRAY_TAIL_PAD = 256;     // vector loads may read up to 15 bytes past the last element
 
 template<typename T>
@@ -98,6 +100,10 @@ struct Timer
 };
 }   // anonymous namespace
 
+// (Everything the host writes into device memory goes through the runner's stream, which does not wait for the legacy one:
+// a plain cudaMemcpy may return while its transfer is still on the way, and a kernel launched behind it on another stream
+// would read what was there before.)
+
 // Device buffer that is freed on every early return of a build function unless it was handed over.
 struct ScopedDevice
 {
@@ -118,6 +124,13 @@ struct b200_runner
     cudaStream_t stream = nullptr;
     StepState *state = nullptr;
     std::unordered_map<void*, size_t> arrays;
+    unsigned char *stage = nullptr;         // STAGE_BYTES, page-locked: pulls of small arrays land here
+    unsigned int *hostWord = nullptr;       // page-locked: the device's error word
+    // recording list (record.cuh): chunk counts, header and pairs on the device, header and pairs on the host
+    unsigned int *recCounts = nullptr;
+    RecordHeader *recList = nullptr, *recHost = nullptr;
+    size_t recChunks = 0, recCapacity = 0;
+    size_t recLast = 0;                     // pairs of the last pull
 
     std::vector<b200_neuron_group> neuronGroups;
     std::vector<b200_synapse_group> synapseGroups;
@@ -455,12 +468,12 @@ int buildFusedTables(b200_runner *r)
         if(e) return e;
     }
     CUDA_TRY(cudaMalloc(&r->fusedSlotStart, sizeof(unsigned int) * slotStart.size()));
-    CUDA_TRY(cudaMemcpy(r->fusedSlotStart, slotStart.data(), sizeof(unsigned int) * slotStart.size(), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->fusedSlotStart, slotStart.data(), sizeof(unsigned int) * slotStart.size(), cudaMemcpyHostToDevice, r->stream));
     if(!sources.empty()) {
         CUDA_TRY(cudaMalloc(&r->fusedSources, sizeof(FusedSource) * sources.size()));
-        CUDA_TRY(cudaMemcpy(r->fusedSources, sources.data(), sizeof(FusedSource) * sources.size(), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(r->fusedSources, sources.data(), sizeof(FusedSource) * sources.size(), cudaMemcpyHostToDevice, r->stream));
         CUDA_TRY(cudaMalloc(&r->fusedItems, sizeof(uint2) * items.size()));
-        CUDA_TRY(cudaMemcpy(r->fusedItems, items.data(), sizeof(uint2) * items.size(), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(r->fusedItems, items.data(), sizeof(uint2) * items.size(), cudaMemcpyHostToDevice, r->stream));
     }
     if(!r->fusedBarrier) CUDA_TRY(cudaMalloc(&r->fusedBarrier, sizeof(unsigned long long)));
     int perSM = r->fusedPerSM, sms = 0, coop = 0;
@@ -553,9 +566,8 @@ int prepare(b200_runner *r)
             fold(g.max_den_delay);
         }
         if(period > (1ull << 30)) return fail(B200_ERR_INVALID, "ring sizes have no common period below 2^30");
-        CUDA_TRY(cudaStreamSynchronize(r->stream));
         const unsigned int ring[2] = {(unsigned int)(r->hostStepsDone % period), (unsigned int)period};
-        CUDA_TRY(cudaMemcpy(&r->state->phase, ring, sizeof(ring), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(&r->state->phase, ring, sizeof(ring), cudaMemcpyHostToDevice, r->stream));
     }
     r->dirty = false;
     return B200_OK;
@@ -694,9 +706,9 @@ int buildNearTables(b200_runner *r, bool forExport = false)
     std::vector<NearSpace> spaces(numNeuronGroups);
     for(size_t ni = 0; ni < numNeuronGroups; ni++) spaces[ni] = NearSpace{r->nearTable + firstCell[ni], shifts[ni], 0u, shifts[ni], 0u};
     CUDA_TRY(cudaMalloc(&r->nearRings, sizeof(NearRing) * rings.size()));
-    CUDA_TRY(cudaMemcpy(r->nearRings, rings.data(), sizeof(NearRing) * rings.size(), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->nearRings, rings.data(), sizeof(NearRing) * rings.size(), cudaMemcpyHostToDevice, r->stream));
     CUDA_TRY(cudaMalloc(&r->nearSpaces, sizeof(NearSpace) * spaces.size()));
-    CUDA_TRY(cudaMemcpy(r->nearSpaces, spaces.data(), sizeof(NearSpace) * spaces.size(), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->nearSpaces, spaces.data(), sizeof(NearSpace) * spaces.size(), cudaMemcpyHostToDevice, r->stream));
     r->schedule = b200_runner::EMIT;
     return B200_OK;
 }
@@ -1126,7 +1138,7 @@ int buildTiled(b200_runner *r)
     for(const auto &T : tiles) smem = std::max(smem, sizeof(float) * T.depth * T.stride);
     auto toDevice = [&](const void *host, size_t bytes, void **out) -> int {
         CUDA_TRY(cudaMalloc(out, std::max<size_t>(bytes, 16)));
-        CUDA_TRY(cudaMemcpy(*out, host, bytes, cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(*out, host, bytes, cudaMemcpyHostToDevice, r->stream));
         return B200_OK;
     };
     int e = toDevice(tiles.data(), sizeof(TiledTile) * tiles.size(), (void**)&r->tiledTiles);
@@ -1354,15 +1366,17 @@ int b200_runner_create(int device, double dt, uint64_t seed, uint32_t batch_size
     r->batch = batch_size;
     CUDA_TRY(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking));
     CUDA_TRY(cudaMalloc(&r->state, sizeof(StepState)));
-    CUDA_TRY(cudaMemset(r->state, 0, sizeof(StepState)));
+    CUDA_TRY(cudaMemsetAsync(r->state, 0, sizeof(StepState), r->stream));
     {
         const unsigned long long limits[3] = {BARRIER_SPIN_LIMIT, EXCHANGE_SPIN_LIMIT, (unsigned long long)STREAM_WAIT_CYCLES};
-        CUDA_TRY(cudaMemcpy(&r->state->barrier_spin_limit, limits, sizeof(limits), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(&r->state->barrier_spin_limit, limits, sizeof(limits), cudaMemcpyHostToDevice, r->stream));
     }
     CUDA_TRY(cudaEventCreate(&r->evA));
     CUDA_TRY(cudaEventCreate(&r->evB));
     CUDA_TRY(cudaEventCreate(&r->evC));
     CUDA_TRY(cudaEventCreate(&r->evD));
+    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&r->stage), STAGE_BYTES + 64, cudaHostAllocPortable));
+    r->hostWord = reinterpret_cast<unsigned int*>(r->stage + STAGE_BYTES);
     *out = r;
     return B200_OK;
 }
@@ -1430,6 +1444,10 @@ int b200_runner_destroy(b200_runner *r)
     for(unsigned int p = 0; p < B200_MAX_RANKS; p++) {
         if(r->peerArena[p] && !r->peerLocal[p]) cudaIpcCloseMemHandle(r->peerArena[p]);
     }
+    if(r->stage) cudaFreeHost(r->stage);
+    if(r->recCounts) cudaFree(r->recCounts);
+    if(r->recList) cudaFree(r->recList);
+    if(r->recHost) cudaFreeHost(r->recHost);
     if(r->peakHost) cudaFreeHost(r->peakHost);
     if(r->peakEvent) cudaEventDestroy(r->peakEvent);
     if(r->ncclComm && ncclApi()) ncclApi()->commDestroy(r->ncclComm);
@@ -1491,7 +1509,8 @@ int b200_exchange_alloc(b200_runner *r, size_t bytes, void **device_ptr)
     void *p = nullptr;
     const size_t total = exchangeTotalBytes(bytes);
     CUDA_TRY(cudaMalloc(&p, total));
-    CUDA_TRY(cudaMemset(p, 0, total));
+    CUDA_TRY(cudaMemsetAsync(p, 0, total, r->stream));
+    CUDA_TRY(cudaStreamSynchronize(r->stream));         // (peers write into it as soon as they know its handle)
     r->arena = static_cast<unsigned char*>(p);
     r->arenaBytes = bytes;
     r->queueOffset = exchangeQueueOffset(bytes);
@@ -1527,7 +1546,7 @@ int b200_exchange_open_peer(b200_runner *r, uint32_t peer_rank, const void *hand
     CUDA_TRY(cudaIpcOpenMemHandle(&p, h, cudaIpcMemLazyEnablePeerAccess));
     r->peerArena[peer_rank] = static_cast<unsigned char*>(p);
     if(!r->peerTable) CUDA_TRY(cudaMalloc(&r->peerTable, sizeof(unsigned char*) * B200_MAX_RANKS));
-    CUDA_TRY(cudaMemcpy(r->peerTable, r->peerArena, sizeof(unsigned char*) * B200_MAX_RANKS, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->peerTable, r->peerArena, sizeof(unsigned char*) * B200_MAX_RANKS, cudaMemcpyHostToDevice, r->stream));
     return B200_OK;
 }
 
@@ -1538,7 +1557,7 @@ int b200_exchange_set_peer(b200_runner *r, uint32_t peer_rank, void *device_ptr)
     CUDA_TRY(cudaSetDevice(r->device));
     r->peerArena[peer_rank] = static_cast<unsigned char*>(device_ptr);
     if(!r->peerTable) CUDA_TRY(cudaMalloc(&r->peerTable, sizeof(unsigned char*) * B200_MAX_RANKS));
-    CUDA_TRY(cudaMemcpy(r->peerTable, r->peerArena, sizeof(unsigned char*) * B200_MAX_RANKS, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->peerTable, r->peerArena, sizeof(unsigned char*) * B200_MAX_RANKS, cudaMemcpyHostToDevice, r->stream));
     r->peerLocal[peer_rank] = true;
     return B200_OK;
 }
@@ -1605,13 +1624,13 @@ int b200_near_import(b200_runner *r, uint32_t peer_rank, const void *handle_64_b
         const size_t rowCells = (size_t)1 << (common + worldShift);
         if(!r->nearImported[ni]) {
             CUDA_TRY(cudaMalloc(&r->nearImported[ni], sizeof(uint2) * (rowCells * ng.num_update + 1)));
-            CUDA_TRY(cudaMemset(r->nearImported[ni], 0, sizeof(uint2) * (rowCells * ng.num_update + 1)));
+            CUDA_TRY(cudaMemsetAsync(r->nearImported[ni], 0, sizeof(uint2) * (rowCells * ng.num_update + 1), r->stream));
             r->nearSpacesAll[ni] = NearSpace{r->nearImported[ni], common + worldShift, ng.first_neuron, common, 0u};
         }
         if(ng.num_update) {
-            CUDA_TRY(cudaMemcpy2D(r->nearImported[ni] + ((size_t)peer_rank << common), sizeof(uint2) * rowCells,
+            CUDA_TRY(cudaMemcpy2DAsync(r->nearImported[ni] + ((size_t)peer_rank << common), sizeof(uint2) * rowCells,
                                   table + meta[3 + 2 * ni] + ((size_t)ng.first_neuron << shift), sizeof(uint2) << shift,
-                                  sizeof(uint2) << shift, ng.num_update, cudaMemcpyDeviceToDevice));
+                                  sizeof(uint2) << shift, ng.num_update, cudaMemcpyDeviceToDevice, r->stream));
         }
     }
     CUDA_TRY(cudaDeviceSynchronize());
@@ -1651,9 +1670,9 @@ int b200_near_finish(b200_runner *r, int agreed)
     if(r->nearRings) cudaFree(r->nearRings);
     if(r->nearSpaces) cudaFree(r->nearSpaces);
     CUDA_TRY(cudaMalloc(&r->nearRings, sizeof(NearRing) * rings.size()));
-    CUDA_TRY(cudaMemcpy(r->nearRings, rings.data(), sizeof(NearRing) * rings.size(), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->nearRings, rings.data(), sizeof(NearRing) * rings.size(), cudaMemcpyHostToDevice, r->stream));
     CUDA_TRY(cudaMalloc(&r->nearSpaces, sizeof(NearSpace) * r->nearSpacesAll.size()));
-    CUDA_TRY(cudaMemcpy(r->nearSpaces, r->nearSpacesAll.data(), sizeof(NearSpace) * r->nearSpacesAll.size(), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(r->nearSpaces, r->nearSpacesAll.data(), sizeof(NearSpace) * r->nearSpacesAll.size(), cudaMemcpyHostToDevice, r->stream));
     r->emitAgreed = true;
     r->queuesAgreed = r->fusedGrid <= NEAR_QUEUE_COUNT;
     for(uint32_t p = 0; p < r->world; p++) {
@@ -1694,6 +1713,14 @@ int b200_array_push(b200_runner *r, void *device_ptr, const void *host, size_t b
 
 int b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t bytes)
 {
+    if(bytes <= STAGE_BYTES) {
+        // to page-locked memory and on from there: the driver's own way into pageable memory takes 15 us however
+        // few the bytes, this one 8 (40 KB)
+        CUDA_TRY(cudaMemcpyAsync(r->stage, device_ptr, bytes, cudaMemcpyDeviceToHost, r->stream));
+        CUDA_TRY(cudaStreamSynchronize(r->stream));
+        memcpy(host, r->stage, bytes);
+        return B200_OK;
+    }
     CUDA_TRY(cudaMemcpyAsync(host, device_ptr, bytes, cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     return B200_OK;
@@ -1824,7 +1851,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
         if(r->fusedProfile && !r->fusedCtaCycles) {
             CUDA_TRY(cudaSetDevice(r->device));
             CUDA_TRY(cudaMalloc(&r->fusedCtaCycles, sizeof(unsigned long long) * 5 * PROFILE_MAX_CTAS));
-            CUDA_TRY(cudaMemset(r->fusedCtaCycles, 0, sizeof(unsigned long long) * 5 * PROFILE_MAX_CTAS));
+            CUDA_TRY(cudaMemsetAsync(r->fusedCtaCycles, 0, sizeof(unsigned long long) * 5 * PROFILE_MAX_CTAS, r->stream));
         }
     }
     else if(n == "fused_blocks_per_sm") { r->fusedBlocksPerSM = (unsigned int)value; r->dirty = true; }
@@ -1838,7 +1865,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
                                 : (n == "exchange_spin_limit") ? &r->state->exchange_spin_limit
                                 : reinterpret_cast<unsigned long long*>(&r->state->stream_wait_cycles);
         CUDA_TRY(cudaStreamSynchronize(r->stream));
-        CUDA_TRY(cudaMemcpy(dst, &v, sizeof(v), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(dst, &v, sizeof(v), cudaMemcpyHostToDevice, r->stream));
     }
     else if(n == "use_tiled") { r->useTiled = (value != 0.0); r->tiledStale = true; }
     else if(n == "tiled_min_events") r->tiledMinEvents = (float)value;
@@ -2119,22 +2146,24 @@ int b200_custom_update_broadcast(b200_runner *r, const char *name)
     return runCustomUpdate(r, name, 2u);
 }
 
+// The device's error word as a status.  A time-out leaves every CTA out of the kernel: the word is cleared for the next one.
+static int reportDeviceError(b200_runner *r, unsigned int err)
+{
+    if(!err) return B200_OK;
+    cudaMemsetAsync(&r->state->error, 0, sizeof(unsigned int), r->stream);
+    return fail(B200_ERR_DEVICE_CHECK, "device-side check failed (flags 0x%x:%s%s%s%s%s)", err,
+                (err & ERR_SPIKE_OVERFLOW) ? " spike list overflow" : "",
+                (err & ERR_IND_RANGE) ? " index or row length out of range" : "",
+                (err & ERR_DELAY_RANGE) ? " a synapse arriving in the same step appeared after the schedule was chosen (option rescan_delays)" : "",
+                (err & ERR_BARRIER_TIMEOUT) ? " grid barrier timed out" : "",
+                (err & ERR_EXCHANGE_TIMEOUT) ? " spikes of another process did not arrive in time" : "");
+}
+
 int b200_synchronize(b200_runner *r)
 {
+    CUDA_TRY(cudaMemcpyAsync(r->hostWord, &r->state->error, sizeof(unsigned int), cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
-    StepState s;
-    CUDA_TRY(cudaMemcpy(&s, r->state, sizeof(s), cudaMemcpyDeviceToHost));
-    if(s.error) {
-        const unsigned int err = s.error;
-        cudaMemset(&r->state->error, 0, sizeof(unsigned int));
-        return fail(B200_ERR_DEVICE_CHECK, "device-side check failed (flags 0x%x:%s%s%s%s%s)", err,
-                    (err & ERR_SPIKE_OVERFLOW) ? " spike list overflow" : "",
-                    (err & ERR_IND_RANGE) ? " index or row length out of range" : "",
-                    (err & ERR_DELAY_RANGE) ? " a synapse arriving in the same step appeared after the schedule was chosen (option rescan_delays)" : "",
-                    (err & ERR_BARRIER_TIMEOUT) ? " grid barrier timed out" : "",
-                    (err & ERR_EXCHANGE_TIMEOUT) ? " spikes of another process did not arrive in time" : "");
-    }
-    return B200_OK;
+    return reportDeviceError(r, *r->hostWord);
 }
 
 int b200_get_timestep(b200_runner *r, uint64_t *timestep)
@@ -2145,9 +2174,8 @@ int b200_get_timestep(b200_runner *r, uint64_t *timestep)
 
 int b200_set_timestep(b200_runner *r, uint64_t timestep)
 {
-    CUDA_TRY(cudaStreamSynchronize(r->stream));
     const unsigned long long t = timestep;
-    CUDA_TRY(cudaMemcpy(&r->state->timestep, &t, sizeof(t), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(&r->state->timestep, &t, sizeof(t), cudaMemcpyHostToDevice, r->stream));
     r->hostTimestep = timestep;
     return B200_OK;
 }
@@ -2315,6 +2343,114 @@ int b200_compact_words(b200_runner *r, const uint32_t *words, uint64_t num_words
     CUDA_TRY(cudaPeekAtLastError());
     r->launches++;
     return B200_OK;
+}
+
+int b200_pull_recording(b200_runner *r, uint32_t num_arrays, const uint32_t *const *words, const uint64_t *num_words,
+                        uint32_t capacity, const void **pairs, uint64_t *num_pairs)
+{
+    if(!r || (num_arrays && (!words || !num_words)) || !pairs || !num_pairs) return fail(B200_ERR_INVALID, "null argument to b200_pull_recording");
+    CUDA_TRY(cudaSetDevice(r->device));
+    *pairs = nullptr;
+    *num_pairs = 0;
+    uint64_t total = 0, chunks = 0;
+    for(uint32_t i = 0; i < num_arrays; i++) {
+        total += num_words[i];
+        chunks += (num_words[i] + RECORD_CHUNK - 1) / RECORD_CHUNK;
+    }
+    if(total > 0xFFFFFFFFull) return fail(B200_ERR_INVALID, "word indices beyond 32 bits");
+    if(chunks == 0) return b200_synchronize(r);
+    if(chunks > r->recChunks || capacity > r->recCapacity) {
+        CUDA_TRY(cudaStreamSynchronize(r->stream));
+        if(r->recCounts) cudaFree(r->recCounts);
+        if(r->recList) cudaFree(r->recList);
+        if(r->recHost) cudaFreeHost(r->recHost);
+        r->recCounts = nullptr; r->recList = nullptr; r->recHost = nullptr;
+        r->recChunks = r->recCapacity = 0;
+        const size_t bytes = sizeof(RecordHeader) + sizeof(uint2) * (size_t)capacity;
+        CUDA_TRY(cudaMalloc(&r->recCounts, sizeof(unsigned int) * chunks));
+        CUDA_TRY(cudaMalloc(&r->recList, bytes));
+        CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&r->recHost), bytes, cudaHostAllocPortable));
+        r->recChunks = chunks;
+        r->recCapacity = capacity;
+    }
+    static_assert(sizeof(RecordHeader) == sizeof(uint2), "the pairs follow the header");
+    uint2 *list = reinterpret_cast<uint2*>(r->recList + 1);
+    auto perArrays = [&](auto launch) {
+        RecordArrays A;
+        A.first_chunk = 0;
+        uint32_t base = 0;
+        for(uint32_t first = 0; first < num_arrays; first += RECORD_ARRAYS) {
+            A.num = 0;
+            A.chunk_start[0] = 0;
+            for(uint32_t i = first; i < std::min(num_arrays, first + RECORD_ARRAYS); i++) {
+                A.words[A.num] = words[i];
+                A.num_words[A.num] = (unsigned int)num_words[i];
+                A.base[A.num] = base;
+                base += (uint32_t)num_words[i];
+                A.num++;
+                A.chunk_start[A.num] = A.chunk_start[A.num - 1] + (unsigned int)((num_words[i] + RECORD_CHUNK - 1) / RECORD_CHUNK);
+            }
+            if(A.chunk_start[A.num]) launch(A);
+            A.first_chunk += A.chunk_start[A.num];
+        }
+    };
+    perArrays([&](const RecordArrays &A) {
+        recordCountKernel<<<A.chunk_start[A.num], RECORD_BLOCK, 0, r->stream>>>(A, r->recCounts);
+        r->launches++;
+    });
+    perArrays([&](const RecordArrays &A) {
+        recordListKernel<<<A.chunk_start[A.num], RECORD_BLOCK, 0, r->stream>>>(A, r->recCounts, (unsigned int)chunks, r->recList, list, capacity, r->state);
+        r->launches++;
+    });
+    CUDA_TRY(cudaPeekAtLastError());
+    // header and, in the same copy, about as many pairs as the last pull brought; what is left in a second one
+    const size_t first = std::min<size_t>(capacity, r->recLast + r->recLast / 4 + 512);
+    CUDA_TRY(cudaMemcpyAsync(r->recHost, r->recList, sizeof(RecordHeader) + sizeof(uint2) * first, cudaMemcpyDeviceToHost, r->stream));
+    CUDA_TRY(cudaStreamSynchronize(r->stream));
+    const size_t count = r->recHost->count;
+    *num_pairs = count;
+    if(count <= capacity) {
+        r->recLast = count;
+        uint2 *host = reinterpret_cast<uint2*>(r->recHost + 1);
+        if(count > first) {
+            CUDA_TRY(cudaMemcpyAsync(host + first, list + first, sizeof(uint2) * (count - first), cudaMemcpyDeviceToHost, r->stream));
+            CUDA_TRY(cudaStreamSynchronize(r->stream));
+        }
+        *pairs = host;
+    }
+    return reportDeviceError(r, r->recHost->error);
+}
+
+int b200_decode_recording(const uint32_t *words, const void *pairs, uint64_t num_pairs, uint32_t base, uint32_t rows, uint32_t batch,
+                          uint32_t words_per_row, uint32_t first_row, uint32_t num_neurons, uint32_t first_id, double start, double dt,
+                          uint64_t *counts, double *const *times, uint32_t *const *ids)
+{
+    if((!words && !pairs && num_pairs) || !counts || !rows || !batch || !words_per_row || first_row >= rows ||
+       num_neurons > 32ull * words_per_row || num_neurons + 32ull <= 32ull * words_per_row || (ids && !times)) {
+        return fail(B200_ERR_INVALID, "bad arguments to b200_decode_recording");
+    }
+    decodeRecording(words, static_cast<const uint32_t*>(pairs), num_pairs, base, rows, batch, words_per_row, first_row, num_neurons, first_id,
+                    start, dt, counts, times, ids);
+    return B200_OK;
+}
+
+int b200_pull_spikes(b200_runner *r, const uint32_t *count_ptr, const uint32_t *list_ptr, uint32_t capacity, uint32_t *ids, uint32_t *num)
+{
+    if(!r || !count_ptr || !list_ptr || !ids || !num) return fail(B200_ERR_INVALID, "null argument to b200_pull_spikes");
+    // count, error word and the first ids in one synchronisation
+    const uint32_t first = std::min<uint32_t>(capacity, STAGE_BYTES / sizeof(uint32_t));
+    CUDA_TRY(cudaMemcpyAsync(r->hostWord + 1, count_ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, r->stream));
+    CUDA_TRY(cudaMemcpyAsync(r->hostWord, &r->state->error, sizeof(uint32_t), cudaMemcpyDeviceToHost, r->stream));
+    if(first) CUDA_TRY(cudaMemcpyAsync(r->stage, list_ptr, sizeof(uint32_t) * first, cudaMemcpyDeviceToHost, r->stream));
+    CUDA_TRY(cudaStreamSynchronize(r->stream));
+    const uint32_t n = std::min(r->hostWord[1], capacity);
+    memcpy(ids, r->stage, sizeof(uint32_t) * std::min(n, first));
+    if(n > first) {
+        CUDA_TRY(cudaMemcpyAsync(ids + first, list_ptr + first, sizeof(uint32_t) * (n - first), cudaMemcpyDeviceToHost, r->stream));
+        CUDA_TRY(cudaStreamSynchronize(r->stream));
+    }
+    *num = n;
+    return reportDeviceError(r, r->hostWord[0]);
 }
 
 int b200_timed_begin(b200_runner *r)

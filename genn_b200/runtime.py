@@ -112,7 +112,6 @@ class Runtime:
         self._pinned = []
         self._rec_host = {}
         self.recording_pairs_capacity = None        # (index, word) pairs a recording pull has room for; None: 1/16 of the words
-        self._rec_compact = None        # device pair list, device counter, their page-locked copies, capacity
         self._rec_pairs, self._rec_layout = None, {}
         self._rec_timestep = 0
         self.shard = shard
@@ -435,9 +434,12 @@ class Runtime:
         name = pop if isinstance(pop, str) else pop.name
         p = self.net.pop(name)
         slot = self.steps_done % p.runtime_slots
-        cnt, spk = self.array(f"{name}.spk_cnt"), self.array(f"{name}.spk")
-        if cnt.ndim == 2:
-            return spk[batch, slot, :int(cnt[batch, slot])].copy()
+        counts, lists = self.plan.arrays[f"{name}.spk_cnt"], self.plan.arrays[f"{name}.spk"]
+        if len(counts.shape) == 2:
+            at = batch * p.runtime_slots + slot
+            ids, n = np.empty(p.n, dtype=np.uint32), C.c_uint32()
+            check(self.lib.b200_pull_spikes(self.handle, counts.ptr + 4 * at, lists.ptr + 4 * at * p.n, p.n, ids.ctypes.data, C.byref(n)))
+            return ids[:n.value]
         # sharded: one section per process; a section's count travels in the low half
         # of its (step, count) word
         tag, wire = self.array(f"{name}.spk_tag"), self.array(f"{name}.spk_wire")
@@ -462,38 +464,34 @@ class Runtime:
     def pull_recording_buffers(self):
         """Bring the spike recording of the last ``num_recording_timesteps`` steps to page-locked host memory
         (Runtime::pullRecordingBuffersFromDevice, runtime.cc:720-746, copies the bit words whole).  A recording is
-        almost all zeros at cortical rates, so the device first lists its non-zero words (b200_compact_words) and
+        almost all zeros at cortical rates, so the device first lists its non-zero words (b200_pull_recording) and
         only (index, word) pairs travel; a recording too dense for the pair buffer is copied whole instead.
         Decoding into (times, ids) happens lazily in :meth:`recorded_spikes`."""
         T = self.num_recording_timesteps
         if not T:
             raise Exception("Recording buffer not allocated - cannot pull from device")
-        self.synchronize()          # (reports device-side checks of the steps behind the recording)
         recs = [(p.name, self.plan.arrays[f"{p.name}.record"]) for p in self.net.pops if f"{p.name}.record" in self.plan.arrays]
         self._rec_pairs, self._rec_layout = None, {}
-        total = sum(int(np.prod(a.shape, dtype=np.int64)) for _, a in recs)
+        sizes = [int(np.prod(a.shape, dtype=np.int64)) for _, a in recs]
+        total = sum(sizes)
         if recs and total < (1 << 32):
-            if self._rec_compact is None:
-                # room for one non-zero word in sixteen unless the caller chose
-                cap = self.recording_pairs_capacity or max(1024, total // 16)
-                self._rec_compact = (self.factory.alloc(cap * 8), self.factory.alloc(4), self.pinned_empty((cap, 2), np.uint32),
-                                     self.pinned_empty((1,), np.uint32), cap)
-            pairs, counter, host_pairs, host_count, cap = self._rec_compact
-            check(self.lib.b200_array_memset(self.handle, counter.ptr, 0, 4))
+            # room for one non-zero word in sixteen unless the caller chose
+            cap = int(self.recording_pairs_capacity or max(1024, total // 16))
+            pairs, count = C.c_void_p(), C.c_uint64()
+            check(self.lib.b200_pull_recording(self.handle, len(recs), (C.c_void_p * len(recs))(*[a.ptr for _, a in recs]),
+                                               (C.c_uint64 * len(recs))(*sizes), cap, C.byref(pairs), C.byref(count)))
             base = 0
-            for name, arr in recs:
-                n = int(np.prod(arr.shape, dtype=np.int64))
-                check(self.lib.b200_compact_words(self.handle, arr.ptr, n, base, pairs.ptr, cap, counter.ptr))
+            for (name, arr), n in zip(recs, sizes):
                 self._rec_layout[name] = (base, arr.shape)
                 base += n
-            check(self.lib.b200_array_pull(self.handle, host_count.ctypes.data, counter.ptr, 4))     # waits for the stream
-            self.factory.d2h_bytes += 4
-            count = int(host_count[0])
-            if count <= cap:
-                if count:
-                    check(self.lib.b200_array_pull(self.handle, host_pairs.ctypes.data, pairs.ptr, count * 8))
-                    self.factory.d2h_bytes += count * 8
-                self._rec_pairs = host_pairs[:count].copy()
+            self.factory.d2h_bytes += 8
+            if pairs.value:
+                n = int(count.value)
+                self.factory.d2h_bytes += n * 8
+                self._rec_pairs = np.empty((n, 2), dtype=np.uint32)
+                C.memmove(self._rec_pairs.ctypes.data, pairs.value, n * 8)
+        else:
+            self.synchronize()          # (reports device-side checks of the steps behind the recording)
         self._rec_timestep = self.timestep
         for name, arr in recs:
             if self._rec_pairs is None:
@@ -527,13 +525,21 @@ class Runtime:
         # a process of a sharded model records the slice of the population it updates
         lo, hi = (p.shard_bounds[self.shard[0]], p.shard_bounds[self.shard[0] + 1]) if self.shard else (0, p.n)
         start = (ts - T) * self.net.dt
-        # the buffer is a ring over timestep % T: rotate so index 0 is the oldest step
-        words = np.roll(self._recording_words(pop), -(ts % T), axis=0)
-        out = []
-        for b in range(self.net.batch_size):
-            bits = np.unpackbits(np.ascontiguousarray(words[:, b, :]).view(np.uint8), axis=1, bitorder="little")
-            step, ids = np.nonzero(bits[:, :hi - lo])
-            out.append((start + step * self.net.dt, (ids + lo).astype(np.uint32)))
+        batch = self.net.batch_size
+        # from the pairs if the pull brought them (in index order), else from the whole array of bit words; the buffer is a
+        # ring over timestep % T
+        if self._rec_pairs is not None:
+            (base, shape), words, pairs, n = self._rec_layout[pop], None, self._rec_pairs.ctypes.data, len(self._rec_pairs)
+        else:
+            base, shape, words, pairs, n = 0, self._rec_host[pop].shape, self._rec_host[pop].ctypes.data, None, 0
+
+        def decode(times, ids):
+            check(self.lib.b200_decode_recording(words, pairs, n, base, T, batch, shape[2], ts % T, hi - lo, lo, start, self.net.dt,
+                                                 counts, times, ids))
+        counts = (C.c_uint64 * batch)()
+        decode(None, None)
+        out = [(np.empty(c, dtype=np.float64), np.empty(c, dtype=np.uint32)) for c in counts]
+        decode((C.c_void_p * batch)(*[t.ctypes.data for t, _ in out]), (C.c_void_p * batch)(*[i.ctypes.data for _, i in out]))
         return out
 
     # -- measurement helpers ------------------------------------------------------

@@ -249,6 +249,21 @@ int  b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes
  * the array itself.  Order of the pairs is arbitrary. */
 int  b200_compact_words(b200_runner *r, const uint32_t *words, uint64_t num_words, uint32_t base_index,
                         void *pairs, uint32_t capacity, uint32_t *counter);
+/* The same for all recorded populations at once, and fetched: waits for the runner's stream and lists the non-zero words of
+ * the arrays, in order, as (index, word) pairs; an array's first word has the index of all words before it.  `*pairs`
+ * points into page-locked memory of the runner that the next call overwrites; it is NULL if more than `capacity` words
+ * (`*num_pairs` of them) are not zero: the caller then copies the arrays.  Reports device-side checks as b200_synchronize does. */
+int  b200_pull_recording(b200_runner *r, uint32_t num_arrays, const uint32_t *const *words, const uint64_t *num_words,
+                         uint32_t capacity, const void **pairs, uint64_t *num_pairs);
+/* The spikes of one population in such a list (host code, no GPU), or in its whole array (`words`): first call with
+ * times = ids = NULL for the counts per batch entry, second call to store them, ordered by time, then id.  `rows` time
+ * steps of [batch][words_per_row] words, row `first_row` is the oldest; time = start + step * dt. */
+int  b200_decode_recording(const uint32_t *words, const void *pairs, uint64_t num_pairs, uint32_t base, uint32_t rows, uint32_t batch,
+                           uint32_t words_per_row, uint32_t first_row, uint32_t num_neurons, uint32_t first_id, double start, double dt,
+                           uint64_t *counts, double *const *times, uint32_t *const *ids);
+/* One spike list: the count at `count_ptr`, at most `capacity` ids from `list_ptr` (device pointers) into host memory.
+ * Waits for the runner's stream; reports device-side checks as b200_synchronize does. */
+int  b200_pull_spikes(b200_runner *r, const uint32_t *count_ptr, const uint32_t *list_ptr, uint32_t capacity, uint32_t *ids, uint32_t *num);
 
 /* ---- spike exchange between processes (no counterpart in the reference, which has no model
  *      sharding: backendCUDAHIP.cc uses NCCL for the all-reduce of custom-update results only).
