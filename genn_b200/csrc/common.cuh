@@ -48,6 +48,7 @@ struct StepState
 constexpr unsigned int ERR_SPIKE_OVERFLOW = 1u;
 constexpr unsigned int ERR_IND_RANGE = 2u;
 constexpr unsigned int ERR_DELAY_RANGE = 4u;
+constexpr unsigned int ERR_BARRIER_TIMEOUT = 8u;
 
 // Block -> merged-group element lookup: block_start[g] is the first block of
 // group g, block_start[num_groups] the grid size.  Linear for a handful of
@@ -82,4 +83,14 @@ __device__ __forceinline__ unsigned int ringSlot(unsigned int k, unsigned int sl
 {
     return k % slots;
 }
+
+// Copy `bytes` (a multiple of 4) from global to shared memory with the whole CTA.
+__device__ __forceinline__ void stageWords(void *dst, const void *src, size_t bytes)
+{
+    unsigned int *d = static_cast<unsigned int*>(dst);
+    const unsigned int *s = static_cast<const unsigned int*>(src);
+    for(size_t w = threadIdx.x; w < bytes / 4; w += blockDim.x) d[w] = __ldg(&s[w]);
+}
+
+__host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 }   // namespace b200

@@ -75,7 +75,6 @@ constexpr int FUSED_BLOCK = 768;          // one CTA per SM, 85 registers per th
 constexpr unsigned int FUSED_CHUNK = 32 * PRE_VEC;          // synapses per warp item
 constexpr unsigned int FUSED_MAX_SOURCES = 256;             // (population, process, delay) spike sources per model
 constexpr unsigned int FUSED_PREFETCH_IDS = 8;              // spike ids fetched together with each count
-constexpr unsigned int ERR_BARRIER_TIMEOUT = 8u;
 constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 24; // default: polls (tens of ms) before giving up
 
 // One spike source as the presynaptic phase sees it: a (population, axonal
@@ -248,16 +247,6 @@ __device__ __forceinline__ void fusedUrgentChunk(const b200_synapse_group &g, co
     }
     redAdd(g.den_delay + (unsigned long long)ringSlot(front, g.max_den_delay) * g.num_trg + e.x, __uint_as_float(e.y));
 }
-
-// Copy `bytes` (a multiple of 4) from global to shared memory with the whole CTA.
-__device__ __forceinline__ void stageWords(void *dst, const void *src, size_t bytes)
-{
-    unsigned int *d = static_cast<unsigned int*>(dst);
-    const unsigned int *s = static_cast<const unsigned int*>(src);
-    for(size_t w = threadIdx.x; w < bytes / 4; w += blockDim.x) d[w] = __ldg(&s[w]);
-}
-
-__host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // The acquire side of every grid barrier invalidates the SM's L1, so a
 // descriptor left in global memory would cost a full L2 round trip per field
@@ -615,4 +604,8 @@ fusedStepKernel(FusedLaunch L)
         state->phase = k;
     }
 }
+
+// instances: persistent.cu
+const void *fusedKernelFor(int npsm, int ncs);
+const void *streamKernelFor(int npsm, int ncs, bool sharded);
 }   // namespace b200

@@ -78,7 +78,7 @@ __device__ __forceinline__ unsigned int nearDelay(unsigned int d, unsigned int D
 }
 
 // counts[row] += near synapses of the row.  One warp per row.
-__global__ void nearCountKernel(const b200_synapse_group g, unsigned int *counts)
+static __global__ void nearCountKernel(const b200_synapse_group g, unsigned int *counts)
 {
     const unsigned int lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
     const unsigned int D = g.max_den_delay;

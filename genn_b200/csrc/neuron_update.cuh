@@ -168,13 +168,21 @@ __device__ __forceinline__ void drawCurrentSources(const NeuronLaunch &L, const 
     }
 }
 
+// Time to the next spike of a Poisson neuron that has none left (neuronModels.h:318-325): depends on nothing a step
+// delivers, so the target-resident kernel draws it while it waits for the step's spikes.
+__device__ __forceinline__ float drawPoissonInterval(const NeuronLaunch &L, const b200_neuron_group &g, unsigned int b, unsigned int i,
+                                                     unsigned long long timestep, float tts)
+{
+    b200_rng rng = b200_rng_sim(L.seed, g.rng_stream, b * g.num_neurons + i, timestep);
+    return B200_FADD(tts, B200_FMUL(g.params[0], -b200_logf(b200_rng_uniform(&rng))));
+}
+
 template<int NPSM, int NCS>
 __device__ __forceinline__ bool neuronCompute(const NeuronLaunch &L, const b200_neuron_group &g, unsigned int b,
                                               unsigned int i, unsigned long long timestep, float t,
                                               NeuronRegs<NPSM, NCS> &r, const float (&front)[NPSM],
-                                              const unsigned int (&csCount)[NCS > 0 ? NCS : 1])
+                                              const unsigned int (&csCount)[NCS > 0 ? NCS : 1], bool intervalDrawn = false)
 {
-    const unsigned int N = g.num_neurons;
     const unsigned int model = g.model;
     float Isyn = 0.0f;
     float V = __uint_as_float(r.v[0]);
@@ -268,10 +276,7 @@ __device__ __forceinline__ bool neuronCompute(const NeuronLaunch &L, const b200_
     }
     else {
         float tts = V;
-        if(tts <= 0.0f) {
-            b200_rng rng = b200_rng_sim(L.seed, g.rng_stream, b * N + i, timestep);
-            tts = B200_FADD(tts, B200_FMUL(g.params[0], -b200_logf(b200_rng_uniform(&rng))));
-        }
+        if(tts <= 0.0f && !intervalDrawn) tts = drawPoissonInterval(L, g, b, i, timestep, tts);
         tts = B200_FSUB(tts, 1.0f);
         spiked = (tts <= 0.0f);
         r.v[0] = __float_as_uint(tts);

@@ -173,7 +173,7 @@ __device__ __forceinline__ void sparseTileSTDP(const b200_synapse_group &g, unsi
 }
 
 // One launch for every SPARSE merged group.
-__global__ void __launch_bounds__(PRE_BLOCK)
+static __global__ void __launch_bounds__(PRE_BLOCK)
 presynapticSparseKernel(const SynapseLaunch L)
 {
     const unsigned int gi = findGroup(L.block_start, L.num_groups, blockIdx.x);
@@ -222,7 +222,7 @@ presynapticSparseKernel(const SynapseLaunch L)
 // to 32 so the 32 lanes of a warp test bits of ONE connectivity word, fetched
 // with a single broadcast load: numPost/8 bytes per spike.  DENSE streams one
 // coalesced weight row per spike: 4*numPost bytes per spike.
-__global__ void __launch_bounds__(PRE_BLOCK)
+static __global__ void __launch_bounds__(PRE_BLOCK)
 presynapticPostSpanKernel(const SynapseLaunch L)
 {
     const unsigned int gi = findGroup(L.block_start, L.num_groups, blockIdx.x);
@@ -299,7 +299,7 @@ presynapticPostSpanKernel(const SynapseLaunch L)
 constexpr unsigned int PROC_BLOCK = 256;
 constexpr unsigned int PROC_HOLD = 48;      // targets of a sub-row kept between its generation and its delivery
 
-__global__ void __launch_bounds__(PROC_BLOCK)
+static __global__ void __launch_bounds__(PROC_BLOCK)
 presynapticProceduralKernel(const SynapseLaunch L)
 {
     const b200_synapse_group &g = L.groups[blockIdx.y];

@@ -1,0 +1,154 @@
+// Target-resident persistent time-step kernel.
+//
+// A step of a batch-1 network is a dependent chain, not traffic: neuron update -> who spiked -> their synapses ->
+// neuron update.  The kernels that share the input buffers between CTAs (fused_step.cuh, stream_step.cuh) pay for that
+// chain at L2 distance several times over: spike-list atomics, a grid barrier with its release and acquire, the
+// lists, the rows, reductions into L2, the buffers read back.  Here everything but the spikes stays inside the CTA:
+//
+//   * neurons are dealt out in units of 32 (one recording word) over the CTAs, unit u to CTA u % G: state in registers,
+//     input buffers and dendritic-delay rings in shared memory;
+//   * every CTA delivers ALL spikes, each onto its own neurons only.  A private copy of the SPARSE groups (built from
+//     the caller's arrays, rebuilt when they change) holds, per source neuron and CTA, the synapses of all groups onto
+//     that CTA's neurons as one run of 8-byte entries (ring slot and column, weight).  Runs of one source population
+//     onto one CTA have the same padded length, so a spike's id leads to its entries in one memory round trip; the
+//     runs of one source neuron lie side by side (one address translation per spike, not one per spike and CTA).
+//     DENSE rows and BITMASK words are read where they are: a unit of 32 targets is 128 bytes or one word of a row;
+//   * the only thing that crosses CTAs is one message per CTA and step: two 64-bit words (step number, spike count, the
+//     first seven ids); further ids wait at the sender.  Every word carries its step number, so readers poll the
+//     cells themselves: the all-gather IS the barrier, with no fence, no counter and no list.  A message is stored
+//     once for every RESIDENT_READERS CTAs: with one copy for all, polling it grew from 1.8 k cycles at 32 CTAs to
+//     8 k at 148, and with a copy for each the sender's stores took 10 cycles apiece, 1.6 k at 148.  A cell is
+//     written again `buffers` steps later; its sender has by then received messages that every reader sent after it had
+//     read this one.
+//
+// What has to be in place before the neuron update of a step is kept small.  Groups of one axonal delay form a class:
+//
+//   IMMEDIATE  the runs (and DENSE / BITMASK rows) of the step's spikes are added before the update;
+//   SPLIT      every group has a delay ring: only synapses of dendritic delay 0 are needed at once.  They lie in rows of
+//              their own, one per source neuron for ALL CTAs (a few per cent of the synapses: the table stays in L2),
+//              and the runs with the rest are fetched behind them, while the neurons are updated, and added after that;
+//   LATE       no group has a ring and the axonal delay is a step or more: the spikes of the NEXT step are known
+//              already, so their runs are fetched and added behind the update too, into the second of two buffers.
+//              CTAs then run up to the delay apart, and no step waits for another SM or for memory.
+//
+// Memory between launches is what every other path leaves: the first steps of a launch take the spikes of the steps
+// before it from the spike lists, the last ones write them.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "neuron_update.cuh"
+
+namespace b200
+{
+constexpr unsigned int RESIDENT_BLOCK = 768;            // most threads of a CTA: 85 registers each
+constexpr unsigned int RESIDENT_UNITS = RESIDENT_BLOCK / 32;    // most units of 32 neurons of a CTA
+constexpr unsigned int RESIDENT_MAX_CTAS = 256;
+constexpr unsigned int RESIDENT_MAX_GROUPS = 64;        // neuron groups (a bit mask says which are sources)
+constexpr unsigned int RESIDENT_CLASSES = 4;            // distinct ring depths / distinct axonal delays
+constexpr unsigned int RESIDENT_LIST = 2048;            // spikes delivered between two barriers of a CTA
+constexpr unsigned int RESIDENT_READERS = 12;           // CTAs that poll one copy of the messages
+constexpr unsigned int RESIDENT_LOADS = 4;              // loads of a run that a lane has in flight
+constexpr unsigned int RESIDENT_CHUNK = 32 * RESIDENT_LOADS;    // entries of a run that one warp takes
+constexpr unsigned int RESIDENT_NEAR_ROWS = 4;          // rows of delay-0 synapses whose loads a warp has in flight
+constexpr unsigned int RESIDENT_DENSE_SPIKES = 8;       // rows of a DENSE group whose loads a lane has in flight
+constexpr unsigned int RESIDENT_NEAR_MOST = 256;        // most delay-0 synapses of a source neuron for a SPLIT class
+constexpr unsigned int RESIDENT_PAD = 0xFFFFFFFFu;      // key of a padding entry
+constexpr unsigned long long RESIDENT_TAG_STEPS = 1ull << 20;       // step numbers of messages are 20 bits
+constexpr unsigned int RESIDENT_HEAD_IDS = 3, RESIDENT_MORE_IDS = 4;    // ids in a first word / in a further word
+constexpr unsigned int RESIDENT_CELL_IDS = RESIDENT_HEAD_IDS + RESIDENT_MORE_IDS;  // ids in the two words of an inbox cell
+
+enum ResidentClass { RESIDENT_IMMEDIATE = 0, RESIDENT_SPLIT = 1, RESIDENT_LATE = 2 };
+
+// entry key of a run: ring class << 30 | delay << 16 | column; of a row of delay-0 synapses: CTA << 24 | ring class << 16 | column
+struct ResidentRun              // runs of one (axonal delay, source population) pair onto one CTA
+{
+    unsigned long long base;    // first entry of the run of source neuron 0
+    unsigned int length;        // entries of a run (0: no synapses), a multiple of four
+    unsigned int row;           // entries between two source neurons: the runs of all CTAs
+};
+
+struct ResidentNear             // delay-0 synapses of a SPLIT class, one row per source neuron of a population
+{
+    unsigned long long base;    // entry of source neuron 0
+    unsigned long long row_base;    // where the runs of source neuron 0 begin
+    unsigned int length;        // entries of a row (0: none), a multiple of four
+    unsigned int pad;
+};
+
+struct ResidentSpan             // a DENSE or BITMASK group
+{
+    const float *g;             // DENSE weights or NULL (constant)
+    const unsigned int *gp;     // BITMASK words or NULL
+    float weight;               // constant weight
+    unsigned int row_stride;    // BITMASK: bits of a row
+    unsigned int num_trg;
+    unsigned int delay_class;
+    unsigned int src_group, trg_group, psm;
+    unsigned int num_src;
+};
+
+// Where the tables of a CTA lie in its dynamic shared memory (bytes): constants of the launch, so no thread keeps pointers.
+struct ResidentLayout
+{
+    unsigned int groups, unit_start, unit_first, columns, runs, near, spans, poisson, history, acc;
+};
+
+struct ResidentLaunch
+{
+    NeuronLaunch neuron;
+    ResidentLayout at;
+    const unsigned int *unit_start;     // [num_groups + 1] units of 32 neurons before each group
+    const unsigned int *unit_first;     // [num_units] neuron group << 24 | first neuron of the unit
+    const unsigned int *columns;        // [grid][RESIDENT_UNITS][B200_MAX_PSM] ring class << 16 | first column
+    const unsigned int *cta_columns;    // [grid][RESIDENT_CLASSES] columns of each ring class
+    const ResidentRun *runs;            // [grid][delay classes][num_groups]
+    const ResidentNear *near;           // [delay classes][num_groups]
+    const uint2 *entries;
+    const uint2 *near_entries;
+    const float *poisson;               // [num_groups][64] distribution of the event count of a group's one Poisson source, or NULL
+    const ResidentSpan *spans;
+    unsigned int num_spans;
+    unsigned int num_units;
+    unsigned int num_depths, depth[RESIDENT_CLASSES];       // buffers per input: ring depths; without a ring 1, or 2 with a LATE class
+    unsigned int num_delays, delay[RESIDENT_CLASSES];       // axonal delays
+    unsigned int kind[RESIDENT_CLASSES];                    // ResidentClass of each delay
+    unsigned long long source_groups;                       // groups with outgoing synapses of any delay
+    unsigned long long sources[RESIDENT_CLASSES];           // neuron groups with outgoing synapses of that delay
+    unsigned int chunks[RESIDENT_CLASSES];                  // warp items of the longest run of that delay (0: no runs)
+    unsigned int near_chunks[RESIDENT_CLASSES];             // the same of the rows of delay-0 synapses
+    unsigned int acc_floats;            // shared memory of the input buffers
+    unsigned int history;               // steps whose spike lists the launch has to leave behind
+    unsigned int buffers;               // message buffers
+    unsigned int more_words;            // words behind the cell a message may need
+    ulonglong2 *inbox;                  // [buffers][copies][sender]
+    unsigned int copies;
+    unsigned int prefetch;              // 1: the runs do not stay in L2: a spiking neuron's are fetched ahead of its message
+    unsigned long long *more;           // [buffers][sender][more_words]
+    unsigned long long *leave;          // steps done when the spike lists may be written at the end of a launch
+    unsigned int num_steps;
+    unsigned int count_events;
+};
+
+// the runs of one pair are counted (pass 0) and placed (pass 1) by one launch each
+struct ResidentBuild
+{
+    const b200_synapse_group *groups;   // the SPARSE groups of one (axonal delay, source population) pair
+    const unsigned int *target;         // per group: neuron group << 8 | postsynaptic model of its target
+    unsigned int num_groups, num_src;
+    const unsigned int *unit_start, *columns;
+    const unsigned int *depth;          // buffers per input, by ring class
+    unsigned int late;                  // 1: LATE class: every synapse arrives one step after its delivery
+    unsigned int split;                 // 1: SPLIT class: delay-0 synapses go into the rows
+    unsigned int *near_longest;         // longest row of delay-0 synapses
+    ResidentNear near;
+    uint2 *near_entries;
+    unsigned int grid;
+    unsigned int runs_stride;           // distance between the pair's runs of two CTAs
+};
+
+// kernels: resident.cu
+const void *residentKernelFor(int npsm, int ncs, bool one_class);
+cudaError_t residentBuild(const ResidentBuild &B, int pass, unsigned int *longest, const ResidentRun *runs, uint2 *entries, StepState *state,
+                          unsigned int blocks, cudaStream_t stream);
+}   // namespace b200

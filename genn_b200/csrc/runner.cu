@@ -28,6 +28,7 @@
 #include "urgent.cuh"
 #include "stream_step.cuh"
 #include "tiled.cuh"
+#include "resident.h"
 #include "record.cuh"
 
 #include <cub/device/device_scan.cuh>
@@ -276,6 +277,28 @@ struct b200_runner
         tiledReady = false;
     }
 
+    // target-resident kernel (resident.h): private copy of the SPARSE groups cut by CTA, message buffers
+    bool useResident = true;
+    bool scheduleChosen = false;            // the caller picked a schedule of the other persistent kernels
+    bool residentStale = true, residentReady = false;
+    std::string residentWhyNot;
+    unsigned int residentCtas = 0, residentWarps = 0;       // 0: chosen by size
+    unsigned int residentGrid = 0, residentBlock = 0;
+    size_t residentSmem = 0;
+    unsigned long long residentTagged = ~0ull;              // steps since the message buffers were last cleared
+    size_t residentMailBytes = 0;
+    const void *residentKernel = nullptr;
+    ResidentLaunch resident{};
+    std::vector<void*> residentBuffers;
+
+    void dropResident()
+    {
+        for(void *p : residentBuffers) cudaFree(p);
+        residentBuffers.clear();
+        residentReady = false;
+        residentTagged = ~0ull;
+    }
+
     // options
     unsigned int spikeLanes = 16;
     bool countEvents = false;
@@ -451,11 +474,9 @@ int buildFusedTables(b200_runner *r)
             return buildFusedTables(r);
         }
         int e = withNeuronShape(r, [&](auto P, auto C) -> int {
-            auto fused = fusedStepKernel<decltype(P)::value, decltype(C)::value>;
-            auto stream = r->sharded() ? streamStepKernel<decltype(P)::value, decltype(C)::value, true>
-                                       : streamStepKernel<decltype(P)::value, decltype(C)::value, false>;
-            auto kernel = r->streamWarps ? stream : fused;
-            r->fusedKernel = (const void*)kernel;
+            const void *kernel = r->streamWarps ? streamKernelFor(decltype(P)::value, decltype(C)::value, r->sharded())
+                                                : fusedKernelFor(decltype(P)::value, decltype(C)::value);
+            r->fusedKernel = kernel;
             if(r->fusedStage) {
                 CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->fusedSmemBytes));
             }
@@ -539,7 +560,7 @@ int prepare(b200_runner *r)
                         !r->neuronGroups.empty());
     r->fusedGroups = sparse;
     r->lagStale = true;
-    r->tiledStale = true;
+    r->tiledStale = r->residentStale = true;
     r->schedule = b200_runner::PLAIN;
     r->dropUrgent();
     {
@@ -1193,6 +1214,384 @@ TiledLaunch tiledLaunch(const b200_runner *r)
     return L;
 }
 
+// (Re)build the tables of the target-resident kernel; leaves residentReady false, with the reason, where the model does
+// not qualify.  Runs when a block of steps is first asked for and after the arrays it copies changed.
+int buildResident(b200_runner *r)
+{
+    r->dropResident();
+    r->residentStale = false;
+    r->residentWhyNot.clear();
+    auto no = [&](const char *why) { r->residentWhyNot = why; return B200_OK; };
+    if(r->batch != 1 || r->sharded()) return no("batch or sharded model");
+    const size_t numGroups = r->neuronGroups.size();
+    if(!numGroups || numGroups > RESIDENT_MAX_GROUPS || r->synapseGroups.empty()) return no("no groups, or too many");
+    int sms = 0, coop = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+    CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, r->device));
+    if(!coop) return no("no cooperative launch");
+    ResidentLaunch &L = r->resident;
+    L = ResidentLaunch{};
+
+    // ---- ring depths, axonal delays, who feeds whom --------------------------------------------------------
+    std::vector<unsigned int> unitStart{0}, depths, delays;
+    unsigned int maxSlots = 0;
+    for(const auto &g : r->neuronGroups) {
+        if(g.first_neuron != 0 || g.num_update != g.num_neurons || g.num_neurons >= (1u << 24)) return no("partly updated population");
+        if(g.spike_times) return no("spike times");
+        unitStart.push_back(unitStart.back() + (g.num_neurons + 31u) / 32u);
+        maxSlots = std::max(maxSlots, g.num_delay_slots);
+        for(unsigned int p = 0; p < g.num_psm; p++) {
+            const unsigned int d = std::max(1u, g.psm[p].max_den_delay);
+            if(std::find(depths.begin(), depths.end(), d) == depths.end()) depths.push_back(d);
+        }
+    }
+    if(depths.empty()) depths.push_back(1u);
+    const unsigned int units = unitStart.back();
+    if(depths.size() > RESIDENT_CLASSES || units == 0) return no("too many ring depths");
+    struct Link { size_t syn; unsigned int src, trg, psm, delayClass; };
+    std::vector<Link> links;
+    for(size_t i = 0; i < r->synapseGroups.size(); i++) {
+        const auto &g = r->synapseGroups[i];
+        if(g.connectivity == B200_CONN_PROCEDURAL || g.wu_model == B200_WU_STDP) return no("procedural or learning group");
+        Link l{i, ~0u, ~0u, 0u, 0u};
+        for(unsigned int ni = 0; ni < numGroups; ni++) {
+            const auto &ng = r->neuronGroups[ni];
+            if(ng.spk_cnt == g.src_spk_cnt && ng.num_neurons == g.num_src) l.src = ni;
+            for(unsigned int p = 0; p < ng.num_psm; p++) {
+                const bool same = g.max_den_delay ? (ng.psm[p].den_delay == g.den_delay && ng.psm[p].max_den_delay == g.max_den_delay)
+                                                  : (!ng.psm[p].max_den_delay && ng.psm[p].out_post == g.out_post);
+                if(same && ng.num_neurons == g.num_trg) { l.trg = ni; l.psm = p; }
+            }
+        }
+        if(l.src == ~0u || l.trg == ~0u) return no("a group's source or target is not a population of the model");
+        auto it = std::find(delays.begin(), delays.end(), g.axonal_delay);
+        if(it == delays.end()) { delays.push_back(g.axonal_delay); it = delays.end() - 1; }
+        l.delayClass = (unsigned int)(it - delays.begin());
+        links.push_back(l);
+    }
+    if(delays.size() > RESIDENT_CLASSES) return no("too many axonal delays");
+    const unsigned int numDelays = (unsigned int)delays.size();
+    // what of each class has to be delivered before the neuron update (resident.h)
+    bool anyLate = false;
+    for(unsigned int a = 0; a < numDelays; a++) {
+        bool rings = true, noRing = true;
+        for(const auto &l : links) {
+            const auto &g = r->synapseGroups[l.syn];
+            if(l.delayClass != a) continue;
+            if(g.connectivity != B200_CONN_SPARSE || g.max_den_delay < 2) rings = false;
+            if(g.max_den_delay) noRing = false;
+        }
+        L.kind[a] = rings ? RESIDENT_SPLIT : (noRing && delays[a] >= 1u) ? RESIDENT_LATE : RESIDENT_IMMEDIATE;
+        anyLate = anyLate || L.kind[a] == RESIDENT_LATE;
+    }
+    // buffers per input: the ring, one, or two that a LATE class fills and empties in turn
+    for(auto &d : depths) if(d == 1u && anyLate) d = 2u;
+    std::sort(depths.begin(), depths.end());
+    depths.erase(std::unique(depths.begin(), depths.end()), depths.end());
+    auto depthOf = [&](const b200_psm &psm) {
+        const unsigned int d = psm.max_den_delay ? psm.max_den_delay : anyLate ? 2u : 1u;
+        return (unsigned int)(std::find(depths.begin(), depths.end(), d) - depths.begin());
+    };
+
+    // ---- how many CTAs, how many warps ----------------------------------------------------------------------
+    const NeuronShape shape = neuronShape(r);
+    cudaFuncAttributes attr{};
+    r->residentKernel = residentKernelFor(shape.npsm, shape.ncs, depths.size() == 1 && numDelays == 1);
+    CUDA_TRY(cudaFuncGetAttributes(&attr, r->residentKernel));
+    unsigned int numSpans = 0;
+    for(const auto &l : links) numSpans += (r->synapseGroups[l.syn].connectivity != B200_CONN_SPARSE);
+    const unsigned int longestDelay = *std::max_element(delays.begin(), delays.end()), shortest = *std::min_element(delays.begin(), delays.end());
+    const unsigned int history = std::min(longestDelay + 1u, maxSlots);
+    // event counts of Poisson sources: the cumulative probabilities b200_poisson_inverse would add up
+    std::vector<float> poisson;
+    if(shape.ncs == 1) {
+        for(const auto &g : r->neuronGroups) {
+            float p = g.num_cs ? g.cs[0].params[2] : 1.0f, sum = p;
+            for(unsigned int i = 0; i < 64u; i++) {
+                poisson.push_back(sum);
+                p = B200_FDIV(B200_FMUL(p, g.cs[0].params[3]), (float)(i + 1u));
+                sum = B200_FADD(sum, p);
+            }
+        }
+    }
+    size_t tables = 0;
+    auto place = [&](size_t bytes) { const unsigned int at = (unsigned int)tables; tables += align16(bytes); return at; };
+    L.at.groups = place(sizeof(b200_neuron_group) * numGroups);
+    L.at.unit_start = place(sizeof(unsigned int) * (numGroups + 1));
+    L.at.unit_first = place(sizeof(unsigned int) * units);
+    L.at.columns = place(sizeof(unsigned int) * RESIDENT_UNITS * B200_MAX_PSM);
+    L.at.runs = place(sizeof(ResidentRun) * numDelays * numGroups);
+    L.at.near = place(sizeof(ResidentNear) * numDelays * numGroups);
+    L.at.spans = place(sizeof(ResidentSpan) * numSpans);
+    L.at.poisson = place(sizeof(float) * poisson.size());
+    L.at.history = place(sizeof(unsigned int) * history * RESIDENT_UNITS);
+    L.at.acc = place(0);
+    int optin = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, r->device));
+    const size_t room = (size_t)optin - attr.sharedSizeBytes;
+    auto groupOf = [&](unsigned int u) { return (unsigned int)(std::upper_bound(unitStart.begin(), unitStart.end(), u) - unitStart.begin()) - 1u; };
+    std::vector<unsigned int> columns, ctaColumns;
+    unsigned int grid = 0;
+    size_t accFloats = 0;
+    auto layOut = [&](unsigned int G) {
+        columns.assign((size_t)G * RESIDENT_UNITS * B200_MAX_PSM, 0u);
+        ctaColumns.assign((size_t)G * RESIDENT_CLASSES, 0u);
+        accFloats = 0;
+        for(unsigned int c = 0; c < G; c++) {
+            size_t floats = 0;
+            for(unsigned int u = c, w = 0; u < units; u += G, w++) {
+                const auto &g = r->neuronGroups[groupOf(u)];
+                for(unsigned int p = 0; p < g.num_psm; p++) {
+                    const unsigned int cls = depthOf(g.psm[p]);
+                    unsigned int &cols = ctaColumns[(size_t)c * RESIDENT_CLASSES + cls];
+                    columns[((size_t)c * RESIDENT_UNITS + w) * B200_MAX_PSM + p] = (cls << 16) | cols;
+                    cols += 32u;
+                }
+            }
+            for(size_t k = 0; k < depths.size(); k++) floats += (size_t)depths[k] * ctaColumns[(size_t)c * RESIDENT_CLASSES + k];
+            accFloats = std::max(accFloats, floats);
+        }
+    };
+    const unsigned int most = std::min<unsigned int>((unsigned int)sms, RESIDENT_MAX_CTAS);
+    {
+        // Units of 32 neurons for a CTA.  More CTAs share the work of a step but lengthen the exchange; measured (us a step at
+        // 32 / 64 / 148 CTAs): 1000 -> 10 000 sparse 1.37 / 1.48 / 1.94; 7 700 neurons with rings 3.3 / 3.1 / 3.3; DENSE
+        // 4096 -> 4096 6.4 / 5.2 / 4.6; BITMASK 2000 -> 5000 4.6 / 4.3 / 4.1
+        bool rings = false;
+        for(unsigned int a = 0; a < numDelays; a++) rings = rings || L.kind[a] == RESIDENT_SPLIT;
+        const unsigned int perCta = numSpans ? 2u : rings ? 4u : 10u;
+        unsigned int G = r->residentCtas ? r->residentCtas : std::max(32u, (units + perCta - 1u) / perCta);
+        G = std::min(std::min(std::max(G, (units + RESIDENT_UNITS - 1u) / RESIDENT_UNITS), most), units);
+        for(;; G = std::min(most, G + (G + 7u) / 8u)) {
+            if((units + G - 1u) / G <= RESIDENT_UNITS) {
+                layOut(G);
+                if(tables + accFloats * sizeof(float) <= room) { grid = G; break; }
+            }
+            if(G == most) break;
+        }
+        if(!grid) return no("more neurons, or deeper rings, than the SMs hold");
+    }
+    const unsigned int neuronWarps = (units + grid - 1u) / grid;
+    // (warps without neurons ask for the messages and build this CTA's own)
+    unsigned int warps = r->residentWarps ? r->residentWarps : std::max(numSpans ? 16u : 8u, neuronWarps + (grid + 31u) / 32u);
+    warps = std::min(std::max(warps, std::max(neuronWarps, (grid + 31u) / 32u)), RESIDENT_UNITS);
+
+    auto device = [&](size_t bytes, void **out) -> int {
+        CUDA_TRY(cudaMalloc(out, std::max<size_t>(bytes, 16)));
+        r->residentBuffers.push_back(*out);
+        return B200_OK;
+    };
+    auto upload = [&](const void *host, size_t bytes, void **out) -> int {
+        if(const int err = device(bytes, out)) return err;
+        CUDA_TRY(cudaMemcpyAsync(*out, host, bytes, cudaMemcpyHostToDevice, r->stream));
+        return B200_OK;
+    };
+    std::vector<unsigned int> unitFirst(units);
+    for(unsigned int u = 0; u < units; u++) unitFirst[u] = (groupOf(u) << 24) | ((u - unitStart[groupOf(u)]) * 32u);
+    unsigned int *dUnitStart = nullptr, *dUnitFirst = nullptr, *dColumns = nullptr, *dCtaColumns = nullptr, *dDepths = nullptr;
+    if(const int err = upload(unitStart.data(), sizeof(unsigned int) * unitStart.size(), (void**)&dUnitStart)) return err;
+    if(const int err = upload(unitFirst.data(), sizeof(unsigned int) * unitFirst.size(), (void**)&dUnitFirst)) return err;
+    if(const int err = upload(columns.data(), sizeof(unsigned int) * columns.size(), (void**)&dColumns)) return err;
+    if(const int err = upload(ctaColumns.data(), sizeof(unsigned int) * ctaColumns.size(), (void**)&dCtaColumns)) return err;
+    if(const int err = upload(depths.data(), sizeof(unsigned int) * depths.size(), (void**)&dDepths)) return err;
+
+    // ---- runs of the SPARSE groups ----------------------------------------------------------------------------
+    const size_t runsPerCta = (size_t)numDelays * numGroups;
+    std::vector<ResidentRun> runs(runsPerCta * grid, ResidentRun{0, 0, 0});
+    std::vector<b200_synapse_group> sorted;
+    std::vector<unsigned int> targets;
+    struct Pair { unsigned int delayClass, src, first, count; };
+    std::vector<Pair> pairs;
+    for(unsigned int a = 0; a < numDelays; a++) {
+        for(unsigned int ni = 0; ni < numGroups; ni++) {
+            Pair pr{a, ni, (unsigned int)sorted.size(), 0u};
+            for(const auto &l : links) {
+                const auto &g = r->synapseGroups[l.syn];
+                if(l.delayClass != a || l.src != ni) continue;
+                L.sources[a] |= 1ull << ni;
+                if(g.connectivity != B200_CONN_SPARSE) continue;
+                sorted.push_back(g);
+                targets.push_back((l.trg << 8) | l.psm);
+                pr.count++;
+            }
+            if(pr.count) pairs.push_back(pr);
+        }
+    }
+    for(unsigned int a = 0; a < numDelays; a++) L.source_groups |= L.sources[a];
+    std::vector<ResidentNear> nears(runsPerCta, ResidentNear{0, 0, 0, 0});
+    ResidentRun *dRuns = nullptr;
+    uint2 *dEntries = nullptr, *dNear = nullptr;
+    if(!pairs.empty()) {
+        unsigned long long cells = 0, nearCells = 0;
+        ScopedDevice longest, sortedHold, targetsHold;
+        CUDA_TRY(cudaMalloc(&sortedHold.p, sizeof(b200_synapse_group) * sorted.size()));
+        CUDA_TRY(cudaMalloc(&targetsHold.p, sizeof(unsigned int) * targets.size()));
+        CUDA_TRY(cudaMemcpyAsync(sortedHold.p, sorted.data(), sizeof(b200_synapse_group) * sorted.size(), cudaMemcpyHostToDevice, r->stream));
+        CUDA_TRY(cudaMemcpyAsync(targetsHold.p, targets.data(), sizeof(unsigned int) * targets.size(), cudaMemcpyHostToDevice, r->stream));
+        // longest run of every (CTA, pair), then longest row of delay-0 synapses of every pair
+        const size_t numLongest = runs.size() + runsPerCta;
+        CUDA_TRY(cudaMalloc(&longest.p, sizeof(unsigned int) * numLongest));
+        auto pass = [&](int which) -> int {
+            for(const auto &pr : pairs) {
+                ResidentBuild B;
+                B.groups = sortedHold.as<b200_synapse_group>() + pr.first;
+                B.target = targetsHold.as<unsigned int>() + pr.first;
+                B.num_groups = pr.count;
+                B.num_src = r->neuronGroups[pr.src].num_neurons;
+                B.unit_start = dUnitStart; B.columns = dColumns; B.depth = dDepths; B.grid = grid;
+                B.runs_stride = (unsigned int)runsPerCta;
+                if(!B.num_src) continue;
+                const size_t at = (size_t)pr.delayClass * numGroups + pr.src;
+                B.late = (L.kind[pr.delayClass] == RESIDENT_LATE);
+                B.split = (L.kind[pr.delayClass] == RESIDENT_SPLIT);
+                B.near_longest = longest.as<unsigned int>() + runs.size() + at;
+                B.near = nears[at];
+                B.near_entries = dNear;
+                CUDA_TRY(residentBuild(B, which, longest.as<unsigned int>() + at, dRuns ? dRuns + at : nullptr, dEntries, r->state,
+                                       std::min(B.num_src, (unsigned int)sms * 8u), r->stream));
+                r->launches++;
+            }
+            return B200_OK;
+        };
+        std::vector<unsigned int> longestHost(numLongest);
+        auto count = [&]() -> int {
+            CUDA_TRY(cudaMemsetAsync(longest.p, 0, sizeof(unsigned int) * numLongest, r->stream));
+            if(const int err = pass(0)) return err;
+            CUDA_TRY(cudaMemcpyAsync(longestHost.data(), longest.p, sizeof(unsigned int) * numLongest, cudaMemcpyDeviceToHost, r->stream));
+            CUDA_TRY(cudaStreamSynchronize(r->stream));
+            return B200_OK;
+        };
+        if(const int err = count()) return err;
+        // every CTA reads the whole row of delay-0 synapses: worth it while that is a few loads
+        bool again = false;
+        for(size_t pair = 0; pair < runsPerCta; pair++) {
+            if(longestHost[runs.size() + pair] > RESIDENT_NEAR_MOST && L.kind[pair / numGroups] == RESIDENT_SPLIT) {
+                L.kind[pair / numGroups] = RESIDENT_IMMEDIATE;
+                again = true;
+            }
+        }
+        if(again) if(const int err = count()) return err;
+        for(size_t pair = 0; pair < runsPerCta; pair++) {
+            unsigned int row = 0;
+            for(unsigned int c = 0; c < grid; c++) {
+                ResidentRun &run = runs[c * runsPerCta + pair];
+                run.base = cells + row;
+                run.length = (longestHost[c * runsPerCta + pair] + 3u) & ~3u;
+                row += run.length;
+                unsigned int &chunks = L.chunks[pair / numGroups];
+                chunks = std::max(chunks, (run.length + RESIDENT_CHUNK - 1u) / RESIDENT_CHUNK);
+            }
+            nears[pair].base = nearCells;
+            nears[pair].row_base = cells;
+            nears[pair].length = (longestHost[runs.size() + pair] + 3u) & ~3u;
+            cells += (unsigned long long)row * r->neuronGroups[pair % numGroups].num_neurons;
+            nearCells += (unsigned long long)nears[pair].length * r->neuronGroups[pair % numGroups].num_neurons;
+            unsigned int &nearChunks = L.near_chunks[pair / numGroups];
+            nearChunks = std::max(nearChunks, (nears[pair].length + 31u) / 32u);
+            for(unsigned int c = 0; c < grid; c++) runs[c * runsPerCta + pair].row = row;
+        }
+        // padded runs of a network with few synapses per (source neuron, CTA) pair can take several times the room of its
+        // arrays: the copy may use a quarter of what is free
+        size_t freeBytes = 0, totalBytes = 0;
+        CUDA_TRY(cudaMemGetInfo(&freeBytes, &totalBytes));
+        if((cells + nearCells) * sizeof(uint2) > freeBytes / 4) { r->dropResident(); return no("the padded copy of the synapses would take more than a quarter of the free memory"); }
+        // (a table that stays in L2 once it has been read needs no fetching ahead: measured on tables of up to half of it)
+        int l2 = 0;
+        CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, r->device));
+        L.prefetch = (cells + nearCells) * sizeof(uint2) > (size_t)l2 / 2 ? 1u : 0u;
+        if(const int err = device(sizeof(uint2) * cells, (void**)&dEntries)) return err;
+        CUDA_TRY(cudaMemsetAsync(dEntries, 0xFF, sizeof(uint2) * cells, r->stream));
+        if(const int err = device(sizeof(uint2) * nearCells, (void**)&dNear)) return err;
+        CUDA_TRY(cudaMemsetAsync(dNear, 0xFF, sizeof(uint2) * nearCells, r->stream));
+        if(const int err = upload(runs.data(), sizeof(ResidentRun) * runs.size(), (void**)&dRuns)) return err;
+        if(const int err = pass(1)) return err;
+        CUDA_TRY(cudaStreamSynchronize(r->stream));         // (the temporaries go out of scope)
+    }
+    else if(const int err = upload(runs.data(), sizeof(ResidentRun) * runs.size(), (void**)&dRuns)) return err;
+
+    // ---- DENSE and BITMASK groups ---------------------------------------------------------------------------------
+    std::vector<ResidentSpan> spans;
+    for(const auto &l : links) {
+        const auto &g = r->synapseGroups[l.syn];
+        if(g.connectivity == B200_CONN_SPARSE) continue;
+        const bool constant = (g.wu_model == B200_WU_STATIC_PULSE_CONSTANT_WEIGHT);
+        spans.push_back(ResidentSpan{constant ? nullptr : g.g, g.connectivity == B200_CONN_BITMASK ? g.gp : nullptr, g.wu_params[0], g.row_stride,
+                                     g.num_trg, l.delayClass, l.src, l.trg, l.psm, g.num_src});
+    }
+    if(const int err = upload(spans.data(), sizeof(ResidentSpan) * spans.size(), (void**)&L.spans)) return err;
+    if(const int err = upload(nears.data(), sizeof(ResidentNear) * nears.size(), (void**)&L.near)) return err;
+    if(!poisson.empty()) {
+        if(const int err = upload(poisson.data(), sizeof(float) * poisson.size(), (void**)&L.poisson)) return err;
+    }
+
+    // ---- messages ---------------------------------------------------------------------------------------------------
+    L.buffers = longestDelay + shortest + 3u;
+    L.history = history;
+    const unsigned int mostIds = neuronWarps * 32u;
+    L.more_words = (mostIds - RESIDENT_CELL_IDS + RESIDENT_MORE_IDS - 1u) / RESIDENT_MORE_IDS;
+    L.copies = (grid + RESIDENT_READERS - 1u) / RESIDENT_READERS;
+    const size_t headWords = (size_t)L.buffers * L.copies * grid * 2u, moreWords = (size_t)L.buffers * grid * L.more_words;
+    void *mail = nullptr;
+    r->residentMailBytes = sizeof(unsigned long long) * (headWords + moreWords + 1u);
+    if(const int err = device(r->residentMailBytes, &mail)) return err;
+    L.inbox = static_cast<ulonglong2*>(mail);
+    L.more = static_cast<unsigned long long*>(mail) + headWords;
+    L.leave = L.more + moreWords;
+
+    L.unit_start = dUnitStart; L.unit_first = dUnitFirst; L.columns = dColumns; L.cta_columns = dCtaColumns; L.runs = dRuns; L.entries = dEntries; L.near_entries = dNear;
+    L.num_spans = numSpans; L.num_units = units;
+    L.num_depths = (unsigned int)depths.size();
+    L.num_delays = numDelays;
+    for(size_t i = 0; i < depths.size(); i++) L.depth[i] = depths[i];
+    for(size_t i = 0; i < delays.size(); i++) L.delay[i] = delays[i];
+    L.acc_floats = (unsigned int)accFloats;
+    r->residentGrid = grid;
+    r->residentBlock = warps * 32u;
+    r->residentSmem = tables + accFloats * sizeof(float);
+    CUDA_TRY(cudaFuncSetAttribute(r->residentKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    r->residentReady = true;
+    return B200_OK;
+}
+
+int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long long numRec)
+{
+    ResidentLaunch &L = r->resident;
+    L.neuron.groups = r->neuronTable.d;
+    L.neuron.block_start = r->neuronTable.blockStart;
+    L.neuron.num_groups = r->neuronTable.num;
+    L.neuron.batch = 1;
+    L.neuron.dt = r->dt;
+    L.neuron.seed = r->seed;
+    L.neuron.num_recording_timesteps = numRec;
+    L.neuron.state = r->state;
+    L.neuron.count_events = r->countEvents ? 1u : 0u;
+    L.count_events = r->countEvents ? 1u : 0u;
+    L.num_steps = (unsigned int)numSteps;
+    // a message word is known by the last 20 bits of its step: before they repeat, no old word may be left
+    if(r->residentTagged == ~0ull || r->residentTagged + numSteps >= RESIDENT_TAG_STEPS - 1ull) {
+        CUDA_TRY(cudaMemsetAsync(L.inbox, 0, r->residentMailBytes, r->stream));
+        r->residentTagged = 0;
+    }
+    r->residentTagged += numSteps;
+    void *args[] = {&L};
+    CUDA_TRY(cudaLaunchCooperativeKernel(r->residentKernel, dim3(r->residentGrid), dim3(r->residentBlock), args, r->residentSmem, r->stream));
+    r->launches++;
+    r->fusedLaunches++;
+    return B200_OK;
+}
+
+// Whether b200_step_time takes the target-resident kernel (its tables are built if they were not).
+int chooseResident(b200_runner *r, bool *yes)
+{
+    *yes = false;
+    if(!r->useFused || !r->useResident || r->scheduleChosen || r->timing || r->sharded() || r->batch != 1) return B200_OK;
+    if(r->residentStale) {
+        if(const int e = buildResident(r)) { r->dropResident(); return e; }
+    }
+    *yes = r->residentReady;
+    return B200_OK;
+}
+
 // Before steps are enqueued (or captured) on the one-launch-per-kernel path.
 int ensureTiled(b200_runner *r)
 {
@@ -1441,6 +1840,7 @@ int b200_runner_destroy(b200_runner *r)
     r->dropNear();
     if(r->fusedCtaCycles) cudaFree(r->fusedCtaCycles);
     r->dropTiled();
+    r->dropResident();
     for(unsigned int p = 0; p < B200_MAX_RANKS; p++) {
         if(r->peerArena[p] && !r->peerLocal[p]) cudaIpcCloseMemHandle(r->peerArena[p]);
     }
@@ -1707,7 +2107,7 @@ int b200_array_push(b200_runner *r, void *device_ptr, const void *host, size_t b
     CUDA_TRY(cudaMemcpyAsync(device_ptr, host, bytes, cudaMemcpyHostToDevice, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     if(touchesDelays(r, device_ptr, bytes)) { r->lagStale = true; r->nearDataStale = true; }
-    if(touchesSparse(r, device_ptr, bytes)) r->tiledStale = true;
+    if(touchesSparse(r, device_ptr, bytes)) r->tiledStale = r->residentStale = true;
     return B200_OK;
 }
 
@@ -1730,7 +2130,7 @@ int b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes)
 {
     CUDA_TRY(cudaMemsetAsync(device_ptr, value, bytes, r->stream));
     if(touchesDelays(r, device_ptr, bytes)) { r->lagStale = true; r->nearDataStale = true; }
-    if(touchesSparse(r, device_ptr, bytes)) r->tiledStale = true;
+    if(touchesSparse(r, device_ptr, bytes)) r->tiledStale = r->residentStale = true;
     return B200_OK;
 }
 
@@ -1830,10 +2230,15 @@ int b200_push_custom_update(b200_runner *r, const char *name, uint32_t idx, cons
 int b200_set_option(b200_runner *r, const char *name, double value)
 {
     const std::string n(name);
+    // (an option that picks a schedule of the other persistent kernels asks for those kernels)
+    if(n == "use_lag" || n == "use_emit" || n == "use_split" || n == "stream_warps") r->scheduleChosen = true;
     if(n == "spike_lanes") r->spikeLanes = std::max(1u, (unsigned int)value);
     else if(n == "count_events") r->countEvents = (value != 0.0);
     else if(n == "use_graph") r->useGraph = (value != 0.0);
     else if(n == "use_fused") r->useFused = (value != 0.0);
+    else if(n == "use_resident") { r->useResident = (value != 0.0); r->scheduleChosen = false; }
+    else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; }
+    else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; }
     else if(n == "use_lag") { r->useLag = (value != 0.0); r->lagStale = true; }
     else if(n == "use_split") { r->useSplit = (value != 0.0); r->lagStale = true; }
     else if(n == "use_near_queues") r->useNearQueues = (value != 0.0);
@@ -1892,7 +2297,7 @@ int b200_init_var(b200_runner *r, void *device_ptr, uint32_t elem_bytes, uint64_
                   uint32_t snippet, const float *params, uint32_t rng_stream)
 {
     r->lagStale = true;
-    r->tiledStale = true;
+    r->tiledStale = r->residentStale = true;
     InitParams prm{};
     for(int i = 0; i < 4; i++) prm.p[i] = params ? params[i] : 0.0f;
     const unsigned int blocks = (unsigned int)std::min<uint64_t>((count + INIT_BLOCK - 1) / INIT_BLOCK, 148u * 32u);
@@ -1915,7 +2320,7 @@ int b200_init_sparse_connectivity(b200_runner *r, uint32_t snippet, const float 
                                   uint32_t *row_length, void *ind, uint32_t rng_stream)
 {
     r->lagStale = true;
-    r->tiledStale = true;
+    r->tiledStale = r->residentStale = true;
     if(trg_end > num_trg || trg_begin >= trg_end) return fail(B200_ERR_INVALID, "bad target range");
     InitParams prm{};
     for(int i = 0; i < 4; i++) prm.p[i] = params ? params[i] : 0.0f;
@@ -1942,7 +2347,7 @@ int b200_init_sparse_vars(b200_runner *r, const uint32_t *row_length, uint32_t n
                           uint32_t snippet, const float *params, uint32_t rng_stream)
 {
     r->lagStale = true;
-    r->tiledStale = true;
+    r->tiledStale = r->residentStale = true;
     InitParams prm{};
     for(int i = 0; i < 4; i++) prm.p[i] = params ? params[i] : 0.0f;
     const uint64_t total = (uint64_t)num_src * row_stride;
@@ -2008,7 +2413,17 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
         return fail(B200_ERR_STATE, "a sharded model runs on the persistent kernel only (batch 1, SPARSE "
                                     "non-learning groups, per-kernel timing off)");
     }
-    if(r->useFused && r->fusedEligible && !r->timing) {
+    bool resident = false;
+    if(num_steps && (e = chooseResident(r, &resident)) != B200_OK) return e;
+    if(resident) {
+        while(left) {
+            const uint64_t n = std::min<uint64_t>(left, RESIDENT_TAG_STEPS / 2);
+            e = launchResident(r, n, num_recording_timesteps);
+            if(e) return e;
+            left -= n;
+        }
+    }
+    else if(r->useFused && r->fusedEligible && !r->timing) {
         while(left) {
             const uint64_t n = std::min<uint64_t>(left, 1ull << 20);
             e = launchFused(r, n, num_recording_timesteps);
@@ -2036,7 +2451,7 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
         e = enqueueStep(r, num_recording_timesteps, false);
         if(e) return e;
     }
-    if(r->tiledReady && !(r->useFused && r->fusedEligible && !r->timing)) {
+    if(r->tiledReady && !resident && !(r->useFused && r->fusedEligible && !r->timing)) {
         e = fetchPeak(r);
         if(e) return e;
     }
@@ -2151,6 +2566,7 @@ static int reportDeviceError(b200_runner *r, unsigned int err)
 {
     if(!err) return B200_OK;
     cudaMemsetAsync(&r->state->error, 0, sizeof(unsigned int), r->stream);
+    r->residentTagged = ~0ull;          // (a launch that gave up may have left messages of steps that count again)
     return fail(B200_ERR_DEVICE_CHECK, "device-side check failed (flags 0x%x:%s%s%s%s%s)", err,
                 (err & ERR_SPIKE_OVERFLOW) ? " spike list overflow" : "",
                 (err & ERR_IND_RANGE) ? " index or row length out of range" : "",
@@ -2197,6 +2613,15 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
             if(e) return e;
         }
         *value = r->streamWarps;
+        return B200_OK;
+    }
+    if(n == "resident") {
+        // whether b200_step_time takes the target-resident kernel
+        int e = prepare(r);
+        bool yes = false;
+        if(!e) e = chooseResident(r, &yes);
+        if(e) return e;
+        *value = yes ? 1u : 0u;
         return B200_OK;
     }
     if(n == "schedule") {

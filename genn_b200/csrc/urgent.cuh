@@ -21,7 +21,7 @@ __device__ __forceinline__ bool urgentDelay(unsigned int d, unsigned int D)
 }
 
 // len[row] = urgent synapses of the row.  One warp per row.
-__global__ void urgentCountKernel(const b200_synapse_group g, unsigned int *len)
+static __global__ void urgentCountKernel(const b200_synapse_group g, unsigned int *len)
 {
     const unsigned int lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
     const unsigned int D = g.max_den_delay;

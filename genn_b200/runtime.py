@@ -386,8 +386,7 @@ class Runtime:
         return int(v.value)
 
     def step_path(self):
-        """(path, reason): 2 target-stationary persistent kernel, 1 persistent kernel with global
-        reductions, 0 one launch per kernel; reason says why path 2 was not taken."""
+        """(path, reason): 1 persistent kernel, 0 one launch per kernel; reason says why not path 1."""
         path = C.c_int()
         why = C.create_string_buffer(256)
         check(self.lib.b200_get_step_path(self.handle, C.byref(path), why, 256))

@@ -1,0 +1,130 @@
+"""The target-resident time-step path (resident.cu) against the reference's golden vectors and the CPU checker: every grid
+size and block size changes which CTA holds a neuron, launches of every length hand over to the other paths, more
+spikes than a message head or the delivery list holds, several axonal delays and ring depths in one model."""
+import numpy as np
+import pytest
+
+from genn_b200 import GeNNModel, init_postsynaptic, init_weight_update
+from genn_b200.resolve import resolve
+from tests import helpers
+from tests.cases import CASES
+from tests.test_gpu_parity import _Adapter, _runtime
+
+pytestmark = pytest.mark.gpu
+NAMES = ["ff_sparse", "ff_sparse_narrow", "ff_bitmask", "ff_dense", "potjans_mini", "potjans_mini_d1", "cond_delay", "izhikevich", "c1_full"]
+
+
+def _resident(name, ctas=0, warps=0):
+    model, steps, dump_every = CASES[name]()
+    net = resolve(model)
+    rt = _runtime(net, steps)
+    rt.set_option("resident_ctas", ctas)
+    rt.set_option("resident_warps", warps)
+    assert rt.counter("resident") == 1
+    return net, rt, steps, dump_every
+
+
+@pytest.mark.parametrize("ctas,warps", [(0, 0), (1, 24), (7, 4), (148, 24)])
+@pytest.mark.parametrize("name", NAMES)
+def test_all_steps_in_one_launch_match_the_reference(name, ctas, warps):
+    net, rt, steps, _ = _resident(name, ctas, warps)
+    rt.set_option("count_events", 1)
+    before = rt.kernel_launches
+    rt.step_time(steps)
+    rt.synchronize()
+    assert rt.kernel_launches == before + 1
+    rt.pull_recording_buffers()
+    want = helpers.load_golden(name)
+    for p in net.pops:
+        if p.record:
+            times, ids = rt.recorded_spikes(p.name)[0]
+            got = helpers.sorted_pairs(np.stack([np.rint(times / net.dt).astype(np.uint32), ids], axis=1))
+            assert np.array_equal(got, want[f"spikes_{p.name}"]), f"recorded spikes of {p.name} differ"
+    final = helpers.snapshot(_Adapter(rt), net, steps)
+    helpers.compare(final, {k: v for k, v in want.items() if k.endswith(f"_{steps}")}, exact_state=False, rtol=1e-5, atol=2e-6)
+    assert rt.counter("spikes") == sum(len(want[f"spikes_{p.name}"]) for p in net.pops)
+    rt.close()
+
+
+@pytest.mark.parametrize("name", ["ff_sparse", "ff_bitmask", "potjans_mini", "cond_delay", "izhikevich"])
+def test_launches_of_every_length_hand_over_to_the_other_paths(name):
+    """Steps on this path alternate with steps on the one-launch-per-kernel path: spike lists, rings and state between
+    launches must be what that path expects, and the current spikes those of the reference."""
+    net, rt, steps, dump_every = _resident(name)
+    chunk = [1, 2, 1, 5, 3, 17, 1, 1, 40]
+    spikes = {p.name: [] for p in net.pops}
+    done = i = 0
+    while done < steps:
+        n = min(chunk[i % len(chunk)], steps - done)
+        rt.set_option("use_fused", 0 if (i % 3 == 2) else 1)
+        rt.step_time(n)
+        done += n
+        i += 1
+        for p in net.pops:
+            spikes[p.name] += [(done - 1, int(j)) for j in rt.current_spikes(p.name)]
+    want = helpers.load_golden(name)
+    for p in net.pops:
+        ends = {s for s, _ in spikes[p.name]}
+        ref = np.array([q for q in want[f"spikes_{p.name}"] if int(q[0]) in ends]).reshape(-1, 2)
+        assert np.array_equal(helpers.sorted_pairs(spikes[p.name]), helpers.sorted_pairs(ref)), p.name
+    final = helpers.snapshot(_Adapter(rt), net, steps)
+    helpers.compare(final, {k: v for k, v in want.items() if k.endswith(f"_{steps}")}, exact_state=False, rtol=1e-5, atol=2e-6)
+    rt.close()
+
+
+def _mixed():
+    """Two populations that all fire at once (more spikes than a message head or the delivery list holds), groups of all
+    three connectivities, axonal delays 0, 2 and 5, inputs with and without a ring."""
+    rng = np.random.default_rng(3)
+    m = GeNNModel("float", "mixed")
+    m.dt = 1.0
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.5, "TauRefrac": 2.0}
+    a = m.add_neuron_population("a", 2500, "LIF", lif, {"V": np.where(rng.random(2500) < 0.9, -50.5, -60.0).astype(np.float32), "RefracTime": 0.0})
+    b = m.add_neuron_population("b", 70, "LIF", lif, {"V": rng.uniform(-65, -50, 70).astype(np.float32), "RefracTime": 0.0})
+    pre = np.repeat(np.arange(2500, dtype=np.uint32), 3)
+    sg = m.add_synapse_population("ab", "SPARSE", a, b, init_weight_update("StaticPulseDendriticDelay", {}, {
+        "g": rng.uniform(0, 1e-3, 7500).astype(np.float32), "d": rng.integers(0, 9, 7500).astype(np.uint8)}), init_postsynaptic("ExpCurr", {"tau": 3.0}))
+    sg.set_sparse_connections(pre, rng.integers(0, 70, 7500).astype(np.uint32))
+    sg.max_dendritic_delay_timesteps = 7        # delays of 7 and 8 steps wrap around
+    sg.axonal_delay_steps = 2
+    m.add_synapse_population("ba", "DENSE", b, a, init_weight_update("StaticPulse", {}, {"g": rng.uniform(0, 0.01, (70, 2500)).astype(np.float32)}),
+                             init_postsynaptic("ExpCurr", {"tau": 5.0}))
+    sg = m.add_synapse_population("aa", "BITMASK", a, a, init_weight_update("StaticPulseConstantWeight", {"g": -2e-4}), init_postsynaptic("ExpCurr", {"tau": 5.0}))
+    sg.set_sparse_connections(rng.integers(0, 2500, 30000).astype(np.uint32), rng.integers(0, 2500, 30000).astype(np.uint32))
+    sg.axonal_delay_steps = 5
+    sg = m.add_synapse_population("aa2", "SPARSE", a, a, init_weight_update("StaticPulse", {}, {"g": rng.uniform(0, 1e-3, 7500).astype(np.float32)}),
+                                  init_postsynaptic("ExpCurr", {"tau": 5.0}))
+    sg.set_sparse_connections(pre, rng.integers(0, 2500, 7500).astype(np.uint32))
+    return m
+
+
+@pytest.mark.parametrize("ctas", [0, 4, 148])
+def test_mixed_groups_and_bursts_match_the_cpu_checker(ctas):
+    from oracle.oracle import OracleRunner
+    net = resolve(_mixed())
+    rt, orc = _runtime(net, 50), OracleRunner(resolve(_mixed()), 50)
+    rt.set_option("resident_ctas", ctas)
+    assert rt.counter("resident") == 1
+    done = 0
+    for n in (1, 1, 3, 4, 11, 20):
+        rt.step_time(n)
+        orc.step(n)
+        done += n
+        for p in net.pops:
+            assert np.array_equal(np.sort(rt.current_spikes(p.name)), np.sort(orc.current_spikes(p.name))), f"step {done} {p.name}"
+            helpers.assert_close(rt.array(f"{p.name}.V")[0], orc.array(f"{p.name}.V")[0], f"step {done} V {p.name}", 1e-5, 2e-6)
+    rt.close()
+    orc.close()
+
+
+def test_pushed_weights_reach_the_private_copy():
+    net, rt, steps, _ = _resident("ff_sparse")
+    other = _runtime(resolve(CASES["ff_sparse"]()[0]), steps)
+    other.set_option("use_fused", 0)
+    for r in (rt, other):
+        r.step_time(20)
+        r.plan.push("syn.g", (net.syn("syn").g * 0.5).astype(np.float32))
+        r.step_time(80)
+    helpers.assert_close(rt.array("psm0.out_post")[0], other.array("psm0.out_post")[0], "out_post after a weight push", 1e-5, 2e-6)
+    rt.close()
+    other.close()
