@@ -29,6 +29,7 @@
 #include "stream_step.cuh"
 #include "tiled.cuh"
 #include "resident.h"
+#include "memory.h"
 #include "record.cuh"
 
 #include <cub/device/device_scan.cuh>
@@ -59,7 +60,8 @@ int fail(int code, const char *fmt, ...)
         }                                                                                        \
     } while(0)
 
-constexpr size_t STAGE_BYTES = 256 * 1024;  // page-locked buffer of a runner through which small arrays reach pageable memory
+constexpr size_t STAGE_BYTES = 256 * 1024 - 64;  // page-locked buffer of a runner through which small arrays reach pageable memory
+constexpr size_t LARGE_PULL = 4u << 20;      // arrays from here on are copied out by several threads
 constexpr size_t ARRAY_TAIL_PAD = 256;     // vector loads may read up to 15 bytes past the last element
 
 template<typename T>
@@ -70,22 +72,22 @@ struct DeviceTable
     unsigned int num = 0;
     unsigned int blocks = 0;
 
-    void release()
+    void release(cudaStream_t s)
     {
-        if(d) cudaFree(d);
-        if(blockStart) cudaFree(blockStart);
+        poolFree(d, s);
+        poolFree(blockStart, s);
         d = nullptr; blockStart = nullptr; num = 0; blocks = 0;
     }
 
     cudaError_t upload(const std::vector<T> &items, const std::vector<unsigned int> &starts, cudaStream_t s)
     {
-        release();
+        release(s);
         num = (unsigned int)items.size();
         if(num == 0) return cudaSuccess;
         blocks = starts.back();
-        cudaError_t e = cudaMalloc(&d, sizeof(T) * num);
+        cudaError_t e = poolAlloc(&d, sizeof(T) * num, s);
         if(e != cudaSuccess) return e;
-        e = cudaMalloc(&blockStart, sizeof(unsigned int) * starts.size());
+        e = poolAlloc(&blockStart, sizeof(unsigned int) * starts.size(), s);
         if(e != cudaSuccess) return e;
         e = cudaMemcpyAsync(d, items.data(), sizeof(T) * num, cudaMemcpyHostToDevice, s);
         if(e != cudaSuccess) return e;
@@ -108,8 +110,10 @@ struct Timer
 // Device buffer that is freed on every early return of a build function unless it was handed over.
 struct ScopedDevice
 {
+    cudaStream_t stream;
     void *p = nullptr;
-    ~ScopedDevice() { if(p) cudaFree(p); }
+    explicit ScopedDevice(cudaStream_t s) : stream(s) {}
+    ~ScopedDevice() { poolFree(p, stream); }
     template<typename T> T *as() const { return static_cast<T*>(p); }
     void *release() { void *q = p; p = nullptr; return q; }
 };
@@ -179,6 +183,7 @@ struct b200_runner
     enum Schedule { PLAIN = 0, SPLIT = 1, LAG = 2, EMIT = 3 };
     // "deliver at emission" mode (near.cuh): near synapses of all groups, one row per source neuron
     bool useEmit = true;
+    bool nearExported = false;              // nearTable is an allocation of its own, which other processes map
     uint2 *nearTable = nullptr;             // rows of every source neuron (synapses onto THIS process's neurons)
     NearRing *nearRings = nullptr;          // device copies, [world][numRings] and [world][neuron groups]
     NearSpace *nearSpaces = nullptr;
@@ -194,23 +199,32 @@ struct b200_runner
     bool nearDataStale = false;                     // synapse arrays changed after the exchange
     Schedule schedule = PLAIN;
 
+    void freeNearTable()
+    {
+        if(nearTable) {
+            if(nearExported) cudaFree(nearTable);
+            else poolFree(nearTable, stream);
+        }
+        nearTable = nullptr;
+    }
+
     void dropNear()
     {
-        if(nearTable) cudaFree(nearTable);
-        if(nearRings) cudaFree(nearRings);
-        if(nearSpaces) cudaFree(nearSpaces);
+        freeNearTable();
+        poolFree(nearRings, stream);
+        poolFree(nearSpaces, stream);
         for(uint2 *p : nearImported) if(p) cudaFree(p);
         nearImported.clear();
-        nearTable = nullptr; nearRings = nullptr; nearSpaces = nullptr; numRings = 0;
+        nearRings = nullptr; nearSpaces = nullptr; numRings = 0;
         emitAgreed = false;
     }
 
     void dropUrgent()
     {
         urgentStride.clear();
-        if(urgentOffsets) cudaFree(urgentOffsets);
-        if(urgentEntries) cudaFree(urgentEntries);
-        if(fusedUrgent) cudaFree(fusedUrgent);
+        poolFree(urgentOffsets, stream);
+        poolFree(urgentEntries, stream);
+        poolFree(fusedUrgent, stream);
         urgentOffsets = nullptr; urgentEntries = nullptr; fusedUrgent = nullptr;
         if(!emitAgreed) dropNear();
     }
@@ -270,7 +284,7 @@ struct b200_runner
     {
         void *bufs[] = {tiledTiles, tiledSources, tiledRunStart, tiledCtaStart, tiledPairBatches, tiledKeys, tiledWeights,
                         tiledPairs, tiledPairPrefix, tiledServed};
-        for(void *b : bufs) if(b) cudaFree(b);
+        for(void *b : bufs) poolFree(b, stream);
         tiledTiles = nullptr; tiledSources = nullptr; tiledRunStart = nullptr; tiledCtaStart = nullptr;
         tiledPairBatches = nullptr; tiledKeys = nullptr; tiledWeights = nullptr; tiledPairs = nullptr;
         tiledPairPrefix = nullptr; tiledServed = nullptr;
@@ -293,7 +307,7 @@ struct b200_runner
 
     void dropResident()
     {
-        for(void *p : residentBuffers) cudaFree(p);
+        for(void *p : residentBuffers) poolFree(p, stream);
         residentBuffers.clear();
         residentReady = false;
         residentTagged = ~0ull;
@@ -371,9 +385,12 @@ int withNeuronShape(const b200_runner *r, F f)
 // sources, the two item lists of each, thread slots, shared-memory budget, grid.
 int buildFusedTables(b200_runner *r)
 {
-    if(r->fusedSlotStart) { cudaFree(r->fusedSlotStart); r->fusedSlotStart = nullptr; }
-    if(r->fusedSources) { cudaFree(r->fusedSources); r->fusedSources = nullptr; }
-    if(r->fusedItems) { cudaFree(r->fusedItems); r->fusedItems = nullptr; }
+    poolFree(r->fusedSlotStart, r->stream);
+    r->fusedSlotStart = nullptr;
+    poolFree(r->fusedSources, r->stream);
+    r->fusedSources = nullptr;
+    poolFree(r->fusedItems, r->stream);
+    r->fusedItems = nullptr;
     if(!r->fusedEligible) return B200_OK;
     const std::vector<b200_synapse_group> &sparse = r->fusedGroups;
     std::vector<unsigned int> slotStart{0};
@@ -488,15 +505,15 @@ int buildFusedTables(b200_runner *r)
         });
         if(e) return e;
     }
-    CUDA_TRY(cudaMalloc(&r->fusedSlotStart, sizeof(unsigned int) * slotStart.size()));
+    CUDA_TRY(poolAlloc(&r->fusedSlotStart, sizeof(unsigned int) * slotStart.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->fusedSlotStart, slotStart.data(), sizeof(unsigned int) * slotStart.size(), cudaMemcpyHostToDevice, r->stream));
     if(!sources.empty()) {
-        CUDA_TRY(cudaMalloc(&r->fusedSources, sizeof(FusedSource) * sources.size()));
+        CUDA_TRY(poolAlloc(&r->fusedSources, sizeof(FusedSource) * sources.size(), r->stream));
         CUDA_TRY(cudaMemcpyAsync(r->fusedSources, sources.data(), sizeof(FusedSource) * sources.size(), cudaMemcpyHostToDevice, r->stream));
-        CUDA_TRY(cudaMalloc(&r->fusedItems, sizeof(uint2) * items.size()));
+        CUDA_TRY(poolAlloc(&r->fusedItems, sizeof(uint2) * items.size(), r->stream));
         CUDA_TRY(cudaMemcpyAsync(r->fusedItems, items.data(), sizeof(uint2) * items.size(), cudaMemcpyHostToDevice, r->stream));
     }
-    if(!r->fusedBarrier) CUDA_TRY(cudaMalloc(&r->fusedBarrier, sizeof(unsigned long long)));
+    if(!r->fusedBarrier) CUDA_TRY(poolAlloc(&r->fusedBarrier, sizeof(unsigned long long), r->stream));
     int perSM = r->fusedPerSM, sms = 0, coop = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
     CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, r->device));
@@ -658,8 +675,8 @@ int buildNearTables(b200_runner *r, bool forExport = false)
     if(totalRows == 0 || totalRows >= (1ull << 31)) return B200_OK;
     // (both freed on every way out of this function; a table left behind by a failed build is dropped with the
     // runner's other near tables)
-    ScopedDevice cursorHold, badHold;
-    CUDA_TRY(cudaMalloc(&cursorHold.p, sizeof(unsigned int) * totalRows));
+    ScopedDevice cursorHold(r->stream), badHold(r->stream);
+    CUDA_TRY(poolAlloc(&cursorHold.p, sizeof(unsigned int) * totalRows, r->stream));
     unsigned int *const cursor = cursorHold.as<unsigned int>();
     CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(unsigned int) * totalRows, r->stream));
     for(size_t gi = 0; gi < n; gi++) {
@@ -691,10 +708,11 @@ int buildNearTables(b200_runner *r, bool forExport = false)
     }
     if(cells >= (1ull << 33)) return B200_OK;      // 64 GB of table: not worth it
     CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(unsigned int) * totalRows, r->stream));
-    CUDA_TRY(cudaMalloc(&badHold.p, sizeof(unsigned int)));
+    CUDA_TRY(poolAlloc(&badHold.p, sizeof(unsigned int), r->stream));
     unsigned int *const bad = badHold.as<unsigned int>();
     CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(unsigned int), r->stream));
-    CUDA_TRY(cudaMalloc(&r->nearTable, sizeof(uint2) * (cells + 1)));
+    r->nearExported = forExport;
+    CUDA_TRY(forExport ? cudaMalloc(&r->nearTable, sizeof(uint2) * (cells + 1)) : poolAlloc(&r->nearTable, sizeof(uint2) * (cells + 1), r->stream));
     CUDA_TRY(cudaMemsetAsync(r->nearTable, 0, sizeof(uint2) * (cells + 1), r->stream));
     for(size_t gi = 0; gi < n; gi++) {
         const auto &g = groups[gi];
@@ -715,8 +733,7 @@ int buildNearTables(b200_runner *r, bool forExport = false)
     CUDA_TRY(cudaMemcpyAsync(&isBad, bad, sizeof(unsigned int), cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     if(isBad) {
-        cudaFree(r->nearTable);
-        r->nearTable = nullptr;
+        r->freeNearTable();
         return B200_OK;
     }
     r->numRings = (unsigned int)rings.size();
@@ -726,9 +743,9 @@ int buildNearTables(b200_runner *r, bool forExport = false)
     if(forExport) return B200_OK;       // the owners of the source neurons take their rows from here
     std::vector<NearSpace> spaces(numNeuronGroups);
     for(size_t ni = 0; ni < numNeuronGroups; ni++) spaces[ni] = NearSpace{r->nearTable + firstCell[ni], shifts[ni], 0u, shifts[ni], 0u};
-    CUDA_TRY(cudaMalloc(&r->nearRings, sizeof(NearRing) * rings.size()));
+    CUDA_TRY(poolAlloc(&r->nearRings, sizeof(NearRing) * rings.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->nearRings, rings.data(), sizeof(NearRing) * rings.size(), cudaMemcpyHostToDevice, r->stream));
-    CUDA_TRY(cudaMalloc(&r->nearSpaces, sizeof(NearSpace) * spaces.size()));
+    CUDA_TRY(poolAlloc(&r->nearSpaces, sizeof(NearSpace) * spaces.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->nearSpaces, spaces.data(), sizeof(NearSpace) * spaces.size(), cudaMemcpyHostToDevice, r->stream));
     r->schedule = b200_runner::EMIT;
     return B200_OK;
@@ -763,7 +780,7 @@ int refreshSchedule(b200_runner *r)
         totalRows += (size_t)g.num_src + 1;
     }
     if((r->useLag || r->useSplit) && anyRing && totalRows < (1ull << 31)) {
-        CUDA_TRY(cudaMalloc(&r->urgentOffsets, sizeof(unsigned int) * (totalRows + 1)));
+        CUDA_TRY(poolAlloc(&r->urgentOffsets, sizeof(unsigned int) * (totalRows + 1), r->stream));
         CUDA_TRY(cudaMemsetAsync(r->urgentOffsets, 0, sizeof(unsigned int) * (totalRows + 1), r->stream));
         for(size_t gi = 0; gi < n; gi++) {
             const auto &g = groups[gi];
@@ -821,7 +838,7 @@ int refreshSchedule(b200_runner *r)
             if(total) {
                 CUDA_TRY(cudaMemcpyAsync(r->urgentOffsets, cells.data(), sizeof(unsigned int) * (totalRows + 1),
                                          cudaMemcpyHostToDevice, r->stream));
-                CUDA_TRY(cudaMalloc(&r->urgentEntries, sizeof(uint2) * total));
+                CUDA_TRY(poolAlloc(&r->urgentEntries, sizeof(uint2) * total, r->stream));
                 std::vector<FusedUrgent> table(n);
                 for(size_t gi = 0; gi < n; gi++) {
                     const auto &g = groups[gi];
@@ -837,13 +854,13 @@ int refreshSchedule(b200_runner *r)
                     CUDA_TRY(cudaPeekAtLastError());
                     r->launches++;
                 }
-                CUDA_TRY(cudaMalloc(&r->fusedUrgent, sizeof(FusedUrgent) * n));
+                CUDA_TRY(poolAlloc(&r->fusedUrgent, sizeof(FusedUrgent) * n, r->stream));
                 CUDA_TRY(cudaMemcpyAsync(r->fusedUrgent, table.data(), sizeof(FusedUrgent) * n, cudaMemcpyHostToDevice, r->stream));
                 CUDA_TRY(cudaStreamSynchronize(r->stream));
             }
         }
         if(!r->urgentEntries) {
-            cudaFree(r->urgentOffsets);
+            poolFree(r->urgentOffsets, r->stream);
             r->urgentOffsets = nullptr;
             r->urgentStride.assign(n, 0u);
         }
@@ -1064,9 +1081,9 @@ int buildTiled(b200_runner *r)
     if(numTiles > 65535u) { r->tiledWhyNot = "more than 65535 tiles"; return B200_OK; }
 
     // ---- count, scan, place ---------------------------------------------------------------------
-    ScopedDevice count, runStart, scanTemp, keys, weights;
-    CUDA_TRY(cudaMalloc(&count.p, sizeof(unsigned int) * ((size_t)entries + 1)));
-    CUDA_TRY(cudaMalloc(&runStart.p, sizeof(unsigned int) * ((size_t)entries + 1)));
+    ScopedDevice count(r->stream), runStart(r->stream), scanTemp(r->stream), keys(r->stream), weights(r->stream);
+    CUDA_TRY(poolAlloc(&count.p, sizeof(unsigned int) * ((size_t)entries + 1), r->stream));
+    CUDA_TRY(poolAlloc(&runStart.p, sizeof(unsigned int) * ((size_t)entries + 1), r->stream));
     CUDA_TRY(cudaMemsetAsync(count.p, 0, sizeof(unsigned int) * ((size_t)entries + 1), r->stream));
     std::vector<TiledBuildGroup> build;
     std::vector<TiledSource> sources;
@@ -1105,13 +1122,13 @@ int buildTiled(b200_runner *r)
     if(const int e = launchBuild(0)) return e;
     size_t tempBytes = 0;
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tempBytes, count.as<unsigned int>(), runStart.as<unsigned int>(), (int)(entries + 1), r->stream));
-    CUDA_TRY(cudaMalloc(&scanTemp.p, std::max<size_t>(tempBytes, 16)));
+    CUDA_TRY(poolAlloc(&scanTemp.p, std::max<size_t>(tempBytes, 16), r->stream));
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(scanTemp.p, tempBytes, count.as<unsigned int>(), runStart.as<unsigned int>(), (int)(entries + 1), r->stream));
     unsigned int total = 0;
     CUDA_TRY(cudaMemcpyAsync(&total, runStart.as<unsigned int>() + entries, sizeof(total), cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
-    CUDA_TRY(cudaMalloc(&keys.p, std::max<size_t>((size_t)total * (key16 ? 2 : 4), 16)));
-    if(anyWeights) CUDA_TRY(cudaMalloc(&weights.p, std::max<size_t>((size_t)total * sizeof(float), 16)));
+    CUDA_TRY(poolAlloc(&keys.p, std::max<size_t>((size_t)total * (key16 ? 2 : 4), 16), r->stream));
+    if(anyWeights) CUDA_TRY(poolAlloc(&weights.p, std::max<size_t>((size_t)total * sizeof(float), 16), r->stream));
     CUDA_TRY(cudaMemsetAsync(count.p, 0, sizeof(unsigned int) * ((size_t)entries + 1), r->stream));
     if(const int e = launchBuild(1)) return e;
 
@@ -1152,13 +1169,13 @@ int buildTiled(b200_runner *r)
     }
     if(pairs.empty()) { r->tiledWhyNot = "no synapses"; return B200_OK; }
     if((unsigned long long)pairs.size() * r->batch >= (1ull << 31)) { r->tiledWhyNot = "too many (tile, source, batch) pairs"; return B200_OK; }
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, r->device));
-    const unsigned int grid = (unsigned int)prop.multiProcessorCount;
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+    const unsigned int grid = (unsigned int)sms;
     size_t smem = 0;
     for(const auto &T : tiles) smem = std::max(smem, sizeof(float) * T.depth * T.stride);
     auto toDevice = [&](const void *host, size_t bytes, void **out) -> int {
-        CUDA_TRY(cudaMalloc(out, std::max<size_t>(bytes, 16)));
+        CUDA_TRY(poolAlloc(out, std::max<size_t>(bytes, 16), r->stream));
         CUDA_TRY(cudaMemcpyAsync(*out, host, bytes, cudaMemcpyHostToDevice, r->stream));
         return B200_OK;
     };
@@ -1170,9 +1187,9 @@ int buildTiled(b200_runner *r)
     // scratch of the per-step work partition
     {
         const size_t perStep = pairs.size() * r->batch;
-        cudaError_t ce = cudaMalloc(&r->tiledPairBatches, sizeof(unsigned int) * perStep);
-        if(ce == cudaSuccess) ce = cudaMalloc(&r->tiledPairPrefix, sizeof(double) * perStep);
-        if(ce == cudaSuccess) ce = cudaMalloc(&r->tiledCtaStart, sizeof(unsigned int) * 2 * (grid + 1));
+        cudaError_t ce = poolAlloc(&r->tiledPairBatches, sizeof(unsigned int) * perStep, r->stream);
+        if(ce == cudaSuccess) ce = poolAlloc(&r->tiledPairPrefix, sizeof(double) * perStep, r->stream);
+        if(ce == cudaSuccess) ce = poolAlloc(&r->tiledCtaStart, sizeof(unsigned int) * 2 * (grid + 1), r->stream);
         if(ce != cudaSuccess) { r->dropTiled(); CUDA_TRY(ce); }
     }
     CUDA_TRY(cudaFuncSetAttribute(tiledKernelFor(key16, anyWeights), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1187,7 +1204,7 @@ int buildTiled(b200_runner *r)
     r->tiledSynapses = total;
     if(!r->peakHost) {
         // where the neuron kernel's spike-count peaks land (allocated here, with the copy; never on the time-step path)
-        CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&r->peakHost), sizeof(unsigned int), cudaHostAllocPortable));
+        CUDA_TRY(hostAcquire(reinterpret_cast<void**>(&r->peakHost), sizeof(unsigned int)));
         CUDA_TRY(cudaEventCreateWithFlags(&r->peakEvent, cudaEventDisableTiming));
         *r->peakHost = 0u;
     }
@@ -1377,7 +1394,7 @@ int buildResident(b200_runner *r)
     warps = std::min(std::max(warps, std::max(neuronWarps, (grid + 31u) / 32u)), RESIDENT_UNITS);
 
     auto device = [&](size_t bytes, void **out) -> int {
-        CUDA_TRY(cudaMalloc(out, std::max<size_t>(bytes, 16)));
+        CUDA_TRY(poolAlloc(out, std::max<size_t>(bytes, 16), r->stream));
         r->residentBuffers.push_back(*out);
         return B200_OK;
     };
@@ -1423,14 +1440,14 @@ int buildResident(b200_runner *r)
     uint2 *dEntries = nullptr, *dNear = nullptr;
     if(!pairs.empty()) {
         unsigned long long cells = 0, nearCells = 0;
-        ScopedDevice longest, sortedHold, targetsHold;
-        CUDA_TRY(cudaMalloc(&sortedHold.p, sizeof(b200_synapse_group) * sorted.size()));
-        CUDA_TRY(cudaMalloc(&targetsHold.p, sizeof(unsigned int) * targets.size()));
+        ScopedDevice longest(r->stream), sortedHold(r->stream), targetsHold(r->stream);
+        CUDA_TRY(poolAlloc(&sortedHold.p, sizeof(b200_synapse_group) * sorted.size(), r->stream));
+        CUDA_TRY(poolAlloc(&targetsHold.p, sizeof(unsigned int) * targets.size(), r->stream));
         CUDA_TRY(cudaMemcpyAsync(sortedHold.p, sorted.data(), sizeof(b200_synapse_group) * sorted.size(), cudaMemcpyHostToDevice, r->stream));
         CUDA_TRY(cudaMemcpyAsync(targetsHold.p, targets.data(), sizeof(unsigned int) * targets.size(), cudaMemcpyHostToDevice, r->stream));
         // longest run of every (CTA, pair), then longest row of delay-0 synapses of every pair
         const size_t numLongest = runs.size() + runsPerCta;
-        CUDA_TRY(cudaMalloc(&longest.p, sizeof(unsigned int) * numLongest));
+        CUDA_TRY(poolAlloc(&longest.p, sizeof(unsigned int) * numLongest, r->stream));
         auto pass = [&](int which) -> int {
             for(const auto &pr : pairs) {
                 ResidentBuild B;
@@ -1492,8 +1509,8 @@ int buildResident(b200_runner *r)
         }
         // padded runs of a network with few synapses per (source neuron, CTA) pair can take several times the room of its
         // arrays: the copy may use a quarter of what is free
-        size_t freeBytes = 0, totalBytes = 0;
-        CUDA_TRY(cudaMemGetInfo(&freeBytes, &totalBytes));
+        size_t freeBytes = POOL_KEEP * 4, totalBytes = 0;       // (what the pool may keep needs no asking)
+        if((cells + nearCells) * sizeof(uint2) > freeBytes / 4) CUDA_TRY(cudaMemGetInfo(&freeBytes, &totalBytes));
         if((cells + nearCells) * sizeof(uint2) > freeBytes / 4) { r->dropResident(); return no("the padded copy of the synapses would take more than a quarter of the free memory"); }
         // (a table that stays in L2 once it has been read needs no fetching ahead: measured on tables of up to half of it)
         int l2 = 0;
@@ -1764,7 +1781,7 @@ int b200_runner_create(int device, double dt, uint64_t seed, uint32_t batch_size
     r->seed = seed;
     r->batch = batch_size;
     CUDA_TRY(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking));
-    CUDA_TRY(cudaMalloc(&r->state, sizeof(StepState)));
+    CUDA_TRY(poolAlloc(&r->state, sizeof(StepState), r->stream));
     CUDA_TRY(cudaMemsetAsync(r->state, 0, sizeof(StepState), r->stream));
     {
         const unsigned long long limits[3] = {BARRIER_SPIN_LIMIT, EXCHANGE_SPIN_LIMIT, (unsigned long long)STREAM_WAIT_CYCLES};
@@ -1774,7 +1791,7 @@ int b200_runner_create(int device, double dt, uint64_t seed, uint32_t batch_size
     CUDA_TRY(cudaEventCreate(&r->evB));
     CUDA_TRY(cudaEventCreate(&r->evC));
     CUDA_TRY(cudaEventCreate(&r->evD));
-    CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&r->stage), STAGE_BYTES + 64, cudaHostAllocPortable));
+    CUDA_TRY(hostAcquire(reinterpret_cast<void**>(&r->stage), STAGE_BYTES + 64));
     r->hostWord = reinterpret_cast<unsigned int*>(r->stage + STAGE_BYTES);
     *out = r;
     return B200_OK;
@@ -1826,36 +1843,36 @@ int b200_runner_destroy(b200_runner *r)
     cudaSetDevice(r->device);
     cudaStreamSynchronize(r->stream);
     r->dropGraph();
-    r->neuronTable.release();
-    r->sparseTable.release();
-    r->postSpanTable.release();
-    r->proceduralTable.release();
-    r->learnTable.release();
-    if(r->fusedSlotStart) cudaFree(r->fusedSlotStart);
-    if(r->fusedSources) cudaFree(r->fusedSources);
-    if(r->fusedItems) cudaFree(r->fusedItems);
-    if(r->fusedBarrier) cudaFree(r->fusedBarrier);
-    if(r->lagScan) cudaFree(r->lagScan);
+    r->neuronTable.release(r->stream);
+    r->sparseTable.release(r->stream);
+    r->postSpanTable.release(r->stream);
+    r->proceduralTable.release(r->stream);
+    r->learnTable.release(r->stream);
+    poolFree(r->fusedSlotStart, r->stream);
+    poolFree(r->fusedSources, r->stream);
+    poolFree(r->fusedItems, r->stream);
+    poolFree(r->fusedBarrier, r->stream);
+    poolFree(r->lagScan, r->stream);
     r->dropUrgent();
     r->dropNear();
-    if(r->fusedCtaCycles) cudaFree(r->fusedCtaCycles);
+    poolFree(r->fusedCtaCycles, r->stream);
     r->dropTiled();
     r->dropResident();
     for(unsigned int p = 0; p < B200_MAX_RANKS; p++) {
         if(r->peerArena[p] && !r->peerLocal[p]) cudaIpcCloseMemHandle(r->peerArena[p]);
     }
-    if(r->stage) cudaFreeHost(r->stage);
-    if(r->recCounts) cudaFree(r->recCounts);
-    if(r->recList) cudaFree(r->recList);
-    if(r->recHost) cudaFreeHost(r->recHost);
-    if(r->peakHost) cudaFreeHost(r->peakHost);
+    hostRelease(r->stage);
+    poolFree(r->recCounts, r->stream);
+    poolFree(r->recList, r->stream);
+    hostRelease(r->recHost);
+    hostRelease(r->peakHost);
     if(r->peakEvent) cudaEventDestroy(r->peakEvent);
     if(r->ncclComm && ncclApi()) ncclApi()->commDestroy(r->ncclComm);
-    if(r->reducePacked) cudaFree(r->reducePacked);
+    poolFree(r->reducePacked, r->stream);
     if(r->arena) cudaFree(r->arena);
-    if(r->peerTable) cudaFree(r->peerTable);
-    for(auto &a : r->arrays) cudaFree(a.first);
-    cudaFree(r->state);
+    poolFree(r->peerTable, r->stream);
+    for(auto &a : r->arrays) poolFree(a.first, r->stream);
+    poolFree(r->state, r->stream);
     cudaEventDestroy(r->evA);
     cudaEventDestroy(r->evB);
     cudaEventDestroy(r->evC);
@@ -1870,7 +1887,7 @@ int b200_array_alloc(b200_runner *r, size_t bytes, void **device_ptr)
     if(!r || !device_ptr) return fail(B200_ERR_INVALID, "bad arguments to b200_array_alloc");
     CUDA_TRY(cudaSetDevice(r->device));
     void *p = nullptr;
-    CUDA_TRY(cudaMalloc(&p, bytes + ARRAY_TAIL_PAD));
+    CUDA_TRY(poolAlloc(&p, bytes + ARRAY_TAIL_PAD, r->stream));
     CUDA_TRY(cudaMemsetAsync(p, 0, bytes + ARRAY_TAIL_PAD, r->stream));
     r->arrays[p] = bytes;
     *device_ptr = p;
@@ -1881,14 +1898,14 @@ int b200_host_alloc(b200_runner *r, size_t bytes, void **host_ptr)
 {
     if(!r || !host_ptr) return fail(B200_ERR_INVALID, "bad arguments to b200_host_alloc");
     CUDA_TRY(cudaSetDevice(r->device));
-    CUDA_TRY(cudaHostAlloc(host_ptr, bytes ? bytes : 1, cudaHostAllocPortable));
+    CUDA_TRY(hostAcquire(host_ptr, bytes ? bytes : 1));
     return B200_OK;
 }
 
 int b200_host_free(b200_runner *r, void *host_ptr)
 {
     (void)r;
-    CUDA_TRY(cudaFreeHost(host_ptr));
+    hostRelease(host_ptr);
     return B200_OK;
 }
 
@@ -2054,8 +2071,7 @@ int b200_near_finish(b200_runner *r, int agreed)
         if(!r->nearPeerDone[p]) return fail(B200_ERR_STATE, "the rows held by process %u have not been imported", p);
         if(p != r->rank && !r->peerArena[p]) return fail(B200_ERR_STATE, "exchange arena of rank %u has not been opened", p);
     }
-    if(r->nearTable) cudaFree(r->nearTable);
-    r->nearTable = nullptr;
+    r->freeNearTable();
     // the rings of every process as this process sees them: same offset in the peer's arena
     std::vector<NearRing> rings((size_t)r->world * r->numRings);
     for(uint32_t p = 0; p < r->world; p++) {
@@ -2067,11 +2083,11 @@ int b200_near_finish(b200_runner *r, int agreed)
             rings[(size_t)p * r->numRings + i] = ring;
         }
     }
-    if(r->nearRings) cudaFree(r->nearRings);
-    if(r->nearSpaces) cudaFree(r->nearSpaces);
-    CUDA_TRY(cudaMalloc(&r->nearRings, sizeof(NearRing) * rings.size()));
+    poolFree(r->nearRings, r->stream);
+    poolFree(r->nearSpaces, r->stream);
+    CUDA_TRY(poolAlloc(&r->nearRings, sizeof(NearRing) * rings.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->nearRings, rings.data(), sizeof(NearRing) * rings.size(), cudaMemcpyHostToDevice, r->stream));
-    CUDA_TRY(cudaMalloc(&r->nearSpaces, sizeof(NearSpace) * r->nearSpacesAll.size()));
+    CUDA_TRY(poolAlloc(&r->nearSpaces, sizeof(NearSpace) * r->nearSpacesAll.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->nearSpaces, r->nearSpacesAll.data(), sizeof(NearSpace) * r->nearSpacesAll.size(), cudaMemcpyHostToDevice, r->stream));
     r->emitAgreed = true;
     r->queuesAgreed = r->fusedGrid <= NEAR_QUEUE_COUNT;
@@ -2097,7 +2113,7 @@ int b200_array_free(b200_runner *r, void *device_ptr)
     auto it = r->arrays.find(device_ptr);
     if(it == r->arrays.end()) return fail(B200_ERR_INVALID, "pointer was not allocated by this runner");
     CUDA_TRY(cudaStreamSynchronize(r->stream));
-    CUDA_TRY(cudaFree(device_ptr));
+    CUDA_TRY(poolFree(device_ptr, r->stream));
     r->arrays.erase(it);
     return B200_OK;
 }
@@ -2121,8 +2137,20 @@ int b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t b
         memcpy(host, r->stage, bytes);
         return B200_OK;
     }
+    if(bytes >= LARGE_PULL) {
+        CUDA_TRY(pullLarge(host, device_ptr, bytes, 1u, false, r->device, r->stream));
+        return B200_OK;
+    }
     CUDA_TRY(cudaMemcpyAsync(host, device_ptr, bytes, cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
+    return B200_OK;
+}
+
+int b200_array_pull_u32(b200_runner *r, uint32_t *host, const void *device_ptr, uint32_t elem_bytes, uint64_t count)
+{
+    if(!r || (count && (!host || !device_ptr))) return fail(B200_ERR_INVALID, "null argument to b200_array_pull_u32");
+    if(elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4) return fail(B200_ERR_INVALID, "element size %u is not 1, 2 or 4", elem_bytes);
+    if(count) CUDA_TRY(pullLarge(host, device_ptr, count, elem_bytes, true, r->device, r->stream));
     return B200_OK;
 }
 
@@ -2255,7 +2283,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
         r->fusedProfile = (value != 0.0);
         if(r->fusedProfile && !r->fusedCtaCycles) {
             CUDA_TRY(cudaSetDevice(r->device));
-            CUDA_TRY(cudaMalloc(&r->fusedCtaCycles, sizeof(unsigned long long) * 5 * PROFILE_MAX_CTAS));
+            CUDA_TRY(poolAlloc(&r->fusedCtaCycles, sizeof(unsigned long long) * 5 * PROFILE_MAX_CTAS, r->stream));
             CUDA_TRY(cudaMemsetAsync(r->fusedCtaCycles, 0, sizeof(unsigned long long) * 5 * PROFILE_MAX_CTAS, r->stream));
         }
     }
@@ -2520,9 +2548,9 @@ static int runCustomUpdate(b200_runner *r, const char *name, unsigned int phases
     }
     if(total > r->reducePackedElements) {
         CUDA_TRY(cudaStreamSynchronize(r->stream));
-        if(r->reducePacked) CUDA_TRY(cudaFree(r->reducePacked));
+        if(r->reducePacked) CUDA_TRY(poolFree(r->reducePacked, r->stream));
         r->reducePacked = nullptr;
-        CUDA_TRY(cudaMalloc(&r->reducePacked, sizeof(float) * total));
+        CUDA_TRY(poolAlloc(&r->reducePacked, sizeof(float) * total, r->stream));
         CUDA_TRY(cudaMemsetAsync(r->reducePacked, 0, sizeof(float) * total, r->stream));
         r->reducePackedElements = total;
     }
@@ -2786,15 +2814,15 @@ int b200_pull_recording(b200_runner *r, uint32_t num_arrays, const uint32_t *con
     if(chunks == 0) return b200_synchronize(r);
     if(chunks > r->recChunks || capacity > r->recCapacity) {
         CUDA_TRY(cudaStreamSynchronize(r->stream));
-        if(r->recCounts) cudaFree(r->recCounts);
-        if(r->recList) cudaFree(r->recList);
-        if(r->recHost) cudaFreeHost(r->recHost);
+        poolFree(r->recCounts, r->stream);
+        poolFree(r->recList, r->stream);
+        hostRelease(r->recHost);
         r->recCounts = nullptr; r->recList = nullptr; r->recHost = nullptr;
         r->recChunks = r->recCapacity = 0;
         const size_t bytes = sizeof(RecordHeader) + sizeof(uint2) * (size_t)capacity;
-        CUDA_TRY(cudaMalloc(&r->recCounts, sizeof(unsigned int) * chunks));
-        CUDA_TRY(cudaMalloc(&r->recList, bytes));
-        CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&r->recHost), bytes, cudaHostAllocPortable));
+        CUDA_TRY(poolAlloc(&r->recCounts, sizeof(unsigned int) * chunks, r->stream));
+        CUDA_TRY(poolAlloc(&r->recList, bytes, r->stream));
+        CUDA_TRY(hostAcquire(reinterpret_cast<void**>(&r->recHost), bytes));
         r->recChunks = chunks;
         r->recCapacity = capacity;
     }

@@ -147,6 +147,7 @@ class Runtime:
             self._push_custom_updates()
             if getattr(model, "timing_enabled", False):
                 check(self.lib.b200_enable_timing(self.handle, 1))
+        self.counter("resident")        # (has the step kernel's copy of the synapses built now, not by the first step)
         self.synchronize()
 
     # -- sharded models: map every peer's exchange arena ---------------------------
@@ -278,7 +279,10 @@ class Runtime:
     def pull_connectivity(self, sg):
         rs = self.net.syn(sg.name)
         sg.row_lengths = self.array(f"{sg.name}.row_length")
-        sg.ind = self.array(f"{sg.name}.ind").astype(np.uint32)
+        ind = self.plan.arrays[f"{sg.name}.ind"]
+        sg.ind = np.empty(ind.shape, dtype=np.uint32)
+        check(self.lib.b200_array_pull_u32(self.handle, sg.ind.ctypes.data, ind.ptr, ind.dtype.itemsize, sg.ind.size))
+        self.factory.d2h_bytes += ind.nbytes
 
     # -- stepping ---------------------------------------------------------------
     def step_time(self, num_steps: int = 1):

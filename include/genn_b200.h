@@ -241,6 +241,8 @@ int  b200_host_alloc(b200_runner *r, size_t bytes, void **host_ptr);
 int  b200_host_free(b200_runner *r, void *host_ptr);
 int  b200_array_push(b200_runner *r, void *device_ptr, const void *host, size_t bytes);
 int  b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t bytes);
+/* An array of 8-, 16- or 32-bit indices, as 32-bit values. */
+int  b200_array_pull_u32(b200_runner *r, uint32_t *host, const void *device_ptr, uint32_t elem_bytes, uint64_t count);
 int  b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes);
 /* Spike recordings are one bit per neuron and time step and almost all zeros (Runtime::pullRecordingBuffersFromDevice,
  * runtime.cc:720-746, copies them whole).  This appends the non-zero 32-bit words of `words` to `pairs` as
