@@ -79,6 +79,31 @@ __device__ __forceinline__ void redAdd(float *addr, float v)
     asm volatile("red.global.add.f32 [%0], %1;" :: "l"(__cvta_generic_to_global(addr)), "f"(v));
 }
 
+// Four neighbouring cells at once (16-byte aligned).
+__device__ __forceinline__ void redAdd4(float *addr, const float4 &v)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" :: "l"(__cvta_generic_to_global(addr)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+}
+
+// The kernels of the one-launch-per-kernel path follow one another as dependent launches: a kernel's blocks may be placed,
+// and read what no kernel writes, while the kernel before it still runs; chainWait() holds them until that one's results
+// are there.  Every kernel says at once that the next one may be placed: nothing of it runs past its own chainWait().
+__device__ __forceinline__ void chainWait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A block of steps advances the counters once, with its last kernel; the kernels of its step number `ahead` count for
+// themselves (an election of a last block in every step cost 2 us a step).
+__device__ __forceinline__ unsigned int chainPhase(const StepState *state, unsigned int ahead)
+{
+    unsigned int k = state->phase + ahead;
+    const unsigned int period = state->ring_period;
+    if(k >= period && period) k %= period;
+    return k;
+}
+
 __device__ __forceinline__ unsigned int ringSlot(unsigned int k, unsigned int slots)
 {
     return k % slots;

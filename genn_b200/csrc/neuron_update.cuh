@@ -26,6 +26,7 @@
 namespace b200
 {
 constexpr int NEURON_BLOCK = 128;
+constexpr unsigned int NEURON_BLOCKS_PER_SM = 8;
 
 // Peers of a sharded model as the neuron update sees them: every spike id is also
 // stored into each peer's exchange arena, at the offset it has in this process's.
@@ -49,6 +50,8 @@ struct NeuronLaunch
     unsigned long long num_recording_timesteps;
     StepState *state;
     unsigned int count_events;
+    unsigned int ahead;                 // steps of this block of steps that come before this one
+    unsigned int advance;               // last kernel of a block of steps: how many it has, else 0
 };
 
 // Loads of data other SMs write between grid barriers (postsynaptic input,
@@ -376,40 +379,40 @@ template<int NPSM, int NCS>
 __global__ void __launch_bounds__(NEURON_BLOCK)
 neuronUpdateKernel(const NeuronLaunch L)
 {
-    const unsigned int gi = findGroup(L.block_start, L.num_groups, blockIdx.x);
-    const b200_neuron_group &g = L.groups[gi];
-    const unsigned int local = (blockIdx.x - __ldg(&L.block_start[gi])) * NEURON_BLOCK + threadIdx.x;
-    const unsigned int k = L.state->phase;
-    const unsigned long long timestep = L.state->timestep;
-    neuronStep<false, NPSM, NCS>(L, g, blockIdx.y, local, k, timestep);
-
-    // ---- last block: queue update for the next step and counter advance -------
-    __shared__ bool isLast;
-    __threadfence();
-    __syncthreads();
-    if(threadIdx.x == 0) {
-        const unsigned int total = gridDim.x * gridDim.y;
-        isLast = (atomicAdd(&L.state->ticket, 1u) == total - 1u);
+    const unsigned int blocks = __ldg(&L.block_start[L.num_groups]), launched = gridDim.x * gridDim.y;
+    const unsigned int rank = blockIdx.y * gridDim.x + blockIdx.x;
+    chainWait();
+    const unsigned int k = chainPhase(L.state, L.ahead);
+    const unsigned long long timestep = L.state->timestep + L.ahead;
+    for(unsigned int item = rank; item < blocks * L.batch; item += launched) {
+        const unsigned int b = item / blocks, block = item - b * blocks;
+        const unsigned int gi = findGroup(L.block_start, L.num_groups, block);
+        neuronStep<false, NPSM, NCS>(L, L.groups[gi], b, (block - __ldg(&L.block_start[gi])) * NEURON_BLOCK + threadIdx.x, k, timestep);
     }
-    __syncthreads();
-    if(isLast) {
+
+    // ---- queue update for the next step: its slot was last read three steps ago at the latest -------
+    if(rank == launched - 1u) {
         __shared__ unsigned int stepSpikes;
         if(threadIdx.x == 0) stepSpikes = 0u;
         __syncthreads();
         for(unsigned int q = threadIdx.x; q < L.num_groups * L.batch; q += blockDim.x) {
             const b200_neuron_group &o = L.groups[q / L.batch];
             const unsigned int ob = q % L.batch;
+            // (the spikes of the step before: this one's are not all there yet)
+            atomicAdd(&stepSpikes, o.spk_cnt[ob * o.num_delay_slots + ringSlot(k, o.num_delay_slots)]);
             o.spk_cnt[ob * o.num_delay_slots + ringSlot(k + 2, o.num_delay_slots)] = 0;
-            atomicAdd(&stepSpikes, __ldcg(&o.spk_cnt[ob * o.num_delay_slots + ringSlot(k + 1, o.num_delay_slots)]));
         }
         __syncthreads();
-        if(threadIdx.x == 0) {
-            atomicMax(&L.state->peak_spikes, stepSpikes);
+        if(threadIdx.x == 0 && stepSpikes) atomicMax(&L.state->peak_spikes, stepSpikes);
+    }
+    // ---- behind a block of steps: the counters, once every block has read them ------------------------
+    if(L.advance) {
+        __syncthreads();
+        if(threadIdx.x == 0 && atomicAdd(&L.state->ticket, 1u) == launched - 1u) {
             L.state->ticket = 0;
             L.state->timestep = timestep + 1;
-            L.state->steps_done = L.state->steps_done + 1;
+            L.state->steps_done = L.state->steps_done + L.advance;
             L.state->phase = (k + 1 == L.state->ring_period) ? 0u : k + 1;
-            __threadfence();
         }
     }
 }

@@ -204,6 +204,8 @@ int b200_update_neurons_noalloc(int device, void *stream, const b200_neuron_grou
     L.num_recording_timesteps = num_recording_timesteps;
     L.state = &scratch->state;
     L.count_events = 0;
+    L.ahead = 0;
+    L.advance = 1;
     const dim3 grid(blockStart[num_groups], batch_size, 1);
     const int P = (maxPSM <= 1) ? 1 : (maxPSM <= 2) ? 2 : B200_MAX_PSM;
     const int C = (maxCS == 0) ? 0 : (maxCS == 1) ? 1 : B200_MAX_CS;

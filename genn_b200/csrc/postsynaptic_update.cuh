@@ -30,7 +30,8 @@ postsynapticUpdateKernel(const SynapseLaunch L)
     const b200_synapse_group &g = L.groups[gi];
     const unsigned int tile = blockIdx.x - __ldg(&L.block_start[gi]);
     const unsigned int b = blockIdx.z;
-    const unsigned int k = L.state->phase;
+    chainWait();
+    const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned int tslots = g.trg_delay_slots;
     const unsigned int rslot = ringSlot(k + tslots - g.back_prop_delay, tslots);
     const unsigned int count = g.trg_spk_cnt[b * tslots + rslot];
@@ -39,7 +40,7 @@ postsynapticUpdateKernel(const SynapseLaunch L)
     const unsigned int sslots = g.src_delay_slots;
     const float *stPre = g.src_spike_times +
         ((unsigned long long)b * sslots + ringSlot(k + sslots - g.axonal_delay, sslots)) * g.num_src;
-    const float t = B200_FMUL((float)L.state->timestep, L.dt);
+    const float t = B200_FMUL((float)(L.state->timestep + L.ahead), L.dt);
     const bool sparse = (g.connectivity == B200_CONN_SPARSE);
     const unsigned long long perBatch = sparse ? (unsigned long long)g.num_src * g.row_stride
                                                : (unsigned long long)g.num_src * g.num_trg;
@@ -53,17 +54,19 @@ postsynapticUpdateKernel(const SynapseLaunch L)
         unsigned long long idSyn;
         unsigned int pre;
         if(sparse) {
-            idSyn = __ldg(&g.remap[(unsigned long long)post * g.col_stride + i]);
-            pre = (unsigned int)(idSyn / g.row_stride);
+            const unsigned int entry = __ldg(&g.remap[(unsigned long long)post * g.col_stride + i]);
+            idSyn = entry;
+            pre = entry / g.row_stride;
         }
         else {
             pre = i;
             idSyn = (unsigned long long)i * g.num_trg + post;
         }
+        const float w = gb[idSyn];          // (on its way together with the spike time)
         const float dts = B200_FSUB(t, B200_FADD(g.wu_params[6], stPre[pre]));
         if(dts > 0.0f) {
             const float timing = expf(B200_FDIV(-dts, g.wu_params[0]));
-            const float nw = B200_FADD(gb[idSyn], B200_FMUL(g.wu_params[2], timing));
+            const float nw = B200_FADD(w, B200_FMUL(g.wu_params[2], timing));
             gb[idSyn] = fmaxf(g.wu_params[4], fminf(g.wu_params[5], nw));
         }
     }

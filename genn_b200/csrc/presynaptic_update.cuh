@@ -45,6 +45,7 @@ struct SynapseLaunch
     unsigned long long seed;
     StepState *state;
     unsigned int count_events;
+    unsigned int ahead;                 // steps of this block of steps that come before this one
     const unsigned char *tiled_served;  // per SPARSE group: 1 if the target-tiled kernel delivers it in heavy steps; or NULL
 };
 
@@ -154,19 +155,26 @@ __device__ __forceinline__ void sparseTileSTDP(const b200_synapse_group &g, unsi
     const float *stPost = g.trg_spike_times +
         ((unsigned long long)b * tslots + ringSlot(k + tslots - g.back_prop_delay, tslots)) * g.num_trg;
     float *out = g.out_post + (unsigned long long)b * g.num_trg;
+    // every load before any store: a store between two loads would make the second wait for the first
+    unsigned int post[PRE_VEC];
+    float w[PRE_VEC], dts[PRE_VEC];
+#pragma unroll
+    for(int j = 0; j < PRE_VEC; j++) {
+        const unsigned int col = tile * PRE_TILE + j * PRE_BLOCK + threadIdx.x;
+        post[j] = (col < len) ? static_cast<const IndT*>(g.ind)[rowStart + col] : 0u;
+        w[j] = (col < len) ? gb[rowStart + col] : 0.0f;
+    }
+#pragma unroll
+    for(int j = 0; j < PRE_VEC; j++) dts[j] = B200_FSUB(t, B200_FADD(g.wu_params[7], stPost[post[j]]));
 #pragma unroll
     for(int j = 0; j < PRE_VEC; j++) {
         const unsigned int col = tile * PRE_TILE + j * PRE_BLOCK + threadIdx.x;
         if(col < len) {
-            const unsigned long long s = rowStart + col;
-            const unsigned int p = static_cast<const IndT*>(g.ind)[s];
-            const float w = gb[s];
-            redAdd(out + p, w);
-            const float dts = B200_FSUB(t, B200_FADD(g.wu_params[7], stPost[p]));
-            if(dts > 0.0f) {
-                const float timing = expf(B200_FDIV(-dts, g.wu_params[1]));
-                const float nw = B200_FSUB(w, B200_FMUL(g.wu_params[3], timing));
-                gb[s] = fmaxf(g.wu_params[4], fminf(g.wu_params[5], nw));
+            redAdd(out + post[j], w[j]);
+            if(dts[j] > 0.0f) {
+                const float timing = expf(B200_FDIV(-dts[j], g.wu_params[1]));
+                const float nw = B200_FSUB(w[j], B200_FMUL(g.wu_params[3], timing));
+                gb[rowStart + col] = fmaxf(g.wu_params[4], fminf(g.wu_params[5], nw));
             }
         }
     }
@@ -180,8 +188,9 @@ presynapticSparseKernel(const SynapseLaunch L)
     const b200_synapse_group &g = L.groups[gi];
     const unsigned int tile = blockIdx.x - __ldg(&L.block_start[gi]);
     const unsigned int b = blockIdx.z;
+    chainWait();
     if(L.tiled_served && L.tiled_served[gi] && L.state->heavy) return;
-    const unsigned int k = L.state->phase;
+    const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned int slots = g.src_delay_slots;
     const unsigned int rslot = ringSlot(k + slots - g.axonal_delay, slots);
     const unsigned int count = g.src_spk_cnt[b * slots + rslot];
@@ -192,7 +201,7 @@ presynapticSparseKernel(const SynapseLaunch L)
     float *target = D ? g.den_delay + (unsigned long long)b * D * g.num_trg
                       : g.out_post + (unsigned long long)b * g.num_trg;
     const bool learn = (g.wu_model == B200_WU_STDP);
-    const float t = B200_FMUL((float)L.state->timestep, L.dt);
+    const float t = B200_FMUL((float)(L.state->timestep + L.ahead), L.dt);
 
     for(unsigned int s = blockIdx.y; s < count; s += gridDim.y) {
         const unsigned int pre = spk[s];
@@ -229,7 +238,8 @@ presynapticPostSpanKernel(const SynapseLaunch L)
     const b200_synapse_group &g = L.groups[gi];
     const unsigned int post = (blockIdx.x - __ldg(&L.block_start[gi])) * PRE_BLOCK + threadIdx.x;
     const unsigned int b = blockIdx.z;
-    const unsigned int k = L.state->phase;
+    chainWait();
+    const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned int slots = g.src_delay_slots;
     const unsigned int rslot = ringSlot(k + slots - g.axonal_delay, slots);
     const unsigned int count = g.src_spk_cnt[b * slots + rslot];
@@ -253,7 +263,7 @@ presynapticPostSpanKernel(const SynapseLaunch L)
     }
     else if(g.wu_model == B200_WU_STDP) {
         if(!valid) return;
-        const float t = B200_FMUL((float)L.state->timestep, L.dt);
+        const float t = B200_FMUL((float)(L.state->timestep + L.ahead), L.dt);
         const unsigned int tslots = g.trg_delay_slots;
         const float stPost = g.trg_spike_times[((unsigned long long)b * tslots +
                                                 ringSlot(k + tslots - g.back_prop_delay, tslots)) * numTrg + post];
@@ -304,8 +314,9 @@ presynapticProceduralKernel(const SynapseLaunch L)
 {
     const b200_synapse_group &g = L.groups[blockIdx.y];
     const unsigned int b = blockIdx.z;
+    chainWait();
     const unsigned int lane = threadIdx.x & 31u;
-    const unsigned int k = L.state->phase;
+    const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned int slots = g.src_delay_slots;
     const unsigned int rslot = ringSlot(k + slots - g.axonal_delay, slots);
     const unsigned int count = g.src_spk_cnt[b * slots + rslot];

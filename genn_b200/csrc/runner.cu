@@ -28,6 +28,8 @@
 #include "urgent.cuh"
 #include "stream_step.cuh"
 #include "tiled.cuh"
+#include "dense_batch.cuh"
+#include "sparse_batch.cuh"
 #include "resident.h"
 #include "memory.h"
 #include "record.cuh"
@@ -143,7 +145,14 @@ struct b200_runner
     bool dirty = true;
 
     DeviceTable<b200_neuron_group> neuronTable;
-    DeviceTable<b200_synapse_group> sparseTable, postSpanTable, learnTable, proceduralTable;
+    DeviceTable<b200_synapse_group> sparseTable, postSpanTable, learnTable, proceduralTable, denseTable, scatterTable;
+    unsigned int ahead = 0, advance = 1;    // place of the step being enqueued in its block of steps (see chainPhase)
+    ScatterTarget *scatterTargets = nullptr;
+    ScatterPart *scatterParts = nullptr;    // sparseBatchKernel: what every CTA does
+    unsigned int scatterGrid = 0;
+    size_t scatterSmem = 0;
+    uint4 *denseParts = nullptr;            // denseBatchKernel: what every CTA does
+    size_t denseSmem = 0;
 
     // persistent fused-step path (batch 1, SPARSE non-learning groups only)
     bool fusedEligible = false;
@@ -293,6 +302,7 @@ struct b200_runner
 
     // target-resident kernel (resident.h): private copy of the SPARSE groups cut by CTA, message buffers
     bool useResident = true;
+    bool tiledChosen = false;               // the caller set what arms the tiled kernels: they serve whatever they can
     bool scheduleChosen = false;            // the caller picked a schedule of the other persistent kernels
     bool residentStale = true, residentReady = false;
     std::string residentWhyNot;
@@ -528,6 +538,105 @@ int buildFusedTables(b200_runner *r)
     return B200_OK;
 }
 
+// What the CTAs of denseBatchKernel do: (columns, sources) parts of every group, about as many as the chip holds at once so
+// that no last wave is nearly empty.  A part has at least 64 sources (below that its sums cost more than its rows) and at
+// most DENSE_WINDOW.
+int buildDense(b200_runner *r, const std::vector<b200_synapse_group> &dense)
+{
+    poolFree(r->denseParts, r->stream);
+    r->denseParts = nullptr;
+    r->denseTable.release(r->stream);
+    if(dense.empty()) return B200_OK;
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+    const unsigned int copies = std::min(r->batch, DENSE_COPIES), words = (r->batch + DENSE_COPIES - 1u) / DENSE_COPIES;
+    const unsigned int perSm = std::min<unsigned int>(6u, (unsigned int)(220u * 1024u / (denseSmemBytes(copies, 1024u) + 1024u)));
+    unsigned long long strips = 0;
+    for(const auto &g : dense) strips += (g.num_trg + DENSE_COLS - 1u) / DENSE_COLS;
+    const unsigned int wanted = std::max(1u, (unsigned int)((unsigned long long)sms * perSm / std::max(1ull, strips * words)));
+    std::vector<uint4> parts;
+    unsigned int window = 0;
+    for(unsigned int gi = 0; gi < dense.size(); gi++) {
+        const auto &g = dense[gi];
+        const unsigned int chunks = std::max(std::min(wanted, std::max(1u, g.num_src / 64u)), (g.num_src + DENSE_WINDOW - 1u) / DENSE_WINDOW);
+        const unsigned int per = chunks ? (g.num_src + chunks - 1u) / chunks : 0u;
+        for(unsigned int first = 0; first < g.num_src; first += per) {
+            const unsigned int n = std::min(per, g.num_src - first);
+            window = std::max(window, n);
+            for(unsigned int col = 0; col < g.num_trg; col += DENSE_COLS) parts.push_back(make_uint4(gi, col, first, n));
+        }
+    }
+    if(parts.empty()) return B200_OK;
+    r->denseSmem = denseSmemBytes(copies, window);
+    CUDA_TRY(cudaFuncSetAttribute(denseBatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->denseSmem));
+    CUDA_TRY(poolAlloc(&r->denseParts, sizeof(uint4) * parts.size(), r->stream));
+    CUDA_TRY(cudaMemcpyAsync(r->denseParts, parts.data(), sizeof(uint4) * parts.size(), cudaMemcpyHostToDevice, r->stream));
+    CUDA_TRY(r->denseTable.upload(dense, {0u, (unsigned int)parts.size()}, r->stream));
+    return B200_OK;
+}
+
+// Whether sparseBatchKernel delivers a SPARSE group: a batched network (one copy has the target-resident kernel, and the
+// tiled kernels where that does not apply), no learning, a target buffer that fits a CTA's shared memory.
+bool scatterServes(const b200_runner *r, const b200_synapse_group &g)
+{
+    if(r->batch < 2 || r->sharded() || r->tiledChosen || g.wu_model == B200_WU_STDP) return false;
+    const unsigned long long cells = (unsigned long long)std::max(1u, g.max_den_delay) * g.num_trg;
+    if(cells > SCATTER_MOST_CELLS) return false;
+    unsigned int groups = 0;
+    for(const auto &o : r->synapseGroups) {
+        if((o.max_den_delay ? o.den_delay : o.out_post) == (g.max_den_delay ? g.den_delay : g.out_post)) groups++;
+    }
+    return groups <= SCATTER_MOST_SOURCES;
+}
+
+// The CTAs of sparseBatchKernel: one per SM as far as there are not more (buffer, copy) pairs; a buffer gets as many as its
+// part of all synapses.
+int buildScatter(b200_runner *r, std::vector<b200_synapse_group> &scatter)
+{
+    poolFree(r->scatterTargets, r->stream);
+    poolFree(r->scatterParts, r->stream);
+    r->scatterTargets = nullptr;
+    r->scatterParts = nullptr;
+    r->scatterTable.release(r->stream);
+    if(scatter.empty()) return B200_OK;
+    auto buffer = [](const b200_synapse_group &g) { return g.max_den_delay ? g.den_delay : g.out_post; };
+    std::stable_sort(scatter.begin(), scatter.end(), [&](const b200_synapse_group &a, const b200_synapse_group &b) { return buffer(a) < buffer(b); });
+    std::vector<ScatterTarget> targets;
+    std::vector<double> weight;
+    double all = 0.0;
+    unsigned int cells = 0;
+    for(unsigned int i = 0; i < scatter.size(); i++) {
+        const auto &g = scatter[i];
+        if(targets.empty() || targets.back().cells != buffer(g)) {
+            targets.push_back(ScatterTarget{buffer(g), std::max(1u, g.max_den_delay) * g.num_trg, i, 0u});
+            weight.push_back(0.0);
+        }
+        targets.back().num_groups++;
+        const double synapses = (double)g.num_src * g.row_stride + 1.0;
+        weight.back() += synapses;
+        all += synapses;
+        cells = std::max(cells, targets.back().num_cells);
+    }
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+    std::vector<ScatterPart> parts;
+    for(unsigned int t = 0; t < targets.size(); t++) {
+        const unsigned int shares = std::max(1u, (unsigned int)((double)sms * weight[t] / all / r->batch));
+        for(unsigned int b = 0; b < r->batch; b++) {
+            for(unsigned int s = 0; s < shares; s++) parts.push_back(ScatterPart{t, b, s, shares});
+        }
+    }
+    r->scatterGrid = (unsigned int)parts.size();
+    r->scatterSmem = (size_t)((cells + 3u) & ~3u) * sizeof(float);
+    CUDA_TRY(cudaFuncSetAttribute(sparseBatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->scatterSmem));
+    CUDA_TRY(poolAlloc(&r->scatterTargets, sizeof(ScatterTarget) * targets.size(), r->stream));
+    CUDA_TRY(cudaMemcpyAsync(r->scatterTargets, targets.data(), sizeof(ScatterTarget) * targets.size(), cudaMemcpyHostToDevice, r->stream));
+    CUDA_TRY(poolAlloc(&r->scatterParts, sizeof(ScatterPart) * parts.size(), r->stream));
+    CUDA_TRY(cudaMemcpyAsync(r->scatterParts, parts.data(), sizeof(ScatterPart) * parts.size(), cudaMemcpyHostToDevice, r->stream));
+    CUDA_TRY(r->scatterTable.upload(scatter, {0u, r->scatterGrid}, r->stream));
+    return B200_OK;
+}
+
 int prepare(b200_runner *r)
 {
     if(!r->dirty) return B200_OK;
@@ -540,13 +649,19 @@ int prepare(b200_runner *r)
         }
         CUDA_TRY(r->neuronTable.upload(r->neuronGroups, starts, r->stream));
     }
-    std::vector<b200_synapse_group> sparse, postSpan, learn, procedural;
+    std::vector<b200_synapse_group> sparse, postSpan, learn, procedural, dense, scatter;
     std::vector<unsigned int> sparseStarts{0}, postSpanStarts{0}, learnStarts{0}, proceduralStarts{0};
     for(const auto &g : r->synapseGroups) {
-        if(g.connectivity == B200_CONN_SPARSE) {
+        if(g.connectivity == B200_CONN_SPARSE && scatterServes(r, g)) {
+            scatter.push_back(g);
+        }
+        else if(g.connectivity == B200_CONN_SPARSE) {
             sparse.push_back(g);
             // +3: tiles are aligned to the array, not to the row
             sparseStarts.push_back(sparseStarts.back() + (g.row_stride + 3 + PRE_TILE - 1) / PRE_TILE);
+        }
+        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src <= DENSE_MOST_SOURCES) {
+            dense.push_back(g);
         }
         else if(g.connectivity == B200_CONN_BITMASK || g.connectivity == B200_CONN_DENSE) {
             postSpan.push_back(g);
@@ -569,11 +684,16 @@ int prepare(b200_runner *r)
     }
     CUDA_TRY(r->sparseTable.upload(sparse, sparseStarts, r->stream));
     CUDA_TRY(r->postSpanTable.upload(postSpan, postSpanStarts, r->stream));
+    {
+        int e = buildDense(r, dense);
+        if(e == B200_OK) e = buildScatter(r, scatter);
+        if(e) return e;
+    }
     CUDA_TRY(r->learnTable.upload(learn, learnStarts, r->stream));
     CUDA_TRY(r->proceduralTable.upload(procedural, proceduralStarts, r->stream));
 
     // ---- tables of the persistent fused-step kernel --------------------------------
-    r->fusedEligible = (r->batch == 1 && postSpan.empty() && learn.empty() && procedural.empty() &&
+    r->fusedEligible = (r->batch == 1 && postSpan.empty() && dense.empty() && scatter.empty() && learn.empty() && procedural.empty() &&
                         !r->neuronGroups.empty());
     r->fusedGroups = sparse;
     r->lagStale = true;
@@ -937,6 +1057,7 @@ int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long 
     L.neuron.num_recording_timesteps = numRec;
     L.neuron.state = r->state;
     L.neuron.count_events = r->countEvents ? 1u : 0u;
+    L.neuron.ahead = L.neuron.advance = 0u;
     L.slot_start = r->fusedSlotStart;
     L.sgroups = r->sparseTable.d;
     L.sources = r->fusedSources;
@@ -988,6 +1109,7 @@ SynapseLaunch synapseLaunch(const b200_runner *r, const DeviceTable<b200_synapse
     L.seed = r->seed;
     L.state = r->state;
     L.count_events = r->countEvents ? 1u : 0u;
+    L.ahead = r->ahead;
     L.tiled_served = nullptr;
     return L;
 }
@@ -1031,7 +1153,7 @@ int buildTiled(b200_runner *r)
     if(r->sharded()) { r->tiledWhyNot = "sharded models run on the persistent kernel"; return B200_OK; }
     // the SPARSE groups in the order of sparseTable; the non-learning ones are served
     std::vector<b200_synapse_group> sparse;
-    for(const auto &g : r->synapseGroups) if(g.connectivity == B200_CONN_SPARSE) sparse.push_back(g);
+    for(const auto &g : r->synapseGroups) if(g.connectivity == B200_CONN_SPARSE && !scatterServes(r, g)) sparse.push_back(g);
     std::vector<unsigned char> served(sparse.size(), 0);
     struct Target { float *ptr; unsigned int n, depth, stride, tiles, firstTile, firstTable, rows, firstSource; std::vector<size_t> groups; };
     std::vector<Target> targets;
@@ -1220,6 +1342,7 @@ int buildTiled(b200_runner *r)
 TiledLaunch tiledLaunch(const b200_runner *r)
 {
     TiledLaunch L;
+    L.ahead = r->ahead;
     L.tiles = r->tiledTiles; L.sources = r->tiledSources; L.run_start = r->tiledRunStart; L.keys = r->tiledKeys;
     L.weights = r->tiledWeights; L.pairs = r->tiledPairs; L.pair_batches = r->tiledPairBatches;
     L.pair_prefix = r->tiledPairPrefix; L.cta_start = r->tiledCtaStart; L.num_pairs = r->tiledNumPairs;
@@ -1582,6 +1705,7 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
     L.neuron.num_recording_timesteps = numRec;
     L.neuron.state = r->state;
     L.neuron.count_events = r->countEvents ? 1u : 0u;
+    L.neuron.ahead = L.neuron.advance = 0u;
     L.count_events = r->countEvents ? 1u : 0u;
     L.num_steps = (unsigned int)numSteps;
     // a message word is known by the last 20 bits of its step: before they repeat, no old word may be left
@@ -1625,6 +1749,33 @@ bool tiledActive(const b200_runner *r, bool force = false)
     return r->tiledReady && (force || r->tiledArmed || r->tiledMinEvents == 0);
 }
 
+// A kernel of the one-launch-per-kernel path: its blocks may be placed while the kernel before it runs (chainWait).
+template<typename P, typename A>
+cudaError_t chain(const b200_runner *r, void (*kernel)(P), dim3 grid, unsigned int block, size_t smem, const A &params)
+{
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3(block);
+    config.dynamicSmemBytes = smem;
+    config.stream = r->stream;
+    config.attrs = &early;
+    config.numAttrs = r->timing ? 0u : 1u;      // (timed kernels do not overlap)
+    return cudaLaunchKernelEx(&config, kernel, params);
+}
+
+// Spikes of a copy that blocks take side by side: with a learning rule an event is a chain of dependent loads, so every
+// block the chip holds at once (16 of 128 threads an SM) should have a spike; without one the rows are long and 16 will do.
+unsigned int spikeLanesFor(const b200_runner *r, unsigned int blocks)
+{
+    if(r->learnTable.num == 0) return r->spikeLanes;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
+    return std::max(r->spikeLanes, std::min(256u, (unsigned int)sms * 16u / std::max(1u, blocks * r->batch)));
+}
+
 int enqueueSynapses(b200_runner *r, bool capturing, bool force = false)
 {
     if(r->sparseTable.num) {
@@ -1633,19 +1784,31 @@ int enqueueSynapses(b200_runner *r, bool capturing, bool force = false)
         if(tiledActive(r, force)) {
             // the step's estimated events decide which of the two kernels delivers the served groups
             const TiledLaunch T = tiledLaunch(r);
-            tiledDecideKernel<<<1, TILED_BLOCK, 0, r->stream>>>(T);
-            tiledKernelFor(r->tiledPostBits == 10u, r->tiledWeights != nullptr)<<<r->tiledGrid, TILED_BLOCK, r->tiledSmemBytes, r->stream>>>(T);
+            CUDA_TRY(chain(r, tiledDecideKernel, 1, TILED_BLOCK, 0, T));
+            CUDA_TRY(chain(r, tiledKernelFor(r->tiledPostBits == 10u, r->tiledWeights != nullptr), r->tiledGrid, TILED_BLOCK, r->tiledSmemBytes, T));
             r->launches += 2;
             S.tiled_served = r->tiledServed;
         }
-        const dim3 grid(r->sparseTable.blocks, r->spikeLanes, r->batch);
-        presynapticSparseKernel<<<grid, PRE_BLOCK, 0, r->stream>>>(S);
+        const dim3 grid(r->sparseTable.blocks, spikeLanesFor(r, r->sparseTable.blocks), r->batch);
+        CUDA_TRY(chain(r, presynapticSparseKernel, grid, PRE_BLOCK, 0, S));
         r->launches++;
     }
     if(r->postSpanTable.num) {
         ScopedTimer tm(r, "presynaptic_update", capturing);
         const dim3 grid(r->postSpanTable.blocks, 1, r->batch);
-        presynapticPostSpanKernel<<<grid, PRE_BLOCK, 0, r->stream>>>(synapseLaunch(r, r->postSpanTable));
+        CUDA_TRY(chain(r, presynapticPostSpanKernel, grid, PRE_BLOCK, 0, synapseLaunch(r, r->postSpanTable)));
+        r->launches++;
+    }
+    if(r->denseTable.num) {
+        ScopedTimer tm(r, "presynaptic_update", capturing);
+        const dim3 grid(r->denseTable.blocks, 1, (r->batch + DENSE_COPIES - 1u) / DENSE_COPIES);
+        CUDA_TRY(chain(r, denseBatchKernel, grid, DENSE_BLOCK, r->denseSmem, DenseLaunch{synapseLaunch(r, r->denseTable), r->denseParts}));
+        r->launches++;
+    }
+    if(r->scatterTable.num) {
+        ScopedTimer tm(r, "presynaptic_update", capturing);
+        CUDA_TRY(chain(r, sparseBatchKernel, r->scatterGrid, SCATTER_BLOCK, r->scatterSmem,
+                       ScatterLaunch{synapseLaunch(r, r->scatterTable), r->scatterTargets, r->scatterParts}));
         r->launches++;
     }
     if(r->proceduralTable.num) {
@@ -1654,13 +1817,13 @@ int enqueueSynapses(b200_runner *r, bool capturing, bool force = false)
         int sms = 0;
         CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
         const dim3 grid((unsigned int)sms * 8u, r->proceduralTable.num, r->batch);
-        presynapticProceduralKernel<<<grid, PROC_BLOCK, 0, r->stream>>>(synapseLaunch(r, r->proceduralTable));
+        CUDA_TRY(chain(r, presynapticProceduralKernel, grid, PROC_BLOCK, 0, synapseLaunch(r, r->proceduralTable)));
         r->launches++;
     }
     if(r->learnTable.num) {
         ScopedTimer tm(r, "postsynaptic_update", capturing);
-        const dim3 grid(r->learnTable.blocks, r->spikeLanes, r->batch);
-        postsynapticUpdateKernel<<<grid, POST_BLOCK, 0, r->stream>>>(synapseLaunch(r, r->learnTable));
+        const dim3 grid(r->learnTable.blocks, spikeLanesFor(r, r->learnTable.blocks), r->batch);
+        CUDA_TRY(chain(r, postsynapticUpdateKernel, grid, POST_BLOCK, 0, synapseLaunch(r, r->learnTable)));
         r->launches++;
     }
     CUDA_TRY(cudaPeekAtLastError());
@@ -1681,9 +1844,15 @@ int enqueueNeurons(b200_runner *r, unsigned long long numRec, bool capturing)
     L.num_recording_timesteps = numRec;
     L.state = r->state;
     L.count_events = r->countEvents ? 1u : 0u;
-    const dim3 grid(r->neuronTable.blocks, r->batch, 1);
+    L.ahead = r->ahead;
+    L.advance = r->advance;
+    // (as many blocks as are on the chip at once: thousands of blocks for a few loads each spend their time starting, and
+    // counting themselves one after another in the ticket)
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+    const dim3 grid((unsigned int)std::min<unsigned long long>((unsigned long long)r->neuronTable.blocks * r->batch, (unsigned long long)sms * NEURON_BLOCKS_PER_SM));
     int e = withNeuronShape(r, [&](auto P, auto C) -> int {
-        neuronUpdateKernel<decltype(P)::value, decltype(C)::value><<<grid, NEURON_BLOCK, 0, r->stream>>>(L);
+        CUDA_TRY(chain(r, neuronUpdateKernel<decltype(P)::value, decltype(C)::value>, grid, NEURON_BLOCK, 0, L));
         return B200_OK;
     });
     if(e) return e;
@@ -1730,7 +1899,7 @@ int enqueueStep(b200_runner *r, unsigned long long numRec, bool capturing)
 
 unsigned int kernelsPerStep(const b200_runner *r)
 {
-    return 1u + (r->sparseTable.num ? (tiledActive(r) ? 3u : 1u) : 0u) + (r->postSpanTable.num ? 1u : 0u) + (r->learnTable.num ? 1u : 0u) +
+    return 1u + (r->sparseTable.num ? (tiledActive(r) ? 3u : 1u) : 0u) + (r->postSpanTable.num ? 1u : 0u) + (r->denseTable.num ? 1u : 0u) + (r->scatterTable.num ? 1u : 0u) + (r->learnTable.num ? 1u : 0u) +
            (r->proceduralTable.num ? 1u : 0u);
 }
 
@@ -1741,7 +1910,13 @@ int buildGraph(b200_runner *r, unsigned int len, unsigned long long numRec)
     const unsigned long long before = r->launches;
     CUDA_TRY(cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal));
     int e = B200_OK;
-    for(unsigned int i = 0; i < len && e == B200_OK; i++) e = enqueueStep(r, numRec, true);
+    for(unsigned int i = 0; i < len && e == B200_OK; i++) {
+        r->ahead = i;
+        r->advance = (i + 1u == len) ? len : 0u;
+        e = enqueueStep(r, numRec, true);
+    }
+    r->ahead = 0;
+    r->advance = 1;
     cudaError_t ce = cudaStreamEndCapture(r->stream, &graph);
     r->launches = before;       // capture enqueues nothing
     if(e) {
@@ -1846,6 +2021,11 @@ int b200_runner_destroy(b200_runner *r)
     r->neuronTable.release(r->stream);
     r->sparseTable.release(r->stream);
     r->postSpanTable.release(r->stream);
+    r->denseTable.release(r->stream);
+    poolFree(r->denseParts, r->stream);
+    r->scatterTable.release(r->stream);
+    poolFree(r->scatterTargets, r->stream);
+    poolFree(r->scatterParts, r->stream);
     r->proceduralTable.release(r->stream);
     r->learnTable.release(r->stream);
     poolFree(r->fusedSlotStart, r->stream);
@@ -2301,7 +2481,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
         CUDA_TRY(cudaMemcpyAsync(dst, &v, sizeof(v), cudaMemcpyHostToDevice, r->stream));
     }
     else if(n == "use_tiled") { r->useTiled = (value != 0.0); r->tiledStale = true; }
-    else if(n == "tiled_min_events") r->tiledMinEvents = (float)value;
+    else if(n == "tiled_min_events") { r->tiledMinEvents = (float)value; r->tiledChosen = r->dirty = true; }
     else if(n == "tiled_ticket_events") { r->tiledTicketEvents = std::max(1.0f, (float)value); r->dropGraph(); }
     else if(n == "tiled_ticket_cost") { r->tiledTicketCost = std::max(0.0f, (float)value); r->dropGraph(); }
     else return fail(B200_ERR_INVALID, "unknown option %s", name);

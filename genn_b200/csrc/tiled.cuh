@@ -89,6 +89,7 @@ __host__ __device__ __forceinline__ unsigned int tiledTicketSpikes(float meanRun
 
 struct TiledLaunch
 {
+    unsigned int ahead;                 // steps of this block of steps that come before this one
     const TiledTile *tiles;
     const TiledSource *sources;
     const TiledPair *pairs;             // [num_pairs], tile-major
@@ -183,7 +184,8 @@ tiledDecideKernel(const TiledLaunch L)
     __shared__ double chunk[TILED_BLOCK];
     __shared__ float partial[32];
     __shared__ unsigned int verdict;
-    const unsigned int k = L.state->phase;
+    chainWait();
+    const unsigned int k = chainPhase(L.state, L.ahead);
     float est = 0.0f;
     for(unsigned int i = threadIdx.x; i < L.num_sources * L.batch; i += TILED_BLOCK) {
         const TiledSource &s = L.sources[i / L.batch];
@@ -267,8 +269,9 @@ tiledDeliverKernel(const TiledLaunch L)
     __shared__ unsigned int pieceCount[TILED_MAX_SOURCES], pieceRows[TILED_MAX_SOURCES], pieceSpikes[TILED_MAX_SOURCES];
     __shared__ float pieceWeight[TILED_MAX_SOURCES];
     __shared__ unsigned int numPieces, nextTicket, segmentEnd;
+    chainWait();
     if(!L.state->heavy) return;
-    const unsigned int k = L.state->phase;
+    const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned int lane = threadIdx.x & 31u;
     const unsigned int postMask = (1u << L.post_bits) - 1u;
     const KeyT *__restrict__ keys = static_cast<const KeyT*>(L.keys);
