@@ -3,13 +3,15 @@
 // The rows are what bounds it.  With 32 copies at 2.5 % a step reaches 55 % of the rows, 1.44 copies each; one pass over the
 // rows per copy (presynapticPostSpanKernel) moves 1.44 times the bytes, and its threads wait for one load after another.
 // Here a CTA owns DENSE_COLS columns and a range of source neurons.  It turns the copies' spike lists into one bit mask per
-// source neuron (bit b: copy b spiked), gathers the sources that have one into a list, and its warps walk the list,
-// DENSE_ROWS rows in flight each (12 warps x 8 x 512 bytes on an SM: what HBM's latency wants in flight).  A row's quad of
-// columns is added to the private sums [copy][column] that every warp keeps in shared memory, where a lane only meets its
-// own columns: plain loads and stores, no atomics.  The warps' sums are combined before one reduction per cell leaves the
-// CTA, 16 bytes wide where the row allows.
+// source neuron (bit b: copy b spiked) and gathers the sources that have one into a list.  The listed rows pass through a
+// ring of DENSE_STAGES stages of 32 rows in shared memory (two CTAs on an SM: 128 KB under way, several times what HBM's
+// latency wants); one warp sends for them, a row a lane, as bulk copies, and the others fall behind one another by as much
+// as the ring holds (with a barrier per stage every stage took as long as its busiest warp).  A warp owns copies: a ballot over the masks of
+// a stage's rows gives the rows its copy needs, which it sums in registers, so that sums cost neither shared memory nor
+// atomics until one 16-byte reduction per four columns at the end.  Instructions decide: sums in shared memory, the masks'
+// bits walked row by row, took 55 us at the size below, stages of half the columns brought in by all threads 42.
 //
-// 8192 x 8192, 32 copies, 25 Hz at 1 ms (149 MB of rows a step): 107 us with presynapticPostSpanKernel, 55 here.
+// 8192 x 8192, 32 copies, 25 Hz at 1 ms (149 MB of rows a step): 107 us with presynapticPostSpanKernel, 33 here.
 #pragma once
 
 #include "common.cuh"
@@ -17,12 +19,15 @@
 
 namespace b200
 {
-constexpr unsigned int DENSE_WARPS = 4;
-constexpr unsigned int DENSE_BLOCK = DENSE_WARPS * 32;
-constexpr unsigned int DENSE_COLS = 128;            // columns of a CTA: four a lane
+constexpr unsigned int DENSE_WARPS = 8;             // warps that add; one more brings the rows in
+constexpr unsigned int DENSE_BLOCK = DENSE_WARPS * 32 + 32;
+constexpr unsigned int DENSE_COLS = 256;            // columns of a CTA: twice four a lane
 constexpr unsigned int DENSE_COPIES = 32;           // copies of a CTA: one mask word
-constexpr unsigned int DENSE_ROWS = 8;              // rows a warp has in flight
-constexpr unsigned int DENSE_WINDOW = 2048;         // most source neurons of a CTA (masks and list: 12 KB)
+constexpr unsigned int DENSE_OWN = DENSE_COPIES / DENSE_WARPS;      // copies of a warp
+constexpr unsigned int DENSE_STAGES = 3;
+constexpr unsigned int DENSE_PER_SM = 2;            // CTAs on an SM: 96 KB of stages each
+constexpr unsigned int DENSE_WAITS = 1u << 18;      // polls for a stage before the step is given up
+constexpr unsigned int DENSE_WINDOW = 1024;         // most source neurons of a CTA (masks and list: 6 KB)
 // A CTA reads all spike lists to find its own sources: worth it while those are a small part of what it reads of the rows.
 constexpr unsigned int DENSE_MOST_SOURCES = 65536;
 
@@ -32,124 +37,88 @@ struct DenseLaunch
     const uint4 *parts;                 // per CTA: group, first column, first source, number of sources
 };
 
-inline size_t denseSmemBytes(unsigned int copies, unsigned int window)
-{
-    return (size_t)DENSE_WARPS * copies * DENSE_COLS * sizeof(float) + window * (sizeof(unsigned int) + sizeof(uint16_t)) + 16u;
-}
+constexpr size_t DENSE_SMEM = DENSE_STAGES * 32 * DENSE_COLS * sizeof(float) + DENSE_WINDOW * (sizeof(unsigned int) + sizeof(uint16_t));
 
-// Four columns of a row: a 16-byte load where rows keep that alignment, else four coalesced words.  (Lanes beyond the row's
-// end read its last columns again; what they add is never flushed.)
-template<bool VEC>
-__device__ __forceinline__ float4 denseLoad(const float *row, unsigned int lane, unsigned int cols)
-{
-    if(VEC) return __ldg(reinterpret_cast<const float4*>(row + min(lane * 4u, cols - 4u)));
-    return make_float4(__ldg(row + min(lane, cols - 1u)), __ldg(row + min(lane + 32u, cols - 1u)),
-                       __ldg(row + min(lane + 64u, cols - 1u)), __ldg(row + min(lane + 96u, cols - 1u)));
-}
+__device__ __forceinline__ unsigned int denseShare(const void *p) { return (unsigned int)__cvta_generic_to_shared(p); }
 
-// A lane's four sums of one copy (its columns as in denseLoad).
-template<bool VEC>
-__device__ __forceinline__ void denseAdd(float *sums, unsigned int lane, const float4 &w)
+// Waits (with a limit) for the bytes of a stage.
+__device__ __forceinline__ bool denseArrived(unsigned long long *bar, unsigned int parity)
 {
-    if(VEC) {
-        float4 *const at = reinterpret_cast<float4*>(sums) + lane;
-        float4 a = *at;
-        a.x = B200_FADD(a.x, w.x); a.y = B200_FADD(a.y, w.y); a.z = B200_FADD(a.z, w.z); a.w = B200_FADD(a.w, w.w);
-        *at = a;
+    for(unsigned int i = 0; i < DENSE_WAITS; i++) {
+        unsigned int done;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(done) : "r"(denseShare(bar)), "r"(parity) : "memory");
+        if(done) return true;
     }
-    else {
-        sums[lane] = B200_FADD(sums[lane], w.x);
-        sums[lane + 32u] = B200_FADD(sums[lane + 32u], w.y);
-        sums[lane + 64u] = B200_FADD(sums[lane + 64u], w.z);
-        sums[lane + 96u] = B200_FADD(sums[lane + 96u], w.w);
-    }
+    return false;
 }
 
-template<bool VEC>
-__device__ __forceinline__ void denseRows(const b200_synapse_group &g, float *sums, const unsigned int *mask, const uint16_t *list,
-                                          unsigned int listed, unsigned int firstColumn, unsigned int firstSource, unsigned int cols,
-                                          unsigned int warp, unsigned int lane)
+__device__ __forceinline__ void denseSum(float4 &sum, const float4 &v)
 {
-    const bool constant = (g.wu_model == B200_WU_STATIC_PULSE_CONSTANT_WEIGHT);
-    const float c = g.wu_params[0];
-    const float *const base = constant ? nullptr : g.g + (unsigned long long)firstSource * g.num_trg + firstColumn;
-    const unsigned int rowStride = g.num_trg;
-    // the next rows are on their way while these are added; behind the list's end its last row is read again and not added
-    auto fetch = [&](float4 (&w)[DENSE_ROWS], unsigned int (&m)[DENSE_ROWS], unsigned int first) {
-        unsigned int s[DENSE_ROWS];
-        #pragma unroll
-        for(unsigned int j = 0; j < DENSE_ROWS; j++) s[j] = list[min(first + j, listed - 1u)];
-        #pragma unroll
-        for(unsigned int j = 0; j < DENSE_ROWS; j++) {
-            w[j] = constant ? make_float4(c, c, c, c) : denseLoad<VEC>(base + (unsigned long long)s[j] * rowStride, lane, cols);
-        }
-        #pragma unroll
-        for(unsigned int j = 0; j < DENSE_ROWS; j++) m[j] = (first + j < listed) ? mask[s[j]] : 0u;
-    };
-    auto add = [&](const float4 (&w)[DENSE_ROWS], const unsigned int (&m)[DENSE_ROWS]) {
-        #pragma unroll
-        for(unsigned int j = 0; j < DENSE_ROWS; j++) {
-            for(unsigned int left = m[j]; left; left &= left - 1u) denseAdd<VEC>(sums + (unsigned int)(__ffs(left) - 1) * DENSE_COLS, lane, w[j]);
-        }
-    };
-    constexpr unsigned int STRIDE = DENSE_WARPS * DENSE_ROWS;
-    float4 wa[DENSE_ROWS], wb[DENSE_ROWS];
-    unsigned int ma[DENSE_ROWS], mb[DENSE_ROWS];
-    unsigned int first = warp * DENSE_ROWS;
-    if(first >= listed) return;
-    fetch(wa, ma, first);
-    while(true) {
-        if(first + STRIDE < listed) fetch(wb, mb, first + STRIDE);
-        add(wa, ma);
-        first += STRIDE;
-        if(first >= listed) break;
-        if(first + STRIDE < listed) fetch(wa, ma, first + STRIDE);
-        add(wb, mb);
-        first += STRIDE;
-        if(first >= listed) break;
-    }
+    sum.x = B200_FADD(sum.x, v.x); sum.y = B200_FADD(sum.y, v.y);
+    sum.z = B200_FADD(sum.z, v.z); sum.w = B200_FADD(sum.w, v.w);
 }
 
-static __global__ void __launch_bounds__(DENSE_BLOCK)
+static __global__ void __launch_bounds__(DENSE_BLOCK, DENSE_PER_SM)
 denseBatchKernel(const DenseLaunch L)
 {
     extern __shared__ __align__(16) unsigned char denseShared[];
     __shared__ unsigned int listed;
-    __shared__ unsigned int counts[DENSE_COPIES];
+    __shared__ __align__(8) unsigned long long arrived[DENSE_STAGES], released[DENSE_STAGES];
     const uint4 part = __ldg(&L.parts[blockIdx.x]);
     const b200_synapse_group &g = L.S.groups[part.x];
     const unsigned int firstCopy = blockIdx.z * DENSE_COPIES, copies = min(DENSE_COPIES, L.S.batch - firstCopy);
+    const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const unsigned int rowStride = g.num_trg, cols = min(DENSE_COLS, rowStride - part.y);
+    const bool vec = (rowStride & 3u) == 0u && ((reinterpret_cast<size_t>(g.g) | reinterpret_cast<size_t>(g.out_post)) & 15u) == 0u;    // rows keep a 16-byte alignment
+    const bool constant = (g.wu_model == B200_WU_STATIC_PULSE_CONSTANT_WEIGHT);
+    float *const stages = reinterpret_cast<float*>(denseShared);
+    unsigned int *const mask = reinterpret_cast<unsigned int*>(stages + DENSE_STAGES * 32u * DENSE_COLS);
+    uint16_t *const list = reinterpret_cast<uint16_t*>(mask + DENSE_WINDOW);
+    if(threadIdx.x == 0u) {
+        listed = 0u;
+        // a stage is complete when its bytes are: the sending warp's first lane announces them, or its lanes' copies arrive
+        for(unsigned int i = 0; i < DENSE_STAGES; i++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(denseShare(&arrived[i])), "r"(vec ? 1u : 32u) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(denseShare(&released[i])), "r"(DENSE_WARPS) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    for(unsigned int i = threadIdx.x; i < part.w; i += DENSE_BLOCK) mask[i] = 0u;
+    __syncthreads();
     chainWait();
     const unsigned int k = chainPhase(L.S.state, L.S.ahead);
     const unsigned int slots = g.src_delay_slots, slot = ringSlot(k + slots - g.axonal_delay, slots);
-    const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const unsigned int cols = min(DENSE_COLS, g.num_trg - part.y);
-    float *const sums = reinterpret_cast<float*>(denseShared);
-    unsigned int *const mask = reinterpret_cast<unsigned int*>(sums + DENSE_WARPS * copies * DENSE_COLS);
-    uint16_t *const list = reinterpret_cast<uint16_t*>(mask + part.w);
 
-    if(threadIdx.x < copies) counts[threadIdx.x] = min(g.src_spk_cnt[(firstCopy + threadIdx.x) * slots + slot], g.num_src);
-    if(threadIdx.x == 0u) listed = 0u;
-    for(unsigned int i = threadIdx.x; i < part.w; i += DENSE_BLOCK) mask[i] = 0u;
-    for(unsigned int i = threadIdx.x; i < DENSE_WARPS * copies * DENSE_COLS / 4u; i += DENSE_BLOCK) {
-        reinterpret_cast<float4*>(sums)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    __syncthreads();
-    // ---- spike lists -> masks of this CTA's sources: a warp takes every DENSE_WARPS-th copy
-    for(unsigned int b = warp; b < copies; b += DENSE_WARPS) {
-        const unsigned int *const spk = g.src_spk + ((unsigned long long)(firstCopy + b) * slots + slot) * g.num_src;
-        const unsigned int n = counts[b];
-        for(unsigned int at = lane; at < n; at += 32u * 8u) {
-            unsigned int id[8];
+    // ---- spike lists -> masks of this CTA's sources: the lists of a warp's copies side by side
+    if(warp < DENSE_WARPS) {
+        const unsigned int *spk[DENSE_OWN];
+        unsigned int n[DENSE_OWN], most = 0u;
+        #pragma unroll
+        for(unsigned int o = 0; o < DENSE_OWN; o++) {
+            const unsigned int b = warp + o * DENSE_WARPS;
+            spk[o] = g.src_spk + ((unsigned long long)(firstCopy + b) * slots + slot) * g.num_src;
+            n[o] = b < copies ? min(g.src_spk_cnt[(firstCopy + b) * slots + slot], g.num_src) : 0u;
+        }
+        #pragma unroll
+        for(unsigned int o = 0; o < DENSE_OWN; o++) most = max(most, n[o]);
+        for(unsigned int at = lane; at < most; at += 32u * 4u) {
+            unsigned int id[DENSE_OWN][4];
             #pragma unroll
-            for(unsigned int j = 0; j < 8u; j++) id[j] = (at + 32u * j < n) ? spk[at + 32u * j] : 0xFFFFFFFFu;
+            for(unsigned int o = 0; o < DENSE_OWN; o++) {
+                #pragma unroll
+                for(unsigned int j = 0; j < 4u; j++) id[o][j] = (at + 32u * j < n[o]) ? spk[o][at + 32u * j] : 0xFFFFFFFFu;
+            }
             #pragma unroll
-            for(unsigned int j = 0; j < 8u; j++) {
-                if(id[j] - part.z < part.w) atomicOr(&mask[id[j] - part.z], 1u << b);
+            for(unsigned int o = 0; o < DENSE_OWN; o++) {
+                #pragma unroll
+                for(unsigned int j = 0; j < 4u; j++) {
+                    if(id[o][j] - part.z < part.w) atomicOr(&mask[id[o][j] - part.z], 1u << (warp + o * DENSE_WARPS));
+                }
             }
         }
-        if(L.S.count_events && lane == 0u && part.y == 0u && part.z == 0u) {
-            atomicAdd(&L.S.state->synaptic_events, (unsigned long long)n * g.num_trg);
+        if(L.S.count_events && part.y == 0u && part.z == 0u && lane == 0u) {
+            atomicAdd(&L.S.state->synaptic_events, (unsigned long long)(n[0] + n[1] + n[2] + n[3]) * g.num_trg);
         }
     }
     __syncthreads();
@@ -164,31 +133,118 @@ denseBatchKernel(const DenseLaunch L)
     __syncthreads();
     const unsigned int rows = listed;
     if(rows == 0u) return;
-    const bool vec = (g.num_trg & 3u) == 0u;
-    float *const own = sums + warp * copies * DENSE_COLS;
-    if(vec) denseRows<true>(g, own, mask, list, rows, part.y, part.z, cols, warp, lane);
-    else denseRows<false>(g, own, mask, list, rows, part.y, part.z, cols, warp, lane);
-    __syncthreads();
-    // ---- the warps' sums together, out to the targets' input
-    const unsigned int quads = copies * DENSE_COLS / 4u;
-    for(unsigned int q = threadIdx.x; q < quads; q += DENSE_BLOCK) {
-        float4 a = reinterpret_cast<const float4*>(sums)[q];
+
+    // ---- rows through the ring
+    const float *const base = constant ? nullptr : g.g + (unsigned long long)part.z * rowStride + part.y;
+    const unsigned int numStages = constant ? 0u : (rows + 31u) / 32u;
+    if(warp == DENSE_WARPS) {
+        bool room = true;
+        for(unsigned int stage = 0; stage < numStages && room; stage++) {
+            const unsigned int ring = stage % DENSE_STAGES;
+            if(stage >= DENSE_STAGES) room = denseArrived(&released[ring], (stage / DENSE_STAGES - 1u) & 1u);
+            if(!room) {
+                atomicOr(&L.S.state->error, ERR_BARRIER_TIMEOUT);
+                break;
+            }
+            float *const to = stages + ring * 32u * DENSE_COLS;
+            const unsigned int n = min(32u, rows - stage * 32u), bar = denseShare(&arrived[ring]);
+            if(vec) {
+                if(lane == 0u) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(n * cols * 4u) : "memory");
+                __syncwarp();
+                if(lane < n) {
+                    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 :: "r"(denseShare(to + lane * DENSE_COLS)), "l"(__cvta_generic_to_global(base + (unsigned long long)list[stage * 32u + lane] * rowStride)),
+                                    "r"(cols * 4u), "r"(bar) : "memory");
+                }
+            }
+            else {
+                for(unsigned int j = 0; j < n; j++) {
+                    const float *const row = base + (unsigned long long)list[stage * 32u + j] * rowStride;
+                    for(unsigned int col = lane; col < cols; col += 32u) {
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(denseShare(to + j * DENSE_COLS + col)), "l"(__cvta_generic_to_global(row + col)) : "memory");
+                    }
+                }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(bar) : "memory");
+            }
+        }
+        return;
+    }
+    // fewer copies than warps: several warps share a copy, each with every `sharers`-th row
+    const unsigned int sharers = copies >= DENSE_WARPS ? 1u : DENSE_WARPS / copies, share = copies >= DENSE_WARPS ? 0u : warp / copies;
+    const unsigned int first = copies >= DENSE_WARPS ? warp : warp % copies;
+    const bool mine = share < sharers && (lane % sharers) == share;
+    float4 sum[DENSE_OWN][2];
+    #pragma unroll
+    for(unsigned int o = 0; o < DENSE_OWN; o++) sum[o][0] = sum[o][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    unsigned int ring = 0, parity = 0;
+    bool there = true;
+    for(unsigned int stage = 0; stage < numStages; stage++) {
+        there = there && denseArrived(&arrived[ring], parity);
+        const unsigned int at = stage * 32u + lane;
+        const unsigned int m = (mine && there && at < rows) ? mask[list[at]] >> first : 0u;
+        const float4 *const w = reinterpret_cast<const float4*>(stages + ring * 32u * DENSE_COLS) + lane;
         #pragma unroll
-        for(unsigned int o = 1; o < DENSE_WARPS; o++) {
-            const float4 x = reinterpret_cast<const float4*>(sums)[o * quads + q];
-            a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+        for(unsigned int o = 0; o < DENSE_OWN; o++) {
+            // two rows at a time: the loads of one behind the other's
+            unsigned int left = __ballot_sync(0xFFFFFFFFu, (m >> (o * DENSE_WARPS)) & 1u);
+            while(left) {
+                const float4 *const row = w + (31 - __clz(left)) * (DENSE_COLS / 4u);
+                left ^= 0x80000000u >> __clz(left);
+                const float4 v0 = row[0], v1 = row[32];
+                if(left) {
+                    const float4 *const next = w + (31 - __clz(left)) * (DENSE_COLS / 4u);
+                    left ^= 0x80000000u >> __clz(left);
+                    const float4 u0 = next[0], u1 = next[32];
+                    denseSum(sum[o][0], v0);
+                    denseSum(sum[o][1], v1);
+                    denseSum(sum[o][0], u0);
+                    denseSum(sum[o][1], u1);
+                }
+                else {
+                    denseSum(sum[o][0], v0);
+                    denseSum(sum[o][1], v1);
+                }
+            }
         }
-        const unsigned int b = q / (DENSE_COLS / 4u), col = (q % (DENSE_COLS / 4u)) * 4u;
-        if(col >= cols || (a.x == 0.0f && a.y == 0.0f && a.z == 0.0f && a.w == 0.0f)) continue;
-        float *const out = g.out_post + (unsigned long long)(firstCopy + b) * g.num_trg + part.y + col;
-        if(vec) {
-            redAdd4(out, a);
+        __syncwarp();
+        if(lane == 0u) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(denseShare(&released[ring])) : "memory");
+        if(!there) atomicOr(&L.S.state->error, ERR_BARRIER_TIMEOUT);
+        if(++ring == DENSE_STAGES) {
+            ring = 0;
+            parity ^= 1u;
         }
-        else {
-            redAdd(out, a.x);
-            if(col + 1u < cols) redAdd(out + 1, a.y);
-            if(col + 2u < cols) redAdd(out + 2, a.z);
-            if(col + 3u < cols) redAdd(out + 3, a.w);
+    }
+    if(constant) {
+        // nothing to read: every listed row adds the same weight
+        const float c = g.wu_params[0];
+        for(unsigned int at = lane; at < ((rows + 31u) & ~31u); at += 32u) {
+            const unsigned int m = (mine && at < rows) ? mask[list[at]] >> first : 0u;
+            #pragma unroll
+            for(unsigned int o = 0; o < DENSE_OWN; o++) {
+                for(unsigned int n = __popc(__ballot_sync(0xFFFFFFFFu, (m >> (o * DENSE_WARPS)) & 1u)); n; n--) {
+                    denseSum(sum[o][0], make_float4(c, c, c, c));
+                }
+                sum[o][1] = sum[o][0];
+            }
+        }
+    }
+
+    // ---- the sums, out to the targets' input
+    #pragma unroll
+    for(unsigned int o = 0; o < DENSE_OWN; o++) {
+        #pragma unroll
+        for(unsigned int half = 0; half < 2u; half++) {
+            const unsigned int b = first + o * DENSE_WARPS, col = half * 128u + lane * 4u;
+            const float4 a = sum[o][half];
+            if(b >= copies || share >= sharers || col >= cols || (a.x == 0.0f && a.y == 0.0f && a.z == 0.0f && a.w == 0.0f)) continue;
+            float *const out = g.out_post + (unsigned long long)(firstCopy + b) * g.num_trg + part.y + col;
+            if(vec) redAdd4(out, a);
+            else {
+                redAdd(out, a.x);
+                if(col + 1u < cols) redAdd(out + 1, a.y);
+                if(col + 2u < cols) redAdd(out + 2, a.z);
+                if(col + 3u < cols) redAdd(out + 3, a.w);
+            }
         }
     }
 }

@@ -26,7 +26,7 @@
 namespace b200
 {
 constexpr int NEURON_BLOCK = 128;
-constexpr unsigned int NEURON_BLOCKS_PER_SM = 8;
+constexpr unsigned int NEURON_BLOCKS_PER_SM = 16;
 
 // Peers of a sharded model as the neuron update sees them: every spike id is also
 // stored into each peer's exchange arena, at the offset it has in this process's.

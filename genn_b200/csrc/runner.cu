@@ -149,10 +149,9 @@ struct b200_runner
     unsigned int ahead = 0, advance = 1;    // place of the step being enqueued in its block of steps (see chainPhase)
     ScatterTarget *scatterTargets = nullptr;
     ScatterPart *scatterParts = nullptr;    // sparseBatchKernel: what every CTA does
-    unsigned int scatterGrid = 0;
+    unsigned int scatterGrid = 0, scatterCells = 0, scatterDepth = 0, scatterPiece = 0;
     size_t scatterSmem = 0;
     uint4 *denseParts = nullptr;            // denseBatchKernel: what every CTA does
-    size_t denseSmem = 0;
 
     // persistent fused-step path (batch 1, SPARSE non-learning groups only)
     bool fusedEligible = false;
@@ -549,26 +548,22 @@ int buildDense(b200_runner *r, const std::vector<b200_synapse_group> &dense)
     if(dense.empty()) return B200_OK;
     int sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
-    const unsigned int copies = std::min(r->batch, DENSE_COPIES), words = (r->batch + DENSE_COPIES - 1u) / DENSE_COPIES;
-    const unsigned int perSm = std::min<unsigned int>(6u, (unsigned int)(220u * 1024u / (denseSmemBytes(copies, 1024u) + 1024u)));
+    const unsigned int words = (r->batch + DENSE_COPIES - 1u) / DENSE_COPIES;
     unsigned long long strips = 0;
     for(const auto &g : dense) strips += (g.num_trg + DENSE_COLS - 1u) / DENSE_COLS;
-    const unsigned int wanted = std::max(1u, (unsigned int)((unsigned long long)sms * perSm / std::max(1ull, strips * words)));
+    const unsigned int wanted = std::max(1u, (unsigned int)((unsigned long long)sms * DENSE_PER_SM / std::max(1ull, strips * words)));
     std::vector<uint4> parts;
-    unsigned int window = 0;
     for(unsigned int gi = 0; gi < dense.size(); gi++) {
         const auto &g = dense[gi];
         const unsigned int chunks = std::max(std::min(wanted, std::max(1u, g.num_src / 64u)), (g.num_src + DENSE_WINDOW - 1u) / DENSE_WINDOW);
         const unsigned int per = chunks ? (g.num_src + chunks - 1u) / chunks : 0u;
         for(unsigned int first = 0; first < g.num_src; first += per) {
             const unsigned int n = std::min(per, g.num_src - first);
-            window = std::max(window, n);
             for(unsigned int col = 0; col < g.num_trg; col += DENSE_COLS) parts.push_back(make_uint4(gi, col, first, n));
         }
     }
     if(parts.empty()) return B200_OK;
-    r->denseSmem = denseSmemBytes(copies, window);
-    CUDA_TRY(cudaFuncSetAttribute(denseBatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->denseSmem));
+    CUDA_TRY(cudaFuncSetAttribute(denseBatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DENSE_SMEM));
     CUDA_TRY(poolAlloc(&r->denseParts, sizeof(uint4) * parts.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->denseParts, parts.data(), sizeof(uint4) * parts.size(), cudaMemcpyHostToDevice, r->stream));
     CUDA_TRY(r->denseTable.upload(dense, {0u, (unsigned int)parts.size()}, r->stream));
@@ -581,7 +576,10 @@ bool scatterServes(const b200_runner *r, const b200_synapse_group &g)
 {
     if(r->batch < 2 || r->sharded() || r->tiledChosen || g.wu_model == B200_WU_STDP) return false;
     const unsigned long long cells = (unsigned long long)std::max(1u, g.max_den_delay) * g.num_trg;
-    if(cells > SCATTER_MOST_CELLS) return false;
+    // (two pieces of the widest kind for every warp have to fit besides)
+    if(cells * sizeof(float) > SCATTER_SMEM - 2u * SCATTER_WARPS * SCATTER_PIECE * 9u - 128u) return false;
+    if(((reinterpret_cast<size_t>(g.ind) | reinterpret_cast<size_t>(g.g) | reinterpret_cast<size_t>(g.d) |
+         reinterpret_cast<size_t>(g.max_den_delay ? g.den_delay : g.out_post)) & 15u) != 0u) return false;
     unsigned int groups = 0;
     for(const auto &o : r->synapseGroups) {
         if((o.max_den_delay ? o.den_delay : o.out_post) == (g.max_den_delay ? g.den_delay : g.out_post)) groups++;
@@ -604,7 +602,7 @@ int buildScatter(b200_runner *r, std::vector<b200_synapse_group> &scatter)
     std::vector<ScatterTarget> targets;
     std::vector<double> weight;
     double all = 0.0;
-    unsigned int cells = 0;
+    unsigned int cells = 0, pieceBytes = 0;
     for(unsigned int i = 0; i < scatter.size(); i++) {
         const auto &g = scatter[i];
         if(targets.empty() || targets.back().cells != buffer(g)) {
@@ -616,6 +614,7 @@ int buildScatter(b200_runner *r, std::vector<b200_synapse_group> &scatter)
         weight.back() += synapses;
         all += synapses;
         cells = std::max(cells, targets.back().num_cells);
+        pieceBytes = std::max(pieceBytes, SCATTER_PIECE * (g.ind_bytes + 4u + (g.max_den_delay ? 1u : 0u)));
     }
     int sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
@@ -627,7 +626,11 @@ int buildScatter(b200_runner *r, std::vector<b200_synapse_group> &scatter)
         }
     }
     r->scatterGrid = (unsigned int)parts.size();
-    r->scatterSmem = (size_t)((cells + 3u) & ~3u) * sizeof(float);
+    r->scatterCells = cells;
+    r->scatterPiece = pieceBytes;
+    const size_t sums = (size_t)((cells + 31u) & ~31u) * sizeof(float);
+    r->scatterDepth = std::min<unsigned int>(SCATTER_MOST_DEPTH, (unsigned int)((SCATTER_SMEM - sums) / (SCATTER_WARPS * pieceBytes)));
+    r->scatterSmem = sums + (size_t)r->scatterDepth * SCATTER_WARPS * pieceBytes;
     CUDA_TRY(cudaFuncSetAttribute(sparseBatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->scatterSmem));
     CUDA_TRY(poolAlloc(&r->scatterTargets, sizeof(ScatterTarget) * targets.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->scatterTargets, targets.data(), sizeof(ScatterTarget) * targets.size(), cudaMemcpyHostToDevice, r->stream));
@@ -1802,13 +1805,13 @@ int enqueueSynapses(b200_runner *r, bool capturing, bool force = false)
     if(r->denseTable.num) {
         ScopedTimer tm(r, "presynaptic_update", capturing);
         const dim3 grid(r->denseTable.blocks, 1, (r->batch + DENSE_COPIES - 1u) / DENSE_COPIES);
-        CUDA_TRY(chain(r, denseBatchKernel, grid, DENSE_BLOCK, r->denseSmem, DenseLaunch{synapseLaunch(r, r->denseTable), r->denseParts}));
+        CUDA_TRY(chain(r, denseBatchKernel, grid, DENSE_BLOCK, DENSE_SMEM, DenseLaunch{synapseLaunch(r, r->denseTable), r->denseParts}));
         r->launches++;
     }
     if(r->scatterTable.num) {
         ScopedTimer tm(r, "presynaptic_update", capturing);
         CUDA_TRY(chain(r, sparseBatchKernel, r->scatterGrid, SCATTER_BLOCK, r->scatterSmem,
-                       ScatterLaunch{synapseLaunch(r, r->scatterTable), r->scatterTargets, r->scatterParts}));
+                       ScatterLaunch{synapseLaunch(r, r->scatterTable), r->scatterTargets, r->scatterParts, r->scatterCells, r->scatterDepth, r->scatterPiece}));
         r->launches++;
     }
     if(r->proceduralTable.num) {

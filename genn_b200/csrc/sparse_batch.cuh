@@ -8,23 +8,28 @@
 // and reduces straight into L2: clearing and flushing them would take longer.
 //
 // Shares: the spikes of all groups onto the buffer stand on one line, each as long as its group's rows; a CTA owns an equal
-// stretch of the line and computes it from the spike counts itself.  Inside, a warp takes pieces of SCATTER_PIECE synapses,
-// the next piece's loads under way while one is added (a piece is 8 bytes of weight and index a lane and load; 32 warps with
-// two pieces in flight keep 50 KB under way on an SM, about what HBM needs).
+// stretch of the line and computes it from the spike counts itself.  Inside, a warp takes pieces of SCATTER_PIECE synapses.
+// They come as bulk copies into a ring of the warp's own (SCATTER_WARPS warps x 2 to 4 pieces of 1.5 to 2.3 KB: 50 KB and
+// more under way on an SM, what HBM's latency wants, and no warp waits for another).  Pieces held in registers instead, one
+// ahead: 27 KB under way and 37 instructions an event besides its addition, 43 us at the size below.
 //
-// 20 000 + 20 000 neurons, 8 copies, 11 M events a step: 90 us with the tiled kernels, 60 here.
+// 20 000 + 20 000 neurons, 8 copies, 11 M events a step: 90 us with the tiled kernels, 31 here.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "presynaptic_update.cuh"
 
 namespace b200
 {
-constexpr unsigned int SCATTER_BLOCK = 1024;
+constexpr unsigned int SCATTER_BLOCK = 768;
 constexpr unsigned int SCATTER_WARPS = SCATTER_BLOCK / 32;
-constexpr unsigned int SCATTER_QUADS = 2;                               // groups of four synapses of a lane in a piece
-constexpr unsigned int SCATTER_PIECE = 32 * 4 * SCATTER_QUADS;
-constexpr unsigned int SCATTER_MOST_CELLS = 52 * 1024;                  // 208 KB of sums
+constexpr unsigned int SCATTER_PIECE = 256;                             // synapses: eight a lane
+constexpr unsigned int SCATTER_ALIGN = 16;                              // synapses: pieces start where every array allows a bulk copy
+constexpr unsigned int SCATTER_MOST_DEPTH = 4;                          // pieces in a warp's ring
+constexpr unsigned int SCATTER_SMEM = 225 * 1024;
+constexpr unsigned int SCATTER_WAITS = 1u << 18;                        // polls for a piece before the step is given up
 constexpr unsigned int SCATTER_MOST_SOURCES = 64;                       // groups onto one buffer
 // An event costs 0.19 ns of an SM's shared memory and 0.78 ns of its share of the L2's reductions; clearing and flushing
 // the sums about 2.5 us.
@@ -48,6 +53,9 @@ struct ScatterLaunch
     SynapseLaunch S;                    // SPARSE groups that do not learn, in the order of their targets
     const ScatterTarget *targets;
     const ScatterPart *parts;
+    unsigned int cells;                 // of the largest buffer
+    unsigned int depth;                 // pieces in a warp's ring
+    unsigned int piece_bytes;
 };
 
 __device__ __forceinline__ void scatterShared(float *cell, float v)
@@ -55,94 +63,184 @@ __device__ __forceinline__ void scatterShared(float *cell, float v)
     asm volatile("red.shared.add.f32 [%0], %1;" :: "r"((unsigned int)__cvta_generic_to_shared(cell)), "f"(v) : "memory");
 }
 
-// Four synapses as they are stored.
-struct ScatterQuad
+__device__ __forceinline__ unsigned int scatterShare(const void *p) { return (unsigned int)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void scatterBulk(unsigned int to, const void *from, unsigned int bytes, unsigned int bar)
 {
-    uint4 ind;
-    float4 w;
-    unsigned int delay;
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(to), "l"(__cvta_generic_to_global(from)), "r"(bytes), "r"(bar) : "memory");
+}
+
+// A warp's ring of pieces.
+struct ScatterRing
+{
+    unsigned char *data;
+    unsigned long long *bars;
+    unsigned int depth, bytes;          // pieces, bytes of one
+    unsigned int sent, taken;           // slots of the next piece sent and taken
+    unsigned int parity;                // of the slot next taken
 };
 
-// One piece of a spike's row between its loads and its additions.
-struct ScatterHeld
+// A lane's item: one piece of a spike's row.
+struct ScatterItem
 {
-    ScatterQuad quad[SCATTER_QUADS];
-    unsigned int length, pre, piece;    // length 0: nothing
+    unsigned long long first;           // synapse in the group's arrays
+    unsigned int low, end;              // the row's synapses in the piece
 };
 
-__device__ __forceinline__ void scatterFetch(const b200_synapse_group &g, ScatterHeld &h, unsigned int lane)
+// Four indices of a piece.
+template<int IND>
+__device__ __forceinline__ void scatterIndices(const unsigned char *data, unsigned int at, unsigned int (&cell)[4])
 {
-    const unsigned long long rowStart = (unsigned long long)h.pre * g.row_stride, all = (unsigned long long)g.num_src * g.row_stride;
-    const bool constant = (g.wu_model == B200_WU_STATIC_PULSE_CONSTANT_WEIGHT);
-    h.length = __ldg(&g.row_length[h.pre]);
-    #pragma unroll
-    for(unsigned int q = 0; q < SCATTER_QUADS; q++) {
-        // quads are aligned to the array, not to the row; past the end of the row they still lie in the array or its padding
-        const unsigned long long idx = (rowStart & ~3ull) + (unsigned long long)h.piece * SCATTER_PIECE + (q * 32u + lane) * 4u;
-        ScatterQuad &Q = h.quad[q];
-        if(idx >= all) continue;
-        if(g.ind_bytes == 2u) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(g.ind) + idx));
-            Q.ind.x = v.x; Q.ind.y = v.y;
-        }
-        else if(g.ind_bytes == 4u) Q.ind = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint32_t*>(g.ind) + idx));
-        else Q.ind.x = __ldg(reinterpret_cast<const unsigned int*>(static_cast<const uint8_t*>(g.ind) + idx));
-        if(!constant) Q.w = __ldg(reinterpret_cast<const float4*>(g.g + idx));
-        if(g.max_den_delay) Q.delay = __ldg(reinterpret_cast<const unsigned int*>(g.d + idx));
+    if(IND == 4) {
+        const uint4 v = *reinterpret_cast<const uint4*>(data + at * 4u);
+        cell[0] = v.x; cell[1] = v.y; cell[2] = v.z; cell[3] = v.w;
+    }
+    else if(IND == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(data + at * 2u);
+        cell[0] = v.x & 0xFFFFu; cell[1] = v.x >> 16; cell[2] = v.y & 0xFFFFu; cell[3] = v.y >> 16;
+    }
+    else {
+        const unsigned int v = *reinterpret_cast<const unsigned int*>(data + at);
+        cell[0] = v & 0xFFu; cell[1] = (v >> 8) & 0xFFu; cell[2] = (v >> 16) & 0xFFu; cell[3] = v >> 24;
     }
 }
 
-__device__ __forceinline__ void scatterAdd(const b200_synapse_group &g, const ScatterHeld &h, float *sums, float *cells, bool few,
-                                           unsigned int front, unsigned int lane, StepState *state)
+// What a warp does of one group's spikes: pieces `item`, `item` + SCATTER_WARPS, ... of the group's; returns how far beyond
+// them its next one lies.  The widths are template parameters: they decide every address.
+template<int IND, bool DELAYS>
+__device__ __forceinline__ unsigned int scatterGroup(const SynapseLaunch &S, const b200_synapse_group &g, const unsigned int *spk, unsigned int spikes,
+                                                     unsigned int item, ScatterRing &R, float *sums, float *cells, bool few, unsigned int front)
 {
+    const unsigned int lane = threadIdx.x & 31u;
+    const unsigned int stride = g.row_stride, numTrg = g.num_trg, D = g.max_den_delay, numSrc = g.num_src;
+    const unsigned int pieces = (stride + SCATTER_ALIGN - 1u + SCATTER_PIECE - 1u) / SCATTER_PIECE, items = spikes * pieces;
+    const unsigned int n = items > item ? (items - item + SCATTER_WARPS - 1u) / SCATTER_WARPS : 0u;
     const bool constant = (g.wu_model == B200_WU_STATIC_PULSE_CONSTANT_WEIGHT);
-    const unsigned int skew = (unsigned int)(((unsigned long long)h.pre * g.row_stride) & 3ull);
-    const unsigned int D = g.max_den_delay, numTrg = g.num_trg, end = skew + h.length;
-    #pragma unroll
-    for(unsigned int q = 0; q < SCATTER_QUADS; q++) {
-        const ScatterQuad &Q = h.quad[q];
-        const unsigned int at = h.piece * SCATTER_PIECE + (q * 32u + lane) * 4u;
-        if(at >= end) continue;
-        unsigned int post[4];
-        if(g.ind_bytes == 2u) {
-            post[0] = Q.ind.x & 0xFFFFu; post[1] = Q.ind.x >> 16; post[2] = Q.ind.y & 0xFFFFu; post[3] = Q.ind.y >> 16;
+    const float c = g.wu_params[0];
+    // a lane looks up one of 32 consecutive items
+    auto look = [&](unsigned int from) {
+        ScatterItem I{0ull, 0u, 0u};
+        const unsigned int turn = from + lane;
+        if(turn < n) {
+            const unsigned int x = item + turn * SCATTER_WARPS, spike = x / pieces, offset = (x - spike * pieces) * SCATTER_PIECE;
+            const unsigned int pre = spk[spike];
+            if(pre < numSrc) {
+                const unsigned int length = __ldg(&g.row_length[pre]);
+                const unsigned long long rowStart = (unsigned long long)pre * stride;
+                const unsigned int skew = (unsigned int)rowStart & (SCATTER_ALIGN - 1u);
+                I.first = rowStart - skew + offset;
+                I.low = skew > offset ? skew - offset : 0u;
+                I.end = skew + length > offset ? min(skew + length - offset, SCATTER_PIECE) : 0u;
+                if(S.count_events && offset == 0u) atomicAdd(&S.state->synaptic_events, (unsigned long long)length);
+            }
+            else atomicOr(&S.state->error, ERR_IND_RANGE);
         }
-        else if(g.ind_bytes == 4u) {
-            post[0] = Q.ind.x; post[1] = Q.ind.y; post[2] = Q.ind.z; post[3] = Q.ind.w;
+        return I;
+    };
+    auto send = [&](const ScatterItem &I) {
+        // (whole groups of SCATTER_ALIGN: behind the arrays' last row that is in their padding)
+        const unsigned int m = (I.end + SCATTER_ALIGN - 1u) & ~(SCATTER_ALIGN - 1u);
+        const unsigned int bar = scatterShare(R.bars + R.sent), to = scatterShare(R.data + R.sent * R.bytes);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(m * (IND + (constant ? 0u : 4u) + (DELAYS ? 1u : 0u))) : "memory");
+        if(m) {
+            scatterBulk(to, static_cast<const unsigned char*>(g.ind) + I.first * IND, m * IND, bar);
+            if(!constant) scatterBulk(to + SCATTER_PIECE * IND, g.g + I.first, m * 4u, bar);
+            if(DELAYS) scatterBulk(to + SCATTER_PIECE * (IND + 4u), g.d + I.first, m, bar);
         }
-        else {
-            post[0] = Q.ind.x & 0xFFu; post[1] = (Q.ind.x >> 8) & 0xFFu; post[2] = (Q.ind.x >> 16) & 0xFFu; post[3] = Q.ind.x >> 24;
-        }
-        const float w[4] = {Q.w.x, Q.w.y, Q.w.z, Q.w.w};
+    };
+    auto next = [&](unsigned int &slot) { slot = (slot + 1u == R.depth) ? 0u : slot + 1u; };
+    auto add = [&](const unsigned char *data, unsigned int low, unsigned int end) {
         #pragma unroll
-        for(unsigned int j = 0; j < 4u; j++) {
-            if(at + j < skew || at + j >= end) continue;
-            unsigned int cell = post[j];
-            if(cell >= numTrg) {
-                atomicOr(&state->error, ERR_IND_RANGE);
-                continue;
+        for(unsigned int q = 0; q < SCATTER_PIECE / 128u; q++) {
+            const unsigned int at = q * 128u + lane * 4u;
+            if(at >= end) break;
+            unsigned int cell[4];
+            scatterIndices<IND>(data, at, cell);
+            const float4 v = constant ? make_float4(c, c, c, c) : *reinterpret_cast<const float4*>(data + SCATTER_PIECE * IND + at * 4u);
+            const float w[4] = {v.x, v.y, v.z, v.w};
+            const unsigned int delay = DELAYS ? *reinterpret_cast<const unsigned int*>(data + SCATTER_PIECE * (IND + 4u) + at) : 0u;
+            auto place = [&](unsigned int j) {
+                if(DELAYS) {
+                    unsigned int slot = front + ((delay >> (8u * j)) & 0xFFu);
+                    while(slot >= D) slot -= D;         // a delay of the ring length or more wraps around
+                    cell[j] += slot * numTrg;
+                }
+            };
+            // the quads inside a row, all but its first and last, need no test of their own for every synapse
+            if(at >= low && at + 4u <= end && max(max(cell[0], cell[1]), max(cell[2], cell[3])) < numTrg) {
+                #pragma unroll
+                for(unsigned int j = 0; j < 4u; j++) place(j);
+                if(few) {
+                    #pragma unroll
+                    for(unsigned int j = 0; j < 4u; j++) redAdd(cells + cell[j], w[j]);
+                }
+                else {
+                    #pragma unroll
+                    for(unsigned int j = 0; j < 4u; j++) scatterShared(sums + cell[j], w[j]);
+                }
             }
-            if(D) {
-                unsigned int slot = front + ((Q.delay >> (8u * j)) & 0xFFu);
-                while(slot >= D) slot -= D;
-                cell += slot * numTrg;
+            else {
+                #pragma unroll
+                for(unsigned int j = 0; j < 4u; j++) {
+                    if(at + j < low || at + j >= end) continue;
+                    if(cell[j] >= numTrg) {
+                        atomicOr(&S.state->error, ERR_IND_RANGE);
+                        continue;
+                    }
+                    place(j);
+                    if(few) redAdd(cells + cell[j], w[j]);
+                    else scatterShared(sums + cell[j], w[j]);
+                }
             }
-            const float v = constant ? g.wu_params[0] : w[j];
-            if(few) redAdd(cells + cell, v);
-            else scatterShared(sums + cell, v);
+        }
+    };
+    ScatterItem here = look(0u), later = {0ull, 0u, 0u};
+    for(unsigned int turn = 0; turn < min(n, R.depth); turn++) {
+        if(lane == turn) send(here);
+        next(R.sent);
+    }
+    for(unsigned int turn = 0; turn < n; turn++) {
+        const unsigned int at = turn & 31u;
+        if(at == 0u) {
+            if(turn) here = later;
+            later = look(turn + 32u);
+        }
+        const unsigned int low = __shfl_sync(0xFFFFFFFFu, here.low, at), end = __shfl_sync(0xFFFFFFFFu, here.end, at);
+        bool there = false;
+        for(unsigned int i = 0; i < SCATTER_WAITS && !there; i++) {
+            unsigned int done;
+            asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                         : "=r"(done) : "r"(scatterShare(R.bars + R.taken)), "r"(R.parity) : "memory");
+            there = done != 0u;
+        }
+        if(there) add(R.data + R.taken * R.bytes, low, end);
+        else atomicOr(&S.state->error, ERR_BARRIER_TIMEOUT);
+        __syncwarp();
+        next(R.taken);
+        if(R.taken == 0u) R.parity ^= 1u;
+        if(turn + R.depth < n) {
+            const unsigned int ahead = (turn + R.depth) & 31u;
+            if(lane == ahead) send(ahead < at ? later : here);
+            next(R.sent);
         }
     }
+    return item + n * SCATTER_WARPS - items;
 }
 
 static __global__ void __launch_bounds__(SCATTER_BLOCK, 1)
 sparseBatchKernel(const ScatterLaunch L)
 {
     extern __shared__ __align__(16) float scatterSums[];
+    __shared__ __align__(8) unsigned long long scatterBars[SCATTER_WARPS][SCATTER_MOST_DEPTH];
     __shared__ unsigned int firstSpike[SCATTER_MOST_SOURCES], spikes[SCATTER_MOST_SOURCES];
     __shared__ unsigned long long line[SCATTER_MOST_SOURCES];
     const ScatterPart part = L.parts[blockIdx.x];
     const ScatterTarget T = L.targets[part.target];
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    if(lane < L.depth) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(scatterShare(&scatterBars[warp][lane])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     chainWait();
     const unsigned int k = chainPhase(L.S.state, L.S.ahead);
     // ---- this CTA's stretch of the line of spikes
@@ -179,41 +277,26 @@ sparseBatchKernel(const ScatterLaunch L)
     }
     __syncthreads();
     float *const cells = T.cells + (unsigned long long)part.copy * T.num_cells;
+    ScatterRing ring{reinterpret_cast<unsigned char*>(scatterSums + ((L.cells + 31u) & ~31u)) + (size_t)warp * L.depth * L.piece_bytes,
+                     scatterBars[warp], L.depth, L.piece_bytes, 0u, 0u, 0u};
     unsigned int item = warp;
     for(unsigned int gi = 0; gi < T.num_groups; gi++) {
         const b200_synapse_group &g = L.S.groups[T.first_group + gi];
-        const unsigned int pieces = (g.row_stride + 3u + SCATTER_PIECE - 1u) / SCATTER_PIECE, items = spikes[gi] * pieces;
         const unsigned int slots = g.src_delay_slots, slot = ringSlot(k + slots - g.axonal_delay, slots);
         const unsigned int *const spk = g.src_spk + ((unsigned long long)part.copy * slots + slot) * g.num_src + firstSpike[gi];
         const unsigned int front = g.max_den_delay ? ringSlot(k + 1u, g.max_den_delay) : 0u;
-        auto spikeOf = [&](unsigned int at) { return at < items ? spk[at / pieces] : 0u; };
-        auto fetch = [&](ScatterHeld &h, unsigned int at, unsigned int pre) {
-            h.length = 0u;
-            if(at >= items) return;
-            if(pre >= g.num_src) {
-                atomicOr(&L.S.state->error, ERR_IND_RANGE);
-                return;
-            }
-            h.pre = pre;
-            h.piece = at % pieces;
-            scatterFetch(g, h, lane);
-            if(L.S.count_events && h.piece == 0u && lane == 0u) atomicAdd(&L.S.state->synaptic_events, (unsigned long long)h.length);
+        auto deliver = [&](auto ind, auto delays) {
+            item = scatterGroup<decltype(ind)::value, decltype(delays)::value>(L.S, g, spk, spikes[gi], item, ring, scatterSums, cells, few, front);
         };
-        ScatterHeld a, b;
-        fetch(a, item, spikeOf(item));
-        unsigned int next = spikeOf(item + SCATTER_WARPS);
-        while(item < items) {
-            fetch(b, item + SCATTER_WARPS, next);
-            next = spikeOf(item + 2u * SCATTER_WARPS);
-            scatterAdd(g, a, scatterSums, cells, few, front, lane, L.S.state);
-            item += SCATTER_WARPS;
-            if(item >= items) break;
-            fetch(a, item + SCATTER_WARPS, next);
-            next = spikeOf(item + 2u * SCATTER_WARPS);
-            scatterAdd(g, b, scatterSums, cells, few, front, lane, L.S.state);
-            item += SCATTER_WARPS;
+        using std::integral_constant;
+        if(g.max_den_delay) {
+            if(g.ind_bytes == 2u) deliver(integral_constant<int, 2>(), integral_constant<bool, true>());
+            else if(g.ind_bytes == 4u) deliver(integral_constant<int, 4>(), integral_constant<bool, true>());
+            else deliver(integral_constant<int, 1>(), integral_constant<bool, true>());
         }
-        item -= items;
+        else if(g.ind_bytes == 2u) deliver(integral_constant<int, 2>(), integral_constant<bool, false>());
+        else if(g.ind_bytes == 4u) deliver(integral_constant<int, 4>(), integral_constant<bool, false>());
+        else deliver(integral_constant<int, 1>(), integral_constant<bool, false>());
     }
     if(few) return;
     __syncthreads();
