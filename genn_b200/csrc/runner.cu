@@ -30,6 +30,7 @@
 #include "tiled.cuh"
 #include "dense_batch.cuh"
 #include "sparse_batch.cuh"
+#include "procedural.cuh"
 #include "resident.h"
 #include "memory.h"
 #include "record.cuh"
@@ -145,7 +146,8 @@ struct b200_runner
     bool dirty = true;
 
     DeviceTable<b200_neuron_group> neuronTable;
-    DeviceTable<b200_synapse_group> sparseTable, postSpanTable, learnTable, proceduralTable, denseTable, scatterTable;
+    DeviceTable<b200_synapse_group> sparseTable, postSpanTable, learnTable, proceduralTable, drawnTable, denseTable, scatterTable;
+    bool drawnNormal = false, drawnWide = false;    // proceduralDrawnKernel: every weight Normal; element numbers beyond 32 bits
     unsigned int ahead = 0, advance = 1;    // place of the step being enqueued in its block of steps (see chainPhase)
     ScatterTarget *scatterTargets = nullptr;
     ScatterPart *scatterParts = nullptr;    // sparseBatchKernel: what every CTA does
@@ -652,7 +654,7 @@ int prepare(b200_runner *r)
         }
         CUDA_TRY(r->neuronTable.upload(r->neuronGroups, starts, r->stream));
     }
-    std::vector<b200_synapse_group> sparse, postSpan, learn, procedural, dense, scatter;
+    std::vector<b200_synapse_group> sparse, postSpan, learn, procedural, drawn, dense, scatter;
     std::vector<unsigned int> sparseStarts{0}, postSpanStarts{0}, learnStarts{0}, proceduralStarts{0};
     for(const auto &g : r->synapseGroups) {
         if(g.connectivity == B200_CONN_SPARSE && scatterServes(r, g)) {
@@ -673,8 +675,15 @@ int prepare(b200_runner *r)
         else if(g.connectivity == B200_CONN_PROCEDURAL) {
             const unsigned int T = connectSubRows(g.proc_connect, g.proc_connect_params);
             if(T > 32u || (T & (T - 1u))) return fail(B200_ERR_INVALID, "procedural group: %u sub-rows per row (a power of two of at most 32 is supported)", T);
-            procedural.push_back(g);
-            proceduralStarts.push_back(proceduralStarts.back() + 1);
+            const bool prob = (g.proc_connect == B200_CONNECT_FIXED_PROBABILITY || g.proc_connect == B200_CONNECT_FIXED_PROBABILITY_NO_AUTAPSE);
+            // drawn weights need a place in the row and most of the work: the two-phase kernel
+            if(prob && g.wu_model != B200_WU_STATIC_PULSE_CONSTANT_WEIGHT) {
+                drawn.push_back(g);
+            }
+            else {
+                procedural.push_back(g);
+                proceduralStarts.push_back(proceduralStarts.back() + 1);
+            }
         }
         else {
             return fail(B200_ERR_INVALID, "connectivity %u is not supported by this build", g.connectivity);
@@ -694,9 +703,16 @@ int prepare(b200_runner *r)
     }
     CUDA_TRY(r->learnTable.upload(learn, learnStarts, r->stream));
     CUDA_TRY(r->proceduralTable.upload(procedural, proceduralStarts, r->stream));
+    CUDA_TRY(r->drawnTable.upload(drawn, {0u, (unsigned int)drawn.size()}, r->stream));
+    r->drawnNormal = true;
+    r->drawnWide = false;
+    for(const auto &g : drawn) {
+        r->drawnNormal = r->drawnNormal && g.proc_weight_init == B200_INIT_NORMAL;
+        r->drawnWide = r->drawnWide || (unsigned long long)g.num_src * g.row_stride > 0xFFFFFFFFull;
+    }
 
     // ---- tables of the persistent fused-step kernel --------------------------------
-    r->fusedEligible = (r->batch == 1 && postSpan.empty() && dense.empty() && scatter.empty() && learn.empty() && procedural.empty() &&
+    r->fusedEligible = (r->batch == 1 && postSpan.empty() && dense.empty() && scatter.empty() && learn.empty() && procedural.empty() && drawn.empty() &&
                         !r->neuronGroups.empty());
     r->fusedGroups = sparse;
     r->lagStale = true;
@@ -1823,6 +1839,18 @@ int enqueueSynapses(b200_runner *r, bool capturing, bool force = false)
         CUDA_TRY(chain(r, presynapticProceduralKernel, grid, PROC_BLOCK, 0, synapseLaunch(r, r->proceduralTable)));
         r->launches++;
     }
+    if(r->drawnTable.num) {
+        ScopedTimer tm(r, "presynaptic_update", capturing);
+        // (the number of spikes is only known on the device: as many blocks as the chip holds take them in turn)
+        int sms = 0;
+        CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+        const dim3 grid((unsigned int)sms * PROC_PER_SM, r->drawnTable.num, r->batch);
+        const ProceduralLaunch P{synapseLaunch(r, r->drawnTable), proceduralKeys(r->seed)};
+        auto kernel = r->drawnNormal ? (r->drawnWide ? proceduralDrawnKernel<true, true> : proceduralDrawnKernel<true, false>)
+                                     : proceduralDrawnKernel<false, true>;
+        CUDA_TRY(chain(r, kernel, grid, DRAWN_BLOCK, 0, P));
+        r->launches++;
+    }
     if(r->learnTable.num) {
         ScopedTimer tm(r, "postsynaptic_update", capturing);
         const dim3 grid(r->learnTable.blocks, spikeLanesFor(r, r->learnTable.blocks), r->batch);
@@ -1903,7 +1931,7 @@ int enqueueStep(b200_runner *r, unsigned long long numRec, bool capturing)
 unsigned int kernelsPerStep(const b200_runner *r)
 {
     return 1u + (r->sparseTable.num ? (tiledActive(r) ? 3u : 1u) : 0u) + (r->postSpanTable.num ? 1u : 0u) + (r->denseTable.num ? 1u : 0u) + (r->scatterTable.num ? 1u : 0u) + (r->learnTable.num ? 1u : 0u) +
-           (r->proceduralTable.num ? 1u : 0u);
+           (r->proceduralTable.num ? 1u : 0u) + (r->drawnTable.num ? 1u : 0u);
 }
 
 int buildGraph(b200_runner *r, unsigned int len, unsigned long long numRec)
@@ -2030,6 +2058,7 @@ int b200_runner_destroy(b200_runner *r)
     poolFree(r->scatterTargets, r->stream);
     poolFree(r->scatterParts, r->stream);
     r->proceduralTable.release(r->stream);
+    r->drawnTable.release(r->stream);
     r->learnTable.release(r->stream);
     poolFree(r->fusedSlotStart, r->stream);
     poolFree(r->fusedSources, r->stream);
