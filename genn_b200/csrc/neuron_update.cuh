@@ -27,6 +27,7 @@ namespace b200
 {
 constexpr int NEURON_BLOCK = 128;
 constexpr unsigned int NEURON_BLOCKS_PER_SM = 16;
+constexpr unsigned int NEURON_WARPS_WANTED = 8;     // of an SM, before a warp takes four words of neurons
 
 // Peers of a sharded model as the neuron update sees them: every spike id is also
 // stored into each peer's exchange arena, at the offset it has in this process's.
@@ -180,36 +181,56 @@ __device__ __forceinline__ float drawPoissonInterval(const NeuronLaunch &L, cons
     return B200_FADD(tts, B200_FMUL(g.params[0], -b200_logf(b200_rng_uniform(&rng))));
 }
 
-template<int NPSM, int NCS>
-__device__ __forceinline__ bool neuronCompute(const NeuronLaunch &L, const b200_neuron_group &g, unsigned int b,
-                                              unsigned int i, unsigned long long timestep, float t,
-                                              NeuronRegs<NPSM, NCS> &r, const float (&front)[NPSM],
-                                              const unsigned int (&csCount)[NCS > 0 ? NCS : 1], bool intervalDrawn = false)
+// WORDS neurons of a thread, 32 apart: what they share (the group's parameters, every branch) is done once for all, and their
+// arithmetic chains run side by side.  Neurons that are not `active` are computed on whatever they hold and never spike.
+template<int NPSM, int NCS, int WORDS>
+__device__ __forceinline__ void neuronComputeWords(const NeuronLaunch &L, const b200_neuron_group &g, unsigned int b,
+                                                   const unsigned int (&i)[WORDS], const bool (&active)[WORDS],
+                                                   unsigned long long timestep, float t,
+                                                   NeuronRegs<NPSM, NCS> (&r)[WORDS], const float (&front)[WORDS][NPSM],
+                                                   const unsigned int (&csCount)[WORDS][NCS > 0 ? NCS : 1], bool (&spiked)[WORDS],
+                                                   bool intervalDrawn = false)
 {
     const unsigned int model = g.model;
-    float Isyn = 0.0f;
-    float V = __uint_as_float(r.v[0]);
+    float Isyn[WORDS], V[WORDS];
+    #pragma unroll
+    for(int w = 0; w < WORDS; w++) {
+        Isyn[w] = 0.0f;
+        V[w] = __uint_as_float(r[w].v[0]);
+        spiked[w] = false;
+    }
 
     // incoming fused postsynaptic models
     #pragma unroll
     for(unsigned int p = 0; p < NPSM; p++) {
         if(p < g.num_psm) {
             const b200_psm &psm = g.psm[p];
-            float linSyn = B200_FADD(r.lin[p], front[p]);
-            if(!psm.max_den_delay) linSyn = r.lin[p];
+            float linSyn[WORDS];
+            #pragma unroll
+            for(int w = 0; w < WORDS; w++) linSyn[w] = psm.max_den_delay ? B200_FADD(r[w].lin[p], front[w][p]) : r[w].lin[p];
             if(psm.model == B200_PSM_EXP_CURR) {
-                Isyn = B200_FADD(Isyn, B200_FMUL(psm.params[0], linSyn));
-                linSyn = B200_FMUL(linSyn, psm.params[1]);
+                const float init = psm.params[0], decay = psm.params[1];
+                #pragma unroll
+                for(int w = 0; w < WORDS; w++) {
+                    Isyn[w] = B200_FADD(Isyn[w], B200_FMUL(init, linSyn[w]));
+                    r[w].lin[p] = B200_FMUL(linSyn[w], decay);
+                }
             }
             else if(psm.model == B200_PSM_EXP_COND) {
-                Isyn = B200_FADD(Isyn, B200_FMUL(linSyn, B200_FSUB(psm.params[1], V)));
-                linSyn = B200_FMUL(linSyn, psm.params[0]);
+                const float decay = psm.params[0], E = psm.params[1];
+                #pragma unroll
+                for(int w = 0; w < WORDS; w++) {
+                    Isyn[w] = B200_FADD(Isyn[w], B200_FMUL(linSyn[w], B200_FSUB(E, V[w])));
+                    r[w].lin[p] = B200_FMUL(linSyn[w], decay);
+                }
             }
             else {
-                Isyn = B200_FADD(Isyn, linSyn);
-                linSyn = 0.0f;
+                #pragma unroll
+                for(int w = 0; w < WORDS; w++) {
+                    Isyn[w] = B200_FADD(Isyn[w], linSyn[w]);
+                    r[w].lin[p] = 0.0f;
+                }
             }
-            r.lin[p] = linSyn;
         }
     }
 
@@ -218,73 +239,111 @@ __device__ __forceinline__ bool neuronCompute(const NeuronLaunch &L, const b200_
     for(unsigned int c = 0; c < NCS; c++) {
         if(c < g.num_cs) {
             const b200_current_source &cs = g.cs[c];
+            const float scale = cs.params[0], decay = cs.params[1];
             if(cs.model == B200_CS_DC) {
-                Isyn = B200_FADD(Isyn, cs.params[0]);
+                #pragma unroll
+                for(int w = 0; w < WORDS; w++) Isyn[w] = B200_FADD(Isyn[w], scale);
             }
             else {
-                float current = r.cs[c];
-                current = B200_FADD(current, B200_FMUL(cs.params[0], (float)csCount[c]));
-                Isyn = B200_FADD(Isyn, current);
-                r.cs[c] = B200_FMUL(current, cs.params[1]);
+                #pragma unroll
+                for(int w = 0; w < WORDS; w++) {
+                    const float current = B200_FADD(r[w].cs[c], B200_FMUL(scale, (float)csCount[w][c]));
+                    Isyn[w] = B200_FADD(Isyn[w], current);
+                    r[w].cs[c] = B200_FMUL(current, decay);
+                }
             }
         }
     }
 
-    bool spiked = false;
     if(model == B200_NEURON_LIF) {
-        float R = __uint_as_float(r.v[1]);
-        if(R <= 0.0f) {
-            const float alpha = B200_FADD(B200_FMUL(B200_FADD(Isyn, g.params[3]), g.params[4]), g.params[2]);
-            V = B200_FSUB(alpha, B200_FMUL(g.params[5], B200_FSUB(alpha, V)));
+        const float threshold = g.params[0], reset = g.params[1], rest = g.params[2], offset = g.params[3], rm = g.params[4],
+                    decay = g.params[5], refractory = g.params[6];
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) {
+            float R = __uint_as_float(r[w].v[1]);
+            if(R <= 0.0f) {
+                const float alpha = B200_FADD(B200_FMUL(B200_FADD(Isyn[w], offset), rm), rest);
+                V[w] = B200_FSUB(alpha, B200_FMUL(decay, B200_FSUB(alpha, V[w])));
+            }
+            else {
+                R = B200_FSUB(R, L.dt);
+            }
+            if(R <= 0.0f && V[w] >= threshold) {
+                spiked[w] = active[w];
+                V[w] = reset;
+                R = refractory;
+            }
+            r[w].v[0] = __float_as_uint(V[w]);
+            r[w].v[1] = __float_as_uint(R);
         }
-        else {
-            R = B200_FSUB(R, L.dt);
-        }
-        if(R <= 0.0f && V >= g.params[0]) {
-            spiked = true;
-            V = g.params[1];
-            R = g.params[6];
-        }
-        r.v[0] = __float_as_uint(V);
-        r.v[1] = __float_as_uint(R);
     }
     else if(model == B200_NEURON_IZHIKEVICH) {
-        float U = __uint_as_float(r.v[1]);
+        const float a = g.params[0], bb = g.params[1], c = g.params[2], d = g.params[3];
         const float dt = L.dt;
-        if(V >= 30.0f) {
-            V = g.params[2];
-            U = B200_FADD(U, g.params[3]);
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) {
+            float U = __uint_as_float(r[w].v[1]), v = V[w];
+            if(v >= 30.0f) {
+                v = c;
+                U = B200_FADD(U, d);
+            }
+            for(int half = 0; half < 2; half++) {
+                // 0.04*V*V + 5*V + 140 - U + Isyn, left to right
+                float x = B200_FMUL(B200_FMUL(0.04f, v), v);
+                x = B200_FADD(x, B200_FMUL(5.0f, v));
+                x = B200_FADD(x, 140.0f);
+                x = B200_FSUB(x, U);
+                x = B200_FADD(x, Isyn[w]);
+                v = B200_FADD(v, B200_FMUL(B200_FMUL(0.5f, x), dt));
+            }
+            U = B200_FADD(U, B200_FMUL(B200_FMUL(a, B200_FSUB(B200_FMUL(bb, v), U)), dt));
+            if(v > 30.0f) v = 30.0f;
+            spiked[w] = active[w] && (v >= 29.99f);
+            r[w].v[0] = __float_as_uint(v);
+            r[w].v[1] = __float_as_uint(U);
         }
-        for(int half = 0; half < 2; half++) {
-            // 0.04*V*V + 5*V + 140 - U + Isyn, left to right
-            float x = B200_FMUL(B200_FMUL(0.04f, V), V);
-            x = B200_FADD(x, B200_FMUL(5.0f, V));
-            x = B200_FADD(x, 140.0f);
-            x = B200_FSUB(x, U);
-            x = B200_FADD(x, Isyn);
-            V = B200_FADD(V, B200_FMUL(B200_FMUL(0.5f, x), dt));
-        }
-        U = B200_FADD(U, B200_FMUL(B200_FMUL(g.params[0], B200_FSUB(B200_FMUL(g.params[1], V), U)), dt));
-        if(V > 30.0f) V = 30.0f;
-        spiked = (V >= 29.99f);
-        r.v[0] = __float_as_uint(V);
-        r.v[1] = __float_as_uint(U);
     }
     else if(model == B200_NEURON_SPIKE_SOURCE_ARRAY) {
-        const unsigned int start = r.v[0], end = r.v[1];
-        if(start != end && t >= __ldg(&g.egp[start])) {
-            spiked = true;
-            r.v[0] = start + 1;
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) {
+            const unsigned int start = r[w].v[0], end = r[w].v[1];
+            if(active[w] && start != end && t >= __ldg(&g.egp[start])) {
+                spiked[w] = true;
+                r[w].v[0] = start + 1;
+            }
         }
     }
     else {
-        float tts = V;
-        if(tts <= 0.0f && !intervalDrawn) tts = drawPoissonInterval(L, g, b, i, timestep, tts);
-        tts = B200_FSUB(tts, 1.0f);
-        spiked = (tts <= 0.0f);
-        r.v[0] = __float_as_uint(tts);
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) {
+            float tts = V[w];
+            if(active[w] && tts <= 0.0f && !intervalDrawn) tts = drawPoissonInterval(L, g, b, i[w], timestep, tts);
+            tts = B200_FSUB(tts, 1.0f);
+            spiked[w] = active[w] && (tts <= 0.0f);
+            r[w].v[0] = __float_as_uint(tts);
+        }
     }
-    return spiked;
+}
+
+template<int NPSM, int NCS>
+__device__ __forceinline__ bool neuronCompute(const NeuronLaunch &L, const b200_neuron_group &g, unsigned int b,
+                                              unsigned int i, unsigned long long timestep, float t,
+                                              NeuronRegs<NPSM, NCS> &r, const float (&front)[NPSM],
+                                              const unsigned int (&csCount)[NCS > 0 ? NCS : 1], bool intervalDrawn = false)
+{
+    const unsigned int one[1] = {i};
+    const bool active[1] = {true};
+    bool spiked[1];
+    NeuronRegs<NPSM, NCS> regs[1] = {r};
+    float fronts[1][NPSM];
+    unsigned int counts[1][NCS > 0 ? NCS : 1];
+    #pragma unroll
+    for(int p = 0; p < NPSM; p++) fronts[0][p] = front[p];
+    #pragma unroll
+    for(int c = 0; c < (NCS > 0 ? NCS : 1); c++) counts[0][c] = csCount[c];
+    neuronComputeWords<NPSM, NCS, 1>(L, g, b, one, active, timestep, t, regs, fronts, counts, spiked, intervalDrawn);
+    r = regs[0];
+    return spiked[0];
 }
 
 // Spike emission (ballot + one atomic per spiking warp), spike times and
@@ -375,19 +434,105 @@ __device__ __forceinline__ void neuronStep(const NeuronLaunch &L, const b200_neu
     neuronEmit<COHERENT>(L, g, b, local, spiked, k, timestep, t, x);
 }
 
-template<int NPSM, int NCS>
+// A warp's WORDS x 32 neurons of one group, one time step with their state in global memory: every load before any store
+// (the pointers are generic: a store between two loads would make the second wait), one place in the spike list for all.
+template<int NPSM, int NCS, int WORDS>
+__device__ __forceinline__ void neuronWords(const NeuronLaunch &L, const b200_neuron_group &g, unsigned int b, unsigned int firstLocal,
+                                            unsigned int k, unsigned long long timestep)
+{
+    const unsigned int lane = threadIdx.x & 31u, N = g.num_neurons, update = g.num_update, slots = g.num_delay_slots;
+    const unsigned int wslot = ringSlot(k + 1, slots);
+    const float t = B200_FMUL((float)timestep, L.dt);
+    NeuronRegs<NPSM, NCS> r[WORDS];
+    float front[WORDS][NPSM], was[WORDS];
+    unsigned int csCount[WORDS][NCS > 0 ? NCS : 1], i[WORDS];
+    bool active[WORDS], spiked[WORDS];
+    float *const times = g.spike_times ? g.spike_times + (unsigned long long)b * slots * N : nullptr;
+    const unsigned int rslot = times ? ringSlot(k, slots) : 0u;
+    #pragma unroll
+    for(int w = 0; w < WORDS; w++) {
+        const unsigned int local = firstLocal + 32u * w + lane;
+        active[w] = local < update;
+        i[w] = g.first_neuron + local;
+        if(active[w]) {
+            loadNeuron<false>(g, (unsigned long long)b * N + i[w], r[w]);
+            if(times) was[w] = times[(unsigned long long)rslot * N + i[w]];
+        }
+    }
+    // front slots of the dendritic-delay rings: read and cleared (neuronUpdateGroupMerged.cc:96-113)
+    #pragma unroll
+    for(unsigned int p = 0; p < NPSM; p++) {
+        const unsigned int D = p < g.num_psm ? g.psm[p].max_den_delay : 0u;
+        float *const slot = D ? &g.psm[p].den_delay[((unsigned long long)b * D + ringSlot(k + 1, D)) * N] : nullptr;
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) front[w][p] = (slot && active[w]) ? slot[i[w]] : 0.0f;
+        if(slot) {
+            #pragma unroll
+            for(int w = 0; w < WORDS; w++) if(active[w]) slot[i[w]] = 0.0f;
+        }
+    }
+    #pragma unroll
+    for(int w = 0; w < WORDS; w++) drawCurrentSources<NCS>(L, g, b, i[w], timestep, csCount[w]);
+    neuronComputeWords<NPSM, NCS, WORDS>(L, g, b, i, active, timestep, t, r, front, csCount, spiked);
+    unsigned int ballot[WORDS], total = 0;
+    #pragma unroll
+    for(int w = 0; w < WORDS; w++) {
+        ballot[w] = __ballot_sync(0xFFFFFFFFu, spiked[w]);
+        total += __popc(ballot[w]);
+    }
+    unsigned int base = 0;
+    if(total && lane == 0) {
+        base = atomicAdd(&g.spk_cnt[b * slots + wslot], total);
+        if(L.count_events) atomicAdd(&L.state->spikes, (unsigned long long)total);
+    }
+    // (the state on its way while the place in the list is fetched)
+    #pragma unroll
+    for(int w = 0; w < WORDS; w++) {
+        if(active[w]) {
+            storeNeuron(g, (unsigned long long)b * N + i[w], r[w], false);
+            // spike times ride in the queue: carry the previous slot forward
+            if(times) times[(unsigned long long)wslot * N + i[w]] = spiked[w] ? t : was[w];
+        }
+    }
+    // recording: bit j%32 of word j/32 for the group's j-th neuron (backendSIMT.cc:617-660 for a whole population)
+    if(g.record_spk && L.num_recording_timesteps) {
+        const unsigned int words = (update + 31u) / 32u;
+        unsigned int *const rec = g.record_spk + ((timestep % L.num_recording_timesteps) * L.batch + b) * words + firstLocal / 32u;
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) if(lane == 0 && firstLocal / 32u + w < words) rec[w] = ballot[w];
+    }
+    if(total) {
+        const unsigned int listStride = g.spk_slot_stride ? g.spk_slot_stride : N;
+        unsigned int *const list = g.spk + ((unsigned long long)b * slots + wslot) * listStride;
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        #pragma unroll
+        for(int w = 0; w < WORDS; w++) {
+            if(spiked[w]) {
+                const unsigned int pos = base + __popc(ballot[w] & ((1u << lane) - 1u));
+                if(pos < listStride) list[pos] = i[w];
+                else atomicOr(&L.state->error, ERR_SPIKE_OVERFLOW);
+            }
+            base += __popc(ballot[w]);
+        }
+    }
+}
+
+// WORDS = 4: a warp takes the 128 neurons of a padded block, a quarter of the instructions for each, as long as that leaves
+// every SM its warps; WORDS = 1: a warp takes 32, for small networks, where the chain of one neuron is all there is.
+template<int NPSM, int NCS, int WORDS>
 __global__ void __launch_bounds__(NEURON_BLOCK)
 neuronUpdateKernel(const NeuronLaunch L)
 {
+    constexpr unsigned int PARTS = NEURON_BLOCK / (32 * WORDS);         // warps of a padded block
     const unsigned int blocks = __ldg(&L.block_start[L.num_groups]), launched = gridDim.x * gridDim.y;
     const unsigned int rank = blockIdx.y * gridDim.x + blockIdx.x;
     chainWait();
     const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned long long timestep = L.state->timestep + L.ahead;
-    for(unsigned int item = rank; item < blocks * L.batch; item += launched) {
-        const unsigned int b = item / blocks, block = item - b * blocks;
+    for(unsigned int unit = rank * (NEURON_BLOCK / 32) + (threadIdx.x >> 5); unit < blocks * L.batch * PARTS; unit += launched * (NEURON_BLOCK / 32)) {
+        const unsigned int item = unit / PARTS, b = item / blocks, block = item - b * blocks;
         const unsigned int gi = findGroup(L.block_start, L.num_groups, block);
-        neuronStep<false, NPSM, NCS>(L, L.groups[gi], b, (block - __ldg(&L.block_start[gi])) * NEURON_BLOCK + threadIdx.x, k, timestep);
+        neuronWords<NPSM, NCS, WORDS>(L, L.groups[gi], b, (block - __ldg(&L.block_start[gi])) * NEURON_BLOCK + (unit % PARTS) * 32u * WORDS, k, timestep);
     }
 
     // ---- queue update for the next step: its slot was last read three steps ago at the latest -------

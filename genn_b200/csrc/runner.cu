@@ -1881,9 +1881,19 @@ int enqueueNeurons(b200_runner *r, unsigned long long numRec, bool capturing)
     // counting themselves one after another in the ticket)
     int sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
-    const dim3 grid((unsigned int)std::min<unsigned long long>((unsigned long long)r->neuronTable.blocks * r->batch, (unsigned long long)sms * NEURON_BLOCKS_PER_SM));
+    const unsigned long long items = (unsigned long long)r->neuronTable.blocks * r->batch;
+    const bool four = items >= (unsigned long long)sms * NEURON_WARPS_WANTED;
+    const dim3 grid((unsigned int)std::min<unsigned long long>(four ? (items + 3u) / 4u : items, (unsigned long long)sms * NEURON_BLOCKS_PER_SM));
     int e = withNeuronShape(r, [&](auto P, auto C) -> int {
-        CUDA_TRY(chain(r, neuronUpdateKernel<decltype(P)::value, decltype(C)::value>, grid, NEURON_BLOCK, 0, L));
+        // (with many inputs or sources four words would not fit the registers)
+        if constexpr(decltype(P)::value + decltype(C)::value <= 4) {
+            if(four) {
+                CUDA_TRY(chain(r, neuronUpdateKernel<decltype(P)::value, decltype(C)::value, 4>, grid, NEURON_BLOCK, 0, L));
+                return B200_OK;
+            }
+        }
+        const dim3 all((unsigned int)std::min<unsigned long long>(items, (unsigned long long)sms * NEURON_BLOCKS_PER_SM));
+        CUDA_TRY(chain(r, neuronUpdateKernel<decltype(P)::value, decltype(C)::value, 1>, all, NEURON_BLOCK, 0, L));
         return B200_OK;
     });
     if(e) return e;
