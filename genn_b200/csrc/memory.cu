@@ -32,7 +32,7 @@ size_t hostClass(size_t bytes)
 }
 
 // Page-locked chunks through which a large pull passes.
-constexpr size_t CHUNK = 512 * 1024;
+constexpr size_t CHUNK = 256 * 1024;
 // (40 + 20 MB into fresh pageable memory, whose page faults bound it, on 16 cores: 9.3 ms of a whole load and pull with 6
 // threads, 8.3 with 8, 7.4 with 12, 7.0 with 16; populating the pages ahead with one call per chunk made it slower)
 constexpr unsigned int MOST_THREADS = 16;
@@ -122,19 +122,33 @@ cudaError_t hostAcquire(void **p, size_t bytes)
 void hostRelease(void *p)
 {
     if(!p) return;
+    // what was used last is likeliest to be used next: it stays, and other idle blocks, the largest first, make room for it
+    std::vector<void*> out;
     {
         std::lock_guard<std::mutex> lock(g_hostMutex);
         auto it = g_hostAll.find(p);
-        if(it != g_hostAll.end()) {
-            if(g_hostIdleBytes + it->second <= HOST_KEEP) {
-                g_hostIdle.emplace(it->second, p);
-                g_hostIdleBytes += it->second;
-                return;
-            }
-            g_hostAll.erase(it);
+        if(it == g_hostAll.end()) return;
+        const size_t c = it->second;
+        while(!g_hostIdle.empty() && g_hostIdleBytes + c > HOST_KEEP) {
+            auto largest = std::prev(g_hostIdle.end());
+            out.push_back(largest->second);
+            g_hostIdleBytes -= largest->first;
+            g_hostIdle.erase(largest);
         }
+        if(c <= HOST_KEEP) {
+            g_hostIdle.emplace(c, p);
+            g_hostIdleBytes += c;
+        }
+        else out.push_back(p);
+        for(void *q : out) g_hostAll.erase(q);
     }
-    cudaFreeHost(p);
+    for(void *q : out) cudaFreeHost(q);
+}
+
+bool hostOwned(const void *p)
+{
+    std::lock_guard<std::mutex> lock(g_hostMutex);
+    return g_hostAll.count(const_cast<void*>(p)) != 0;
 }
 
 cudaError_t pullLarge(void *host, const void *device, size_t count, unsigned int elemBytes, bool widen, int deviceIndex, cudaStream_t stream)

@@ -2118,8 +2118,8 @@ int b200_array_alloc(b200_runner *r, size_t bytes, void **device_ptr)
 
 int b200_host_alloc(b200_runner *r, size_t bytes, void **host_ptr)
 {
-    if(!r || !host_ptr) return fail(B200_ERR_INVALID, "bad arguments to b200_host_alloc");
-    CUDA_TRY(cudaSetDevice(r->device));
+    if(!host_ptr) return fail(B200_ERR_INVALID, "bad arguments to b200_host_alloc");
+    if(r) CUDA_TRY(cudaSetDevice(r->device));
     CUDA_TRY(hostAcquire(host_ptr, bytes ? bytes : 1));
     return B200_OK;
 }
@@ -2359,7 +2359,7 @@ int b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t b
         memcpy(host, r->stage, bytes);
         return B200_OK;
     }
-    if(bytes >= LARGE_PULL) {
+    if(bytes >= LARGE_PULL && !hostOwned(host)) {
         CUDA_TRY(pullLarge(host, device_ptr, bytes, 1u, false, r->device, r->stream));
         return B200_OK;
     }

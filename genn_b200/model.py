@@ -168,7 +168,7 @@ class Variable:
         if self._view is None:
             if self._array is None:
                 raise RuntimeError(f"variable '{self.name}' is not loaded")
-            self._view = np.zeros(self.shape, dtype=self.dtype)     # host side made on first use
+            self._view = self._array.host_view(self.shape, self.dtype)     # host side made on first use
         return self._view
 
     @property
