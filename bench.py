@@ -600,7 +600,8 @@ def run_probe(args):
             therefore row lengths unchanged), --probe-fraction of every population marked as having
             spiked, --probe-reps launches of the presynaptic update.  The device holds about
             2.6 GB x scale; one launch reads about scale x fraction x 2.1 GB (twice L2 at the defaults).
-    phases: --probe-warm + --probe-steps time steps of the persistent kernel at natural rates with its
+    phases: --probe-warm + --probe-steps time steps of the persistent kernel (--option use_resident=0 for those with a grid
+    barrier, which alone keep a phase record) at natural rates with its
             clock64 phase counters on.
     e2e:    where one GeNNModel.step_time + recording pull spends its time.
     dense:  batched DENSE presynaptic update, this library's row gather beside the same update as a contraction
@@ -848,6 +849,8 @@ def main():
         opt_name, opt_value = item.split("=")
         rt.set_option(opt_name, float(opt_value))
     bpe = bytes_per_event(net)
+    # (asking builds the target-resident kernel's tables, if that is the one that runs)
+    resident = bool(rt.counter("resident"))
 
     def barrier():
         if world > 1:
@@ -907,6 +910,7 @@ def main():
         rates[p.name] = round(len(ids) / max(1, n_local) / (block * DT_MS * 1e-3), 3)
 
     # ---- where a step's time goes inside the persistent kernel (clock64 per phase, CTA 0) ---
+    # (the target-resident kernel keeps no such record: phase_cycles stays empty)
     probe_steps = min(args.steps * block, 2000)
     rt.set_option("fused_profile", 1)
     names = ["cycles_presynaptic", "cycles_barrier_a", "cycles_neuron", "cycles_barrier_b"] + [f"probe{i}" for i in range(12)]
@@ -917,9 +921,9 @@ def main():
     rt.synchronize()
     barrier()
     pev, psp = rt.counter("synaptic_events") - pev0, rt.counter("spikes") - psp0
-    phase_cycles = {n: (rt.counter(n) - b) / probe_steps for n, b in zip(names, before)}
+    phase_cycles = {} if resident else {n: (rt.counter(n) - b) / probe_steps for n, b in zip(names, before)}
     cta = rt.cta_cycles().astype(np.float64) / probe_steps
-    if len(cta):
+    if len(cta) and not resident:
         # spike-header wait (counts and first ids of every source) inside the presynaptic phase, per CTA
         head = np.asarray(rt.header_cycles, dtype=np.float64) / probe_steps
         phase_cycles["header_median"] = float(np.median(head))
@@ -953,20 +957,20 @@ def main():
         launch_bytes = float(ev1 - ev0) * bpe + float(sp1 - sp0) * ALGO_BYTES_PER_SPIKE
         launch_gbs = launch_bytes / seconds / 1e9
         timed_steps = args.steps * block
-        per_step, traffic_note = (captured_traffic("streamStepKernel")
-                                  if (scale == 1.0 and args.min_delay == 0.0 and rt.schedule == 3)
+        step_kernel = "residentStepKernel" if resident else ["fusedStepKernel", "fusedStepKernel", "fusedStepKernel", "streamStepKernel"][rt.schedule]
+        per_step, traffic_note = (captured_traffic(step_kernel)
+                                  if (scale == 1.0 and args.min_delay == 0.0 and step_kernel in ("residentStepKernel", "streamStepKernel"))
                                   else (None, "no capture for this configuration"))
         traffic = per_step * timed_steps if per_step is not None else None
-        roofline = {"kernel": ["fusedStepKernel", "fusedStepKernel", "fusedStepKernel", "streamStepKernel"][rt.schedule]
-                              + f" (persistent: {timed_steps} time steps in one launch)",
+        roofline = {"kernel": step_kernel + f" (persistent: {timed_steps} time steps in one launch)",
                     "bound": "hbm", "achieved": launch_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": launch_gbs / hbm_peak,
                     "traffic": traffic, "peak_source": peak_kind, "launches": 1, "avg_launch_ms": ms,
                     "algorithmic_bytes_per_launch": launch_bytes,
                     "persistent_kernel_phase_cycles_per_step": phase_cycles,
                     "per_kernel_path": per_kernel,
                     "note": "natural firing rates: about 0.7 MB of synapse rows per time step, so a step is bound by "
-                            "latency (grid barrier, dependent loads), not by HBM; roofline_saturated shows the same "
-                            "delivery code with enough spikes to be bandwidth-relevant.  traffic: " + traffic_note}
+                            "latency (the exchange of the step's spikes, dependent loads), not by HBM; roofline_saturated shows "
+                            "SPARSE delivery with enough spikes to be bandwidth-relevant.  traffic: " + traffic_note}
     else:
         # a sharded model runs on the persistent kernel only: its presynaptic phase is timed with clock64
         pre_s = phase_cycles["cycles_presynaptic"] * probe_steps / sm_hz
@@ -1041,7 +1045,9 @@ def main():
                                    f"published in-degrees, SPARSE with dendritic delays, PoissonExp background, "
                                    f"dt=0.1 ms; one bench step = {block} time steps ({block * 1e-4:g} s biological)",
                        "parallelism": f"postsynaptic sharding over {world} GPU(s)" if world > 1 else "single GPU",
-                       "schedule": ["persistent kernel, every synapse delivered before the neuron update",
+                       "schedule": "target-resident persistent kernel: neurons, input buffers and delay rings stay in one CTA, spikes "
+                                   "travel as tagged messages; no grid barrier" if resident else
+                                   ["persistent kernel, every synapse delivered before the neuron update",
                                     "persistent kernel, split delivery: synapses that arrive in the same step before the "
                                     "neuron update, all others behind it in the shadow of the second grid barrier",
                                     "persistent kernel, spikes delivered one step late (no synapse arrives in the same "
