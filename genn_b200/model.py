@@ -169,6 +169,7 @@ class Variable:
             if self._array is None:
                 raise RuntimeError(f"variable '{self.name}' is not loaded")
             self._view = self._array.host_view(self.shape, self.dtype)     # host side made on first use
+            self._address = self._view.ctypes.data      # (asking numpy for it takes as long as the call that uses it)
         return self._view
 
     @property
@@ -183,7 +184,8 @@ class Variable:
         self._array.push(self.view)
 
     def pull_from_device(self):
-        self._array.pull(self.view)
+        view = self.view
+        self._array.pull_to(self._address, view.nbytes)
 
     @property
     def device_pointer(self) -> int:

@@ -68,6 +68,11 @@ class DeviceArray:
     def push(self, host: np.ndarray):
         self._rt.push(self, host)
 
+    def pull_to(self, address: int, nbytes: int):
+        rt = self._rt
+        check(rt.lib.b200_array_pull(rt.handle, address, self.ptr, nbytes))
+        rt.d2h_bytes += nbytes
+
     def host_view(self, shape, dtype) -> np.ndarray:
         return _host_view(self._rt, shape, np.dtype(dtype))
 
