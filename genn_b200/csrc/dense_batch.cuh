@@ -6,12 +6,13 @@
 // source neuron (bit b: copy b spiked) and gathers the sources that have one into a list.  The listed rows pass through a
 // ring of DENSE_STAGES stages of 32 rows in shared memory (two CTAs on an SM: 128 KB under way, several times what HBM's
 // latency wants); one warp sends for them, a row a lane, as bulk copies, and the others fall behind one another by as much
-// as the ring holds (with a barrier per stage every stage took as long as its busiest warp).  A warp owns copies: a ballot over the masks of
-// a stage's rows gives the rows its copy needs, which it sums in registers, so that sums cost neither shared memory nor
-// atomics until one 16-byte reduction per four columns at the end.  Instructions decide: sums in shared memory, the masks'
-// bits walked row by row, took 55 us at the size below, stages of half the columns brought in by all threads 42.
+// as the ring holds (with a barrier per stage every stage took as long as its busiest warp).  A warp owns copies: a ballot
+// over the masks of a stage's rows gives the rows its copy needs, which it sums in registers, so that sums cost neither
+// shared memory nor atomics until one 16-byte reduction per four columns at the end.  Instructions decide: sums in shared
+// memory, the masks' bits walked row by row, took 55 us at the size below, stages of half the columns brought in by all
+// threads 42, eight adding warps 33.
 //
-// 8192 x 8192, 32 copies, 25 Hz at 1 ms (149 MB of rows a step): 107 us with presynapticPostSpanKernel, 33 here.
+// 8192 x 8192, 32 copies, 25 Hz at 1 ms (149 MB of rows a step): 107 us with presynapticPostSpanKernel, 32 here.
 #pragma once
 
 #include "common.cuh"
@@ -19,7 +20,7 @@
 
 namespace b200
 {
-constexpr unsigned int DENSE_WARPS = 8;             // warps that add; one more brings the rows in
+constexpr unsigned int DENSE_WARPS = 16;            // warps that add; one more brings the rows in
 constexpr unsigned int DENSE_BLOCK = DENSE_WARPS * 32 + 32;
 constexpr unsigned int DENSE_COLS = 256;            // columns of a CTA: twice four a lane
 constexpr unsigned int DENSE_COPIES = 32;           // copies of a CTA: one mask word
@@ -117,8 +118,11 @@ denseBatchKernel(const DenseLaunch L)
                 }
             }
         }
+        unsigned long long spikes = 0;
+        #pragma unroll
+        for(unsigned int o = 0; o < DENSE_OWN; o++) spikes += n[o];
         if(L.S.count_events && part.y == 0u && part.z == 0u && lane == 0u) {
-            atomicAdd(&L.S.state->synaptic_events, (unsigned long long)(n[0] + n[1] + n[2] + n[3]) * g.num_trg);
+            atomicAdd(&L.S.state->synaptic_events, spikes * g.num_trg);
         }
     }
     __syncthreads();
