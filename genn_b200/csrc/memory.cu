@@ -145,12 +145,6 @@ void hostRelease(void *p)
     for(void *q : out) cudaFreeHost(q);
 }
 
-bool hostOwned(const void *p)
-{
-    std::lock_guard<std::mutex> lock(g_hostMutex);
-    return g_hostAll.count(const_cast<void*>(p)) != 0;
-}
-
 cudaError_t pullLarge(void *host, const void *device, size_t count, unsigned int elemBytes, bool widen, int deviceIndex, cudaStream_t stream)
 {
     const size_t perChunk = CHUNK / elemBytes, chunks = (count + perChunk - 1) / perChunk;

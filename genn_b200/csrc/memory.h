@@ -34,7 +34,6 @@ cudaError_t poolAlloc(T **p, size_t bytes, cudaStream_t stream)
 // Page-locked memory.
 cudaError_t hostAcquire(void **p, size_t bytes);
 void hostRelease(void *p);
-bool hostOwned(const void *p);          // whether `p` is the start of a block that hostAcquire returned
 
 // Copies `count` elements of `elemBytes` (1, 2 or 4; `widen`: stored as 32-bit values) from the device behind what `stream`
 // holds, and waits.

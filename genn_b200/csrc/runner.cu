@@ -665,7 +665,8 @@ int prepare(b200_runner *r)
             // +3: tiles are aligned to the array, not to the row
             sparseStarts.push_back(sparseStarts.back() + (g.row_stride + 3 + PRE_TILE - 1) / PRE_TILE);
         }
-        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src <= DENSE_MOST_SOURCES) {
+        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src <= DENSE_MOST_SOURCES &&
+                (unsigned long long)g.num_src * g.num_trg >= DENSE_LEAST_WEIGHTS) {
             dense.push_back(g);
         }
         else if(g.connectivity == B200_CONN_BITMASK || g.connectivity == B200_CONN_DENSE) {
@@ -2118,9 +2119,23 @@ int b200_array_alloc(b200_runner *r, size_t bytes, void **device_ptr)
 
 int b200_host_alloc(b200_runner *r, size_t bytes, void **host_ptr)
 {
-    if(!host_ptr) return fail(B200_ERR_INVALID, "bad arguments to b200_host_alloc");
-    if(r) CUDA_TRY(cudaSetDevice(r->device));
+    if(!r || !host_ptr) return fail(B200_ERR_INVALID, "bad arguments to b200_host_alloc");
+    CUDA_TRY(cudaSetDevice(r->device));
     CUDA_TRY(hostAcquire(host_ptr, bytes ? bytes : 1));
+    return B200_OK;
+}
+
+int b200_host_register(void *host_ptr, size_t bytes)
+{
+    const cudaError_t e = cudaHostRegister(host_ptr, bytes, cudaHostRegisterPortable);
+    if(e == cudaSuccess) return B200_OK;
+    cudaGetLastError();         // (a page that is locked already, say: not an error of anything that follows)
+    return fail(B200_ERR_CUDA, "%s (page-locking %llu bytes)", cudaGetErrorString(e), (unsigned long long)bytes);
+}
+
+int b200_host_unregister(void *host_ptr)
+{
+    CUDA_TRY(cudaHostUnregister(host_ptr));
     return B200_OK;
 }
 
@@ -2359,7 +2374,7 @@ int b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t b
         memcpy(host, r->stage, bytes);
         return B200_OK;
     }
-    if(bytes >= LARGE_PULL && !hostOwned(host)) {
+    if(bytes >= LARGE_PULL) {
         CUDA_TRY(pullLarge(host, device_ptr, bytes, 1u, false, r->device, r->stream));
         return B200_OK;
     }

@@ -161,6 +161,7 @@ class Variable:
         self.init = init
         self.shape = tuple(shape)
         self._view: Optional[np.ndarray] = None
+        self._pulls = 0
         self._array = None      # runtime.DeviceArray once loaded
 
     @property
@@ -168,7 +169,7 @@ class Variable:
         if self._view is None:
             if self._array is None:
                 raise RuntimeError(f"variable '{self.name}' is not loaded")
-            self._view = self._array.host_view(self.shape, self.dtype)     # host side made on first use
+            self._view = np.zeros(self.shape, dtype=self.dtype)     # host side made on first use
             self._address = self._view.ctypes.data      # (asking numpy for it takes as long as the call that uses it)
         return self._view
 
@@ -186,6 +187,9 @@ class Variable:
     def pull_from_device(self):
         view = self.view
         self._array.pull_to(self._address, view.nbytes)
+        self._pulls += 1
+        if self._pulls == 16:           # (worth page-locking it: see runtime.lock_view)
+            self._array.lock(view)
 
     @property
     def device_pointer(self) -> int:

@@ -20,41 +20,38 @@ from .plan import ArrayFactory, Plan
 from .resolve import Net, resolve
 
 
-# Host views of device arrays in page-locked memory, which the device writes by itself: a pull of 1 MB takes 25 us instead of
-# the 100 of the driver's way into pageable memory.  Below VIEW_LEAST bytes the library's staging buffer is as fast, above
-# VIEW_MOST page-locking (1 ms a MB, once) takes longer than several threads' copies do in many pulls; VIEW_TOTAL bounds what is page-locked at a time.
+# A host view that is pulled again and again is page-locked where it lies, so that the device writes it by itself: a pull of
+# 1 MB takes 25 us instead of the 90 of the driver's way into pageable memory.  Page-locking takes 1 to 3 ms, which sixteen
+# pulls show to be worth it.  Below VIEW_LEAST bytes the library's staging buffer is as fast, above VIEW_MOST
+# page-locking costs more than it gives; VIEW_TOTAL bounds what is page-locked at a time.
 VIEW_LEAST, VIEW_MOST, VIEW_TOTAL = 256 * 1024, 1 << 20, 32 << 20
 _view_lock = threading.Lock()
 _view_bytes = 0
 
 
-def _release_view(lib, ptr: int, nbytes: int):
+def _unlock_view(lib, address: int, nbytes: int):
     global _view_bytes
+    lib.b200_host_unregister(address)
     with _view_lock:
         _view_bytes -= nbytes
-    lib.b200_host_free(None, ptr)
 
 
-def _host_view(factory, shape, dtype) -> np.ndarray:
-    """Zeros, page-locked if the array's size is worth it; the memory goes back when the last view of it does."""
+def lock_view(view: np.ndarray):
+    """Page-locks a view's memory (if its size is worth it and there is room) until the view goes."""
     global _view_bytes
-    nbytes = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
-    if VIEW_LEAST < nbytes <= VIEW_MOST:
+    if not VIEW_LEAST < view.nbytes <= VIEW_MOST:
+        return
+    with _view_lock:
+        if _view_bytes + view.nbytes > VIEW_TOTAL:
+            return
+        _view_bytes += view.nbytes
+    lib, address = abi.load_library(), view.ctypes.data
+    if lib.b200_host_register(address, view.nbytes) == 0:
+        # (slices of the view hold it; the reference is cleared before its memory is freed)
+        weakref.finalize(view, _unlock_view, lib, address, view.nbytes).atexit = False
+    else:
         with _view_lock:
-            room = _view_bytes + nbytes <= VIEW_TOTAL
-            if room:
-                _view_bytes += nbytes
-        if room:
-            p = C.c_void_p()
-            if factory.lib.b200_host_alloc(None, nbytes, C.byref(p)) == 0:
-                buffer = (C.c_byte * nbytes).from_address(p.value)
-                weakref.finalize(buffer, _release_view, factory.lib, p.value, nbytes).atexit = False
-                view = np.frombuffer(buffer, dtype=dtype).reshape(shape)
-                view[...] = 0
-                return view
-            with _view_lock:
-                _view_bytes -= nbytes
-    return np.zeros(shape, dtype=dtype)
+            _view_bytes -= view.nbytes
 
 
 class DeviceArray:
@@ -68,16 +65,13 @@ class DeviceArray:
     def push(self, host: np.ndarray):
         self._rt.push(self, host)
 
+    def lock(self, view: np.ndarray):
+        lock_view(view)
+
     def pull_to(self, address: int, nbytes: int):
         rt = self._rt
         check(rt.lib.b200_array_pull(rt.handle, address, self.ptr, nbytes))
         rt.d2h_bytes += nbytes
-
-    def host_view(self, shape, dtype) -> np.ndarray:
-        return _host_view(self._rt, shape, np.dtype(dtype))
-
-    def pull(self, host: np.ndarray):
-        self._rt.pull(self, host)
 
 
 class DeviceFactory(ArrayFactory):

@@ -238,6 +238,9 @@ int  b200_array_free(b200_runner *r, void *device_ptr);
 /* Page-locked host memory for the host side of an array (the reference's Array::allocate
  * uses cudaHostAlloc, src/genn/backends/cuda/backend.cc:88-101). */
 int  b200_host_alloc(b200_runner *r, size_t bytes, void **host_ptr);
+/* Page-locks memory of the caller's where it lies; to be undone before that memory is freed. */
+int  b200_host_register(void *host_ptr, size_t bytes);
+int  b200_host_unregister(void *host_ptr);
 int  b200_host_free(b200_runner *r, void *host_ptr);
 int  b200_array_push(b200_runner *r, void *device_ptr, const void *host, size_t bytes);
 int  b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t bytes);

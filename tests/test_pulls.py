@@ -33,3 +33,26 @@ def test_pull(runner, dtype, nbytes):
     abi.check(lib.b200_array_free(handle, ptr))
     np.testing.assert_array_equal(got, want)
     np.testing.assert_array_equal(wide, want.astype(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [65536, 65537, 262144, 262145])
+def test_a_view_pulled_often_stays_right_and_outlives_its_model(n):
+    from genn_b200 import GeNNModel
+    m = GeNNModel("float", "views")
+    m.dt = 1.0
+    pop = m.add_neuron_population("pop", n, "LIF", {"C": 1.0, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.0,
+                                                    "TauRefrac": 2.0}, {"V": -65.0, "RefracTime": 0.0})
+    m.build()
+    m.load()
+    v = pop.vars["V"]
+    for i in range(20):
+        v.view[...] = np.arange(n, dtype=np.float32) + i
+        v.push_to_device()
+        v.view[...] = 0.0
+        v.pull_from_device()
+        np.testing.assert_array_equal(v.view, np.arange(n, dtype=np.float32).reshape(v.view.shape) + i)
+    part = v.view.reshape(-1)[1:]
+    m.unload()
+    del m, pop, v
+    np.testing.assert_array_equal(part, np.arange(1, n, dtype=np.float32) + 19)
