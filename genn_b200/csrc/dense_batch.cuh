@@ -31,8 +31,10 @@ constexpr unsigned int DENSE_WAITS = 1u << 18;      // polls for a stage before 
 constexpr unsigned int DENSE_WINDOW = 1024;         // most source neurons of a CTA (masks and list: 6 KB)
 // A CTA reads all spike lists to find its own sources: worth it while those are a small part of what it reads of the rows.
 constexpr unsigned int DENSE_MOST_SOURCES = 65536;
-// Below this many weights a copy's few rows are read before the masks are made (67 000 weights, 8 copies: 1 % slower).
-constexpr unsigned int DENSE_LEAST_WEIGHTS = 128 * 1024;
+// With fewer sources a thread per column that walks a copy's few spikes one after another is done before the masks are made:
+// a step of 2 / 8 / 32 copies takes 7.7 / 7.7 / 8.6 us with it and 7.9 / 8.4 / 9.7 here at 600 x 2400, but 9.1 / 9.6 / 10.2
+// against 7.6 / 8.3 / 9.9 at 1200 x 1200 and 12.9 / 13.3 / 14.2 against 7.7 / 8.3 / 9.6 at 2400 x 600.
+constexpr unsigned int DENSE_LEAST_SOURCES = 1024;
 
 struct DenseLaunch
 {

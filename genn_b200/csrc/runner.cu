@@ -665,8 +665,8 @@ int prepare(b200_runner *r)
             // +3: tiles are aligned to the array, not to the row
             sparseStarts.push_back(sparseStarts.back() + (g.row_stride + 3 + PRE_TILE - 1) / PRE_TILE);
         }
-        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src <= DENSE_MOST_SOURCES &&
-                (unsigned long long)g.num_src * g.num_trg >= DENSE_LEAST_WEIGHTS) {
+        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src >= DENSE_LEAST_SOURCES &&
+                g.num_src <= DENSE_MOST_SOURCES) {
             dense.push_back(g);
         }
         else if(g.connectivity == B200_CONN_BITMASK || g.connectivity == B200_CONN_DENSE) {
