@@ -1043,6 +1043,13 @@ bool touchesSparse(const b200_runner *r, const void *p, size_t bytes)
     return false;
 }
 
+// [p, p + bytes) gets other values: the private copies made from it have to be made again before they are next used.
+void arrayWritten(b200_runner *r, const void *p, size_t bytes)
+{
+    if(touchesDelays(r, p, bytes)) { r->lagStale = true; r->nearDataStale = true; }
+    if(touchesSparse(r, p, bytes)) r->tiledStale = r->residentStale = true;
+}
+
 int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long numRec)
 {
     if(r->lagStale) {
@@ -2359,8 +2366,7 @@ int b200_array_push(b200_runner *r, void *device_ptr, const void *host, size_t b
 {
     CUDA_TRY(cudaMemcpyAsync(device_ptr, host, bytes, cudaMemcpyHostToDevice, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
-    if(touchesDelays(r, device_ptr, bytes)) { r->lagStale = true; r->nearDataStale = true; }
-    if(touchesSparse(r, device_ptr, bytes)) r->tiledStale = r->residentStale = true;
+    arrayWritten(r, device_ptr, bytes);
     return B200_OK;
 }
 
@@ -2394,8 +2400,7 @@ int b200_array_pull_u32(b200_runner *r, uint32_t *host, const void *device_ptr, 
 int b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes)
 {
     CUDA_TRY(cudaMemsetAsync(device_ptr, value, bytes, r->stream));
-    if(touchesDelays(r, device_ptr, bytes)) { r->lagStale = true; r->nearDataStale = true; }
-    if(touchesSparse(r, device_ptr, bytes)) r->tiledStale = r->residentStale = true;
+    arrayWritten(r, device_ptr, bytes);
     return B200_OK;
 }
 
@@ -2762,6 +2767,11 @@ static int runCustomUpdate(b200_runner *r, const char *name, unsigned int phases
     ScopedTimer tm(r, std::string("custom_update_") + name, false);
     const bool combine = r->ncclComm && r->ncclWorld > 1 && phases == 3u;
     auto blocksFor = [](uint64_t n) { return (unsigned int)std::min<uint64_t>((n + REDUCE_BLOCK - 1) / REDUCE_BLOCK, 148u * 16u); };
+    // (a write-back changes the variable itself: weights, say, that private copies hold)
+    for(const auto &u : it->second) {
+        arrayWritten(r, u.target, sizeof(float) * u.num_elements);
+        if(u.broadcast && (phases & 2u)) arrayWritten(r, u.source, sizeof(float) * u.num_elements * r->batch);
+    }
     if(!combine) {
         for(const auto &u : it->second) {
             if(u.num_elements == 0) continue;

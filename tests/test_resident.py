@@ -128,3 +128,43 @@ def test_pushed_weights_reach_the_private_copy():
     helpers.assert_close(rt.array("psm0.out_post")[0], other.array("psm0.out_post")[0], "out_post after a weight push", 1e-5, 2e-6)
     rt.close()
     other.close()
+
+
+def _weights_reduced(ring):
+    """A batch-1 network whose weights a custom update halves."""
+    rng = np.random.default_rng(5)
+    m = GeNNModel("float", "reduced")
+    m.dt = 1.0
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.3, "TauRefrac": 2.0}
+    pops = [m.add_neuron_population(n, 200, "LIF", lif, {"V": rng.uniform(-65, -50, 200).astype(np.float32), "RefracTime": 0.0}) for n in "ab"]
+    params = {"g": rng.uniform(0, 2e-3, 4000).astype(np.float32)}
+    if ring:
+        params["d"] = rng.integers(0, 4, 4000).astype(np.uint8)
+    sg = m.add_synapse_population("syn", "SPARSE", *pops, init_weight_update("StaticPulseDendriticDelay" if ring else "StaticPulse", {}, params),
+                                  init_postsynaptic("ExpCurr", {"tau": 5.0}))
+    sg.set_sparse_connections(np.repeat(np.arange(200, dtype=np.uint32), 20), rng.integers(0, 200, 4000).astype(np.uint32))
+    if ring:
+        sg.max_dendritic_delay_timesteps = 4
+    m.add_custom_update("halved", "train", "SUM", (sg, "g"), broadcast=True, scale=0.5)
+    m.build()
+    m.load()
+    return m
+
+
+@pytest.mark.parametrize("options", [{}, {"use_resident": 0}], ids=["resident", "grid barrier"])
+@pytest.mark.parametrize("ring", [False, True])
+def test_weights_changed_by_a_custom_update_reach_the_private_copies(ring, options):
+    """The paths that deliver out of private copies against the one that reads the arrays."""
+    runs = [(_weights_reduced(ring), o) for o in (options, {"use_fused": 0, "use_tiled": 0})]
+    for m, opts in runs:
+        for k, v in opts.items():
+            m._runtime.set_option(k, v)
+        m.step_time(30)
+        for _ in range(3):
+            m.custom_update("train")
+            m.step_time(15)
+    got, want = (m._runtime.array("psm0.out_post")[0] for m, _ in runs)
+    assert np.abs(want).max() > 0
+    helpers.assert_close(got, want, "out_post after custom updates", 1e-5, 2e-6)
+    for m, _ in runs:
+        m.unload()
