@@ -303,6 +303,8 @@ struct b200_runner
 
     // target-resident kernel (resident.h): private copy of the SPARSE groups cut by CTA, message buffers
     bool useResident = true;
+    bool residentAsked = false;             // the caller asked for it by name (and says so when it writes an exposed array)
+    std::vector<void*> exposed;             // arrays that the program writes by itself (b200_array_expose)
     bool tiledChosen = false;               // the caller set what arms the tiled kernels: they serve whatever they can
     bool scheduleChosen = false;            // the caller picked a schedule of the other persistent kernels
     bool residentStale = true, residentReady = false;
@@ -1752,6 +1754,8 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
 int chooseResident(b200_runner *r, bool *yes)
 {
     *yes = false;
+    // (a private copy would not see what the program writes into an array by itself)
+    for(void *p : r->exposed) if(!r->residentAsked && touchesSparse(r, p, 1)) return B200_OK;
     if(!r->useFused || !r->useResident || r->scheduleChosen || r->timing || r->sharded() || r->batch != 1) return B200_OK;
     if(r->residentStale) {
         if(const int e = buildResident(r)) { r->dropResident(); return e; }
@@ -2359,6 +2363,7 @@ int b200_array_free(b200_runner *r, void *device_ptr)
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     CUDA_TRY(poolFree(device_ptr, r->stream));
     r->arrays.erase(it);
+    r->exposed.erase(std::remove(r->exposed.begin(), r->exposed.end(), device_ptr), r->exposed.end());
     return B200_OK;
 }
 
@@ -2401,6 +2406,13 @@ int b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes)
 {
     CUDA_TRY(cudaMemsetAsync(device_ptr, value, bytes, r->stream));
     arrayWritten(r, device_ptr, bytes);
+    return B200_OK;
+}
+
+int b200_array_expose(b200_runner *r, void *device_ptr)
+{
+    if(!r || r->arrays.find(device_ptr) == r->arrays.end()) return fail(B200_ERR_INVALID, "pointer was not allocated by this runner");
+    if(std::find(r->exposed.begin(), r->exposed.end(), device_ptr) == r->exposed.end()) r->exposed.push_back(device_ptr);
     return B200_OK;
 }
 
@@ -2506,7 +2518,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
     else if(n == "count_events") r->countEvents = (value != 0.0);
     else if(n == "use_graph") r->useGraph = (value != 0.0);
     else if(n == "use_fused") r->useFused = (value != 0.0);
-    else if(n == "use_resident") { r->useResident = (value != 0.0); r->scheduleChosen = false; }
+    else if(n == "use_resident") { r->useResident = r->residentAsked = (value != 0.0); r->scheduleChosen = false; }
     else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; }
     else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; }
     else if(n == "use_lag") { r->useLag = (value != 0.0); r->lagStale = true; }
@@ -2519,7 +2531,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
     else if(n == "use_emit") { r->useEmit = (value != 0.0); r->lagStale = true; }
     else if(n == "stream_warps") { r->streamWarpsWanted = (int)value; r->lagStale = true; }
     else if(n == "lag_agreed") { r->lagAgreed = (value != 0.0); r->lagStale = true; }
-    else if(n == "rescan_delays") r->lagStale = true;
+    else if(n == "rescan_delays") r->lagStale = r->tiledStale = r->residentStale = true;
     else if(n == "fused_profile") {
         // (the per-CTA cycle counters are allocated here, not on the time-step path)
         r->fusedProfile = (value != 0.0);

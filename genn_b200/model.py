@@ -193,7 +193,7 @@ class Variable:
 
     @property
     def device_pointer(self) -> int:
-        return self._array.ptr
+        return self._array.expose()
 
 
 class NeuronGroup:

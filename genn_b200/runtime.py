@@ -68,6 +68,11 @@ class DeviceArray:
     def lock(self, view: np.ndarray):
         lock_view(view)
 
+    def expose(self) -> int:
+        """The array's address, for a program that may write it by itself (include/genn_b200.h: b200_array_expose)."""
+        check(self._rt.lib.b200_array_expose(self._rt.handle, self.ptr))
+        return self.ptr
+
     def pull_to(self, address: int, nbytes: int):
         rt = self._rt
         check(rt.lib.b200_array_pull(rt.handle, address, self.ptr, nbytes))

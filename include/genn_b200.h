@@ -247,6 +247,10 @@ int  b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t 
 /* An array of 8-, 16- or 32-bit indices, as 32-bit values. */
 int  b200_array_pull_u32(b200_runner *r, uint32_t *host, const void *device_ptr, uint32_t elem_bytes, uint64_t count);
 int  b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes);
+/* The program will write this array by itself (its own kernels or copies, not b200_array_push).  The target-resident kernel
+ * works on a private copy of the SPARSE groups' arrays and is not chosen while one of them is exposed, unless option
+ * "use_resident" asks for it; the program then says "rescan_delays" behind everything it writes. */
+int  b200_array_expose(b200_runner *r, void *device_ptr);
 /* Spike recordings are one bit per neuron and time step and almost all zeros (Runtime::pullRecordingBuffersFromDevice,
  * runtime.cc:720-746, copies them whole).  This appends the non-zero 32-bit words of `words` to `pairs` as
  * (base_index + word index, word), 8 bytes each, on the runner's stream; `counter` (a device word the caller has
@@ -378,8 +382,9 @@ int  b200_get_counter(b200_runner *r, const char *name, uint64_t *value);
  * "use_lag" (default 1: when no synapse has dendritic delay 0 the persistent kernel delivers each spike one
  * step later into the ring slot one nearer, same result, one grid barrier per step instead of two),
  * "lag_agreed" (sharded model: the caller has checked "lag_eligible" on EVERY process; without it a sharded
- * model keeps the two-barrier schedule), "rescan_delays" (delay arrays were changed by something other than
- * this library's push / init calls), "use_near_queues" (default 1: a sharded model on the
+ * model keeps the two-barrier schedule), "rescan_delays" (connectivity, weights or delays of a SPARSE group were
+ * changed by something other than this library's push, memset, init and custom update calls: every private copy is made
+ * again, see b200_array_expose), "use_near_queues" (default 1: a sharded model on the
  * "deliver at emission" schedule sends near synapses between processes through per-CTA queues of self-validating
  * words; 0: reduces them straight into the other process's rings and fences) / "near_queue_words" (capacity of
  * one queue, 2 .. 2048; what does not fit goes the direct way), "use_tiled" / "tiled_min_events" (target-tiled SPARSE delivery of steps

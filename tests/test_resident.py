@@ -168,3 +168,57 @@ def test_weights_changed_by_a_custom_update_reach_the_private_copies(ring, optio
     helpers.assert_close(got, want, "out_post after custom updates", 1e-5, 2e-6)
     for m, _ in runs:
         m.unload()
+
+
+def _delivering(seed=8):
+    """A batch-1 SPARSE network that fires in every few steps; its weights do not learn."""
+    rng = np.random.default_rng(seed)
+    m = GeNNModel("float", "delivering")
+    m.dt = 1.0
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.3, "TauRefrac": 2.0}
+    pops = [m.add_neuron_population(n, 200, "LIF", lif, {"V": rng.uniform(-65, -50, 200).astype(np.float32), "RefracTime": 0.0}) for n in "ab"]
+    sg = m.add_synapse_population("syn", "SPARSE", *pops, init_weight_update("StaticPulse", {}, {"g": rng.uniform(0, 2e-3, 4000).astype(np.float32)}),
+                                  init_postsynaptic("ExpCurr", {"tau": 5.0}))
+    sg.set_sparse_connections(np.repeat(np.arange(200, dtype=np.uint32), 20), rng.integers(0, 200, 4000).astype(np.uint32))
+    m.build()
+    m.load()
+    return m, sg
+
+
+class _Foreign:
+    """Device memory of the library's as another one sees it."""
+
+    def __init__(self, pointer, shape):
+        self.__cuda_array_interface__ = {"data": (pointer, False), "shape": shape, "typestr": "<f4", "version": 3}
+
+
+@pytest.mark.parametrize("asked", [False, True])
+def test_weights_written_through_the_device_pointer_reach_the_step(asked):
+    """By default the next step sees them; a program that asks for the target-resident kernel all the same says when it wrote."""
+    import torch
+    (m, sg), (other, _) = _delivering(), _delivering()
+    other._runtime.set_option("use_fused", 0)
+    other._runtime.set_option("use_tiled", 0)
+    rt = m._runtime
+    assert rt.counter("resident") == 1
+    m.neuron_populations["b"].vars["V"].device_pointer          # (neuron state is read and written where it lies)
+    assert rt.counter("resident") == 1
+    if asked:
+        rt.set_option("use_resident", 1)
+    for x in (m, other):
+        x.step_time(30)
+    weights = [torch.as_tensor(_Foreign(x.synapse_populations["syn"].vars["g"].device_pointer, sg.vars["g"].shape), device="cuda") for x in (m, other)]
+    assert rt.counter("resident") == (1 if asked else 0)
+    for _ in range(3):
+        for x, w in zip((m, other), weights):
+            x._runtime.synchronize()
+            w.mul_(0.5)
+            torch.cuda.synchronize()
+            if asked:
+                x._runtime.set_option("rescan_delays", 1)
+            x.step_time(15)
+    got, want = (x._runtime.array("psm0.out_post")[0] for x in (m, other))
+    assert np.abs(want).max() > 0
+    helpers.assert_close(got, want, "out_post", 1e-5, 2e-6)
+    for x in (m, other):
+        x.unload()
