@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -134,6 +135,7 @@ struct b200_runner
     std::unordered_map<void*, size_t> arrays;
     unsigned char *stage = nullptr;         // STAGE_BYTES, page-locked: pulls of small arrays land here
     unsigned int *hostWord = nullptr;       // page-locked: the device's error word
+    std::mutex staging;                     // held by the thread whose transfer uses either
     // recording list (record.cuh): chunk counts, header and pairs on the device, header and pairs on the host
     unsigned int *recCounts = nullptr;
     RecordHeader *recList = nullptr, *recHost = nullptr;
@@ -2380,6 +2382,7 @@ int b200_array_pull(b200_runner *r, void *host, const void *device_ptr, size_t b
     if(bytes <= STAGE_BYTES) {
         // to page-locked memory and on from there: the driver's own way into pageable memory takes 15 us however
         // few the bytes, this one 8 (40 KB)
+        std::lock_guard<std::mutex> lock(r->staging);
         CUDA_TRY(cudaMemcpyAsync(r->stage, device_ptr, bytes, cudaMemcpyDeviceToHost, r->stream));
         CUDA_TRY(cudaStreamSynchronize(r->stream));
         memcpy(host, r->stage, bytes);
@@ -2864,6 +2867,7 @@ static int reportDeviceError(b200_runner *r, unsigned int err)
 
 int b200_synchronize(b200_runner *r)
 {
+    std::lock_guard<std::mutex> lock(r->staging);
     CUDA_TRY(cudaMemcpyAsync(r->hostWord, &r->state->error, sizeof(unsigned int), cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     return reportDeviceError(r, *r->hostWord);
@@ -3151,6 +3155,7 @@ int b200_pull_spikes(b200_runner *r, const uint32_t *count_ptr, const uint32_t *
     if(!r || !count_ptr || !list_ptr || !ids || !num) return fail(B200_ERR_INVALID, "null argument to b200_pull_spikes");
     // count, error word and the first ids in one synchronisation
     const uint32_t first = std::min<uint32_t>(capacity, STAGE_BYTES / sizeof(uint32_t));
+    std::lock_guard<std::mutex> lock(r->staging);
     CUDA_TRY(cudaMemcpyAsync(r->hostWord + 1, count_ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->hostWord, &r->state->error, sizeof(uint32_t), cudaMemcpyDeviceToHost, r->stream));
     if(first) CUDA_TRY(cudaMemcpyAsync(r->stage, list_ptr, sizeof(uint32_t) * first, cudaMemcpyDeviceToHost, r->stream));

@@ -1,5 +1,6 @@
 """Arrays on their way out of the device: every size class, and indices widened on the way."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -56,3 +57,36 @@ def test_a_view_pulled_often_stays_right_and_outlives_its_model(n):
     m.unload()
     del m, pop, v
     np.testing.assert_array_equal(part, np.arange(1, n, dtype=np.float32) + 19)
+
+
+@pytest.mark.gpu
+def test_threads_that_pull_from_one_runner_each_get_their_own(runner):
+    """Small arrays, spike lists and the error word pass through one staging buffer of the runner."""
+    lib, handle = runner
+    wrong, arrays = [], []
+    for k in range(4):
+        want = np.arange(1000 + 900 * k, dtype=np.uint32) + 100000 * k
+        want[0] = want.size - 1         # (as a spike list: the count, then the ids)
+        ptr = C.c_void_p()
+        abi.check(lib.b200_array_alloc(handle, want.nbytes, C.byref(ptr)))
+        abi.check(lib.b200_array_push(handle, ptr, want.ctypes.data, want.nbytes))
+        arrays.append((want, ptr))
+
+    def work(k):
+        want, ptr = arrays[k]
+        n, got, ids, num = want.size, np.zeros_like(want), np.zeros_like(want), C.c_uint32()
+        for _ in range(1500):
+            got[:] = 0
+            abi.check(lib.b200_array_pull(handle, got.ctypes.data, ptr, got.nbytes))
+            abi.check(lib.b200_pull_spikes(handle, ptr.value, ptr.value + 4, n - 1, ids.ctypes.data, C.byref(num)))
+            abi.check(lib.b200_synchronize(handle))
+            if num.value != n - 1 or not np.array_equal(got, want) or not np.array_equal(ids[:n - 1], want[1:]):
+                wrong.append(k)
+                return
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
