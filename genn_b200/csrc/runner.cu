@@ -314,7 +314,7 @@ struct b200_runner
     unsigned int residentCtas = 0, residentWarps = 0;       // 0: chosen by size
     unsigned int residentGrid = 0, residentBlock = 0;
     size_t residentSmem = 0;
-    unsigned long long residentTagged = ~0ull;              // steps since the message buffers were last cleared
+    unsigned long long residentCleared = ~0ull;             // steps done when the message buffers were last cleared (~0: they are not)
     size_t residentMailBytes = 0;
     const void *residentKernel = nullptr;
     ResidentLaunch resident{};
@@ -325,7 +325,7 @@ struct b200_runner
         for(void *p : residentBuffers) poolFree(p, stream);
         residentBuffers.clear();
         residentReady = false;
-        residentTagged = ~0ull;
+        residentCleared = ~0ull;
     }
 
     // options
@@ -1724,7 +1724,8 @@ int buildResident(b200_runner *r)
     return B200_OK;
 }
 
-int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long long numRec)
+// `done`: steps done when the launch begins.
+int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long long numRec, unsigned long long done)
 {
     ResidentLaunch &L = r->resident;
     L.neuron.groups = r->neuronTable.d;
@@ -1739,12 +1740,12 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
     L.neuron.ahead = L.neuron.advance = 0u;
     L.count_events = r->countEvents ? 1u : 0u;
     L.num_steps = (unsigned int)numSteps;
-    // a message word is known by the last 20 bits of its step: before they repeat, no old word may be left
-    if(r->residentTagged == ~0ull || r->residentTagged + numSteps >= RESIDENT_TAG_STEPS - 1ull) {
+    // a message word is known by the last 20 bits of its step: before they repeat, no old word may be left.  (Steps on other
+    // paths count too: they leave the words of earlier steps where they are.)
+    if(r->residentCleared == ~0ull || done + numSteps - r->residentCleared >= RESIDENT_TAG_STEPS - 1ull) {
         CUDA_TRY(cudaMemsetAsync(L.inbox, 0, r->residentMailBytes, r->stream));
-        r->residentTagged = 0;
+        r->residentCleared = done;
     }
-    r->residentTagged += numSteps;
     void *args[] = {&L};
     CUDA_TRY(cudaLaunchCooperativeKernel(r->residentKernel, dim3(r->residentGrid), dim3(r->residentBlock), args, r->residentSmem, r->stream));
     r->launches++;
@@ -2703,7 +2704,7 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
     if(resident) {
         while(left) {
             const uint64_t n = std::min<uint64_t>(left, RESIDENT_TAG_STEPS / 2);
-            e = launchResident(r, n, num_recording_timesteps);
+            e = launchResident(r, n, num_recording_timesteps, r->hostStepsDone + (num_steps - left));
             if(e) return e;
             left -= n;
         }
@@ -2856,7 +2857,7 @@ static int reportDeviceError(b200_runner *r, unsigned int err)
 {
     if(!err) return B200_OK;
     cudaMemsetAsync(&r->state->error, 0, sizeof(unsigned int), r->stream);
-    r->residentTagged = ~0ull;          // (a launch that gave up may have left messages of steps that count again)
+    r->residentCleared = ~0ull;         // (a launch that gave up may have left messages of steps that count again)
     return fail(B200_ERR_DEVICE_CHECK, "device-side check failed (flags 0x%x:%s%s%s%s%s)", err,
                 (err & ERR_SPIKE_OVERFLOW) ? " spike list overflow" : "",
                 (err & ERR_IND_RANGE) ? " index or row length out of range" : "",

@@ -222,3 +222,31 @@ def test_weights_written_through_the_device_pointer_reach_the_step(asked):
     helpers.assert_close(got, want, "out_post", 1e-5, 2e-6)
     for x in (m, other):
         x.unload()
+
+
+def test_messages_of_steps_long_ago_are_not_taken_for_new_ones():
+    """Message words carry the last 20 bits of their step.  Four steps on this path, in the first of which every source fires,
+    then as many on another as bring the same bits (and the same one of the four message buffers) round again."""
+    m = GeNNModel("float", "tags")
+    m.dt = 1.0
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.0, "TauRefrac": 2.0}
+    a = m.add_neuron_population("a", 2368, "LIF", lif, {"V": -40.0, "RefracTime": 0.0})
+    b = m.add_neuron_population("b", 2368, "LIF", dict(lif, Vthresh=1000.0), {"V": -65.0, "RefracTime": 0.0})
+    for delay in (0, 1):
+        sg = m.add_synapse_population(f"syn{delay}", "SPARSE", a, b, init_weight_update("StaticPulseConstantWeight", {"g": 0.1}),
+                                      init_postsynaptic("ExpCurr", {"tau": 5.0}))
+        sg.set_sparse_connections(np.repeat(np.arange(2368, dtype=np.uint32), 20), np.random.default_rng(delay).integers(0, 2368, 47360).astype(np.uint32))
+        sg.axonal_delay_steps = delay
+    rt = _runtime(resolve(m), 10)
+    rt.set_option("resident_ctas", 148)         # (many CTAs, some of which read before others write)
+    assert rt.counter("resident") == 1
+    rt.step_time(4)
+    assert rt.array("psm0.out_post").max() > 1.0 and rt.array("psm1.out_post").max() > 1.0
+    rt.set_option("use_resident", 0)
+    rt.step_time((1 << 20) - 4)
+    rt.set_option("use_resident", 1)
+    rt.set_option("count_events", 1)
+    rt.step_time(8)
+    assert rt.counter("synaptic_events") == 0
+    assert rt.array("psm0.out_post").max() < 1e-30 and rt.array("psm1.out_post").max() < 1e-30
+    rt.close()
