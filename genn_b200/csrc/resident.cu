@@ -715,6 +715,11 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         buf = (buf + 1u == L.buffers) ? 0u : buf + 1u;
         histAt = (histAt + 1u == L.history) ? 0u : histAt + 1u;
         if(++recAt == (unsigned int)L.neuron.num_recording_timesteps) recAt = 0u;
+        // (a lane adds far less than 2^31 events in a step: that many synapses of one CTA do not fit the device)
+        if(L.count_events && (deliver.events >> 24)) {
+            atomicAdd(&state->synaptic_events, (unsigned long long)deliver.events);
+            deliver.events = 0u;
+        }
     }
 
     // ---------------- what the launch leaves in memory ----------------------------------------------------
@@ -775,8 +780,10 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         }
     }
     if(L.count_events) {
-        const unsigned int e = __reduce_add_sync(0xFFFFFFFFu, deliver.events);
-        if(lane == 0 && e) atomicAdd(&state->synaptic_events, (unsigned long long)e);
+        // (halves, so that the sum over a warp does not pass 32 bits)
+        const unsigned long long e = __reduce_add_sync(0xFFFFFFFFu, deliver.events & 0xFFFFu) +
+                                     ((unsigned long long)__reduce_add_sync(0xFFFFFFFFu, deliver.events >> 16) << 16);
+        if(lane == 0 && e) atomicAdd(&state->synaptic_events, e);
         if(spikes) atomicAdd(&state->spikes, (unsigned long long)spikes);
     }
     // (every CTA has sent the message of the last step, so every CTA has read the counters)

@@ -250,3 +250,31 @@ def test_messages_of_steps_long_ago_are_not_taken_for_new_ones():
     assert rt.counter("synaptic_events") == 0
     assert rt.array("psm0.out_post").max() < 1e-30 and rt.array("psm1.out_post").max() < 1e-30
     rt.close()
+
+
+def test_more_events_in_one_launch_than_32_bits_hold():
+    """Every neuron of one CTA fires in every step and reaches every neuron through four groups: 4.9e9 events a warp, 1.5e8
+    a lane."""
+    m = GeNNModel("float", "events")
+    m.dt = 1.0
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 50.0, "TauRefrac": 0.0}
+    n, groups, steps = 128, 4, 300000
+    a = m.add_neuron_population("a", n, "LIF", lif, {"V": -40.0, "RefracTime": 0.0})
+    m.fuse_postsynaptic_models = True
+    for i in range(groups):
+        sg = m.add_synapse_population(f"syn{i}", "BITMASK", a, a, init_weight_update("StaticPulseConstantWeight", {"g": 0.0}),
+                                      init_postsynaptic("ExpCurr", {"tau": 5.0}))
+        sg.set_sparse_connections(np.repeat(np.arange(n, dtype=np.uint32), n), np.tile(np.arange(n, dtype=np.uint32), n))
+    rt = _runtime(resolve(m), 10)
+    rt.set_option("resident_ctas", 1)
+    rt.set_option("resident_warps", 4)
+    assert rt.counter("resident") == 1
+    rt.set_option("count_events", 1)
+    rt.step_time(1)
+    assert rt.counter("spikes") == n and rt.counter("synaptic_events") == 0
+    before = rt.kernel_launches
+    rt.step_time(steps)
+    assert rt.kernel_launches == before + 1
+    assert rt.counter("spikes") == n * (steps + 1)
+    assert rt.counter("synaptic_events") == groups * n * n * steps
+    rt.close()
