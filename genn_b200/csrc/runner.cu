@@ -181,7 +181,6 @@ struct b200_runner
     bool lagAgreed = false;         // sharded model: the host checked that every process is eligible
     bool lagStale = true;           // delay arrays may have changed since the last scan
     bool lagEligible = false;
-    unsigned int *lagScan = nullptr;
     std::vector<b200_synapse_group> fusedGroups;    // host copy of the SPARSE groups the kernel serves
     // split delivery (fused_step.cuh): private tables of the synapses that arrive in the same step
     bool useSplit = true;
@@ -2089,7 +2088,6 @@ int b200_runner_destroy(b200_runner *r)
     poolFree(r->fusedSources, r->stream);
     poolFree(r->fusedItems, r->stream);
     poolFree(r->fusedBarrier, r->stream);
-    poolFree(r->lagScan, r->stream);
     r->dropUrgent();
     r->dropNear();
     poolFree(r->fusedCtaCycles, r->stream);
@@ -2213,7 +2211,7 @@ int b200_exchange_open_peer(b200_runner *r, uint32_t peer_rank, const void *hand
     void *p = nullptr;
     CUDA_TRY(cudaIpcOpenMemHandle(&p, h, cudaIpcMemLazyEnablePeerAccess));
     r->peerArena[peer_rank] = static_cast<unsigned char*>(p);
-    if(!r->peerTable) CUDA_TRY(cudaMalloc(&r->peerTable, sizeof(unsigned char*) * B200_MAX_RANKS));
+    if(!r->peerTable) CUDA_TRY(poolAlloc(&r->peerTable, sizeof(unsigned char*) * B200_MAX_RANKS, r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->peerTable, r->peerArena, sizeof(unsigned char*) * B200_MAX_RANKS, cudaMemcpyHostToDevice, r->stream));
     return B200_OK;
 }
@@ -2224,7 +2222,7 @@ int b200_exchange_set_peer(b200_runner *r, uint32_t peer_rank, void *device_ptr)
     if(r->peerArena[peer_rank]) return fail(B200_ERR_STATE, "peer %u already opened", peer_rank);
     CUDA_TRY(cudaSetDevice(r->device));
     r->peerArena[peer_rank] = static_cast<unsigned char*>(device_ptr);
-    if(!r->peerTable) CUDA_TRY(cudaMalloc(&r->peerTable, sizeof(unsigned char*) * B200_MAX_RANKS));
+    if(!r->peerTable) CUDA_TRY(poolAlloc(&r->peerTable, sizeof(unsigned char*) * B200_MAX_RANKS, r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->peerTable, r->peerArena, sizeof(unsigned char*) * B200_MAX_RANKS, cudaMemcpyHostToDevice, r->stream));
     r->peerLocal[peer_rank] = true;
     return B200_OK;
