@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <thread>
@@ -184,8 +185,14 @@ cudaError_t pullLarge(void *host, const void *device, size_t count, unsigned int
         }
     };
     std::vector<std::thread> helpers;
-    for(unsigned int t = 1; t < threads; t++) helpers.emplace_back(work, t);
+    unsigned int started = 1;
+    try {
+        helpers.reserve(threads);
+        for(; started < threads; started++) helpers.emplace_back(work, started);
+    }
+    catch(const std::exception&) {}         // (no more threads to be had: this one does their part)
     work(0);
+    for(unsigned int t = started; t < threads; t++) work(t);
     for(auto &h : helpers) h.join();
     hostRelease(staged);
     return (cudaError_t)failed.load();
