@@ -169,7 +169,7 @@ class Variable:
         if self._view is None:
             if self._array is None:
                 raise RuntimeError(f"variable '{self.name}' is not loaded")
-            self._view = np.zeros(self.shape, dtype=self.dtype)     # host side made on first use
+            self._view = self._array.new_view(self.shape, self.dtype)       # host side made on first use
             self._address = self._view.ctypes.data      # (asking numpy for it takes as long as the call that uses it)
         return self._view
 

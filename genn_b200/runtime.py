@@ -6,6 +6,7 @@ this module without the built library raises.
 from __future__ import annotations
 
 import ctypes as C
+import mmap
 import threading
 import weakref
 import os
@@ -20,11 +21,12 @@ from .plan import ArrayFactory, Plan
 from .resolve import Net, resolve
 
 
-# A host view that is pulled again and again is page-locked where it lies, so that the device writes it by itself: a pull of
+# A host view that is pulled again and again is page-locked in pages of its own, so that the device writes it by itself: a pull of
 # 1 MB takes 25 us instead of the 90 of the driver's way into pageable memory.  Page-locking takes 1 to 3 ms, which sixteen
 # pulls show to be worth it.  Below VIEW_LEAST bytes the library's staging buffer is as fast, above VIEW_MOST
 # page-locking costs more than it gives; VIEW_TOTAL bounds what is page-locked at a time.
 VIEW_LEAST, VIEW_MOST, VIEW_TOTAL = 256 * 1024, 1 << 20, 32 << 20
+PAGE = mmap.PAGESIZE
 _view_lock = threading.Lock()
 _view_bytes = 0
 
@@ -36,22 +38,35 @@ def _unlock_view(lib, address: int, nbytes: int):
         _view_bytes -= nbytes
 
 
+def page_view(shape, dtype) -> np.ndarray:
+    """Zeros in whole pages of their own: page-locking them touches no neighbour's memory, and no neighbour's theirs."""
+    dtype = np.dtype(dtype)
+    nbytes = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
+    room = np.zeros(-(-nbytes // PAGE) * PAGE + PAGE, dtype=np.uint8)
+    at = -room.ctypes.data % PAGE
+    return room[at:at + nbytes].view(dtype).reshape(shape)
+
+
 def lock_view(view: np.ndarray):
-    """Page-locks a view's memory (if its size is worth it and there is room) until the view goes."""
+    """Page-locks a view made by page_view (if its size is worth it and there is room) until its memory goes."""
     global _view_bytes
-    if not VIEW_LEAST < view.nbytes <= VIEW_MOST:
+    if not VIEW_LEAST < view.nbytes <= VIEW_MOST or view.ctypes.data % PAGE:
         return
+    nbytes = -(-view.nbytes // PAGE) * PAGE
     with _view_lock:
-        if _view_bytes + view.nbytes > VIEW_TOTAL:
+        if _view_bytes + nbytes > VIEW_TOTAL:
             return
-        _view_bytes += view.nbytes
+        _view_bytes += nbytes
     lib, address = abi.load_library(), view.ctypes.data
-    if lib.b200_host_register(address, view.nbytes) == 0:
-        # (slices of the view hold it; the reference is cleared before its memory is freed)
-        weakref.finalize(view, _unlock_view, lib, address, view.nbytes).atexit = False
+    if lib.b200_host_register(address, nbytes) == 0:
+        # (every slice holds the array that owns the memory; its references are cleared before the memory is freed)
+        owner = view
+        while isinstance(owner.base, np.ndarray):
+            owner = owner.base
+        weakref.finalize(owner, _unlock_view, lib, address, nbytes).atexit = False
     else:
         with _view_lock:
-            _view_bytes -= view.nbytes
+            _view_bytes -= nbytes
 
 
 class DeviceArray:
@@ -64,6 +79,10 @@ class DeviceArray:
 
     def push(self, host: np.ndarray):
         self._rt.push(self, host)
+
+    def new_view(self, shape, dtype) -> np.ndarray:
+        nbytes = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+        return page_view(shape, dtype) if VIEW_LEAST < nbytes <= VIEW_MOST else np.zeros(shape, dtype=dtype)
 
     def lock(self, view: np.ndarray):
         lock_view(view)

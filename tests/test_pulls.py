@@ -1,5 +1,6 @@
 """Arrays on their way out of the device: every size class, and indices widened on the way."""
 import ctypes as C
+import mmap
 import threading
 
 import numpy as np
@@ -57,6 +58,52 @@ def test_a_view_pulled_often_stays_right_and_outlives_its_model(n):
     m.unload()
     del m, pop, v
     np.testing.assert_array_equal(part, np.arange(1, n, dtype=np.float32) + 19)
+
+
+class _Registered:
+    """What the library's page-locking calls were given."""
+
+    def __init__(self):
+        self.now, self.ever = {}, []
+
+    def b200_host_register(self, address, nbytes):
+        self.now[address] = nbytes
+        self.ever.append((address, nbytes))
+        return 0
+
+    def b200_host_unregister(self, address):
+        del self.now[address]
+
+
+@pytest.mark.parametrize("n", [65537, 100003, 262144])
+def test_page_locked_views_lie_in_pages_of_their_own_and_are_unlocked_with_their_memory(n, monkeypatch):
+    from genn_b200 import runtime
+    from genn_b200.model import Variable
+    lib = _Registered()
+    monkeypatch.setattr(abi, "load_library", lambda: lib)
+    views = []
+    for i in range(5):
+        v = Variable(f"v{i}", np.float32, None, (1, n))
+        v._array = runtime.DeviceArray.__new__(runtime.DeviceArray)
+        assert v.view.shape == (1, n) and v.view.dtype == np.float32 and not v.view.any()
+        v._array.lock(v.view)
+        views.append(v)
+    assert len(lib.now) == 5 and len(lib.ever) == 5
+    spans = sorted(lib.ever)
+    for (a, na), (b, _) in zip(spans, spans[1:] + [(1 << 63, 0)]):
+        assert a % mmap.PAGESIZE == 0 and na % mmap.PAGESIZE == 0 and na >= 4 * n and a + na <= b
+    for v in views:
+        owner = v.view
+        while isinstance(owner.base, np.ndarray):
+            owner = owner.base
+        at, size = v.view.ctypes.data, lib.now[v.view.ctypes.data]
+        assert owner.ctypes.data <= at and at + size <= owner.ctypes.data + owner.nbytes
+    part = views[0].view.reshape(-1)[10:20]
+    held = views[0].view.ctypes.data
+    del v, owner, views
+    assert list(lib.now) == [held]
+    del part
+    assert not lib.now and runtime._view_bytes == 0
 
 
 @pytest.mark.gpu
