@@ -53,6 +53,7 @@ struct NeuronLaunch
     unsigned int count_events;
     unsigned int ahead;                 // steps of this block of steps that come before this one
     unsigned int advance;               // last kernel of a block of steps: how many it has, else 0
+    unsigned long long peak_groups = ~0ull;     // which of the first 64 groups' spikes count for StepState::peak_spikes
 };
 
 // Loads of data other SMs write between grid barriers (postsynaptic input,
@@ -544,7 +545,9 @@ neuronUpdateKernel(const NeuronLaunch L)
             const b200_neuron_group &o = L.groups[q / L.batch];
             const unsigned int ob = q % L.batch;
             // (the spikes of the step before: this one's are not all there yet)
-            atomicAdd(&stepSpikes, o.spk_cnt[ob * o.num_delay_slots + ringSlot(k, o.num_delay_slots)]);
+            if(q / L.batch >= 64u || ((L.peak_groups >> (q / L.batch)) & 1ull)) {
+                atomicAdd(&stepSpikes, o.spk_cnt[ob * o.num_delay_slots + ringSlot(k, o.num_delay_slots)]);
+            }
             o.spk_cnt[ob * o.num_delay_slots + ringSlot(k + 2, o.num_delay_slots)] = 0;
         }
         __syncthreads();

@@ -149,12 +149,19 @@ struct b200_runner
 
     DeviceTable<b200_neuron_group> neuronTable;
     DeviceTable<b200_synapse_group> sparseTable, postSpanTable, learnTable, proceduralTable, drawnTable, denseTable, scatterTable;
+    DeviceTable<b200_synapse_group> scatterRows;    // the groups of scatterTable, for presynapticSparseKernel
     bool drawnNormal = false, drawnWide = false;    // proceduralDrawnKernel: every weight Normal; element numbers beyond 32 bits
     unsigned int ahead = 0, advance = 1;    // place of the step being enqueued in its block of steps (see chainPhase)
     ScatterTarget *scatterTargets = nullptr;
     ScatterPart *scatterParts = nullptr;    // sparseBatchKernel: what every CTA does
     unsigned int scatterGrid = 0, scatterCells = 0, scatterDepth = 0, scatterPiece = 0;
     size_t scatterSmem = 0;
+    // sparseBatchKernel's start and flush take longer than presynapticSparseKernel needs for a few spikes: it is used ("armed")
+    // while the largest spike count of the steps before (peakHost below) reaches this many spikes a copy
+    float scatterMinSpikes = SCATTER_MIN_SPIKES;
+    bool scatterArmed = false;
+    unsigned int scatterQuiet = 0;
+    unsigned long long scatterSources = ~0ull;      // neuron groups whose spikes it delivers
     uint4 *denseParts = nullptr;            // denseBatchKernel: what every CTA does
 
     // persistent fused-step path (batch 1, SPARSE non-learning groups only)
@@ -275,7 +282,8 @@ struct b200_runner
     bool tiledArmed = false;
     unsigned int *peakHost = nullptr;
     cudaEvent_t peakEvent = nullptr;
-    bool peakPending = false;
+    bool peakPending = false, peakSeen = false;
+    unsigned int peakSteps = 0;             // steps since the count was last fetched
     unsigned int quietBlocks = 0;
     double eventsPerSpike = 0.0;
     std::string tiledWhyNot;
@@ -581,7 +589,8 @@ bool scatterServes(const b200_runner *r, const b200_synapse_group &g)
 {
     if(r->batch < 2 || r->sharded() || r->tiledChosen || g.wu_model == B200_WU_STDP) return false;
     const unsigned long long cells = (unsigned long long)std::max(1u, g.max_den_delay) * g.num_trg;
-    // (two pieces of the widest kind for every warp have to fit besides)
+    // (two pieces of the widest kind for every warp have to fit besides: the groups of a model share one ring size, so a model
+    // without delays stops at 29 900 targets where its own six bytes a synapse would do for 34 500)
     if(cells * sizeof(float) > SCATTER_SMEM - 2u * SCATTER_WARPS * SCATTER_PIECE * 9u - 128u) return false;
     if(((reinterpret_cast<size_t>(g.ind) | reinterpret_cast<size_t>(g.g) | reinterpret_cast<size_t>(g.d) |
          reinterpret_cast<size_t>(g.max_den_delay ? g.den_delay : g.out_post)) & 15u) != 0u) return false;
@@ -590,6 +599,16 @@ bool scatterServes(const b200_runner *r, const b200_synapse_group &g)
         if((o.max_den_delay ? o.den_delay : o.out_post) == (g.max_den_delay ? g.den_delay : g.out_post)) groups++;
     }
     return groups <= SCATTER_MOST_SOURCES;
+}
+
+// Where the neuron kernel's spike-count peaks land (allocated with the tables that need them; never on the time-step path).
+int ensurePeak(b200_runner *r)
+{
+    if(r->peakHost) return B200_OK;
+    CUDA_TRY(hostAcquire(reinterpret_cast<void**>(&r->peakHost), sizeof(unsigned int)));
+    CUDA_TRY(cudaEventCreateWithFlags(&r->peakEvent, cudaEventDisableTiming));
+    *r->peakHost = 0u;
+    return B200_OK;
 }
 
 // The CTAs of sparseBatchKernel: one per SM as far as there are not more (buffer, copy) pairs; a buffer gets as many as its
@@ -601,6 +620,7 @@ int buildScatter(b200_runner *r, std::vector<b200_synapse_group> &scatter)
     r->scatterTargets = nullptr;
     r->scatterParts = nullptr;
     r->scatterTable.release(r->stream);
+    r->scatterRows.release(r->stream);
     if(scatter.empty()) return B200_OK;
     auto buffer = [](const b200_synapse_group &g) { return g.max_den_delay ? g.den_delay : g.out_post; };
     std::stable_sort(scatter.begin(), scatter.end(), [&](const b200_synapse_group &a, const b200_synapse_group &b) { return buffer(a) < buffer(b); });
@@ -642,6 +662,25 @@ int buildScatter(b200_runner *r, std::vector<b200_synapse_group> &scatter)
     CUDA_TRY(poolAlloc(&r->scatterParts, sizeof(ScatterPart) * parts.size(), r->stream));
     CUDA_TRY(cudaMemcpyAsync(r->scatterParts, parts.data(), sizeof(ScatterPart) * parts.size(), cudaMemcpyHostToDevice, r->stream));
     CUDA_TRY(r->scatterTable.upload(scatter, {0u, r->scatterGrid}, r->stream));
+    std::vector<unsigned int> starts{0u};
+    for(const auto &g : scatter) starts.push_back(starts.back() + (g.row_stride + 3u + PRE_TILE - 1u) / PRE_TILE);
+    CUDA_TRY(r->scatterRows.upload(scatter, starts, r->stream));
+    if(const int e = ensurePeak(r)) return e;
+    r->scatterSources = 0;
+    for(size_t ni = 0; ni < std::min<size_t>(r->neuronGroups.size(), 64); ni++) {
+        for(const auto &g : scatter) if(g.src_spk_cnt == r->neuronGroups[ni].spk_cnt) r->scatterSources |= 1ull << ni;
+    }
+    if(!r->peakSeen) {
+        // before anything has been counted: twenty spikes a second of every source neuron
+        std::vector<const void*> sources;
+        double neurons = 0.0;
+        for(const auto &g : scatter) {
+            if(std::find(sources.begin(), sources.end(), g.src_spk_cnt) != sources.end()) continue;
+            sources.push_back(g.src_spk_cnt);
+            neurons += g.num_src;
+        }
+        r->scatterArmed = neurons * 20.0e-3 * r->dt >= r->scatterMinSpikes;
+    }
     return B200_OK;
 }
 
@@ -1354,12 +1393,7 @@ int buildTiled(b200_runner *r)
     r->tiledGrid = grid;
     r->tiledSmemBytes = smem;
     r->tiledSynapses = total;
-    if(!r->peakHost) {
-        // where the neuron kernel's spike-count peaks land (allocated here, with the copy; never on the time-step path)
-        CUDA_TRY(hostAcquire(reinterpret_cast<void**>(&r->peakHost), sizeof(unsigned int)));
-        CUDA_TRY(cudaEventCreateWithFlags(&r->peakEvent, cudaEventDisableTiming));
-        *r->peakHost = 0u;
-    }
+    if(const int err = ensurePeak(r)) return err;
     r->tiledReady = true;
     {
         unsigned long long neurons = 0;
@@ -1782,6 +1816,12 @@ bool tiledActive(const b200_runner *r, bool force = false)
     return r->tiledReady && (force || r->tiledArmed || r->tiledMinEvents == 0);
 }
 
+// Whether sparseBatchKernel delivers the groups it can.
+bool scatterActive(const b200_runner *r)
+{
+    return r->scatterArmed || r->scatterMinSpikes <= 0.0f;
+}
+
 // A kernel of the one-launch-per-kernel path: its blocks may be placed while the kernel before it runs (chainWait).
 template<typename P, typename A>
 cudaError_t chain(const b200_runner *r, void (*kernel)(P), dim3 grid, unsigned int block, size_t smem, const A &params)
@@ -1838,7 +1878,13 @@ int enqueueSynapses(b200_runner *r, bool capturing, bool force = false)
         CUDA_TRY(chain(r, denseBatchKernel, grid, DENSE_BLOCK, DENSE_SMEM, DenseLaunch{synapseLaunch(r, r->denseTable), r->denseParts}));
         r->launches++;
     }
-    if(r->scatterTable.num) {
+    if(r->scatterTable.num && !force && !scatterActive(r)) {
+        ScopedTimer tm(r, "presynaptic_update", capturing);
+        const dim3 grid(r->scatterRows.blocks, spikeLanesFor(r, r->scatterRows.blocks), r->batch);
+        CUDA_TRY(chain(r, presynapticSparseKernel, grid, PRE_BLOCK, 0, synapseLaunch(r, r->scatterRows)));
+        r->launches++;
+    }
+    else if(r->scatterTable.num) {
         ScopedTimer tm(r, "presynaptic_update", capturing);
         CUDA_TRY(chain(r, sparseBatchKernel, r->scatterGrid, SCATTER_BLOCK, r->scatterSmem,
                        ScatterLaunch{synapseLaunch(r, r->scatterTable), r->scatterTargets, r->scatterParts, r->scatterCells, r->scatterDepth, r->scatterPiece}));
@@ -1891,6 +1937,7 @@ int enqueueNeurons(b200_runner *r, unsigned long long numRec, bool capturing)
     L.count_events = r->countEvents ? 1u : 0u;
     L.ahead = r->ahead;
     L.advance = r->advance;
+    L.peak_groups = (r->scatterTable.num && !r->tiledReady) ? r->scatterSources : ~0ull;
     // (as many blocks as are on the chip at once: thousands of blocks for a few loads each spend their time starting, and
     // counting themselves one after another in the ticket)
     int sms = 0;
@@ -1924,24 +1971,39 @@ int fetchPeak(b200_runner *r)
     CUDA_TRY(cudaMemsetAsync(&r->state->peak_spikes, 0, sizeof(unsigned int), r->stream));
     CUDA_TRY(cudaEventRecord(r->peakEvent, r->stream));
     r->peakPending = true;
+    r->peakSteps = 0;
     return B200_OK;
 }
 
-// Before a block of steps: arm or disarm the tiled kernels from the last spike count that has arrived.
+// Before a block of steps: choose kernels by the last spike count that has arrived.
 int pollPeak(b200_runner *r)
 {
-    if(!r->tiledReady || !r->peakPending || cudaEventQuery(r->peakEvent) != cudaSuccess) return B200_OK;
+    if(!r->peakPending || cudaEventQuery(r->peakEvent) != cudaSuccess) return B200_OK;
     r->peakPending = false;
-    const double estimate = (double)*r->peakHost * r->eventsPerSpike;
-    const bool was = r->tiledArmed;
-    if(estimate * 4.0 >= (double)r->tiledMinEvents) {
-        r->tiledArmed = true;
-        r->quietBlocks = 0;
+    r->peakSeen = true;
+    const double peak = (double)*r->peakHost;
+    if(r->tiledReady) {
+        const double estimate = peak * r->eventsPerSpike;
+        const bool was = r->tiledArmed;
+        if(estimate * 4.0 >= (double)r->tiledMinEvents) {
+            r->tiledArmed = true;
+            r->quietBlocks = 0;
+        }
+        else if(r->tiledArmed && estimate * 16.0 < (double)r->tiledMinEvents && ++r->quietBlocks >= 3) {
+            r->tiledArmed = false;
+        }
+        if(was != r->tiledArmed) r->dropGraph();        // the captured steps launch other kernels now
     }
-    else if(r->tiledArmed && estimate * 16.0 < (double)r->tiledMinEvents && ++r->quietBlocks >= 3) {
-        r->tiledArmed = false;
+    if(r->scatterTable.num) {
+        const double least = (double)r->scatterMinSpikes * r->batch;
+        const bool was = r->scatterArmed;
+        if(peak >= least) {
+            r->scatterArmed = true;
+            r->scatterQuiet = 0;
+        }
+        else if(r->scatterArmed && peak * 2.0 < least && ++r->scatterQuiet >= 3) r->scatterArmed = false;
+        if(was != r->scatterArmed) r->dropGraph();
     }
-    if(was != r->tiledArmed) r->dropGraph();        // the captured steps launch other kernels now
     return B200_OK;
 }
 
@@ -2079,6 +2141,7 @@ int b200_runner_destroy(b200_runner *r)
     r->denseTable.release(r->stream);
     poolFree(r->denseParts, r->stream);
     r->scatterTable.release(r->stream);
+    r->scatterRows.release(r->stream);
     poolFree(r->scatterTargets, r->stream);
     poolFree(r->scatterParts, r->stream);
     r->proceduralTable.release(r->stream);
@@ -2556,6 +2619,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
         CUDA_TRY(cudaStreamSynchronize(r->stream));
         CUDA_TRY(cudaMemcpyAsync(dst, &v, sizeof(v), cudaMemcpyHostToDevice, r->stream));
     }
+    else if(n == "scatter_min_spikes") { r->scatterMinSpikes = (float)value; r->peakSeen = false; r->dirty = true; }
     else if(n == "use_tiled") { r->useTiled = (value != 0.0); r->tiledStale = true; }
     else if(n == "tiled_min_events") { r->tiledMinEvents = (float)value; r->tiledChosen = r->dirty = true; }
     else if(n == "tiled_ticket_events") { r->tiledTicketEvents = std::max(1.0f, (float)value); r->dropGraph(); }
@@ -2729,15 +2793,27 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
             CUDA_TRY(cudaGraphLaunch(r->graphExec, r->stream));
             r->launches += (unsigned long long)r->graphLen * kernelsPerStep(r);
             left -= r->graphLen;
+            if(r->scatterTable.num && !r->peakSeen && left >= 4ull * r->graphLen) {
+                // a model's first steps, and many more behind them: worth waiting, once, for what they have to say
+                if((e = fetchPeak(r)) != B200_OK) return e;
+                CUDA_TRY(cudaEventSynchronize(r->peakEvent));
+                const unsigned int len = r->graphLen;
+                if((e = pollPeak(r)) != B200_OK) return e;
+                if(!r->graphExec && (e = buildGraph(r, len, num_recording_timesteps)) != B200_OK) return e;
+            }
         }
     }
     for(; left; left--) {
         e = enqueueStep(r, num_recording_timesteps, false);
         if(e) return e;
     }
-    if(r->tiledReady && !resident && !(r->useFused && r->fusedEligible && !r->timing)) {
-        e = fetchPeak(r);
-        if(e) return e;
+    if((r->tiledReady || r->scatterTable.num) && !resident && !(r->useFused && r->fusedEligible && !r->timing)) {
+        // (three more entries in the stream: not behind every call of a few steps)
+        r->peakSteps += (unsigned int)std::min<uint64_t>(num_steps, 1u << 20);
+        if(r->tiledReady || r->peakSteps >= 64u || !r->peakSeen) {
+            e = fetchPeak(r);
+            if(e) return e;
+        }
     }
     r->hostTimestep += num_steps;
     r->hostStepsDone += num_steps;
@@ -2929,6 +3005,14 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
     if(n == "tiled_armed") {
         // whether the next block of steps on the one-launch-per-kernel path launches the tiled kernels
         *value = tiledActive(r) ? 1u : 0u;
+        return B200_OK;
+    }
+    if(n == "scatter_armed") {
+        // whether the next block of steps of a batched network sums its SPARSE groups in shared memory
+        int e = prepare(r);
+        if(!e) e = pollPeak(r);
+        if(e) return e;
+        *value = (r->scatterTable.num && scatterActive(r)) ? 1u : 0u;
         return B200_OK;
     }
     if(n == "tiled_ready" || n == "tiled_synapses" || n == "heavy") {

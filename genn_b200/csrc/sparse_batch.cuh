@@ -34,6 +34,11 @@ constexpr unsigned int SCATTER_MOST_SOURCES = 64;                       // group
 // An event costs 0.19 ns of an SM's shared memory and 0.78 ns of its share of the L2's reductions; clearing and flushing
 // the sums about 2.5 us.
 constexpr unsigned int SCATTER_FEW = 4096;
+// Spikes of a copy and step from which the kernel is used.  presynapticSparseKernel takes sixteen spikes of a copy side by side
+// and the next sixteen behind them; this one starts its rings, clears and flushes whatever there is to do.  A step takes, with
+// it / here: 1000 neurons, p = 0.1, 8 copies, 5 spikes a copy 5.9 / 7.8 us, 50 spikes 8.0 / 8.4; 3000 neurons, 15 spikes
+// 6.6 / 7.8, 150 spikes 20.4 / 12.0; 10 000 neurons, 50 spikes 14.5 / 11.6 (p = 0.02: 10.0 / 9.3, with 32 copies 13.7 / 15.8).
+constexpr float SCATTER_MIN_SPIKES = 64.0f;
 
 struct ScatterTarget
 {

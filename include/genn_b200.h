@@ -393,6 +393,8 @@ int  b200_get_counter(b200_runner *r, const char *name, uint64_t *value);
  * "tiled_armed"; b200_update_synapses always launches them), "tiled_ticket_events" / "tiled_ticket_cost" (the
  * tiled kernel's unit of work, handed to one warp, is sized for about that many synaptic events, default 2048;
  * its fixed cost in synaptic events when a step's work is cut into equal stretches per CTA, default 256),
+ * "scatter_min_spikes" (batched networks: spikes of a copy and step, by the largest count of the steps before, from which SPARSE
+ * groups whose target buffer fits an SM's shared memory are summed there, default 64; 0: always; counter "scatter_armed"),
  * "barrier_spin_limit" / "exchange_spin_limit" (polls) and "stream_wait_cycles" (SM cycles): how long a wait
  * inside a persistent kernel lasts before the launch gives up and b200_synchronize reports
  * B200_ERR_DEVICE_CHECK (defaults: tens of milliseconds; about two seconds). */

@@ -56,3 +56,45 @@ def test_every_copy_matches_the_cpu_checker(pre, post, degree, batch, rate, narr
     assert rt.counter("tiled_ready") == 0
     rt.close()
     orc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("least", [0, 1e9], ids=["shared sums", "row by row"])
+@pytest.mark.parametrize("pre,post,degree,batch,rate,narrow,delays,constant", [
+    (5, 3, 1, 2, 500.0, False, 0, False), (301, 250, 30, 3, 50.0, True, 0, False), (97, 5003, 700, 2, 40.0, True, 0, False),
+    (129, 300, 60, 9, 90.0, True, 5, False), (700, 257, 90, 2, 900.0, True, 0, True)])
+def test_either_kernel_matches_the_cpu_checker(pre, post, degree, batch, rate, narrow, delays, constant, least):
+    from genn_b200.runtime import Runtime
+    from oracle.oracle import OracleRunner
+    args = (pre, post, degree, batch, rate, narrow, delays, constant)
+    rt, orc = Runtime(None, net=_net(*args)), OracleRunner(_net(*args))
+    rt.set_option("scatter_min_spikes", least)
+    for chunk in (1, 2, 6):
+        assert rt.counter("scatter_armed") == (1 if least == 0 else 0)
+        rt.step_time(chunk)
+        orc.step(chunk)
+        for name in [n for n in rt.plan.arrays if n.endswith((".out_post", ".den_delay", ".V"))]:
+            helpers.assert_close(rt.array(name).reshape(-1), orc.array(name).reshape(-1), f"{name} after {chunk}", 1e-5, 2e-5)
+    rt.close()
+    orc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pre,rate,armed", [(400, 20.0, 0), (400, 400.0, 1), (4000, 2.0, 0), (4000, 50.0, 1)])
+@pytest.mark.parametrize("calls", [[600], [70] * 8])
+def test_the_kernel_is_chosen_by_the_spikes_of_the_steps_before(pre, rate, armed, calls):
+    """Whatever is assumed of a model at first: one long call, in which the choice may change, or several short ones."""
+    from genn_b200.runtime import Runtime
+    from oracle.oracle import OracleRunner
+    args = (pre, 100, 10, 2, rate, True, 0, False)
+    rt, orc = Runtime(None, net=_net(*args)), OracleRunner(_net(*args))
+    assert rt.counter("scatter_armed") == (1 if pre == 4000 else 0)
+    for n in calls:
+        rt.step_time(n)
+        rt.synchronize()
+        orc.step(n)
+    assert rt.counter("scatter_armed") == armed or (len(calls) == 1 and pre == 4000 and not armed)      # (three quiet blocks)
+    for name in [n for n in rt.plan.arrays if n.endswith((".out_post", ".V"))]:
+        helpers.assert_close(rt.array(name).reshape(-1), orc.array(name).reshape(-1), name, 1e-5, 5e-5)
+    rt.close()
+    orc.close()
