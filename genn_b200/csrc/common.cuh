@@ -43,6 +43,11 @@ struct StepState
     unsigned long long barrier_spin_limit;
     unsigned long long exchange_spin_limit;
     long long stream_wait_cycles;
+    // target-resident kernel (resident.h: "Busy networks"): what it has lost to the kernel with a grid barrier (ns), the step
+    // until which that one goes on in its place, and for how many steps it last did
+    unsigned int resident_debt;
+    unsigned int resident_rest;
+    unsigned long long resident_hold;
 };
 
 constexpr unsigned int ERR_SPIKE_OVERFLOW = 1u;

@@ -125,6 +125,7 @@ struct FusedLaunch
     unsigned int profile;                // accumulate phase cycles (thread 0 of every CTA)
     unsigned long long *cta_cycles;      // [gridDim][4] or NULL
     unsigned long long num_steps;
+    unsigned long long goal;             // if not 0: steps done when the launch ends, in place of num_steps (none, if they are done)
     unsigned long long *barrier;         // monotonic arrival counter
     // spike exchange between the processes of a sharded model (world == 1: unused)
     unsigned int rank;
@@ -252,10 +253,23 @@ __device__ __forceinline__ void fusedUrgentChunk(const b200_synapse_group &g, co
 // descriptor left in global memory would cost a full L2 round trip per field
 // and per step, one after another along the dependency chain.  All merged-group
 // tables are therefore staged into shared memory once per launch.
+// What the launch of the target-resident kernel in front of this one has left to do.  (`steps_done` changes behind the last
+// grid barrier only: every CTA sees the same.)
+__device__ __forceinline__ bool stepsLeft(FusedLaunch &L)
+{
+    if(L.goal) {
+        const unsigned long long done = L.neuron.state->steps_done;
+        if(done >= L.goal) return false;
+        L.num_steps = L.goal - done;
+    }
+    return true;
+}
+
 template<int NPSM, int NCS>
 __global__ void __launch_bounds__(FUSED_BLOCK, 1)
 fusedStepKernel(FusedLaunch L)
 {
+    if(!stepsLeft(L)) return;
     extern __shared__ __align__(16) unsigned char fusedSmem[];
     __shared__ bool barrierOk;
     __shared__ long long publishedAt;        // profile mode: when the counts of the last step went out

@@ -45,12 +45,14 @@ __global__ void __launch_bounds__(256)
 residentBuildKernel(const ResidentBuild B, int pass, unsigned int *longest, const ResidentRun *runs, uint2 *entries, StepState *state)
 {
     __shared__ unsigned int cursor[RESIDENT_MAX_CTAS + 1];      // per CTA; the last one: delay-0 synapses
+    unsigned long long synapses = 0;
     for(unsigned int pre = blockIdx.x; pre < B.num_src; pre += gridDim.x) {
         for(unsigned int c = threadIdx.x; c <= RESIDENT_MAX_CTAS; c += blockDim.x) cursor[c] = 0u;
         __syncthreads();
         for(unsigned int gi = 0; gi < B.num_groups; gi++) {
             const b200_synapse_group &g = B.groups[gi];
             const unsigned int len = min(g.row_length[pre], g.row_stride);
+            synapses += len;
             const unsigned int trg = B.target[gi] >> 8, psm = B.target[gi] & 0xFFu;
             const unsigned int firstUnit = B.unit_start[trg];
             const bool constant = (g.wu_model == B200_WU_STATIC_PULSE_CONSTANT_WEIGHT);
@@ -86,6 +88,7 @@ residentBuildKernel(const ResidentBuild B, int pass, unsigned int *longest, cons
         }
         __syncthreads();
     }
+    if(pass == 0 && threadIdx.x == 0 && synapses) atomicAdd(B.synapses, synapses);
 }
 
 // ---- time steps ----------------------------------------------------------------------------------
@@ -104,13 +107,16 @@ struct ResidentShared
     // (three of each, in turn: warps are at most one barrier apart, and a step may have only one)
     unsigned int list[3][RESIDENT_LIST];        // neuron group << 24 | neuron
     unsigned int listed[3];                     // spikes in the list (counts on beyond its end)
-    unsigned int stop[3];
+    unsigned int stop[3];                       // 1: a wait ran out, 2: this launch has lost enough, 4: more spikes than the list holds
     unsigned int sent[2];                       // this CTA's spikes of the step, and how many
     __align__(16) unsigned short ids[2][RESIDENT_BLOCK];
     unsigned int firstWarp[RESIDENT_MAX_GROUPS + 1];    // warps of this CTA before those of each group
     unsigned long long done;                    // StepState at the start of the launch
     unsigned int phase, period;
     unsigned int limit;                         // polls of a wait
+    int debt;                                   // ns lost, by thread 0's account up to the step `accounted`
+    unsigned int accounted;
+    unsigned int steps;                         // of this launch (every thread writes a smaller number for itself when it ends early)
     __align__(16) ResidentLif lif[RESIDENT_MAX_GROUPS];
 };
 
@@ -127,6 +133,21 @@ struct ResidentFronts
 };
 
 extern __shared__ __align__(16) unsigned char residentSmem[];
+
+// Thread 0's account of a step with more than a few spikes (resident.h: "Busy networks"); the steps since the last such one made
+// up for half of `spare` each at least.  (Nothing is done in the others: every instruction is on the chain of the step.)
+__device__ __forceinline__ void residentAccount(ResidentShared &sh, unsigned int weight, unsigned int spare, unsigned int patience, unsigned int step,
+                                             unsigned int spikes, unsigned int *stop)
+{
+    int debt = sh.debt;
+    if(sh.accounted <= step) {
+        debt = max(debt - (int)(min(step - sh.accounted, 1u << 14) * (spare / 2u)), 0) - (int)spare;
+        sh.accounted = step + 1u;
+    }
+    debt = min(debt + (int)(min(spikes, RESIDENT_LIST) * weight) + (spikes > RESIDENT_LIST ? (int)RESIDENT_PIECE_COST : 0), (int)RESIDENT_MOST_DEBT);
+    sh.debt = debt;
+    if(debt > 0 && (unsigned int)debt > patience) atomicOr(stop, 2u);
+}
 
 template<typename T>
 __device__ __forceinline__ T *residentTable(unsigned int at)
@@ -369,8 +390,9 @@ __device__ __forceinline__ bool residentLif(const ResidentLif &q, float dt, Neur
     return spiked;
 }
 
-template<int NPSM, int NCS, bool ONE>
-__global__ void __launch_bounds__(RESIDENT_BLOCK, 1)
+// BLOCK: most threads.  With 640 a thread has 96 registers and next to nothing is spilled, with 768 it has 80.
+template<int NPSM, int NCS, bool ONE, unsigned int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1)
 residentStepKernel(const __grid_constant__ ResidentLaunch L)
 {
     __shared__ ResidentShared sh;
@@ -392,7 +414,14 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     if(L.poisson) stageWords(residentSmem + L.at.poisson, L.poisson, sizeof(float) * 64u * numGroups);
     StepState *const state = L.neuron.state;
     const unsigned long long t0 = state->timestep;
+    if(L.may_leave) {
+        if(me == 0 && threadIdx.x == 0) *L.barrier = 0ull;
+        if(state->steps_done < state->resident_hold) return;        // (the same for every CTA: both change at the end of a launch)
+    }
     if(threadIdx.x == 0) {
+        sh.debt = (int)state->resident_debt;
+        sh.accounted = 0u;
+        sh.steps = L.num_steps;
         unsigned int base = 0;
         for(unsigned int c = 0; c < RESIDENT_CLASSES; c++) {
             const unsigned int n = (c < L.num_depths) ? L.cta_columns[me * RESIDENT_CLASSES + c] : 0u;
@@ -476,7 +505,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     auto gaveUp = [&](unsigned int &polls, unsigned int *stop) -> bool {
         if(++polls <= sh.limit) return false;
         atomicOr(&state->error, ERR_BARRIER_TIMEOUT);
-        *stop = 1u;
+        atomicOr(stop, 1u);
         return true;
     };
     // the sender's cell of the step with number `no` (bounded wait); the second word only if it is needed
@@ -520,8 +549,11 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                 csCount[0] = residentPoisson(draws.draw(L.neuron.seed, g.cs[0].rng_stream, local, t0 + step), residentTable<const float>(L.at.poisson) + 64u * group);
             }
             else drawCurrentSources<NCS>(L.neuron, g, 0u, local, t0 + step, csCount);
-            if(g.model == B200_NEURON_POISSON && __uint_as_float(regs.v[0]) <= 0.0f) {
-                regs.v[0] = __float_as_uint(drawPoissonInterval(L.neuron, g, 0u, local, t0 + step, __uint_as_float(regs.v[0])));
+            if(g.model == B200_NEURON_POISSON) {
+                residentTable<unsigned int>(L.at.undrawn)[threadIdx.x] = regs.v[0];
+                if(__uint_as_float(regs.v[0]) <= 0.0f) {
+                    regs.v[0] = __float_as_uint(drawPoissonInterval(L.neuron, g, 0u, local, t0 + step, __uint_as_float(regs.v[0])));
+                }
             }
         }
 
@@ -535,13 +567,14 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                 // spikes from before this launch come from the spike lists, one piece after the other (a LATE class: in the
                 // first step also those that are due in it)
                 for(unsigned int ahead = (late && step == 0u) ? 0u : late; ahead <= late; ahead++) {
-                    if(step + ahead >= L.delay[a] + 1u || (late && ahead && step + 1u == L.num_steps)) continue;
+                    if(step + ahead >= L.delay[a] + 1u || (late && ahead && (step + 1u == L.num_steps || (numDelays > 1u && step + 1u == sh.steps)))) continue;
                     __syncthreads();
                     for(unsigned int gi = 0; gi < numGroups; gi++) {
                         if(!((L.sources[a] >> gi) & 1ull)) continue;
                         const b200_neuron_group &g = groups[gi];
                         const unsigned int slots = g.num_delay_slots, slot = ringSlot(sh.phase + step + ahead + slots - L.delay[a], slots);
                         const unsigned int n = min(__ldcg(&g.spk_cnt[slot]), g.num_neurons);
+                        if(threadIdx.x == 0 && n > L.quiet[a]) residentAccount(sh, L.weight[a], L.spare, L.may_leave ? L.patience : ~0u, step, min(n, RESIDENT_LIST), &sh.stop[turn]);
                         for(unsigned int from = 0; from < n; from += RESIDENT_LIST) {
                             const unsigned int m = min(RESIDENT_LIST, n - from);
                             for(unsigned int i = threadIdx.x; i < m; i += blockDim.x) {
@@ -564,7 +597,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                     }
                 }
             }
-            if(late && step + 1u == L.num_steps) {
+            if(late && (step + 1u == L.num_steps || (numDelays > 1u && step + 1u == sh.steps))) {
                 __syncthreads();            // (the next launch takes those; the update still waits for what the last step added)
                 continue;
             }
@@ -583,6 +616,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                     if(n > had) {
                         if(ONE) {
                             unsigned int at = atomicAdd(&sh.listed[turn], n - had);
+                            if(at + (n - had) > RESIDENT_LIST && first && L.may_leave) atomicOr(&sh.stop[turn], 4u);
                             for(; had < n && at < RESIDENT_LIST; had++, at++) list[at] = spikeOf(w, had, from, no, &sh.stop[turn]);
                         }
                         else {
@@ -591,16 +625,39 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                                 const unsigned int spike = spikeOf(w, had, from, no, &sh.stop[turn]);
                                 if(!((L.sources[a] >> (spike >> 24)) & 1ull)) continue;
                                 const unsigned int at = atomicAdd(&sh.listed[turn], 1u);
-                                if(at >= RESIDENT_LIST) break;
+                                if(at >= RESIDENT_LIST) {
+                                    if(first && L.may_leave && numDelays == 1u) atomicOr(&sh.stop[turn], 4u);
+                                    break;
+                                }
                                 list[at] = spike;
                             }
                         }
                     }
                 }
                 __syncthreads();
-                if(sh.stop[turn]) return;           // (written in front of the barrier only: the same for every thread)
+                if(const unsigned int stop = sh.stop[turn]) {       // (written in front of the barrier only: the same for every thread)
+                    if(stop & 1u) return;
+                    if(first && a == 0u) {                          // 2 and 4: with `may_leave` only
+                        if(numDelays > 1u || (BLOCK > RESIDENT_FEW && !late)) sh.steps = step + 1u;     // (this step is the last)
+                        else if(late) {
+                            // (the next step's spikes, which the next launch takes)
+                            sh.steps = step + 1u;
+                            break;
+                        }
+                        else if constexpr(BLOCK <= RESIDENT_FEW) {
+                            // (this step is the other kernel's: drawn again, the same, with it.  The jump costs registers that
+                            // the larger blocks do not have: +0.2 us a step)
+                            if(mine && active && groups[group].model == B200_NEURON_POISSON) regs.v[0] = residentTable<unsigned int>(L.at.undrawn)[threadIdx.x];
+                            sh.steps = step;
+                            goto ended;
+                        }
+                    }
+                }
                 const unsigned int all = sh.listed[turn], m = min(all, RESIDENT_LIST);
-                if(threadIdx.x == 0) sh.listed[turn == 0u ? 2u : turn - 1u] = 0u;
+                if(threadIdx.x == 0) {
+                    sh.listed[turn == 0u ? 2u : turn - 1u] = 0u;
+                    if(all > L.quiet[a]) residentAccount(sh, L.weight[a], L.spare, L.may_leave ? L.patience : ~0u, step, all, &sh.stop[turn == 2u ? 0u : turn + 1u]);
+                }
                 turn = (turn == 2u) ? 0u : turn + 1u;
                 if(m) {
                     // runs of the last class that may wait for the neuron update
@@ -621,7 +678,6 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                 if(all <= RESIDENT_LIST) break;
             }
         }
-
         // ---------------- neuron update -------------------------------------------------------------------
         const unsigned int par = step & 1u;
         unsigned int ballot = 0;
@@ -720,18 +776,21 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
             atomicAdd(&state->synaptic_events, (unsigned long long)deliver.events);
             deliver.events = 0u;
         }
+        if(step + 1u == sh.steps) break;
     }
 
+ended: __attribute__((unused));
     // ---------------- what the launch leaves in memory ----------------------------------------------------
     // every CTA is through its last step: nobody reads the spike lists any more
-    const unsigned long long doneNow = sh.done + L.num_steps;
-    const unsigned int k = (sh.phase + L.num_steps) % sh.period, period = sh.period;
+    const unsigned int step = sh.steps;
+    const unsigned long long doneNow = sh.done + step;
+    const unsigned int k = (sh.phase + step) % sh.period, period = sh.period;
     __syncthreads();
-    if(asked < G) awaitCell(buf == 0u ? L.buffers - 1u : buf - 1u, no0 + L.num_steps, &sh.stop[turn]);
+    if(asked < G) awaitCell(buf == 0u ? L.buffers - 1u : buf - 1u, no0 + step, &sh.stop[turn]);
     __syncthreads();
-    if(sh.stop[turn]) return;
+    if(sh.stop[turn] & 1u) return;
     // lists of the last steps: emptied by the first CTA (and the one the next step writes), filled by all
-    const unsigned int lists = min(L.history, L.num_steps);
+    const unsigned int lists = min(L.history, step);
     if(me == 0) {
         for(unsigned int i = threadIdx.x; i < numGroups * (lists + 1u); i += blockDim.x) {
             const b200_neuron_group &g = groups[i % numGroups];
@@ -788,15 +847,34 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     }
     // (every CTA has sent the message of the last step, so every CTA has read the counters)
     if(me == 0 && threadIdx.x == 0) {
-        state->timestep = t0 + L.num_steps;
+        state->timestep = t0 + step;
         state->steps_done = doneNow;
         state->phase = k;
+        const unsigned int quiet = (step > sh.accounted) ? min(step - sh.accounted, 1u << 14) : 0u;
+        const unsigned int debt = (unsigned int)max(sh.debt - (int)(quiet * (L.spare / 2u)), 0);
+        if(step < L.num_steps || debt > L.patience) {
+            const unsigned int rest = min(max(2u * state->resident_rest, RESIDENT_REST), RESIDENT_MOST_REST);
+            state->resident_rest = rest;
+            state->resident_hold = doneNow + rest;
+            state->resident_debt = min(debt, L.patience - L.patience / 4u);       // (the next time it is seen sooner)
+            *reinterpret_cast<volatile unsigned long long*>(L.hold) = doneNow + rest;
+        }
+        else {
+            // (as many steps without that make up for one time)
+            state->resident_rest -= min(state->resident_rest, step);
+            state->resident_debt = debt;
+        }
     }
 }
 
-const void *residentKernelFor(int npsm, int ncs, bool one_class)
+const void *residentKernelFor(int npsm, int ncs, bool one_class, unsigned int threads)
 {
-#define B200_RESIDENT(P, C) if(npsm == P && ncs == C) return one_class ? (const void*)residentStepKernel<P, C, true> : (const void*)residentStepKernel<P, C, false>
+    const bool few = threads <= RESIDENT_FEW;
+#define B200_RESIDENT(P, C) \
+    if(npsm == P && ncs == C) { \
+        if(few) return one_class ? (const void*)residentStepKernel<P, C, true, RESIDENT_FEW> : (const void*)residentStepKernel<P, C, false, RESIDENT_FEW>; \
+        return one_class ? (const void*)residentStepKernel<P, C, true, RESIDENT_BLOCK> : (const void*)residentStepKernel<P, C, false, RESIDENT_BLOCK>; \
+    }
     B200_RESIDENT(1, 0); B200_RESIDENT(1, 1); B200_RESIDENT(1, B200_MAX_CS);
     B200_RESIDENT(2, 0); B200_RESIDENT(2, 1); B200_RESIDENT(2, B200_MAX_CS);
     B200_RESIDENT(B200_MAX_PSM, 0); B200_RESIDENT(B200_MAX_PSM, 1); B200_RESIDENT(B200_MAX_PSM, B200_MAX_CS);

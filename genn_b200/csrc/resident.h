@@ -31,6 +31,19 @@
 //              already, so their runs are fetched and added behind the update too, into the second of two buffers.
 //              CTAs then run up to the delay apart, and no step waits for another SM or for memory.
 //
+// Busy networks.  Every CTA handles every spike, so a spike costs each of them the same, however many they are: about
+// RESIDENT_RUN_COST ns of a warp for every chunk of its run and RESIDENT_NEAR_COST for every chunk of its delay-0 row, where
+// the kernels with a grid barrier share its synapses out (8.5 ps each; 20 with rings) behind a step that costs 2 to 4 us more
+// to begin with.  A step of 10 000 + 10 000 neurons, 1000 synapses each: 3.3 us at 10 spikes a step (6.6 with the barrier),
+// 7.5 at 100 (7.7), 16.5 at 300 (11.3), 163 at 3000 (62); 20 000 + 20 000, 200 synapses: 3.3 (6.5), 6.3 (6.8), 12.2 (6.9), 107
+// (15); 4000 + 4000 with rings of 16, 1000 synapses: 3.7 (5.8), 17.6 (8.2), 49 (11.9), 161 at 1000 (22).  So a launch keeps
+// account of what it loses: every spike delivered adds its class's `weight`, every step takes off `spare`, and when the sum
+// passes `patience` the launch ends with the next step's list.  A launch of the other
+// kernel that the host has put behind it does the rest up to the same step and goes on for `resident_rest` steps, twice as many every time
+// this happens, before this kernel is tried again.  All CTAs count the same spikes, so they leave at the same step without
+// a word.  More spikes in one step than the list holds are left to the other kernel at once (models with one delay, up to
+// 20 units a CTA): the messages' further ids are fetched by one lane per sender, 0.3 ms for every 2048 of them.
+//
 // Memory between launches is what every other path leaves: the first steps of a launch take the spikes of the steps
 // before it from the spike lists, the last ones write them.
 #pragma once
@@ -41,7 +54,8 @@
 
 namespace b200
 {
-constexpr unsigned int RESIDENT_BLOCK = 768;            // most threads of a CTA: 85 registers each
+constexpr unsigned int RESIDENT_BLOCK = 768;            // most threads of a CTA: 80 registers each
+constexpr unsigned int RESIDENT_FEW = 640;              // threads up to which another instance has 96
 constexpr unsigned int RESIDENT_UNITS = RESIDENT_BLOCK / 32;    // most units of 32 neurons of a CTA
 constexpr unsigned int RESIDENT_MAX_CTAS = 256;
 constexpr unsigned int RESIDENT_MAX_GROUPS = 64;        // neuron groups (a bit mask says which are sources)
@@ -53,6 +67,11 @@ constexpr unsigned int RESIDENT_CHUNK = 32 * RESIDENT_LOADS;    // entries of a 
 constexpr unsigned int RESIDENT_NEAR_ROWS = 4;          // rows of delay-0 synapses whose loads a warp has in flight
 constexpr unsigned int RESIDENT_DENSE_SPIKES = 8;       // rows of a DENSE group whose loads a lane has in flight
 constexpr unsigned int RESIDENT_NEAR_MOST = 256;        // most delay-0 synapses of a source neuron for a SPLIT class
+constexpr float RESIDENT_RUN_COST = 560.0f, RESIDENT_NEAR_COST = 280.0f;        // ns of a warp for a chunk of a run / of a delay-0 row
+constexpr unsigned int RESIDENT_PIECE_COST = 300000;    // ns of a step with more spikes than the list holds, for every list of them
+constexpr unsigned int RESIDENT_MOST_WEIGHT = 1000, RESIDENT_MOST_DEBT = 1u << 30;      // ns
+constexpr unsigned int RESIDENT_REST = 64;              // steps on the other kernel, the first time
+constexpr unsigned int RESIDENT_MOST_REST = 1u << 20;
 constexpr unsigned int RESIDENT_PAD = 0xFFFFFFFFu;      // key of a padding entry
 constexpr unsigned long long RESIDENT_TAG_STEPS = 1ull << 20;       // step numbers of messages are 20 bits
 constexpr unsigned int RESIDENT_HEAD_IDS = 3, RESIDENT_MORE_IDS = 4;    // ids in a first word / in a further word
@@ -91,7 +110,7 @@ struct ResidentSpan             // a DENSE or BITMASK group
 // Where the tables of a CTA lie in its dynamic shared memory (bytes): constants of the launch, so no thread keeps pointers.
 struct ResidentLayout
 {
-    unsigned int groups, unit_start, unit_first, columns, runs, near, spans, poisson, history, acc;
+    unsigned int groups, unit_start, unit_first, columns, runs, near, spans, poisson, undrawn, history, acc;
 };
 
 struct ResidentLaunch
@@ -128,6 +147,13 @@ struct ResidentLaunch
     unsigned long long *leave;          // steps done when the spike lists may be written at the end of a launch
     unsigned int num_steps;
     unsigned int count_events;
+    unsigned int weight[RESIDENT_CLASSES];  // ns that a spike of that delay costs above what it costs the other kernel
+    unsigned int quiet[RESIDENT_CLASSES];   // spikes of a step that cost half of `spare`: up to there nothing is accounted
+    unsigned int spare;                     // ns that a step without spikes costs less than there
+    unsigned int patience;                  // ns
+    unsigned int may_leave;                 // 1: a launch of the other kernel follows that does what this one leaves
+    unsigned long long *hold;               // page-locked: the host's copy of StepState::resident_hold
+    unsigned long long *barrier;            // of the launch that follows: zeroed by this one
 };
 
 // the runs of one pair are counted (pass 0) and placed (pass 1) by one launch each
@@ -141,6 +167,7 @@ struct ResidentBuild
     unsigned int late;                  // 1: LATE class: every synapse arrives one step after its delivery
     unsigned int split;                 // 1: SPLIT class: delay-0 synapses go into the rows
     unsigned int *near_longest;         // longest row of delay-0 synapses
+    unsigned long long *synapses;       // all of the pair
     ResidentNear near;
     uint2 *near_entries;
     unsigned int grid;
@@ -148,7 +175,7 @@ struct ResidentBuild
 };
 
 // kernels: resident.cu
-const void *residentKernelFor(int npsm, int ncs, bool one_class);
+const void *residentKernelFor(int npsm, int ncs, bool one_class, unsigned int threads);
 cudaError_t residentBuild(const ResidentBuild &B, int pass, unsigned int *longest, const ResidentRun *runs, uint2 *entries, StepState *state,
                           unsigned int blocks, cudaStream_t stream);
 }   // namespace b200

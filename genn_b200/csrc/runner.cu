@@ -66,6 +66,9 @@ int fail(int code, const char *fmt, ...)
 
 constexpr size_t STAGE_BYTES = 256 * 1024 - 64;  // page-locked buffer of a runner through which small arrays reach pageable memory
 constexpr size_t LARGE_PULL = 4u << 20;      // arrays from here on are copied out by several threads
+constexpr uint64_t FIRST_BLOCK = 2048;       // steps of the first launch of the target-resident kernel in a call, the next has twice as many
+constexpr uint64_t LONG_CALL = 10000;        // steps of a call from which the kernel that may have to take over is prepared first (and of any call once it had to)
+constexpr double MOST_LOSS = 1.0e6;          // ns that a call of the target-resident kernel may lose with no launch behind it
 constexpr size_t ARRAY_TAIL_PAD = 256;     // vector loads may read up to 15 bytes past the last element
 
 template<typename T>
@@ -326,6 +329,12 @@ struct b200_runner
     const void *residentKernel = nullptr;
     ResidentLaunch resident{};
     std::vector<void*> residentBuffers;
+    // busy networks (resident.h): the kernel with a grid barrier takes over
+    volatile unsigned long long *residentHold = nullptr;    // page-locked: until which step it goes on
+    bool residentHandsOver = false;         // the model's other path is that kernel (else: one launch per kernel, call by call)
+    float residentPatience = 200.0f;        // us
+    bool residentPatienceChosen = false;
+    double residentWorst = 0.0;             // ns that a step could lose, were every neuron to fire
 
     void dropResident()
     {
@@ -1092,9 +1101,19 @@ void arrayWritten(b200_runner *r, const void *p, size_t bytes)
     if(touchesSparse(r, p, bytes)) r->tiledStale = r->residentStale = true;
 }
 
-int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long numRec)
+// `goal`: not 0: the launch does what a launch of the target-resident kernel in front of it leaves of the steps up to there.
+int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long numRec, unsigned long long goal = 0)
 {
-    if(r->lagStale) {
+    if(goal && r->lagStale) {
+        // no time to look at the arrays: the schedule that needs no private copies of them (at a hundred spikes a step and more
+        // it is as fast as the others)
+        if(r->schedule != b200_runner::PLAIN) {
+            r->schedule = b200_runner::PLAIN;
+            r->dropUrgent();
+            if(const int e = buildFusedTables(r)) return e;
+        }
+    }
+    else if(r->lagStale) {
         const bool was = r->lagEligible;
         const int e = refreshSchedule(r);
         if(e) return e;
@@ -1139,6 +1158,7 @@ int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long 
     L.profile = r->fusedProfile ? 1u : 0u;
     L.cta_cycles = (r->fusedProfile && r->fusedGrid <= PROFILE_MAX_CTAS) ? r->fusedCtaCycles : nullptr;
     L.num_steps = numSteps;
+    L.goal = goal;
     L.barrier = r->fusedBarrier;
     L.rank = r->rank;
     L.world = r->world;
@@ -1158,11 +1178,11 @@ int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long 
             }
         }
     }
-    CUDA_TRY(cudaMemsetAsync(r->fusedBarrier, 0, sizeof(unsigned long long), r->stream));
+    if(!goal) CUDA_TRY(cudaMemsetAsync(r->fusedBarrier, 0, sizeof(unsigned long long), r->stream));      // (else the launch in front of it did)
     void *args[] = {&L};
     CUDA_TRY(cudaLaunchCooperativeKernel(r->fusedKernel, dim3(r->fusedGrid), dim3(FUSED_BLOCK), args,
                                          r->fusedStage ? r->fusedSmemBytes : 0, r->stream));
-    r->launches++;
+    if(!goal) r->launches++;        // (two launches that share their steps count as one)
     r->fusedLaunches++;
     return B200_OK;
 }
@@ -1435,6 +1455,7 @@ int buildResident(b200_runner *r)
     if(!coop) return no("no cooperative launch");
     ResidentLaunch &L = r->resident;
     L = ResidentLaunch{};
+    r->residentHandsOver = r->fusedEligible;
 
     // ---- ring depths, axonal delays, who feeds whom --------------------------------------------------------
     std::vector<unsigned int> unitStart{0}, depths, delays;
@@ -1500,8 +1521,8 @@ int buildResident(b200_runner *r)
     // ---- how many CTAs, how many warps ----------------------------------------------------------------------
     const NeuronShape shape = neuronShape(r);
     cudaFuncAttributes attr{};
-    r->residentKernel = residentKernelFor(shape.npsm, shape.ncs, depths.size() == 1 && numDelays == 1);
-    CUDA_TRY(cudaFuncGetAttributes(&attr, r->residentKernel));
+    const bool oneClass = depths.size() == 1 && numDelays == 1;
+    CUDA_TRY(cudaFuncGetAttributes(&attr, residentKernelFor(shape.npsm, shape.ncs, oneClass, RESIDENT_BLOCK)));     // (both instances share as much)
     unsigned int numSpans = 0;
     for(const auto &l : links) numSpans += (r->synapseGroups[l.syn].connectivity != B200_CONN_SPARSE);
     const unsigned int longestDelay = *std::max_element(delays.begin(), delays.end()), shortest = *std::min_element(delays.begin(), delays.end());
@@ -1528,6 +1549,9 @@ int buildResident(b200_runner *r)
     L.at.near = place(sizeof(ResidentNear) * numDelays * numGroups);
     L.at.spans = place(sizeof(ResidentSpan) * numSpans);
     L.at.poisson = place(sizeof(float) * poisson.size());
+    bool draws = false;
+    for(const auto &g : r->neuronGroups) draws = draws || g.model == B200_NEURON_POISSON;
+    L.at.undrawn = place(draws ? sizeof(unsigned int) * RESIDENT_BLOCK : 0);
     L.at.history = place(sizeof(unsigned int) * history * RESIDENT_UNITS);
     L.at.acc = place(0);
     int optin = 0;
@@ -1578,7 +1602,9 @@ int buildResident(b200_runner *r)
     const unsigned int neuronWarps = (units + grid - 1u) / grid;
     // (warps without neurons ask for the messages and build this CTA's own)
     unsigned int warps = r->residentWarps ? r->residentWarps : std::max(numSpans ? 16u : 8u, neuronWarps + (grid + 31u) / 32u);
+    if(neuronWarps <= RESIDENT_FEW / 32u && !r->residentWarps) warps = std::min(warps, RESIDENT_FEW / 32u);
     warps = std::min(std::max(warps, std::max(neuronWarps, (grid + 31u) / 32u)), RESIDENT_UNITS);
+    r->residentKernel = residentKernelFor(shape.npsm, shape.ncs, oneClass, warps * 32u);
 
     auto device = [&](size_t bytes, void **out) -> int {
         CUDA_TRY(poolAlloc(out, std::max<size_t>(bytes, 16), r->stream));
@@ -1627,7 +1653,7 @@ int buildResident(b200_runner *r)
     uint2 *dEntries = nullptr, *dNear = nullptr;
     if(!pairs.empty()) {
         unsigned long long cells = 0, nearCells = 0;
-        ScopedDevice longest(r->stream), sortedHold(r->stream), targetsHold(r->stream);
+        ScopedDevice totals(r->stream), longest(r->stream), sortedHold(r->stream), targetsHold(r->stream);
         CUDA_TRY(poolAlloc(&sortedHold.p, sizeof(b200_synapse_group) * sorted.size(), r->stream));
         CUDA_TRY(poolAlloc(&targetsHold.p, sizeof(unsigned int) * targets.size(), r->stream));
         CUDA_TRY(cudaMemcpyAsync(sortedHold.p, sorted.data(), sizeof(b200_synapse_group) * sorted.size(), cudaMemcpyHostToDevice, r->stream));
@@ -1635,6 +1661,8 @@ int buildResident(b200_runner *r)
         // longest run of every (CTA, pair), then longest row of delay-0 synapses of every pair
         const size_t numLongest = runs.size() + runsPerCta;
         CUDA_TRY(poolAlloc(&longest.p, sizeof(unsigned int) * numLongest, r->stream));
+        CUDA_TRY(poolAlloc(&totals.p, sizeof(unsigned long long) * runsPerCta, r->stream));
+        std::vector<unsigned long long> synapses(runsPerCta, 0ull);
         auto pass = [&](int which) -> int {
             for(const auto &pr : pairs) {
                 ResidentBuild B;
@@ -1651,6 +1679,7 @@ int buildResident(b200_runner *r)
                 B.near_longest = longest.as<unsigned int>() + runs.size() + at;
                 B.near = nears[at];
                 B.near_entries = dNear;
+                B.synapses = totals.as<unsigned long long>() + at;
                 CUDA_TRY(residentBuild(B, which, longest.as<unsigned int>() + at, dRuns ? dRuns + at : nullptr, dEntries, r->state,
                                        std::min(B.num_src, (unsigned int)sms * 8u), r->stream));
                 r->launches++;
@@ -1660,7 +1689,9 @@ int buildResident(b200_runner *r)
         std::vector<unsigned int> longestHost(numLongest);
         auto count = [&]() -> int {
             CUDA_TRY(cudaMemsetAsync(longest.p, 0, sizeof(unsigned int) * numLongest, r->stream));
+            CUDA_TRY(cudaMemsetAsync(totals.p, 0, sizeof(unsigned long long) * runsPerCta, r->stream));
             if(const int err = pass(0)) return err;
+            CUDA_TRY(cudaMemcpyAsync(synapses.data(), totals.p, sizeof(unsigned long long) * runsPerCta, cudaMemcpyDeviceToHost, r->stream));
             CUDA_TRY(cudaMemcpyAsync(longestHost.data(), longest.p, sizeof(unsigned int) * numLongest, cudaMemcpyDeviceToHost, r->stream));
             CUDA_TRY(cudaStreamSynchronize(r->stream));
             return B200_OK;
@@ -1694,6 +1725,28 @@ int buildResident(b200_runner *r)
             nearChunks = std::max(nearChunks, (nears[pair].length + 31u) / 32u);
             for(unsigned int c = 0; c < grid; c++) runs[c * runsPerCta + pair].row = row;
         }
+        // what a spike costs here above what it costs the kernel with a grid barrier
+        r->residentWorst = 0.0;
+        for(unsigned int a = 0; a < numDelays; a++) {
+            double sources = 0.0, all = 0.0;
+            for(size_t ni = 0; ni < numGroups; ni++) {
+                if(!((L.sources[a] >> ni) & 1ull)) continue;
+                sources += r->neuronGroups[ni].num_neurons;
+                all += (double)synapses[a * numGroups + ni];
+            }
+            const double here = (RESIDENT_RUN_COST * L.chunks[a] + RESIDENT_NEAR_COST * L.near_chunks[a]) / warps;
+            // (a model that the grid-barrier kernels do not take has only presynapticSparseKernel, no faster than this one per
+            // spike, and the tiled kernels, whose launches and flush take some 35 us)
+            const double there = !r->residentHandsOver ? 0.0 : (L.kind[a] == RESIDENT_SPLIT ? 0.02 : 0.0085) * all / std::max(1.0, sources);
+            L.weight[a] = (unsigned int)std::min(std::max(0.0, here - there) + 0.5, (double)RESIDENT_MOST_WEIGHT);
+            r->residentWorst += sources * L.weight[a] + std::max(0.0, sources / RESIDENT_LIST - 1.0) * RESIDENT_PIECE_COST;
+            // (with rings the exchange, which grows with the grid, and the delay-0 rows stand in front of the update: at ten spikes a
+            // step 63 CTAs gain 2.3 us on the other kernel, 148 gain 1.5)
+            const unsigned int spare = !r->residentHandsOver ? 35000u : (L.kind[a] == RESIDENT_LATE) ? 4000u :
+                (L.kind[a] == RESIDENT_SPLIT) ? 4500u - std::min(2500u, 15u * grid) : 3300u;
+            L.spare = L.spare ? std::min(L.spare, spare) : spare;
+        }
+        for(unsigned int a = 0; a < numDelays; a++) L.quiet[a] = L.weight[a] ? L.spare / (2u * L.weight[a]) : RESIDENT_LIST;
         // padded runs of a network with few synapses per (source neuron, CTA) pair can take several times the room of its
         // arrays: the copy may use a quarter of what is free
         size_t freeBytes = POOL_KEEP * 4, totalBytes = 0;       // (what the pool may keep needs no asking)
@@ -1753,12 +1806,19 @@ int buildResident(b200_runner *r)
     r->residentBlock = warps * 32u;
     r->residentSmem = tables + accFloats * sizeof(float);
     CUDA_TRY(cudaFuncSetAttribute(r->residentKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    if(!r->residentHold) {
+        void *word = nullptr;
+        CUDA_TRY(hostAcquire(&word, sizeof(unsigned long long)));
+        r->residentHold = static_cast<volatile unsigned long long*>(word);
+        *r->residentHold = 0ull;
+    }
+    L.hold = const_cast<unsigned long long*>(r->residentHold);
     r->residentReady = true;
     return B200_OK;
 }
 
-// `done`: steps done when the launch begins.
-int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long long numRec, unsigned long long done)
+// `done`: steps done when the launch begins; `leave`: a launch of the kernel with a grid barrier follows for what it leaves.
+int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long long numRec, unsigned long long done, bool leave)
 {
     ResidentLaunch &L = r->resident;
     L.neuron.groups = r->neuronTable.d;
@@ -1773,6 +1833,9 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
     L.neuron.ahead = L.neuron.advance = 0u;
     L.count_events = r->countEvents ? 1u : 0u;
     L.num_steps = (unsigned int)numSteps;
+    L.may_leave = leave ? 1u : 0u;
+    L.patience = (unsigned int)std::min(1000.0 * r->residentPatience, (double)RESIDENT_MOST_DEBT - 1.0);
+    L.barrier = r->fusedBarrier;
     // a message word is known by the last 20 bits of its step: before they repeat, no old word may be left.  (Steps on other
     // paths count too: they leave the words of earlier steps where they are.)
     if(r->residentCleared == ~0ull || done + numSteps - r->residentCleared >= RESIDENT_TAG_STEPS - 1ull) {
@@ -2164,6 +2227,7 @@ int b200_runner_destroy(b200_runner *r)
     poolFree(r->recList, r->stream);
     hostRelease(r->recHost);
     hostRelease(r->peakHost);
+    hostRelease(const_cast<unsigned long long*>(r->residentHold));
     if(r->peakEvent) cudaEventDestroy(r->peakEvent);
     if(r->ncclComm && ncclApi()) ncclApi()->commDestroy(r->ncclComm);
     poolFree(r->reducePacked, r->stream);
@@ -2586,6 +2650,11 @@ int b200_set_option(b200_runner *r, const char *name, double value)
     else if(n == "use_resident") { r->useResident = r->residentAsked = (value != 0.0); r->scheduleChosen = false; }
     else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; }
     else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; }
+    else if(n == "resident_patience") {
+        // (0: leaves in front of the first spike that costs more here)
+        r->residentPatience = (float)std::max(0.0, value);
+        r->residentPatienceChosen = true;
+    }
     else if(n == "use_lag") { r->useLag = (value != 0.0); r->lagStale = true; }
     else if(n == "use_split") { r->useSplit = (value != 0.0); r->lagStale = true; }
     else if(n == "use_near_queues") r->useNearQueues = (value != 0.0);
@@ -2763,12 +2832,30 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
     }
     bool resident = false;
     if(num_steps && (e = chooseResident(r, &resident)) != B200_OK) return e;
+    // (a busy network without the kernel with a grid barrier: one launch per kernel, call by call)
+    if(resident && !r->residentHandsOver && r->hostStepsDone < *r->residentHold) resident = false;
     if(resident) {
+        // The launches of a call grow, so that a network that was busy at first is tried again.  A call whose few steps cannot
+        // lose much has no second launch behind it (4 us).
+        const bool mayTakeOver = r->residentHandsOver && r->residentWorst > 0.0 && (num_steps >= LONG_CALL || *r->residentHold);
+        if(mayTakeOver && r->lagStale && (e = refreshSchedule(r)) != B200_OK) return e;
+        uint64_t block = r->residentHandsOver ? FIRST_BLOCK : RESIDENT_TAG_STEPS / 2;
         while(left) {
-            const uint64_t n = std::min<uint64_t>(left, RESIDENT_TAG_STEPS / 2);
-            e = launchResident(r, n, num_recording_timesteps, r->hostStepsDone + (num_steps - left));
+            const uint64_t done = r->hostStepsDone + (num_steps - left);
+            if(r->residentHandsOver && done < *r->residentHold) {
+                const uint64_t n = std::min<uint64_t>(left, *r->residentHold - done);
+                e = launchFused(r, n, num_recording_timesteps);
+                if(e) return e;
+                left -= n;
+                continue;
+            }
+            const uint64_t n = std::min<uint64_t>(left, std::min<uint64_t>(block, RESIDENT_TAG_STEPS / 2));
+            const bool leave = r->residentHandsOver && (r->residentPatienceChosen || (double)n * r->residentWorst > MOST_LOSS);
+            e = launchResident(r, n, num_recording_timesteps, done, leave);
+            if(e == B200_OK && leave) e = launchFused(r, n, num_recording_timesteps, done + n);
             if(e) return e;
             left -= n;
+            block *= 2;
         }
     }
     else if(r->useFused && r->fusedEligible && !r->timing) {
@@ -2988,6 +3075,12 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
         if(!e) e = chooseResident(r, &yes);
         if(e) return e;
         *value = yes ? 1u : 0u;
+        return B200_OK;
+    }
+    if(n == "resident_hold") {
+        // the step until which the kernel with a grid barrier takes a busy network's steps
+        CUDA_TRY(cudaStreamSynchronize(r->stream));
+        *value = r->residentHold ? *r->residentHold : 0u;
         return B200_OK;
     }
     if(n == "schedule") {

@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, 1)
 streamStepKernel(FusedLaunch L)
 {
     if(!SHARDED) L.world = 1u;
+    if(!SHARDED && !stepsLeft(L)) return;
     extern __shared__ __align__(16) unsigned char fusedSmem[];
     __shared__ StreamShared sh;
     __shared__ unsigned char *peerArena[B200_MAX_RANKS];

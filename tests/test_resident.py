@@ -278,3 +278,67 @@ def test_more_events_in_one_launch_than_32_bits_hold():
     assert rt.counter("spikes") == n * (steps + 1)
     assert rt.counter("synaptic_events") == groups * n * n * steps
     rt.close()
+
+
+def _busy(kind, synchronous):
+    """Sources that fire in every step, or two populations of which one fires as a whole in some steps."""
+    rng = np.random.default_rng(11)
+    m = GeNNModel("float", "busy")
+    m.dt, m.seed = 1.0, 23
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.3, "TauRefrac": 2.0}
+    src = m.add_neuron_population("in", 300, "Poisson", {"rate": 600.0 if synchronous else 150.0}, {"timeStepToSpike": 0.0})
+    trg = m.add_neuron_population("out", 3000 if synchronous else 200, "LIF", lif,
+                                  {"V": -65.0 if synchronous else rng.uniform(-65, -50, 200).astype(np.float32), "RefracTime": 0.0})
+    n = trg.num_neurons
+    for name, pop, delay in (("syn", src, 0), ("rec", trg, 0)) if kind != "two delays" else (("syn", src, 2), ("rec", trg, 0)):
+        pre = np.repeat(np.arange(pop.num_neurons, dtype=np.uint32), 10)
+        params = {"g": rng.uniform(0, 1e-5, len(pre)).astype(np.float32)}
+        if kind == "rings":
+            params["d"] = rng.integers(0, 6, len(pre)).astype(np.uint8)
+        sg = m.add_synapse_population(name, "BITMASK" if kind == "bit mask" and pop is src else "SPARSE", pop, trg,
+                                      init_weight_update("StaticPulseConstantWeight", {"g": 1e-5}) if kind == "bit mask" and pop is src else
+                                      init_weight_update("StaticPulseDendriticDelay" if kind == "rings" else "StaticPulse", {}, params), init_postsynaptic("ExpCurr", {"tau": 5.0}))
+        sg.set_sparse_connections(pre, rng.integers(0, n, len(pre)).astype(np.uint32))
+        sg.axonal_delay_steps = 3 if kind == "late" else delay
+        if kind == "rings":
+            sg.max_dendritic_delay_timesteps = 6
+    return m
+
+
+@pytest.mark.parametrize("synchronous", [False, True], ids=["patience 0", "more than the list holds"])
+@pytest.mark.parametrize("kind", ["immediate", "late", "rings", "two delays", "bit mask"])
+def test_a_busy_network_is_handed_over_and_taken_back(kind, synchronous):
+    """Launches that end early, the other kernel's share of their steps, and this kernel again: spikes and state of the CPU
+    checker at every end of a call, also where a step that had begun is left to the other kernel."""
+    from oracle.oracle import OracleRunner
+    net = resolve(_busy(kind, synchronous))
+    rt, orc = _runtime(net, 200), OracleRunner(resolve(_busy(kind, synchronous)), 200)
+    assert rt.counter("resident") == 1
+    rt.set_option("resident_patience", 1e6 if synchronous and kind != "bit mask" else 0)
+    holds, done = set(), 0
+    for n in (1, 2, 3, 5, 60, 1, 1, 40, 87):
+        rt.step_time(n)
+        orc.step(n)
+        done += n
+        holds.add(rt.counter("resident_hold"))
+        for p in net.pops:
+            assert np.array_equal(np.sort(rt.current_spikes(p.name)), np.sort(orc.current_spikes(p.name))), f"step {done} {p.name}"
+        helpers.assert_close(rt.array("out.V")[0], orc.array("out.V")[0], f"step {done} V", 1e-5, 5e-6)
+        for i in range(len(net.psms)):
+            helpers.assert_close(rt.array(f"psm{i}.out_post")[0], orc.array(f"psm{i}.out_post")[0], f"step {done} input {i}", 1e-5, 2e-6)
+    if (kind, synchronous) in (("two delays", True), ("bit mask", False)):
+        assert holds == {0}             # (several delays: lists are worked off one by one; too few spikes for the other path's kernels)
+    elif kind == "bit mask":
+        assert len(holds) >= 2, holds   # (from call to call)
+    else:
+        assert len(holds) >= 3, holds   # (left more than once)
+    rt.close()
+    orc.close()
+
+
+def test_a_quiet_network_stays():
+    net, rt, steps, _ = _resident("potjans_mini")
+    for n in (1, 40, 59):
+        rt.step_time(n)
+    assert rt.counter("resident_hold") == 0
+    rt.close()
