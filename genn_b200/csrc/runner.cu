@@ -320,6 +320,17 @@ struct b200_runner
     bool tiledChosen = false;               // the caller set what arms the tiled kernels: they serve whatever they can
     bool scheduleChosen = false;            // the caller picked a schedule of the other persistent kernels
     bool residentStale = true, residentReady = false;
+    bool residentOld = false;               // only weights have changed since the copy was made: it is filled again where it lies
+    // A program that changes the synapses again and again would pay for a copy every time: it is made (or filled) again when the steps on
+    // the model's other path, which reads the arrays, have cost as much as that
+    unsigned long long residentRent = 0;    // steps left to do there
+    double residentCells = 0.0;             // entries of the copy, millions
+    unsigned long long residentBuilds = 0;
+    struct ResidentPair { unsigned int delay_class, src, first, count; };
+    std::vector<ResidentPair> residentPairs;            // what the copy is filled from
+    std::vector<ResidentNear> residentNears;
+    const b200_synapse_group *residentGroups = nullptr; // (device)
+    const unsigned int *residentTargets = nullptr, *residentDepths = nullptr;
     std::string residentWhyNot;
     unsigned int residentCtas = 0, residentWarps = 0;       // 0: chosen by size
     unsigned int residentGrid = 0, residentBlock = 0;
@@ -769,6 +780,7 @@ int prepare(b200_runner *r)
     r->fusedGroups = sparse;
     r->lagStale = true;
     r->tiledStale = r->residentStale = true;
+    r->residentRent = 0;
     r->schedule = b200_runner::PLAIN;
     r->dropUrgent();
     {
@@ -1077,28 +1089,43 @@ bool touchesDelays(const b200_runner *r, const void *p, size_t bytes)
     return false;
 }
 
-// true if [p, p + bytes) overlaps an array the tile-major copy of the SPARSE groups was made from
-bool touchesSparse(const b200_runner *r, const void *p, size_t bytes)
+// Which arrays of SPARSE groups that private copies are made from [p, p + bytes) overlaps: 1 weights, 2 any other.
+unsigned int touchesSparse(const b200_runner *r, const void *p, size_t bytes)
 {
     const unsigned char *a = static_cast<const unsigned char*>(p), *b = a + bytes;
     auto overlaps = [&](const void *start, size_t size) {
         const unsigned char *s0 = static_cast<const unsigned char*>(start);
         return s0 && a < s0 + size && b > s0;
     };
+    unsigned int which = 0;
     for(const auto &g : r->synapseGroups) {
         if(g.connectivity != B200_CONN_SPARSE || g.wu_model == B200_WU_STDP) continue;
         const size_t synapses = (size_t)g.num_src * g.row_stride;
-        if(overlaps(g.d, synapses) || overlaps(g.row_length, sizeof(unsigned int) * g.num_src) ||
-           overlaps(g.ind, synapses * g.ind_bytes) || overlaps(g.g, synapses * sizeof(float))) return true;
+        if(overlaps(g.g, synapses * sizeof(float))) which |= 1u;
+        if(overlaps(g.d, synapses) || overlaps(g.row_length, sizeof(unsigned int) * g.num_src) || overlaps(g.ind, synapses * g.ind_bytes)) which |= 2u;
     }
-    return false;
+    return which;
 }
 
 // [p, p + bytes) gets other values: the private copies made from it have to be made again before they are next used.
 void arrayWritten(b200_runner *r, const void *p, size_t bytes)
 {
     if(touchesDelays(r, p, bytes)) { r->lagStale = true; r->nearDataStale = true; }
-    if(touchesSparse(r, p, bytes)) r->tiledStale = r->residentStale = true;
+    const unsigned int which = touchesSparse(r, p, bytes);
+    if(!which) return;
+    r->tiledStale = true;
+    if(!r->residentReady || r->residentStale) {
+        r->residentStale = true;
+        return;
+    }
+    if(which & 2u) r->residentStale = true;
+    else r->residentOld = true;
+    // Filling takes 12 us and 6.2 for every million entries, making anew 100 and 60 (allocations, two waits); a step here takes some
+    // 3.3 us less.  With rings the other path would have to make its own table of delay-0 and -1 synapses first, which takes longer.
+    bool rings = false;
+    for(unsigned int a = 0; a < r->resident.num_delays; a++) rings = rings || r->resident.kind[a] == RESIDENT_SPLIT;
+    const double cost = r->residentStale ? 100.0 + 60.0 * r->residentCells : 12.0 + 6.2 * r->residentCells;
+    r->residentRent = rings ? 0ull : (unsigned long long)(cost / 3.3);
 }
 
 // `goal`: not 0: the launch does what a launch of the target-resident kernel in front of it leaves of the steps up to there.
@@ -1438,12 +1465,46 @@ TiledLaunch tiledLaunch(const b200_runner *r)
     return L;
 }
 
+// Counts (pass 0) or places (pass 1) the synapses of the target-resident kernel's copy.  Placed again over what it holds, other
+// weights of the same synapses fill the same places (in another order within a run).
+int residentPass(b200_runner *r, int which, unsigned int *longest, unsigned long long *totals)
+{
+    const ResidentLaunch &L = r->resident;
+    const size_t numGroups = r->neuronGroups.size(), runsPerCta = (size_t)r->residentNears.size();
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
+    for(const auto &pr : r->residentPairs) {
+        ResidentBuild B;
+        B.groups = r->residentGroups + pr.first;
+        B.target = r->residentTargets + pr.first;
+        B.num_groups = pr.count;
+        B.num_src = r->neuronGroups[pr.src].num_neurons;
+        B.unit_start = L.unit_start; B.columns = L.columns; B.depth = r->residentDepths; B.grid = r->residentGrid;
+        B.runs_stride = (unsigned int)runsPerCta;
+        if(!B.num_src) continue;
+        const size_t at = (size_t)pr.delay_class * numGroups + pr.src;
+        B.late = (L.kind[pr.delay_class] == RESIDENT_LATE);
+        B.split = (L.kind[pr.delay_class] == RESIDENT_SPLIT);
+        // longest run of every (CTA, pair), then longest row of delay-0 synapses of every pair
+        B.near_longest = longest ? longest + runsPerCta * r->residentGrid + at : nullptr;
+        B.near = r->residentNears[at];
+        B.near_entries = const_cast<uint2*>(L.near_entries);
+        B.synapses = totals ? totals + at : nullptr;
+        CUDA_TRY(residentBuild(B, which, longest ? longest + at : nullptr, L.runs ? L.runs + at : nullptr, const_cast<uint2*>(L.entries), r->state,
+                               std::min(B.num_src, (unsigned int)sms * 8u), r->stream));
+        r->launches++;
+    }
+    return B200_OK;
+}
+
 // (Re)build the tables of the target-resident kernel; leaves residentReady false, with the reason, where the model does
 // not qualify.  Runs when a block of steps is first asked for and after the arrays it copies changed.
 int buildResident(b200_runner *r)
 {
     r->dropResident();
-    r->residentStale = false;
+    r->residentStale = r->residentOld = false;
+    r->residentRent = 0;
+    r->residentBuilds++;
     r->residentWhyNot.clear();
     auto no = [&](const char *why) { r->residentWhyNot = why; return B200_OK; };
     if(r->batch != 1 || r->sharded()) return no("batch or sharded model");
@@ -1630,11 +1691,11 @@ int buildResident(b200_runner *r)
     std::vector<ResidentRun> runs(runsPerCta * grid, ResidentRun{0, 0, 0});
     std::vector<b200_synapse_group> sorted;
     std::vector<unsigned int> targets;
-    struct Pair { unsigned int delayClass, src, first, count; };
-    std::vector<Pair> pairs;
+    std::vector<b200_runner::ResidentPair> &pairs = r->residentPairs;
+    pairs.clear();
     for(unsigned int a = 0; a < numDelays; a++) {
         for(unsigned int ni = 0; ni < numGroups; ni++) {
-            Pair pr{a, ni, (unsigned int)sorted.size(), 0u};
+            b200_runner::ResidentPair pr{a, ni, (unsigned int)sorted.size(), 0u};
             for(const auto &l : links) {
                 const auto &g = r->synapseGroups[l.syn];
                 if(l.delayClass != a || l.src != ni) continue;
@@ -1648,49 +1709,29 @@ int buildResident(b200_runner *r)
         }
     }
     for(unsigned int a = 0; a < numDelays; a++) L.source_groups |= L.sources[a];
-    std::vector<ResidentNear> nears(runsPerCta, ResidentNear{0, 0, 0, 0});
+    std::vector<ResidentNear> &nears = r->residentNears;
+    nears.assign(runsPerCta, ResidentNear{0, 0, 0, 0});
+    r->residentCells = 0.0;
     ResidentRun *dRuns = nullptr;
     uint2 *dEntries = nullptr, *dNear = nullptr;
     if(!pairs.empty()) {
         unsigned long long cells = 0, nearCells = 0;
-        ScopedDevice totals(r->stream), longest(r->stream), sortedHold(r->stream), targetsHold(r->stream);
-        CUDA_TRY(poolAlloc(&sortedHold.p, sizeof(b200_synapse_group) * sorted.size(), r->stream));
-        CUDA_TRY(poolAlloc(&targetsHold.p, sizeof(unsigned int) * targets.size(), r->stream));
-        CUDA_TRY(cudaMemcpyAsync(sortedHold.p, sorted.data(), sizeof(b200_synapse_group) * sorted.size(), cudaMemcpyHostToDevice, r->stream));
-        CUDA_TRY(cudaMemcpyAsync(targetsHold.p, targets.data(), sizeof(unsigned int) * targets.size(), cudaMemcpyHostToDevice, r->stream));
-        // longest run of every (CTA, pair), then longest row of delay-0 synapses of every pair
+        ScopedDevice totals(r->stream), longest(r->stream);
+        if(const int err = upload(sorted.data(), sizeof(b200_synapse_group) * sorted.size(), (void**)&r->residentGroups)) return err;
+        if(const int err = upload(targets.data(), sizeof(unsigned int) * targets.size(), (void**)&r->residentTargets)) return err;
+        r->residentDepths = dDepths;
+        L.unit_start = dUnitStart;
+        L.columns = dColumns;
+        r->residentGrid = grid;
         const size_t numLongest = runs.size() + runsPerCta;
         CUDA_TRY(poolAlloc(&longest.p, sizeof(unsigned int) * numLongest, r->stream));
         CUDA_TRY(poolAlloc(&totals.p, sizeof(unsigned long long) * runsPerCta, r->stream));
         std::vector<unsigned long long> synapses(runsPerCta, 0ull);
-        auto pass = [&](int which) -> int {
-            for(const auto &pr : pairs) {
-                ResidentBuild B;
-                B.groups = sortedHold.as<b200_synapse_group>() + pr.first;
-                B.target = targetsHold.as<unsigned int>() + pr.first;
-                B.num_groups = pr.count;
-                B.num_src = r->neuronGroups[pr.src].num_neurons;
-                B.unit_start = dUnitStart; B.columns = dColumns; B.depth = dDepths; B.grid = grid;
-                B.runs_stride = (unsigned int)runsPerCta;
-                if(!B.num_src) continue;
-                const size_t at = (size_t)pr.delayClass * numGroups + pr.src;
-                B.late = (L.kind[pr.delayClass] == RESIDENT_LATE);
-                B.split = (L.kind[pr.delayClass] == RESIDENT_SPLIT);
-                B.near_longest = longest.as<unsigned int>() + runs.size() + at;
-                B.near = nears[at];
-                B.near_entries = dNear;
-                B.synapses = totals.as<unsigned long long>() + at;
-                CUDA_TRY(residentBuild(B, which, longest.as<unsigned int>() + at, dRuns ? dRuns + at : nullptr, dEntries, r->state,
-                                       std::min(B.num_src, (unsigned int)sms * 8u), r->stream));
-                r->launches++;
-            }
-            return B200_OK;
-        };
         std::vector<unsigned int> longestHost(numLongest);
         auto count = [&]() -> int {
             CUDA_TRY(cudaMemsetAsync(longest.p, 0, sizeof(unsigned int) * numLongest, r->stream));
             CUDA_TRY(cudaMemsetAsync(totals.p, 0, sizeof(unsigned long long) * runsPerCta, r->stream));
-            if(const int err = pass(0)) return err;
+            if(const int err = residentPass(r, 0, longest.as<unsigned int>(), totals.as<unsigned long long>())) return err;
             CUDA_TRY(cudaMemcpyAsync(synapses.data(), totals.p, sizeof(unsigned long long) * runsPerCta, cudaMemcpyDeviceToHost, r->stream));
             CUDA_TRY(cudaMemcpyAsync(longestHost.data(), longest.p, sizeof(unsigned int) * numLongest, cudaMemcpyDeviceToHost, r->stream));
             CUDA_TRY(cudaStreamSynchronize(r->stream));
@@ -1761,7 +1802,11 @@ int buildResident(b200_runner *r)
         if(const int err = device(sizeof(uint2) * nearCells, (void**)&dNear)) return err;
         CUDA_TRY(cudaMemsetAsync(dNear, 0xFF, sizeof(uint2) * nearCells, r->stream));
         if(const int err = upload(runs.data(), sizeof(ResidentRun) * runs.size(), (void**)&dRuns)) return err;
-        if(const int err = pass(1)) return err;
+        L.runs = dRuns;
+        L.entries = dEntries;
+        L.near_entries = dNear;
+        r->residentCells = 1e-6 * (double)(cells + nearCells);
+        if(const int err = residentPass(r, 1, nullptr, nullptr)) return err;
         CUDA_TRY(cudaStreamSynchronize(r->stream));         // (the temporaries go out of scope)
     }
     else if(const int err = upload(runs.data(), sizeof(ResidentRun) * runs.size(), (void**)&dRuns)) return err;
@@ -1856,10 +1901,26 @@ int chooseResident(b200_runner *r, bool *yes)
     // (a private copy would not see what the program writes into an array by itself)
     for(void *p : r->exposed) if(!r->residentAsked && touchesSparse(r, p, 1)) return B200_OK;
     if(!r->useFused || !r->useResident || r->scheduleChosen || r->timing || r->sharded() || r->batch != 1) return B200_OK;
-    if(r->residentStale) {
+    if(r->residentStale && !(r->residentReady && r->residentRent)) {
         if(const int e = buildResident(r)) { r->dropResident(); return e; }
     }
     *yes = r->residentReady;
+    return B200_OK;
+}
+
+// The copy as the arrays are now (nothing, if it is).
+int refreshResident(b200_runner *r)
+{
+    r->residentRent = 0;
+    if(r->residentStale) {
+        const int e = buildResident(r);
+        if(e) r->dropResident();
+        return e;
+    }
+    if(r->residentOld) {
+        r->residentOld = false;
+        return residentPass(r, 1, nullptr, nullptr);
+    }
     return B200_OK;
 }
 
@@ -2648,8 +2709,8 @@ int b200_set_option(b200_runner *r, const char *name, double value)
     else if(n == "use_graph") r->useGraph = (value != 0.0);
     else if(n == "use_fused") r->useFused = (value != 0.0);
     else if(n == "use_resident") { r->useResident = r->residentAsked = (value != 0.0); r->scheduleChosen = false; }
-    else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; }
-    else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; }
+    else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; r->residentRent = 0; }
+    else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; r->residentRent = 0; }
     else if(n == "resident_patience") {
         // (0: leaves in front of the first spike that costs more here)
         r->residentPatience = (float)std::max(0.0, value);
@@ -2665,7 +2726,10 @@ int b200_set_option(b200_runner *r, const char *name, double value)
     else if(n == "use_emit") { r->useEmit = (value != 0.0); r->lagStale = true; }
     else if(n == "stream_warps") { r->streamWarpsWanted = (int)value; r->lagStale = true; }
     else if(n == "lag_agreed") { r->lagAgreed = (value != 0.0); r->lagStale = true; }
-    else if(n == "rescan_delays") r->lagStale = r->tiledStale = r->residentStale = true;
+    else if(n == "rescan_delays") {
+        r->lagStale = true;
+        for(const auto &g : r->synapseGroups) if(g.row_length) arrayWritten(r, g.row_length, sizeof(unsigned int) * g.num_src);
+    }
     else if(n == "fused_profile") {
         // (the per-CTA cycle counters are allocated here, not on the time-step path)
         r->fusedProfile = (value != 0.0);
@@ -2833,7 +2897,17 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
     bool resident = false;
     if(num_steps && (e = chooseResident(r, &resident)) != B200_OK) return e;
     // (a busy network without the kernel with a grid barrier: one launch per kernel, call by call)
-    if(resident && !r->residentHandsOver && r->hostStepsDone < *r->residentHold) resident = false;
+    if(resident && !r->residentHandsOver) {
+        if(r->hostStepsDone < *r->residentHold) resident = false;
+        else if(num_steps <= r->residentRent) {
+            r->residentRent -= num_steps;
+            resident = false;
+        }
+        else {
+            if((e = refreshResident(r)) != B200_OK) return e;
+            resident = r->residentReady;
+        }
+    }
     if(resident) {
         // The launches of a call grow, so that a network that was busy at first is tried again.  A call whose few steps cannot
         // lose much has no second launch behind it (4 us).
@@ -2847,6 +2921,19 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
                 e = launchFused(r, n, num_recording_timesteps);
                 if(e) return e;
                 left -= n;
+                r->residentRent -= std::min<unsigned long long>(r->residentRent, n);
+                continue;
+            }
+            if(r->residentRent || !r->residentReady) {
+                const uint64_t n = r->residentReady ? std::min<uint64_t>(left, r->residentRent) : left;
+                e = launchFused(r, n, num_recording_timesteps);
+                if(e) return e;
+                left -= n;
+                r->residentRent -= std::min<unsigned long long>(r->residentRent, n);
+                continue;
+            }
+            if(r->residentStale || r->residentOld) {
+                if((e = refreshResident(r)) != B200_OK) return e;
                 continue;
             }
             const uint64_t n = std::min<uint64_t>(left, std::min<uint64_t>(block, RESIDENT_TAG_STEPS / 2));
@@ -3075,6 +3162,11 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
         if(!e) e = chooseResident(r, &yes);
         if(e) return e;
         *value = yes ? 1u : 0u;
+        return B200_OK;
+    }
+    if(n == "resident_builds") {
+        // how often the copy has been made (not: filled again with other weights)
+        *value = r->residentBuilds;
         return B200_OK;
     }
     if(n == "resident_hold") {

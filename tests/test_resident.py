@@ -342,3 +342,34 @@ def test_a_quiet_network_stays():
         rt.step_time(n)
     assert rt.counter("resident_hold") == 0
     rt.close()
+
+
+@pytest.mark.parametrize("kind", ["immediate", "late", "rings", "two delays", "bit mask"])
+def test_synapses_changed_between_calls_of_every_length(kind):
+    """Weights, then rows, pushed in front of calls of one step and of many: on the other path, on a copy filled again, on a copy
+    made again and in the middle of a call, the arrays are those pushed last."""
+    net = resolve(_busy(kind, False))
+    rt, other = _runtime(net, 10), _runtime(resolve(_busy(kind, False)), 10)
+    other.set_option("use_fused", 0)
+    other.set_option("use_tiled", 0)
+    assert rt.counter("resident") == 1 and rt.counter("resident_builds") == 1
+    rng = np.random.default_rng(5)
+    g, rows = net.syn("rec").g.copy(), net.syn("rec").row_length.copy()
+    for n in (1, 1, 2, 300, 1, 40, 1):
+        g = (g * rng.uniform(0.2, 3.0)).astype(np.float32)
+        for r in (rt, other):
+            r.plan.push("rec.g", g)
+            r.step_time(n)
+        helpers.assert_close(rt.array("out.V")[0], other.array("out.V")[0], f"V after {n} steps", 1e-5, 5e-6)
+    for i in range(len(net.psms)):
+        helpers.assert_close(rt.array(f"psm{i}.out_post")[0], other.array(f"psm{i}.out_post")[0], f"input {i}", 1e-5, 2e-6)
+    assert rt.counter("resident_builds") == 1, "other weights of the same synapses fill the copy where it lies"
+    for n in (1, 2, 600, 1):
+        rows = np.minimum(rows, rng.integers(3, 11, len(rows)).astype(np.uint32))
+        for r in (rt, other):
+            r.plan.push("rec.row_length", rows)
+            r.step_time(n)
+        helpers.assert_close(rt.array("out.V")[0], other.array("out.V")[0], f"V after {n} steps", 1e-5, 5e-6)
+    assert rt.counter("resident") == 1 and 1 < rt.counter("resident_builds") <= 5
+    rt.close()
+    other.close()
