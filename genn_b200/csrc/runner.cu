@@ -2708,7 +2708,17 @@ int b200_set_option(b200_runner *r, const char *name, double value)
     else if(n == "count_events") r->countEvents = (value != 0.0);
     else if(n == "use_graph") r->useGraph = (value != 0.0);
     else if(n == "use_fused") r->useFused = (value != 0.0);
-    else if(n == "use_resident") { r->useResident = r->residentAsked = (value != 0.0); r->scheduleChosen = false; }
+    else if(n == "use_resident") {
+        r->useResident = r->residentAsked = (value != 0.0);
+        r->scheduleChosen = false;
+        if(!r->useResident && !r->residentBuffers.empty()) {
+            // its copy of the synapses goes back
+            CUDA_TRY(cudaSetDevice(r->device));
+            r->dropResident();
+            r->residentStale = true;
+            r->residentRent = 0;
+        }
+    }
     else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; r->residentRent = 0; }
     else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; r->residentRent = 0; }
     else if(n == "resident_patience") {
@@ -3162,6 +3172,10 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
         if(!e) e = chooseResident(r, &yes);
         if(e) return e;
         *value = yes ? 1u : 0u;
+        return B200_OK;
+    }
+    if(n == "resident_bytes") {
+        *value = r->residentReady ? (uint64_t)(r->residentCells * 1e6 * sizeof(uint2) + 0.5) : 0u;
         return B200_OK;
     }
     if(n == "resident_builds") {

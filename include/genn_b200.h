@@ -394,7 +394,8 @@ int  b200_get_counter(b200_runner *r, const char *name, uint64_t *value);
  * tiled kernel's unit of work, handed to one warp, is sized for about that many synaptic events, default 2048;
  * its fixed cost in synaptic events when a step's work is cut into equal stretches per CTA, default 256),
  * "use_resident" (default 1: batch-1 networks without learning and PROCEDURAL groups run on the target-resident kernel, which
- * works on a private copy of the SPARSE groups; counter "resident": whether the next steps do), "resident_ctas" /
+ * works on a private copy of the SPARSE groups, 8 bytes an entry, padded per block of targets: 12 to 26 bytes a synapse,
+ * measured; 0 gives it back.  Counter "resident": whether the next steps run on it, "resident_bytes": the copy's size), "resident_ctas" /
  * "resident_warps" (its grid and block; 0: chosen by size), "resident_patience" (microseconds that it may lose to the kernel with a
  * grid barrier, which is faster from some 100 spikes a step on, before that one takes over for a while; default 200; counter
  * "resident_hold": the step until which; "resident_builds": how often the copy was made),

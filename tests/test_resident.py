@@ -242,7 +242,7 @@ def test_messages_of_steps_long_ago_are_not_taken_for_new_ones():
     assert rt.counter("resident") == 1
     rt.step_time(4)
     assert rt.array("psm0.out_post").max() > 1.0 and rt.array("psm1.out_post").max() > 1.0
-    rt.set_option("use_resident", 0)
+    rt.set_option("use_lag", 1)                 # (one of the kernels with a grid barrier; the message buffers stay)
     rt.step_time((1 << 20) - 4)
     rt.set_option("use_resident", 1)
     rt.set_option("count_events", 1)
@@ -373,3 +373,33 @@ def test_synapses_changed_between_calls_of_every_length(kind):
     assert rt.counter("resident") == 1 and 1 < rt.counter("resident_builds") <= 5
     rt.close()
     other.close()
+
+
+def test_the_private_copy_goes_back_when_the_kernel_is_switched_off():
+    import torch
+    rng = np.random.default_rng(1)
+    m = GeNNModel("float", "memory")
+    m.dt = 1.0
+    lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.0, "TauRefrac": 2.0}
+    a = m.add_neuron_population("a", 40000, "LIF", lif, {"V": -65.0, "RefracTime": 0.0})
+    sg = m.add_synapse_population("syn", "SPARSE", a, a, init_weight_update("StaticPulseConstantWeight", {"g": 0.1}), init_postsynaptic("ExpCurr", {"tau": 5.0}))
+    pre = np.repeat(np.arange(40000, dtype=np.uint32), 500)
+    sg.set_sparse_connections(pre, rng.integers(0, 40000, len(pre)).astype(np.uint32), presorted=True)
+    m.build()
+    m.load()
+    rt = m._runtime
+    assert rt.counter("resident") == 1
+    size = rt.counter("resident_bytes")
+    assert 8 * len(pre) <= size <= 5 * 8 * len(pre)
+    rt.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    rt.set_option("use_resident", 0)
+    rt.step_time(5)
+    rt.synchronize()
+    assert rt.counter("resident_bytes") == 0
+    assert torch.cuda.mem_get_info()[0] - before >= size          # (more than the pool keeps for one allocation)
+    rt.set_option("use_resident", 1)
+    rt.step_time(5)
+    rt.synchronize()
+    assert rt.counter("resident_bytes") == size
+    m.unload()
