@@ -43,6 +43,8 @@ struct StepState
     unsigned long long barrier_spin_limit;
     unsigned long long exchange_spin_limit;
     long long stream_wait_cycles;
+    // polls for a copy into shared memory (dense_batch.cuh, sparse_batch.cuh)
+    unsigned int copy_wait_limit;
     // target-resident kernel (resident.h: "Busy networks"): what it has lost to the kernel with a grid barrier (ns), the step
     // until which that one goes on in its place, and for how many steps it last did
     unsigned int resident_debt;
@@ -54,6 +56,23 @@ constexpr unsigned int ERR_SPIKE_OVERFLOW = 1u;
 constexpr unsigned int ERR_IND_RANGE = 2u;
 constexpr unsigned int ERR_DELAY_RANGE = 4u;
 constexpr unsigned int ERR_BARRIER_TIMEOUT = 8u;
+constexpr unsigned int ERR_COPY_TIMEOUT = 64u;          // (32: ERR_EXCHANGE_TIMEOUT)
+
+// Polls for a copy into shared memory, unless the host set another limit.  A kernel that gives up waits, this long again, for what
+// it has sent for: nothing may arrive in a block's shared memory after the block.
+constexpr unsigned int COPY_WAITS = 1u << 18;
+
+// Waits for a phase of a shared-memory barrier.
+__device__ __forceinline__ bool copyArrived(const unsigned long long *bar, unsigned int parity, unsigned int polls)
+{
+    for(unsigned int i = 0; i < polls; i++) {
+        unsigned int done;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(done) : "r"((unsigned int)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
+        if(done) return true;
+    }
+    return false;
+}
 
 // Block -> merged-group element lookup: block_start[g] is the first block of
 // group g, block_start[num_groups] the grid size.  Linear for a handful of

@@ -27,7 +27,6 @@ constexpr unsigned int DENSE_COPIES = 32;           // copies of a CTA: one mask
 constexpr unsigned int DENSE_OWN = DENSE_COPIES / DENSE_WARPS;      // copies of a warp
 constexpr unsigned int DENSE_STAGES = 3;
 constexpr unsigned int DENSE_PER_SM = 2;            // CTAs on an SM: 96 KB of stages each
-constexpr unsigned int DENSE_WAITS = 1u << 18;      // polls for a stage before the step is given up
 constexpr unsigned int DENSE_WINDOW = 1024;         // most source neurons of a CTA (masks and list: 6 KB)
 // A CTA reads all spike lists to find its own sources: worth it while those are a small part of what it reads of the rows.
 constexpr unsigned int DENSE_MOST_SOURCES = 65536;
@@ -45,17 +44,6 @@ struct DenseLaunch
 constexpr size_t DENSE_SMEM = DENSE_STAGES * 32 * DENSE_COLS * sizeof(float) + DENSE_WINDOW * (sizeof(unsigned int) + sizeof(uint16_t));
 
 __device__ __forceinline__ unsigned int denseShare(const void *p) { return (unsigned int)__cvta_generic_to_shared(p); }
-
-// Waits (with a limit) for the bytes of a stage.
-__device__ __forceinline__ bool denseArrived(unsigned long long *bar, unsigned int parity)
-{
-    for(unsigned int i = 0; i < DENSE_WAITS; i++) {
-        unsigned int done;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(done) : "r"(denseShare(bar)), "r"(parity) : "memory");
-        if(done) return true;
-    }
-    return false;
-}
 
 __device__ __forceinline__ void denseSum(float4 &sum, const float4 &v)
 {
@@ -92,7 +80,7 @@ denseBatchKernel(const DenseLaunch L)
     for(unsigned int i = threadIdx.x; i < part.w; i += DENSE_BLOCK) mask[i] = 0u;
     __syncthreads();
     chainWait();
-    const unsigned int k = chainPhase(L.S.state, L.S.ahead);
+    const unsigned int k = chainPhase(L.S.state, L.S.ahead), polls = L.S.state->copy_wait_limit;
     const unsigned int slots = g.src_delay_slots, slot = ringSlot(k + slots - g.axonal_delay, slots);
 
     // ---- spike lists -> masks of this CTA's sources: the lists of a warp's copies side by side
@@ -146,12 +134,11 @@ denseBatchKernel(const DenseLaunch L)
     const float *const base = constant ? nullptr : g.g + (unsigned long long)part.z * rowStride + part.y;
     const unsigned int numStages = constant ? 0u : (rows + 31u) / 32u;
     if(warp == DENSE_WARPS) {
-        bool room = true;
-        for(unsigned int stage = 0; stage < numStages && room; stage++) {
+        unsigned int stage = 0;
+        for(; stage < numStages; stage++) {
             const unsigned int ring = stage % DENSE_STAGES;
-            if(stage >= DENSE_STAGES) room = denseArrived(&released[ring], (stage / DENSE_STAGES - 1u) & 1u);
-            if(!room) {
-                atomicOr(&L.S.state->error, ERR_BARRIER_TIMEOUT);
+            if(stage >= DENSE_STAGES && !__all_sync(0xFFFFFFFFu, copyArrived(&released[ring], (stage / DENSE_STAGES - 1u) & 1u, polls))) {
+                if(lane == 0u) atomicOr(&L.S.state->error, ERR_COPY_TIMEOUT);
                 break;
             }
             float *const to = stages + ring * 32u * DENSE_COLS;
@@ -175,6 +162,10 @@ denseBatchKernel(const DenseLaunch L)
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(bar) : "memory");
             }
         }
+        // (the others wait for every stage too, unless they have given up)
+        for(unsigned int sent = stage > DENSE_STAGES ? stage - DENSE_STAGES : 0u; sent < stage; sent++) {
+            copyArrived(&arrived[sent % DENSE_STAGES], (sent / DENSE_STAGES) & 1u, COPY_WAITS);
+        }
         return;
     }
     // fewer copies than warps: several warps share a copy, each with every `sharers`-th row
@@ -185,11 +176,13 @@ denseBatchKernel(const DenseLaunch L)
     #pragma unroll
     for(unsigned int o = 0; o < DENSE_OWN; o++) sum[o][0] = sum[o][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     unsigned int ring = 0, parity = 0;
-    bool there = true;
     for(unsigned int stage = 0; stage < numStages; stage++) {
-        there = there && denseArrived(&arrived[ring], parity);
+        if(!__all_sync(0xFFFFFFFFu, copyArrived(&arrived[ring], parity, polls))) {
+            if(lane == 0u) atomicOr(&L.S.state->error, ERR_COPY_TIMEOUT);
+            return;
+        }
         const unsigned int at = stage * 32u + lane;
-        const unsigned int m = (mine && there && at < rows) ? mask[list[at]] >> first : 0u;
+        const unsigned int m = (mine && at < rows) ? mask[list[at]] >> first : 0u;
         const float4 *const w = reinterpret_cast<const float4*>(stages + ring * 32u * DENSE_COLS) + lane;
         #pragma unroll
         for(unsigned int o = 0; o < DENSE_OWN; o++) {
@@ -216,7 +209,6 @@ denseBatchKernel(const DenseLaunch L)
         }
         __syncwarp();
         if(lane == 0u) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(denseShare(&released[ring])) : "memory");
-        if(!there) atomicOr(&L.S.state->error, ERR_BARRIER_TIMEOUT);
         if(++ring == DENSE_STAGES) {
             ring = 0;
             parity ^= 1u;

@@ -2202,6 +2202,8 @@ int b200_runner_create(int device, double dt, uint64_t seed, uint32_t batch_size
     {
         const unsigned long long limits[3] = {BARRIER_SPIN_LIMIT, EXCHANGE_SPIN_LIMIT, (unsigned long long)STREAM_WAIT_CYCLES};
         CUDA_TRY(cudaMemcpyAsync(&r->state->barrier_spin_limit, limits, sizeof(limits), cudaMemcpyHostToDevice, r->stream));
+        const unsigned int polls = COPY_WAITS;
+        CUDA_TRY(cudaMemcpyAsync(&r->state->copy_wait_limit, &polls, sizeof(polls), cudaMemcpyHostToDevice, r->stream));
     }
     CUDA_TRY(cudaEventCreate(&r->evA));
     CUDA_TRY(cudaEventCreate(&r->evB));
@@ -2762,6 +2764,12 @@ int b200_set_option(b200_runner *r, const char *name, double value)
         CUDA_TRY(cudaStreamSynchronize(r->stream));
         CUDA_TRY(cudaMemcpyAsync(dst, &v, sizeof(v), cudaMemcpyHostToDevice, r->stream));
     }
+    else if(n == "copy_wait_limit") {
+        // polls for a copy into shared memory; 0: none is waited for, so that every step of the kernels that use them fails
+        const unsigned int polls = (unsigned int)std::min(std::max(0.0, value), 4.0e9);
+        CUDA_TRY(cudaStreamSynchronize(r->stream));
+        CUDA_TRY(cudaMemcpyAsync(&r->state->copy_wait_limit, &polls, sizeof(polls), cudaMemcpyHostToDevice, r->stream));
+    }
     else if(n == "scatter_min_spikes") { r->scatterMinSpikes = (float)value; r->peakSeen = false; r->dirty = true; }
     else if(n == "use_tiled") { r->useTiled = (value != 0.0); r->tiledStale = true; }
     else if(n == "tiled_min_events") { r->tiledMinEvents = (float)value; r->tiledChosen = r->dirty = true; }
@@ -3116,12 +3124,13 @@ static int reportDeviceError(b200_runner *r, unsigned int err)
     if(!err) return B200_OK;
     cudaMemsetAsync(&r->state->error, 0, sizeof(unsigned int), r->stream);
     r->residentCleared = ~0ull;         // (a launch that gave up may have left messages of steps that count again)
-    return fail(B200_ERR_DEVICE_CHECK, "device-side check failed (flags 0x%x:%s%s%s%s%s)", err,
+    return fail(B200_ERR_DEVICE_CHECK, "device-side check failed (flags 0x%x:%s%s%s%s%s%s)", err,
                 (err & ERR_SPIKE_OVERFLOW) ? " spike list overflow" : "",
                 (err & ERR_IND_RANGE) ? " index or row length out of range" : "",
                 (err & ERR_DELAY_RANGE) ? " a synapse arriving in the same step appeared after the schedule was chosen (option rescan_delays)" : "",
                 (err & ERR_BARRIER_TIMEOUT) ? " grid barrier timed out" : "",
-                (err & ERR_EXCHANGE_TIMEOUT) ? " spikes of another process did not arrive in time" : "");
+                (err & ERR_EXCHANGE_TIMEOUT) ? " spikes of another process did not arrive in time" : "",
+                (err & ERR_COPY_TIMEOUT) ? " a copy into shared memory was not waited for any longer" : "");
 }
 
 int b200_synchronize(b200_runner *r)

@@ -29,7 +29,6 @@ constexpr unsigned int SCATTER_PIECE = 256;                             // synap
 constexpr unsigned int SCATTER_ALIGN = 16;                              // synapses: pieces start where every array allows a bulk copy
 constexpr unsigned int SCATTER_MOST_DEPTH = 4;                          // pieces in a warp's ring
 constexpr unsigned int SCATTER_SMEM = 225 * 1024;
-constexpr unsigned int SCATTER_WAITS = 1u << 18;                        // polls for a piece before the step is given up
 constexpr unsigned int SCATTER_MOST_SOURCES = 64;                       // groups onto one buffer
 // An event costs 0.19 ns of an SM's shared memory and 0.78 ns of its share of the L2's reductions; clearing and flushing
 // the sums about 2.5 us.
@@ -84,6 +83,8 @@ struct ScatterRing
     unsigned int depth, bytes;          // pieces, bytes of one
     unsigned int sent, taken;           // slots of the next piece sent and taken
     unsigned int parity;                // of the slot next taken
+    unsigned int polls;                 // for a piece before the step is given up
+    bool failed;                        // it has been
 };
 
 // A lane's item: one piece of a spike's row.
@@ -212,15 +213,18 @@ __device__ __forceinline__ unsigned int scatterGroup(const SynapseLaunch &S, con
             later = look(turn + 32u);
         }
         const unsigned int low = __shfl_sync(0xFFFFFFFFu, here.low, at), end = __shfl_sync(0xFFFFFFFFu, here.end, at);
-        bool there = false;
-        for(unsigned int i = 0; i < SCATTER_WAITS && !there; i++) {
-            unsigned int done;
-            asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                         : "=r"(done) : "r"(scatterShare(R.bars + R.taken)), "r"(R.parity) : "memory");
-            there = done != 0u;
+        if(__all_sync(0xFFFFFFFFu, copyArrived(R.bars + R.taken, R.parity, R.polls))) add(R.data + R.taken * R.bytes, low, end);
+        else {
+            if(lane == 0u) atomicOr(&S.state->error, ERR_COPY_TIMEOUT);
+            // (what is on its way has to arrive before the block ends)
+            for(unsigned int sent = turn; sent < min(n, turn + R.depth); sent++) {
+                copyArrived(R.bars + R.taken, R.parity, COPY_WAITS);
+                next(R.taken);
+                if(R.taken == 0u) R.parity ^= 1u;
+            }
+            R.failed = true;
+            break;
         }
-        if(there) add(R.data + R.taken * R.bytes, low, end);
-        else atomicOr(&S.state->error, ERR_BARRIER_TIMEOUT);
         __syncwarp();
         next(R.taken);
         if(R.taken == 0u) R.parity ^= 1u;
@@ -247,7 +251,7 @@ sparseBatchKernel(const ScatterLaunch L)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     chainWait();
-    const unsigned int k = chainPhase(L.S.state, L.S.ahead);
+    const unsigned int k = chainPhase(L.S.state, L.S.ahead), polls = L.S.state->copy_wait_limit;
     // ---- this CTA's stretch of the line of spikes
     if(threadIdx.x < T.num_groups) {
         const b200_synapse_group &g = L.S.groups[T.first_group + threadIdx.x];
@@ -283,9 +287,9 @@ sparseBatchKernel(const ScatterLaunch L)
     __syncthreads();
     float *const cells = T.cells + (unsigned long long)part.copy * T.num_cells;
     ScatterRing ring{reinterpret_cast<unsigned char*>(scatterSums + ((L.cells + 31u) & ~31u)) + (size_t)warp * L.depth * L.piece_bytes,
-                     scatterBars[warp], L.depth, L.piece_bytes, 0u, 0u, 0u};
+                     scatterBars[warp], L.depth, L.piece_bytes, 0u, 0u, 0u, polls, false};
     unsigned int item = warp;
-    for(unsigned int gi = 0; gi < T.num_groups; gi++) {
+    for(unsigned int gi = 0; gi < T.num_groups && !ring.failed; gi++) {
         const b200_synapse_group &g = L.S.groups[T.first_group + gi];
         const unsigned int slots = g.src_delay_slots, slot = ringSlot(k + slots - g.axonal_delay, slots);
         const unsigned int *const spk = g.src_spk + ((unsigned long long)part.copy * slots + slot) * g.num_src + firstSpike[gi];

@@ -403,7 +403,8 @@ int  b200_get_counter(b200_runner *r, const char *name, uint64_t *value);
  * groups whose target buffer fits an SM's shared memory are summed there, default 64; 0: always; counter "scatter_armed"),
  * "barrier_spin_limit" / "exchange_spin_limit" (polls) and "stream_wait_cycles" (SM cycles): how long a wait
  * inside a persistent kernel lasts before the launch gives up and b200_synchronize reports
- * B200_ERR_DEVICE_CHECK (defaults: tens of milliseconds; about two seconds). */
+ * B200_ERR_DEVICE_CHECK (defaults: tens of milliseconds; about two seconds), "copy_wait_limit" (polls for a copy into shared
+ * memory in the kernels of batched networks; 0: none, every such step fails and says so). */
 int  b200_set_option(b200_runner *r, const char *name, double value);
 
 /* Which time-step path b200_step_time takes for the registered model: 1 = persistent kernel (one

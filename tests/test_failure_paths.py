@@ -58,3 +58,55 @@ def test_wait_limits_are_options():
         with pytest.raises(abi.B200Error):
             rt.set_option(name, 0)
     rt.close()
+
+
+def test_a_missing_message_of_the_target_resident_kernel_runs_into_the_wait_limit():
+    """Two polls are fewer than a message needs from one CTA to the next."""
+    from genn_b200.runtime import Runtime
+    from tests import helpers
+    from tests.cases import CASES
+    rt = Runtime(None, 10, net=resolve(CASES["c1_full"]()[0]))
+    assert rt.counter("resident") == 1
+    rt.set_option("resident_ctas", 148)
+    rt.set_option("barrier_spin_limit", 1)
+    rt.step_time(200)
+    with pytest.raises(abi.B200Error, match="timed out"):
+        rt.synchronize()
+    rt.close()
+    ok = Runtime(None, 400, net=_net())
+    assert ok.counter("resident") == 1
+    ok.step_time(400)
+    ok.synchronize()
+    want = helpers.load_golden("potjans_mini")
+    for p in ok.net.pops:
+        helpers.assert_close(ok.array(f"{p.name}.V")[0], want[f"V_{p.name}_400"], f"V {p.name}", 1e-5, 2e-6)
+    ok.close()
+
+
+@pytest.mark.parametrize("pre,post,weight", [(1100, 260, "drawn"), (5000, 257, "drawn"), (1100, 260, "sparse"), (300, 5003, "sparse")])
+def test_a_copy_that_is_not_waited_for_ends_the_step_with_an_error(pre, post, weight):
+    """The kernels of batched networks, told to give up at once: rows and pieces are on their way into shared memory when they do, and
+    land before the blocks end; the same kernels are right again when they may wait."""
+    from genn_b200.runtime import Runtime
+    from oracle.oracle import OracleRunner
+    from tests import helpers, test_dense_batch, test_sparse_batch
+
+    def net():
+        return (test_sparse_batch._net(pre, post, 60, 4, 300.0, True, 0, False) if weight == "sparse" else
+                test_dense_batch._net(pre, post, 4, 300.0, weight))
+    rt = Runtime(None, net=net())
+    rt.set_option("scatter_min_spikes", 0)
+    rt.set_option("copy_wait_limit", 0)
+    rt.step_time(6)
+    with pytest.raises(abi.B200Error, match="copy into shared memory"):
+        rt.synchronize()
+    rt.close()
+    rt, orc = Runtime(None, net=net()), OracleRunner(net())
+    rt.set_option("scatter_min_spikes", 0)
+    rt.set_option("copy_wait_limit", 1 << 18)
+    rt.step_time(6)
+    orc.step(6)
+    for name in [n for n in rt.plan.arrays if n.endswith((".out_post", ".V"))]:
+        helpers.assert_close(rt.array(name).reshape(-1), orc.array(name).reshape(-1), name, 1e-5, 2e-5)
+    rt.close()
+    orc.close()
