@@ -106,7 +106,6 @@ _PROTOTYPES = {
     "b200_array_expose": [C.c_void_p, C.c_void_p],
     "b200_array_memset": [C.c_void_p, C.c_void_p, C.c_int, C.c_size_t],
     "b200_exchange_alloc": [C.c_void_p, C.c_size_t, C.POINTER(C.c_void_p)],
-    "b200_compact_words": [C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p],
     "b200_pull_recording": [C.c_void_p, C.c_uint32, C.POINTER(C.c_void_p), C.POINTER(C.c_uint64), C.c_uint32, C.POINTER(C.c_void_p),
                             C.POINTER(C.c_uint64)],
     "b200_decode_recording": [C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32,

@@ -67,7 +67,7 @@ __device__ __forceinline__ float proceduralUniform(unsigned int x)
     return B200_FADD(__uint_as_float((x >> 9) | 0x3F800000u), -0.999999940395355224609375f);
 }
 
-// b200_logf for the uniforms, equal for every one of them (checked over all 2^23).  The quotient of numbers in [-0.3, 0.42]
+// b200_logf for the uniforms, equal for every one of the 2^23 (tests/test_procedural_math.py, as are the others here).  The quotient of numbers in [-0.3, 0.42]
 // and [1.7, 2.42] needs no scaling: an approximate reciprocal, and the quotient corrected by its exact remainder (Markstein,
 // IBM J. Res. Dev. 34, 1990).
 __device__ __forceinline__ float proceduralLog(float u)

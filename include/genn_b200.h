@@ -252,14 +252,8 @@ int  b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes
  * "use_resident" asks for it; the program then says "rescan_delays" behind everything it writes. */
 int  b200_array_expose(b200_runner *r, void *device_ptr);
 /* Spike recordings are one bit per neuron and time step and almost all zeros (Runtime::pullRecordingBuffersFromDevice,
- * runtime.cc:720-746, copies them whole).  This appends the non-zero 32-bit words of `words` to `pairs` as
- * (base_index + word index, word), 8 bytes each, on the runner's stream; `counter` (a device word the caller has
- * zeroed) counts every non-zero word, also those that found no room below `capacity`: the caller then copies
- * the array itself.  Order of the pairs is arbitrary. */
-int  b200_compact_words(b200_runner *r, const uint32_t *words, uint64_t num_words, uint32_t base_index,
-                        void *pairs, uint32_t capacity, uint32_t *counter);
-/* The same for all recorded populations at once, and fetched: waits for the runner's stream and lists the non-zero words of
- * the arrays, in order, as (index, word) pairs; an array's first word has the index of all words before it.  `*pairs`
+ * runtime.cc:720-746, copies them whole).  This waits for the runner's stream and fetches the non-zero 32-bit words of all
+ * recorded populations, in order, as (index, word) pairs; an array's first word has the index of all words before it.  `*pairs`
  * points into page-locked memory of the runner that the next call overwrites; it is NULL if more than `capacity` words
  * (`*num_pairs` of them) are not zero: the caller then copies the arrays.  Reports device-side checks as b200_synchronize does. */
 int  b200_pull_recording(b200_runner *r, uint32_t num_arrays, const uint32_t *const *words, const uint64_t *num_words,
