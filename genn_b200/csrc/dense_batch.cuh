@@ -28,8 +28,9 @@ constexpr unsigned int DENSE_OWN = DENSE_COPIES / DENSE_WARPS;      // copies of
 constexpr unsigned int DENSE_STAGES = 3;
 constexpr unsigned int DENSE_PER_SM = 2;            // CTAs on an SM: 96 KB of stages each
 constexpr unsigned int DENSE_WINDOW = 1024;         // most source neurons of a CTA (masks and list: 6 KB)
-// A CTA reads all spike lists to find its own sources: worth it while those are a small part of what it reads of the rows.
-constexpr unsigned int DENSE_MOST_SOURCES = 65536;
+// (There is no upper limit: every CTA reads all spike lists to find its own sources, but 100 000 x 512 with 2 / 8 / 32 copies takes 25 / 26
+// / 59 us a step at 20 Hz, 400 000 x 128 81 / 97 / 219, where the kernel with a thread per column takes 468 / 491 / 536 and 1842
+// / 1942 / 2189.)
 // With fewer sources a thread per column that walks a copy's few spikes one after another is done before the masks are made:
 // a step of 2 / 8 / 32 copies takes 7.7 / 7.7 / 8.6 us with it and 7.9 / 8.4 / 9.7 here at 600 x 2400, but 9.1 / 9.6 / 10.2
 // against 7.6 / 8.3 / 9.9 at 1200 x 1200 and 12.9 / 13.3 / 14.2 against 7.7 / 8.3 / 9.6 at 2400 x 600.

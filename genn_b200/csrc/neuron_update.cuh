@@ -27,7 +27,10 @@ namespace b200
 {
 constexpr int NEURON_BLOCK = 128;
 constexpr unsigned int NEURON_BLOCKS_PER_SM = 16;
-constexpr unsigned int NEURON_WARPS_WANTED = 8;     // of an SM, before a warp takes four words of neurons
+// Warps of an SM before a warp takes four words of neurons.  us a step of a network of 80 000 / 150 000 / 200 000 / 300 000 / 1 200 000
+// neurons with one word a warp 4.4 / 4.7 / 6.7 / 7.4 / 15.1, with four 5.3 / 5.6 / 5.5 / 5.5 / 11.9; with a Poisson source each 5.3 / 5.6 /
+// 8.0 / 9.0 / 21.7 and 7.2 / 8.1 / 8.2 / 7.9 / 21.8: the line, 152 000 neurons, is where the second wave of blocks begins.
+constexpr unsigned int NEURON_WARPS_WANTED = 8;
 
 // Peers of a sharded model as the neuron update sees them: every spike id is also
 // stored into each peer's exchange arena, at the offset it has in this process's.

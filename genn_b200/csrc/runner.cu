@@ -727,8 +727,7 @@ int prepare(b200_runner *r)
             // +3: tiles are aligned to the array, not to the row
             sparseStarts.push_back(sparseStarts.back() + (g.row_stride + 3 + PRE_TILE - 1) / PRE_TILE);
         }
-        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src >= DENSE_LEAST_SOURCES &&
-                g.num_src <= DENSE_MOST_SOURCES) {
+        else if(r->batch > 1 && g.connectivity == B200_CONN_DENSE && g.wu_model != B200_WU_STDP && g.num_src >= DENSE_LEAST_SOURCES) {
             dense.push_back(g);
         }
         else if(g.connectivity == B200_CONN_BITMASK || g.connectivity == B200_CONN_DENSE) {
@@ -1643,9 +1642,12 @@ int buildResident(b200_runner *r)
     };
     const unsigned int most = std::min<unsigned int>((unsigned int)sms, RESIDENT_MAX_CTAS);
     {
-        // Units of 32 neurons for a CTA.  More CTAs share the work of a step but lengthen the exchange; measured (us a step at
-        // 32 / 64 / 148 CTAs): 1000 -> 10 000 sparse 1.37 / 1.48 / 1.94; 7 700 neurons with rings 3.3 / 3.1 / 3.3; DENSE
-        // 4096 -> 4096 6.4 / 5.2 / 4.6; BITMASK 2000 -> 5000 4.6 / 4.3 / 4.1
+        // Units of 32 neurons for a CTA.  More CTAs share the work of a step but lengthen the exchange.  us a step, this rule / the
+        // best of seven grids from 16 to 148 CTAs (at which): SPARSE 1000 + 1000 3.0 / 2.9 (64), 3000 3.5 / 3.5, 5000 4.2 / 4.2,
+        // 10 000 4.4 / 3.8 (32), 20 000 6.3 / 5.3 (64), 50 000 6.8 / 6.7; with rings 1000 2.6 / 2.5, 3000 3.4 / 3.1 (16), 8000 5.9
+        // / 4.4 (32), 20 000 7.9 / 7.8; DENSE 1000 x 1000 2.9 / 2.7 (64), 2000 x 2000 3.5 / 3.2 (148), 1000 x 4000 3.3 / 3.2, 8000 x
+        // 8000 8.1 / 8.1; BITMASK 2000 x 2000 3.7 / 3.2 (148), 1000 x 4000 3.5 / 3.1 (32), 8000 x 8000 5.0 / 4.8.  So the lines are
+        // coarse: within a fifth of the best in all of 25 but one.
         bool rings = false;
         for(unsigned int a = 0; a < numDelays; a++) rings = rings || L.kind[a] == RESIDENT_SPLIT;
         const unsigned int perCta = numSpans ? 2u : rings ? 4u : 10u;

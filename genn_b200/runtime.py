@@ -21,11 +21,12 @@ from .plan import ArrayFactory, Plan
 from .resolve import Net, resolve
 
 
-# A host view that is pulled again and again is page-locked in pages of its own, so that the device writes it by itself: a pull of
-# 1 MB takes 25 us instead of the 90 of the driver's way into pageable memory.  Page-locking takes 1 to 3 ms, which sixteen
-# pulls show to be worth it.  Below VIEW_LEAST bytes the library's staging buffer is as fast, above VIEW_MOST
-# page-locking costs more than it gives; VIEW_TOTAL bounds what is page-locked at a time.
-VIEW_LEAST, VIEW_MOST, VIEW_TOTAL = 256 * 1024, 1 << 20, 32 << 20
+# A host view that is pulled again and again is page-locked in pages of its own, so that the device writes it by itself.  Measured, us
+# a pull pageable / page-locked, and pulls that pay for locking and unlocking: 300 KB 36 / 17, 30; 512 KB 51 / 21, 17; 1 MB 86 / 30,
+# 12; 2 MB 147 / 48, 10; 3 MB 201 / 66, 7; 4 MB 257 / 83, 15.  Sixteen pulls show that there will be more.  Up to VIEW_LEAST
+# the library's staging buffer is as fast (255 KB: 26.5 either way); from 4 MB on several threads copy, page-locked or not
+# (6 MB: 567 / 610).  VIEW_TOTAL bounds what is page-locked at a time.
+VIEW_LEAST, VIEW_MOST, VIEW_TOTAL = 256 * 1024, (4 << 20) - 1, 32 << 20
 PAGE = mmap.PAGESIZE
 _view_lock = threading.Lock()
 _view_bytes = 0

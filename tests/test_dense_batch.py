@@ -26,7 +26,7 @@ def _net(pre, post, batch, rate, weight):
 @pytest.mark.parametrize("pre,post,batch,rate,weight", [
     (1, 1, 2, 900.0, "drawn"), (1023, 129, 3, 100.0, "drawn"), (1024, 127, 32, 50.0, "drawn"), (2049, 260, 5, 30.0, "drawn"),
     (1070, 4, 33, 100.0, "drawn"), (5000, 130, 2, 20.0, "drawn"), (1029, 128, 8, 990.0, "drawn"), (1090, 513, 4, 100.0, "constant"),
-    (1025, 1, 2, 100.0, "drawn")])
+    (1025, 1, 2, 100.0, "drawn"), (70001, 5, 3, 3.0, "drawn")])
 def test_every_copy_matches_the_cpu_checker(pre, post, batch, rate, weight):
     from genn_b200.runtime import Runtime
     from oracle.oracle import OracleRunner

@@ -75,7 +75,7 @@ class _Registered:
         del self.now[address]
 
 
-@pytest.mark.parametrize("n", [65537, 100003, 262144])
+@pytest.mark.parametrize("n", [65537, 100003, 262144, 1048575])
 def test_page_locked_views_lie_in_pages_of_their_own_and_are_unlocked_with_their_memory(n, monkeypatch):
     from genn_b200 import runtime
     from genn_b200.model import Variable
