@@ -659,7 +659,8 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                     if(all > L.quiet[a]) residentAccount(sh, L.weight[a], L.spare, L.may_leave ? L.patience : ~0u, step, all, &sh.stop[turn == 2u ? 0u : turn + 1u]);
                 }
                 turn = (turn == 2u) ? 0u : turn + 1u;
-                if(m) {
+                // (a LATE class in a step that has just become the last: for the next launch)
+                if(m && !(numDelays > 1u && late && step + 1u == sh.steps)) {
                     // runs of the last class that may wait for the neuron update
                     if(kind != RESIDENT_IMMEDIATE && all <= RESIDENT_LIST && a + 1u == numDelays) {
                         deliver.fetch(held, list, a, m, warp);

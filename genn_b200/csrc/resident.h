@@ -38,11 +38,11 @@
 // 7.5 at 100 (7.7), 16.5 at 300 (11.3), 163 at 3000 (62); 20 000 + 20 000, 200 synapses: 3.3 (6.5), 6.3 (6.8), 12.2 (6.9), 107
 // (15); 4000 + 4000 with rings of 16, 1000 synapses: 3.7 (5.8), 17.6 (8.2), 49 (11.9), 161 at 1000 (22).  So a launch keeps
 // account of what it loses: every spike delivered adds its class's `weight`, every step takes off `spare`, and when the sum
-// passes `patience` the launch ends with the next step's list.  A launch of the other
-// kernel that the host has put behind it does the rest up to the same step and goes on for `resident_rest` steps, twice as many every time
-// this happens, before this kernel is tried again.  All CTAs count the same spikes, so they leave at the same step without
-// a word.  More spikes in one step than the list holds are left to the other kernel at once (models with one delay, up to
-// 20 units a CTA): the messages' further ids are fetched by one lane per sender, 0.3 ms for every 2048 of them.
+// passes `patience` the launch ends with the next step's list.  A launch of the other kernel that the host has put behind it does the rest
+// up to the same step, and goes on for `resident_rest` steps, twice as many every time this happens, before this kernel is tried again.  All
+// CTAs count the same spikes, so they leave at the same step without a word.  More spikes in one step than the list holds are left to
+// the other kernel at once (models with one delay, up to 20 units a CTA): the messages' further ids are fetched by one lane per
+// sender, 0.3 ms for every 2048 of them.
 //
 // Memory between launches is what every other path leaves: the first steps of a launch take the spikes of the steps
 // before it from the spike lists, the last ones write them.
@@ -70,7 +70,7 @@ constexpr unsigned int RESIDENT_NEAR_MOST = 256;        // most delay-0 synapses
 constexpr float RESIDENT_RUN_COST = 560.0f, RESIDENT_NEAR_COST = 280.0f;        // ns of a warp for a chunk of a run / of a delay-0 row
 constexpr unsigned int RESIDENT_PIECE_COST = 300000;    // ns of a step with more spikes than the list holds, for every list of them
 constexpr unsigned int RESIDENT_MOST_WEIGHT = 1000, RESIDENT_MOST_DEBT = 1u << 30;      // ns
-constexpr unsigned int RESIDENT_REST = 64;              // steps on the other kernel, the first time
+constexpr unsigned int RESIDENT_REST = 48;              // steps on the other kernel, the first time
 constexpr unsigned int RESIDENT_MOST_REST = 1u << 20;
 constexpr unsigned int RESIDENT_PAD = 0xFFFFFFFFu;      // key of a padding entry
 constexpr unsigned long long RESIDENT_TAG_STEPS = 1ull << 20;       // step numbers of messages are 20 bits

@@ -66,9 +66,12 @@ int fail(int code, const char *fmt, ...)
 
 constexpr size_t STAGE_BYTES = 256 * 1024 - 64;  // page-locked buffer of a runner through which small arrays reach pageable memory
 constexpr size_t LARGE_PULL = 4u << 20;      // arrays from here on are copied out by several threads
-constexpr uint64_t FIRST_BLOCK = 2048;       // steps of the first launch of the target-resident kernel in a call, the next has twice as many
-constexpr uint64_t LONG_CALL = 10000;        // steps of a call from which the kernel that may have to take over is prepared first (and of any call once it had to)
-constexpr double MOST_LOSS = 1.0e6;          // ns that a call of the target-resident kernel may lose with no launch behind it
+constexpr uint64_t FIRST_BLOCK = 64;         // steps of the first launch of the target-resident kernel in a call, the next has twice as many:
+constexpr uint64_t QUIET_BLOCK = 2048;       // a network that was busy at first is soon tried again; once a call has passed quietly
+constexpr uint64_t LONG_CALL = 10000;        // steps of a call from which the kernel that may have to take over is prepared first,
+constexpr uint64_t LONG_HOLD = 512;          // and of its turn from which it is prepared then (with rings: 2 - 10 ms)
+constexpr double MOST_LOSS = 1.0e6;          // ns that a call of the target-resident kernel may lose with no launch behind it, for each of the
+constexpr unsigned int MOST_QUIET = 50;      // quiet calls before it, up to this many (a launch for nothing: 4 us, a tenth of a short call)
 constexpr size_t ARRAY_TAIL_PAD = 256;     // vector loads may read up to 15 bytes past the last element
 
 template<typename T>
@@ -346,6 +349,9 @@ struct b200_runner
     float residentPatience = 200.0f;        // us
     bool residentPatienceChosen = false;
     double residentWorst = 0.0;             // ns that a step could lose, were every neuron to fire
+    double residentSources = 0.0;           // neurons with synapses
+    unsigned long long residentHoldSeen = 0;
+    unsigned int residentQuiet = 0;         // calls since the host last saw that it had to
 
     void dropResident()
     {
@@ -1128,11 +1134,11 @@ void arrayWritten(b200_runner *r, const void *p, size_t bytes)
 }
 
 // `goal`: not 0: the launch does what a launch of the target-resident kernel in front of it leaves of the steps up to there.
-int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long numRec, unsigned long long goal = 0)
+// `quick`: no time to look at the arrays.
+int launchFused(b200_runner *r, unsigned long long numSteps, unsigned long long numRec, unsigned long long goal = 0, bool quick = false)
 {
-    if(goal && r->lagStale) {
-        // no time to look at the arrays: the schedule that needs no private copies of them (at a hundred spikes a step and more
-        // it is as fast as the others)
+    if((goal || quick) && r->lagStale) {
+        // the schedule that needs no private copies of them (at a hundred spikes a step and more it is as fast as the others)
         if(r->schedule != b200_runner::PLAIN) {
             r->schedule = b200_runner::PLAIN;
             r->dropUrgent();
@@ -1769,7 +1775,7 @@ int buildResident(b200_runner *r)
             for(unsigned int c = 0; c < grid; c++) runs[c * runsPerCta + pair].row = row;
         }
         // what a spike costs here above what it costs the kernel with a grid barrier
-        r->residentWorst = 0.0;
+        r->residentWorst = r->residentSources = 0.0;
         for(unsigned int a = 0; a < numDelays; a++) {
             double sources = 0.0, all = 0.0;
             for(size_t ni = 0; ni < numGroups; ni++) {
@@ -1782,6 +1788,7 @@ int buildResident(b200_runner *r)
             // spike, and the tiled kernels, whose launches and flush take some 35 us)
             const double there = !r->residentHandsOver ? 0.0 : (L.kind[a] == RESIDENT_SPLIT ? 0.02 : 0.0085) * all / std::max(1.0, sources);
             L.weight[a] = (unsigned int)std::min(std::max(0.0, here - there) + 0.5, (double)RESIDENT_MOST_WEIGHT);
+            r->residentSources += sources;
             r->residentWorst += sources * L.weight[a] + std::max(0.0, sources / RESIDENT_LIST - 1.0) * RESIDENT_PIECE_COST;
             // (with rings the exchange, which grows with the grid, and the delay-0 rows stand in front of the update: at ten spikes a
             // step 63 CTAs gain 2.3 us on the other kernel, 148 gain 1.5)
@@ -2929,16 +2936,19 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
         }
     }
     if(resident) {
-        // The launches of a call grow, so that a network that was busy at first is tried again.  A call whose few steps cannot
-        // lose much has no second launch behind it (4 us).
-        const bool mayTakeOver = r->residentHandsOver && r->residentWorst > 0.0 && (num_steps >= LONG_CALL || *r->residentHold);
-        if(mayTakeOver && r->lagStale && (e = refreshSchedule(r)) != B200_OK) return e;
-        uint64_t block = r->residentHandsOver ? FIRST_BLOCK : RESIDENT_TAG_STEPS / 2;
+        if(*r->residentHold != r->residentHoldSeen) {
+            r->residentHoldSeen = *r->residentHold;
+            r->residentQuiet = 0;
+        }
+        if(r->residentHandsOver && r->lagStale && r->residentWorst > 0.0 && num_steps >= LONG_CALL && (e = refreshSchedule(r)) != B200_OK) return e;
+        // (one step of it could use up the patience, or be more than the list holds, and how it begins is not known yet)
+        const bool sudden = r->residentHandsOver && !r->residentQuiet && r->residentSources > RESIDENT_LIST;
+        uint64_t block = !r->residentHandsOver ? RESIDENT_TAG_STEPS / 2 : sudden ? FIRST_BLOCK : QUIET_BLOCK;
         while(left) {
             const uint64_t done = r->hostStepsDone + (num_steps - left);
             if(r->residentHandsOver && done < *r->residentHold) {
                 const uint64_t n = std::min<uint64_t>(left, *r->residentHold - done);
-                e = launchFused(r, n, num_recording_timesteps);
+                e = launchFused(r, n, num_recording_timesteps, 0, *r->residentHold - done < LONG_HOLD);
                 if(e) return e;
                 left -= n;
                 r->residentRent -= std::min<unsigned long long>(r->residentRent, n);
@@ -2957,13 +2967,14 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
                 continue;
             }
             const uint64_t n = std::min<uint64_t>(left, std::min<uint64_t>(block, RESIDENT_TAG_STEPS / 2));
-            const bool leave = r->residentHandsOver && (r->residentPatienceChosen || (double)n * r->residentWorst > MOST_LOSS);
+            const bool leave = r->residentHandsOver && (r->residentPatienceChosen || (double)n * r->residentWorst > MOST_LOSS * (1u + std::min(r->residentQuiet, MOST_QUIET)));
             e = launchResident(r, n, num_recording_timesteps, done, leave);
             if(e == B200_OK && leave) e = launchFused(r, n, num_recording_timesteps, done + n);
             if(e) return e;
             left -= n;
             block *= 2;
         }
+        r->residentQuiet++;
     }
     else if(r->useFused && r->fusedEligible && !r->timing) {
         while(left) {

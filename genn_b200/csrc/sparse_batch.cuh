@@ -1,8 +1,8 @@
 // SPARSE delivery of a batched network whose target buffers fit an SM's shared memory.
 //
 // One reduction into L2 per synaptic event is bound by the 1.9e11 scattered reductions a second that the L2 takes (measured;
-// 11 M events: 59 us), one addition in shared memory by 8e11 (random cells of
-// 80 KB and of 4 MB, all SMs, nothing else: 803 and 193 G a second).  A CTA takes one copy of one target buffer (outPost, or a whole
+// 8 M events: 42 us), one addition in shared memory by 8e11 (random cells
+// of 4 MB and of 80 KB, all SMs, nothing else: 193 and 803 G a second).  A CTA takes one copy of one target buffer (outPost, or a whole
 // dendritic-delay ring) into its shared memory as private sums, a share of that copy's spikes, and adds their rows as they
 // lie in the model's arrays: whole rows, 6 to 9 bytes a synapse, no second copy of the synapses and no table of runs.  The
 // sums go to the target once at the end, 16 bytes a reduction.  A share with few events (SCATTER_FEW) leaves the sums alone
@@ -14,7 +14,7 @@
 // more under way on an SM, what HBM's latency wants, and no warp waits for another).  Pieces held in registers instead, one
 // ahead: 27 KB under way and 37 instructions an event besides its addition, 43 us at the size below.
 //
-// 20 000 + 20 000 neurons, 8 copies, 11 M events a step: 90 us with the tiled kernels, 31 here.
+// 20 000 + 20 000 neurons, 8 copies, 8 M events a step: 90 us with the tiled kernels, 31 here (shared-memory pipe 53 %, issue slots 36 %).
 #pragma once
 
 #include <type_traits>

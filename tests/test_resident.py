@@ -313,12 +313,19 @@ def test_a_busy_network_is_handed_over_and_taken_back(kind, synchronous):
     from oracle.oracle import OracleRunner
     net = resolve(_busy(kind, synchronous))
     rt, orc = _runtime(net, 200), OracleRunner(resolve(_busy(kind, synchronous)), 200)
+    other = _runtime(resolve(_busy(kind, synchronous)), 200)       # (the same events are counted)
+    other.set_option("use_fused", 0)
+    for r in (rt, other):
+        r.set_option("count_events", 1)
+    rt.set_option("resident_warps", 4)          # (few warps: a spike costs the more)
     assert rt.counter("resident") == 1
     rt.set_option("resident_patience", 1e6 if synchronous and kind != "bit mask" else 0)
     holds, done = set(), 0
     for n in (1, 2, 3, 5, 60, 1, 1, 40, 87):
         rt.step_time(n)
+        other.step_time(n)
         orc.step(n)
+        assert rt.counter("synaptic_events") == other.counter("synaptic_events") and rt.counter("spikes") == other.counter("spikes")
         done += n
         holds.add(rt.counter("resident_hold"))
         for p in net.pops:
@@ -333,6 +340,7 @@ def test_a_busy_network_is_handed_over_and_taken_back(kind, synchronous):
     else:
         assert len(holds) >= 3, holds   # (left more than once)
     rt.close()
+    other.close()
     orc.close()
 
 
