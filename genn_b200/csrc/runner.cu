@@ -2938,7 +2938,7 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
     if(resident) {
         if(*r->residentHold != r->residentHoldSeen) {
             r->residentHoldSeen = *r->residentHold;
-            r->residentQuiet = 0;
+            r->residentQuiet = r->hostStepsDone > r->residentHoldSeen + 2u * FIRST_BLOCK ? 1u : 0u;       // (it has gone on since)
         }
         if(r->residentHandsOver && r->lagStale && r->residentWorst > 0.0 && num_steps >= LONG_CALL && (e = refreshSchedule(r)) != B200_OK) return e;
         // (one step of it could use up the patience, or be more than the list holds, and how it begins is not known yet)
