@@ -953,7 +953,9 @@ def main():
                       "neuron_kernel_avg_launch_us": neu_s / probe_steps * 1e6,
                       "algorithmic_bytes_per_launch": nat_bytes / probe_steps,
                       "note": "the one-launch-per-kernel path at the same firing rates (CUDA event pair around every launch)"}
-        # the kernel of the timed region: ONE persistent launch runs all its time steps
+        # the kernel of the timed region: a few persistent launches (the target-resident kernel's grow from 2048 steps on) run all
+        # its time steps
+        timed_launches = max(1, int(l1 - l0))
         launch_bytes = float(ev1 - ev0) * bpe + float(sp1 - sp0) * ALGO_BYTES_PER_SPIKE
         launch_gbs = launch_bytes / seconds / 1e9
         timed_steps = args.steps * block
@@ -961,11 +963,11 @@ def main():
         per_step, traffic_note = (captured_traffic(step_kernel)
                                   if (scale == 1.0 and args.min_delay == 0.0 and step_kernel in ("residentStepKernel", "streamStepKernel"))
                                   else (None, "no capture for this configuration"))
-        traffic = per_step * timed_steps if per_step is not None else None
-        roofline = {"kernel": step_kernel + f" (persistent: {timed_steps} time steps in one launch)",
+        traffic = per_step * timed_steps / timed_launches if per_step is not None else None
+        roofline = {"kernel": step_kernel + f" (persistent: {timed_steps} time steps in {timed_launches} launch{'es' if timed_launches > 1 else ''})",
                     "bound": "hbm", "achieved": launch_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": launch_gbs / hbm_peak,
-                    "traffic": traffic, "peak_source": peak_kind, "launches": 1, "avg_launch_ms": ms,
-                    "algorithmic_bytes_per_launch": launch_bytes,
+                    "traffic": traffic, "peak_source": peak_kind, "launches": timed_launches, "avg_launch_ms": ms / timed_launches,
+                    "algorithmic_bytes_per_launch": launch_bytes / timed_launches,
                     "persistent_kernel_phase_cycles_per_step": phase_cycles,
                     "per_kernel_path": per_kernel,
                     "note": "natural firing rates: about 0.7 MB of synapse rows per time step, so a step is bound by "

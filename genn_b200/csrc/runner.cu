@@ -68,8 +68,8 @@ constexpr size_t STAGE_BYTES = 256 * 1024 - 64;  // page-locked buffer of a runn
 constexpr size_t LARGE_PULL = 4u << 20;      // arrays from here on are copied out by several threads
 constexpr uint64_t FIRST_BLOCK = 64;         // steps of the first launch of the target-resident kernel in a call, the next has twice as many:
 constexpr uint64_t QUIET_BLOCK = 2048;       // a network that was busy at first is soon tried again; once a call has passed quietly
-constexpr uint64_t LONG_CALL = 10000;        // steps of a call from which the kernel that may have to take over is prepared first,
-constexpr uint64_t LONG_HOLD = 512;          // and of its turn from which it is prepared then (with rings: 2 - 10 ms)
+constexpr uint64_t LONG_CALL = 10000;        // steps of a first call in the middle of which the host looks whether the other kernel has taken over
+constexpr uint64_t LONG_HOLD = 512;          // steps of that kernel's turn from which its own tables are made (with rings: 2 - 20 ms)
 constexpr double MOST_LOSS = 1.0e6;          // ns that a call of the target-resident kernel may lose with no launch behind it, for each of the
 constexpr unsigned int MOST_QUIET = 50;      // quiet calls before it, up to this many (a launch for nothing: 4 us, a tenth of a short call)
 constexpr size_t ARRAY_TAIL_PAD = 256;     // vector loads may read up to 15 bytes past the last element
@@ -350,6 +350,7 @@ struct b200_runner
     bool residentPatienceChosen = false;
     double residentWorst = 0.0;             // ns that a step could lose, were every neuron to fire
     double residentSources = 0.0;           // neurons with synapses
+    bool residentSteeper = false;           // groups with rings, whose spikes cost more here
     unsigned long long residentHoldSeen = 0;
     unsigned int residentQuiet = 0;         // calls since the host last saw that it had to
 
@@ -1776,6 +1777,7 @@ int buildResident(b200_runner *r)
         }
         // what a spike costs here above what it costs the kernel with a grid barrier
         r->residentWorst = r->residentSources = 0.0;
+        r->residentSteeper = false;
         for(unsigned int a = 0; a < numDelays; a++) {
             double sources = 0.0, all = 0.0;
             for(size_t ni = 0; ni < numGroups; ni++) {
@@ -1789,6 +1791,7 @@ int buildResident(b200_runner *r)
             const double there = !r->residentHandsOver ? 0.0 : (L.kind[a] == RESIDENT_SPLIT ? 0.02 : 0.0085) * all / std::max(1.0, sources);
             L.weight[a] = (unsigned int)std::min(std::max(0.0, here - there) + 0.5, (double)RESIDENT_MOST_WEIGHT);
             r->residentSources += sources;
+            r->residentSteeper = r->residentSteeper || (L.kind[a] == RESIDENT_SPLIT && L.weight[a]);
             r->residentWorst += sources * L.weight[a] + std::max(0.0, sources / RESIDENT_LIST - 1.0) * RESIDENT_PIECE_COST;
             // (with rings the exchange, which grows with the grid, and the delay-0 rows stand in front of the update: at ten spikes a
             // step 63 CTAs gain 2.3 us on the other kernel, 148 gain 1.5)
@@ -2612,7 +2615,8 @@ int b200_array_memset(b200_runner *r, void *device_ptr, int value, size_t bytes)
 
 int b200_array_expose(b200_runner *r, void *device_ptr)
 {
-    if(!r || r->arrays.find(device_ptr) == r->arrays.end()) return fail(B200_ERR_INVALID, "pointer was not allocated by this runner");
+    // (also one inside the exchange arena of a sharded model: nothing is copied from there)
+    if(!r || !device_ptr) return fail(B200_ERR_INVALID, "null argument to b200_array_expose");
     if(std::find(r->exposed.begin(), r->exposed.end(), device_ptr) == r->exposed.end()) r->exposed.push_back(device_ptr);
     return B200_OK;
 }
@@ -2940,12 +2944,19 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
             r->residentHoldSeen = *r->residentHold;
             r->residentQuiet = r->hostStepsDone > r->residentHoldSeen + 2u * FIRST_BLOCK ? 1u : 0u;       // (it has gone on since)
         }
-        if(r->residentHandsOver && r->lagStale && r->residentWorst > 0.0 && num_steps >= LONG_CALL && (e = refreshSchedule(r)) != B200_OK) return e;
+        // (a model's first call, of many steps and with rings: worth waiting once, behind its first blocks, for whether the other kernel has
+        // taken over, since that one is faster with tables of its own)
+        bool look = r->residentHandsOver && r->residentSteeper && r->lagStale && !r->residentQuiet && num_steps >= LONG_CALL;
         // (one step of it could use up the patience, or be more than the list holds, and how it begins is not known yet)
         const bool sudden = r->residentHandsOver && !r->residentQuiet && r->residentSources > RESIDENT_LIST;
         uint64_t block = !r->residentHandsOver ? RESIDENT_TAG_STEPS / 2 : sudden ? FIRST_BLOCK : QUIET_BLOCK;
         while(left) {
             const uint64_t done = r->hostStepsDone + (num_steps - left);
+            if(look && num_steps - left >= LONG_HOLD) {
+                look = false;
+                CUDA_TRY(cudaStreamSynchronize(r->stream));
+                if(done < *r->residentHold && (e = refreshSchedule(r)) != B200_OK) return e;
+            }
             if(r->residentHandsOver && done < *r->residentHold) {
                 const uint64_t n = std::min<uint64_t>(left, *r->residentHold - done);
                 e = launchFused(r, n, num_recording_timesteps, 0, *r->residentHold - done < LONG_HOLD);

@@ -410,6 +410,7 @@ int  b200_get_step_path(b200_runner *r, int *path, char *why, size_t why_bytes);
 int  b200_enable_timing(b200_runner *r, int enabled);
 int  b200_get_timer(b200_runner *r, const char *name, double *seconds);
 int  b200_reset_timers(b200_runner *r);
+/* (The launch behind the target-resident kernel's that does what that one leaves, mostly nothing, counts with it.) */
 int  b200_get_kernel_launches(b200_runner *r, uint64_t *launches);
 /* SM cycles thread 0 of every CTA of the persistent kernel spent in {presynaptic work, barrier,
  * neuron work, barrier}, accumulated while option "fused_profile" is on: out[cta*4 + phase]. */

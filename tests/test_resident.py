@@ -4,7 +4,7 @@ spikes than a message head or the delivery list holds, several axonal delays and
 import numpy as np
 import pytest
 
-from genn_b200 import GeNNModel, init_postsynaptic, init_weight_update
+from genn_b200 import GeNNModel, abi, init_postsynaptic, init_weight_update
 from genn_b200.resolve import resolve
 from tests import helpers
 from tests.cases import CASES
@@ -201,6 +201,7 @@ def test_weights_written_through_the_device_pointer_reach_the_step(asked):
     other._runtime.set_option("use_tiled", 0)
     rt = m._runtime
     assert rt.counter("resident") == 1
+    abi.check(rt.lib.b200_array_expose(rt.handle, m.neuron_populations["b"].vars["V"].device_pointer + 256))    # (not an array's first byte)
     m.neuron_populations["b"].vars["V"].device_pointer          # (neuron state is read and written where it lies)
     assert rt.counter("resident") == 1
     if asked:
