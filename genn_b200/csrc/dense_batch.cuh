@@ -178,12 +178,9 @@ denseBatchKernel(const DenseLaunch L)
     for(unsigned int o = 0; o < DENSE_OWN; o++) sum[o][0] = sum[o][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     unsigned int ring = 0, parity = 0;
     for(unsigned int stage = 0; stage < numStages; stage++) {
-        if(!__all_sync(0xFFFFFFFFu, copyArrived(&arrived[ring], parity, polls))) {
-            if(lane == 0u) atomicOr(&L.S.state->error, ERR_COPY_TIMEOUT);
-            return;
-        }
+        const bool there = copyArrived(&arrived[ring], parity, polls);
         const unsigned int at = stage * 32u + lane;
-        const unsigned int m = (mine && at < rows) ? mask[list[at]] >> first : 0u;
+        const unsigned int m = (mine && there && at < rows) ? mask[list[at]] >> first : 0u;
         const float4 *const w = reinterpret_cast<const float4*>(stages + ring * 32u * DENSE_COLS) + lane;
         #pragma unroll
         for(unsigned int o = 0; o < DENSE_OWN; o++) {
@@ -207,6 +204,11 @@ denseBatchKernel(const DenseLaunch L)
                     denseSum(sum[o][1], v1);
                 }
             }
+        }
+        // the lanes' vote after the stage, not before it: each waits for itself
+        if(!__all_sync(0xFFFFFFFFu, there)) {
+            if(lane == 0u) atomicOr(&L.S.state->error, ERR_COPY_TIMEOUT);
+            return;
         }
         __syncwarp();
         if(lane == 0u) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(denseShare(&released[ring])) : "memory");

@@ -113,6 +113,21 @@ __device__ __forceinline__ void scatterIndices(const unsigned char *data, unsign
     }
 }
 
+// A wait ran out: the pieces on their way have to arrive before the block ends.  (Out of line: six instances of its caller wait for
+// instructions as it is.)
+static __device__ __noinline__ void scatterGiveUp(StepState *state, const unsigned long long *bars, unsigned int depth, unsigned int slot,
+                                                  unsigned int parity, unsigned int sent)
+{
+    atomicOr(&state->error, ERR_COPY_TIMEOUT);
+    for(; sent; sent--) {
+        copyArrived(bars + slot, parity, COPY_WAITS);
+        if(++slot == depth) {
+            slot = 0;
+            parity ^= 1u;
+        }
+    }
+}
+
 // What a warp does of one group's spikes: pieces `item`, `item` + SCATTER_WARPS, ... of the group's; returns how far beyond
 // them its next one lies.  The widths are template parameters: they decide every address.
 template<int IND, bool DELAYS>
@@ -214,15 +229,11 @@ __device__ __forceinline__ unsigned int scatterGroup(const SynapseLaunch &S, con
             later = look(turn + 32u);
         }
         const unsigned int low = __shfl_sync(0xFFFFFFFFu, here.low, at), end = __shfl_sync(0xFFFFFFFFu, here.end, at);
-        if(__all_sync(0xFFFFFFFFu, copyArrived(R.bars + R.taken, R.parity, R.polls))) add(R.data + R.taken * R.bytes, low, end);
-        else {
-            if(lane == 0u) atomicOr(&S.state->error, ERR_COPY_TIMEOUT);
-            // (what is on its way has to arrive before the block ends)
-            for(unsigned int sent = turn; sent < min(n, turn + R.depth); sent++) {
-                copyArrived(R.bars + R.taken, R.parity, COPY_WAITS);
-                next(R.taken);
-                if(R.taken == 0u) R.parity ^= 1u;
-            }
+        const bool there = copyArrived(R.bars + R.taken, R.parity, R.polls);
+        if(there) add(R.data + R.taken * R.bytes, low, end);
+        // the lanes' vote after the piece, not before it: each waits for itself
+        if(!__all_sync(0xFFFFFFFFu, there)) {
+            scatterGiveUp(S.state, R.bars, R.depth, R.taken, R.parity, min(n, turn + R.depth) - turn);
             R.failed = true;
             break;
         }
