@@ -24,19 +24,21 @@
 // What has to be in place before the neuron update of a step is kept small.  Groups of one axonal delay form a class:
 //
 //   IMMEDIATE  the runs (and DENSE / BITMASK rows) of the step's spikes are added before the update;
-//   SPLIT      every group has a delay ring: only synapses of dendritic delay 0 are needed at once.  They lie in rows of
-//              their own, one per source neuron for ALL CTAs (a few per cent of the synapses: the table stays in L2),
-//              and the runs with the rest are fetched behind them, while the neurons are updated, and added after that;
+//   SPLIT      every group has a delay ring: only synapses of dendritic delay 0 are needed at once.  They stand at the head of
+//              every run, all heads of a step's spikes are one line of entries for the threads of the CTA, and the rest is
+//              fetched behind them, while the neurons are updated, and added after that.  (They were rows of their own, one
+//              per source neuron, which every CTA read whole.  us a step before / now, rings of 16, 1000 synapses: 4000 + 4000
+//              neurons 3.74 / 3.00 at 10 spikes a step, 17.6 / 8.5 at 100; 40 000 + 40 000 neurons 3.56 / 2.89, 10.9 / 5.5);
 //   LATE       no group has a ring and the axonal delay is a step or more: the spikes of the NEXT step are known
 //              already, so their runs are fetched and added behind the update too, into the second of two buffers.
 //              CTAs then run up to the delay apart, and no step waits for another SM or for memory.
 //
 // Busy networks.  Every CTA handles every spike, so a spike costs each of them the same, however many they are: about
-// RESIDENT_RUN_COST ns of a warp for every chunk of its run and RESIDENT_NEAR_COST for every chunk of its delay-0 row, where
+// RESIDENT_RUN_COST ns of a warp for every chunk of its run and RESIDENT_NEAR_COST for every 32 entries of its head, where
 // the kernels with a grid barrier share its synapses out (8.5 ps each; 20 with rings) behind a step that costs 2 to 4 us more
 // to begin with.  A step of 10 000 + 10 000 neurons, 1000 synapses each: 3.3 us at 10 spikes a step (6.6 with the barrier),
 // 7.5 at 100 (7.7), 16.5 at 300 (11.3), 163 at 3000 (62); 20 000 + 20 000, 200 synapses: 3.3 (6.5), 6.3 (6.8), 12.2 (6.9), 107
-// (15); 4000 + 4000 with rings of 16, 1000 synapses: 3.7 (5.8), 17.6 (8.2), 49 (11.9), 161 at 1000 (22).  So a launch keeps
+// (15); 4000 + 4000 with rings of 16, 1000 synapses: 3.0 (6.0), 8.5 (8.3), 22 (11.9), 69 at 1000 (23).  So a launch keeps
 // account of what it loses: every spike delivered adds its class's `weight`, every step takes off `spare`, and when the sum
 // passes `patience` the launch ends with the next step's list.  A launch of the other kernel that the host has put behind it does the rest
 // up to the same step, and goes on for `resident_rest` steps, twice as many every time this happens, before this kernel is tried again.  All
@@ -64,10 +66,10 @@ constexpr unsigned int RESIDENT_LIST = 2048;            // spikes delivered betw
 constexpr unsigned int RESIDENT_READERS = 12;           // CTAs that poll one copy of the messages
 constexpr unsigned int RESIDENT_LOADS = 4;              // loads of a run that a lane has in flight
 constexpr unsigned int RESIDENT_CHUNK = 32 * RESIDENT_LOADS;    // entries of a run that one warp takes
-constexpr unsigned int RESIDENT_NEAR_ROWS = 4;          // rows of delay-0 synapses whose loads a warp has in flight
+constexpr unsigned int RESIDENT_NEAR_LOADS = 4;         // entries of the runs' heads that a lane has in flight
 constexpr unsigned int RESIDENT_DENSE_SPIKES = 8;       // rows of a DENSE group whose loads a lane has in flight
-constexpr unsigned int RESIDENT_NEAR_MOST = 256;        // most delay-0 synapses of a source neuron for a SPLIT class
-constexpr float RESIDENT_RUN_COST = 560.0f, RESIDENT_NEAR_COST = 280.0f;        // ns of a warp for a chunk of a run / of a delay-0 row
+constexpr unsigned int RESIDENT_NEAR_MOST = 64;         // most delay-0 synapses of a run for a SPLIT class
+constexpr float RESIDENT_RUN_COST = 560.0f, RESIDENT_NEAR_COST = 280.0f;        // ns of a warp for a chunk of a run / of heads
 constexpr unsigned int RESIDENT_PIECE_COST = 300000;    // ns of a step with more spikes than the list holds, for every list of them
 constexpr unsigned int RESIDENT_MOST_WEIGHT = 1000, RESIDENT_MOST_DEBT = 1u << 30;      // ns
 constexpr unsigned int RESIDENT_REST = 48;              // steps on the other kernel, the first time
@@ -79,20 +81,14 @@ constexpr unsigned int RESIDENT_CELL_IDS = RESIDENT_HEAD_IDS + RESIDENT_MORE_IDS
 
 enum ResidentClass { RESIDENT_IMMEDIATE = 0, RESIDENT_SPLIT = 1, RESIDENT_LATE = 2 };
 
-// entry key of a run: ring class << 30 | delay << 16 | column; of a row of delay-0 synapses: CTA << 24 | ring class << 16 | column
+// entry key of a run: ring class << 30 | delay << 16 | column
 struct ResidentRun              // runs of one (axonal delay, source population) pair onto one CTA
 {
-    unsigned long long base;    // first entry of the run of source neuron 0
-    unsigned int length;        // entries of a run (0: no synapses), a multiple of four
+    unsigned long long place;   // entries of the head (delay-0 synapses of a SPLIT class) << 48 | first entry of the run of source neuron 0
+    unsigned int length;        // entries behind the head (0: none); with the head a multiple of four
     unsigned int row;           // entries between two source neurons: the runs of all CTAs
-};
-
-struct ResidentNear             // delay-0 synapses of a SPLIT class, one row per source neuron of a population
-{
-    unsigned long long base;    // entry of source neuron 0
-    unsigned long long row_base;    // where the runs of source neuron 0 begin
-    unsigned int length;        // entries of a row (0: none), a multiple of four
-    unsigned int pad;
+    __host__ __device__ unsigned int near() const { return (unsigned int)(place >> 48); }
+    __host__ __device__ unsigned long long base() const { return place & 0xFFFFFFFFFFFFull; }
 };
 
 struct ResidentSpan             // a DENSE or BITMASK group
@@ -110,7 +106,7 @@ struct ResidentSpan             // a DENSE or BITMASK group
 // Where the tables of a CTA lie in its dynamic shared memory (bytes): constants of the launch, so no thread keeps pointers.
 struct ResidentLayout
 {
-    unsigned int groups, unit_start, unit_first, columns, runs, near, spans, poisson, undrawn, history, acc;
+    unsigned int groups, unit_start, unit_first, columns, runs, rows, spans, poisson, undrawn, history, acc;
 };
 
 struct ResidentLaunch
@@ -122,9 +118,8 @@ struct ResidentLaunch
     const unsigned int *columns;        // [grid][RESIDENT_UNITS][B200_MAX_PSM] ring class << 16 | first column
     const unsigned int *cta_columns;    // [grid][RESIDENT_CLASSES] columns of each ring class
     const ResidentRun *runs;            // [grid][delay classes][num_groups]
-    const ResidentNear *near;           // [delay classes][num_groups]
+    const unsigned long long *rows;     // [delay classes][num_groups] where the runs of source neuron 0 begin
     const uint2 *entries;
-    const uint2 *near_entries;
     const float *poisson;               // [num_groups][64] distribution of the event count of a group's one Poisson source, or NULL
     const ResidentSpan *spans;
     unsigned int num_spans;
@@ -135,7 +130,8 @@ struct ResidentLaunch
     unsigned long long source_groups;                       // groups with outgoing synapses of any delay
     unsigned long long sources[RESIDENT_CLASSES];           // neuron groups with outgoing synapses of that delay
     unsigned int chunks[RESIDENT_CLASSES];                  // warp items of the longest run of that delay (0: no runs)
-    unsigned int near_chunks[RESIDENT_CLASSES];             // the same of the rows of delay-0 synapses
+    unsigned int near_most[RESIDENT_CLASSES];               // entries of the longest head of that delay (0: no heads)
+    unsigned int near_share[RESIDENT_CLASSES];              // 2^32 / near_most, rounded up
     unsigned int acc_floats;            // shared memory of the input buffers
     unsigned int history;               // steps whose spike lists the launch has to leave behind
     unsigned int buffers;               // message buffers
@@ -166,10 +162,8 @@ struct ResidentBuild
     const unsigned int *depth;          // buffers per input, by ring class
     unsigned int late;                  // 1: LATE class: every synapse arrives one step after its delivery
     unsigned int split;                 // 1: SPLIT class: delay-0 synapses go into the rows
-    unsigned int *near_longest;         // longest row of delay-0 synapses
+    unsigned int *near_longest;         // longest head of a run
     unsigned long long *synapses;       // all of the pair
-    ResidentNear near;
-    uint2 *near_entries;
     unsigned int grid;
     unsigned int runs_stride;           // distance between the pair's runs of two CTAs
 };

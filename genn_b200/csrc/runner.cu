@@ -331,7 +331,6 @@ struct b200_runner
     unsigned long long residentBuilds = 0;
     struct ResidentPair { unsigned int delay_class, src, first, count; };
     std::vector<ResidentPair> residentPairs;            // what the copy is filled from
-    std::vector<ResidentNear> residentNears;
     const b200_synapse_group *residentGroups = nullptr; // (device)
     const unsigned int *residentTargets = nullptr, *residentDepths = nullptr;
     std::string residentWhyNot;
@@ -1476,7 +1475,7 @@ TiledLaunch tiledLaunch(const b200_runner *r)
 int residentPass(b200_runner *r, int which, unsigned int *longest, unsigned long long *totals)
 {
     const ResidentLaunch &L = r->resident;
-    const size_t numGroups = r->neuronGroups.size(), runsPerCta = (size_t)r->residentNears.size();
+    const size_t numGroups = r->neuronGroups.size(), runsPerCta = (size_t)L.num_delays * numGroups;
     int sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
     for(const auto &pr : r->residentPairs) {
@@ -1491,10 +1490,8 @@ int residentPass(b200_runner *r, int which, unsigned int *longest, unsigned long
         const size_t at = (size_t)pr.delay_class * numGroups + pr.src;
         B.late = (L.kind[pr.delay_class] == RESIDENT_LATE);
         B.split = (L.kind[pr.delay_class] == RESIDENT_SPLIT);
-        // longest run of every (CTA, pair), then longest row of delay-0 synapses of every pair
+        // longest run of every (CTA, pair), then longest head of every pair
         B.near_longest = longest ? longest + runsPerCta * r->residentGrid + at : nullptr;
-        B.near = r->residentNears[at];
-        B.near_entries = const_cast<uint2*>(L.near_entries);
         B.synapses = totals ? totals + at : nullptr;
         CUDA_TRY(residentBuild(B, which, longest ? longest + at : nullptr, L.runs ? L.runs + at : nullptr, const_cast<uint2*>(L.entries), r->state,
                                std::min(B.num_src, (unsigned int)sms * 8u), r->stream));
@@ -1613,7 +1610,7 @@ int buildResident(b200_runner *r)
     L.at.unit_first = place(sizeof(unsigned int) * units);
     L.at.columns = place(sizeof(unsigned int) * RESIDENT_UNITS * B200_MAX_PSM);
     L.at.runs = place(sizeof(ResidentRun) * numDelays * numGroups);
-    L.at.near = place(sizeof(ResidentNear) * numDelays * numGroups);
+    L.at.rows = place(sizeof(unsigned long long) * numDelays * numGroups);
     L.at.spans = place(sizeof(ResidentSpan) * numSpans);
     L.at.poisson = place(sizeof(float) * poisson.size());
     bool draws = false;
@@ -1718,13 +1715,13 @@ int buildResident(b200_runner *r)
         }
     }
     for(unsigned int a = 0; a < numDelays; a++) L.source_groups |= L.sources[a];
-    std::vector<ResidentNear> &nears = r->residentNears;
-    nears.assign(runsPerCta, ResidentNear{0, 0, 0, 0});
+    std::vector<unsigned long long> rowStarts(runsPerCta, 0ull);
     r->residentCells = 0.0;
+    L.num_delays = numDelays;
     ResidentRun *dRuns = nullptr;
-    uint2 *dEntries = nullptr, *dNear = nullptr;
+    uint2 *dEntries = nullptr;
     if(!pairs.empty()) {
-        unsigned long long cells = 0, nearCells = 0;
+        unsigned long long cells = 0;
         ScopedDevice totals(r->stream), longest(r->stream);
         if(const int err = upload(sorted.data(), sizeof(b200_synapse_group) * sorted.size(), (void**)&r->residentGroups)) return err;
         if(const int err = upload(targets.data(), sizeof(unsigned int) * targets.size(), (void**)&r->residentTargets)) return err;
@@ -1747,7 +1744,7 @@ int buildResident(b200_runner *r)
             return B200_OK;
         };
         if(const int err = count()) return err;
-        // every CTA reads the whole row of delay-0 synapses: worth it while that is a few loads
+        // the heads stand in front of the update: worth it while they are a few loads
         bool again = false;
         for(size_t pair = 0; pair < runsPerCta; pair++) {
             if(longestHost[runs.size() + pair] > RESIDENT_NEAR_MOST && L.kind[pair / numGroups] == RESIDENT_SPLIT) {
@@ -1757,24 +1754,21 @@ int buildResident(b200_runner *r)
         }
         if(again) if(const int err = count()) return err;
         for(size_t pair = 0; pair < runsPerCta; pair++) {
+            const unsigned int near = longestHost[runs.size() + pair], a = (unsigned int)(pair / numGroups);
             unsigned int row = 0;
             for(unsigned int c = 0; c < grid; c++) {
                 ResidentRun &run = runs[c * runsPerCta + pair];
-                run.base = cells + row;
-                run.length = (longestHost[c * runsPerCta + pair] + 3u) & ~3u;
-                row += run.length;
-                unsigned int &chunks = L.chunks[pair / numGroups];
-                chunks = std::max(chunks, (run.length + RESIDENT_CHUNK - 1u) / RESIDENT_CHUNK);
+                run.place = ((unsigned long long)near << 48) | (cells + row);
+                run.length = ((near + longestHost[c * runsPerCta + pair] + 3u) & ~3u) - near;
+                row += near + run.length;
+                L.chunks[a] = std::max(L.chunks[a], (run.length + RESIDENT_CHUNK - 1u) / RESIDENT_CHUNK);
             }
-            nears[pair].base = nearCells;
-            nears[pair].row_base = cells;
-            nears[pair].length = (longestHost[runs.size() + pair] + 3u) & ~3u;
+            rowStarts[pair] = cells;
             cells += (unsigned long long)row * r->neuronGroups[pair % numGroups].num_neurons;
-            nearCells += (unsigned long long)nears[pair].length * r->neuronGroups[pair % numGroups].num_neurons;
-            unsigned int &nearChunks = L.near_chunks[pair / numGroups];
-            nearChunks = std::max(nearChunks, (nears[pair].length + 31u) / 32u);
+            L.near_most[a] = std::max(L.near_most[a], near);
             for(unsigned int c = 0; c < grid; c++) runs[c * runsPerCta + pair].row = row;
         }
+        for(unsigned int a = 0; a < numDelays; a++) L.near_share[a] = L.near_most[a] ? (unsigned int)(((1ull << 32) + L.near_most[a] - 1u) / L.near_most[a]) : 0u;
         // what a spike costs here above what it costs the kernel with a grid barrier
         r->residentWorst = r->residentSources = 0.0;
         r->residentSteeper = false;
@@ -1785,7 +1779,7 @@ int buildResident(b200_runner *r)
                 sources += r->neuronGroups[ni].num_neurons;
                 all += (double)synapses[a * numGroups + ni];
             }
-            const double here = (RESIDENT_RUN_COST * L.chunks[a] + RESIDENT_NEAR_COST * L.near_chunks[a]) / warps;
+            const double here = (RESIDENT_RUN_COST * L.chunks[a] + RESIDENT_NEAR_COST * L.near_most[a] / 32.0) / warps;
             // (a model that the grid-barrier kernels do not take has only presynapticSparseKernel, no faster than this one per
             // spike, and the tiled kernels, whose launches and flush take some 35 us)
             const double there = !r->residentHandsOver ? 0.0 : (L.kind[a] == RESIDENT_SPLIT ? 0.02 : 0.0085) * all / std::max(1.0, sources);
@@ -1793,8 +1787,8 @@ int buildResident(b200_runner *r)
             r->residentSources += sources;
             r->residentSteeper = r->residentSteeper || (L.kind[a] == RESIDENT_SPLIT && L.weight[a]);
             r->residentWorst += sources * L.weight[a] + std::max(0.0, sources / RESIDENT_LIST - 1.0) * RESIDENT_PIECE_COST;
-            // (with rings the exchange, which grows with the grid, and the delay-0 rows stand in front of the update: at ten spikes a
-            // step 63 CTAs gain 2.3 us on the other kernel, 148 gain 1.5)
+            // (with rings the exchange, which grows with the grid, and the heads stand in front of the update: at ten spikes a step
+            // 63 CTAs gain 3.0 us on the other kernel, 148 gain 1.5)
             const unsigned int spare = !r->residentHandsOver ? 35000u : (L.kind[a] == RESIDENT_LATE) ? 4000u :
                 (L.kind[a] == RESIDENT_SPLIT) ? 4500u - std::min(2500u, 15u * grid) : 3300u;
             L.spare = L.spare ? std::min(L.spare, spare) : spare;
@@ -1803,21 +1797,18 @@ int buildResident(b200_runner *r)
         // padded runs of a network with few synapses per (source neuron, CTA) pair can take several times the room of its
         // arrays: the copy may use a quarter of what is free
         size_t freeBytes = POOL_KEEP * 4, totalBytes = 0;       // (what the pool may keep needs no asking)
-        if((cells + nearCells) * sizeof(uint2) > freeBytes / 4) CUDA_TRY(cudaMemGetInfo(&freeBytes, &totalBytes));
-        if((cells + nearCells) * sizeof(uint2) > freeBytes / 4) { r->dropResident(); return no("the padded copy of the synapses would take more than a quarter of the free memory"); }
+        if(cells * sizeof(uint2) > freeBytes / 4) CUDA_TRY(cudaMemGetInfo(&freeBytes, &totalBytes));
+        if(cells * sizeof(uint2) > freeBytes / 4) { r->dropResident(); return no("the padded copy of the synapses would take more than a quarter of the free memory"); }
         // (a table that stays in L2 once it has been read needs no fetching ahead: measured on tables of up to half of it)
         int l2 = 0;
         CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, r->device));
-        L.prefetch = (cells + nearCells) * sizeof(uint2) > (size_t)l2 / 2 ? 1u : 0u;
+        L.prefetch = cells * sizeof(uint2) > (size_t)l2 / 2 ? 1u : 0u;
         if(const int err = device(sizeof(uint2) * cells, (void**)&dEntries)) return err;
         CUDA_TRY(cudaMemsetAsync(dEntries, 0xFF, sizeof(uint2) * cells, r->stream));
-        if(const int err = device(sizeof(uint2) * nearCells, (void**)&dNear)) return err;
-        CUDA_TRY(cudaMemsetAsync(dNear, 0xFF, sizeof(uint2) * nearCells, r->stream));
         if(const int err = upload(runs.data(), sizeof(ResidentRun) * runs.size(), (void**)&dRuns)) return err;
         L.runs = dRuns;
         L.entries = dEntries;
-        L.near_entries = dNear;
-        r->residentCells = 1e-6 * (double)(cells + nearCells);
+        r->residentCells = 1e-6 * (double)cells;
         if(const int err = residentPass(r, 1, nullptr, nullptr)) return err;
         CUDA_TRY(cudaStreamSynchronize(r->stream));         // (the temporaries go out of scope)
     }
@@ -1833,7 +1824,7 @@ int buildResident(b200_runner *r)
                                      g.num_trg, l.delayClass, l.src, l.trg, l.psm, g.num_src});
     }
     if(const int err = upload(spans.data(), sizeof(ResidentSpan) * spans.size(), (void**)&L.spans)) return err;
-    if(const int err = upload(nears.data(), sizeof(ResidentNear) * nears.size(), (void**)&L.near)) return err;
+    if(const int err = upload(rowStarts.data(), sizeof(unsigned long long) * rowStarts.size(), (void**)&L.rows)) return err;
     if(!poisson.empty()) {
         if(const int err = upload(poisson.data(), sizeof(float) * poisson.size(), (void**)&L.poisson)) return err;
     }
@@ -1852,7 +1843,7 @@ int buildResident(b200_runner *r)
     L.more = static_cast<unsigned long long*>(mail) + headWords;
     L.leave = L.more + moreWords;
 
-    L.unit_start = dUnitStart; L.unit_first = dUnitFirst; L.columns = dColumns; L.cta_columns = dCtaColumns; L.runs = dRuns; L.entries = dEntries; L.near_entries = dNear;
+    L.unit_start = dUnitStart; L.unit_first = dUnitFirst; L.columns = dColumns; L.cta_columns = dCtaColumns; L.runs = dRuns; L.entries = dEntries;
     L.num_spans = numSpans; L.num_units = units;
     L.num_depths = (unsigned int)depths.size();
     L.num_delays = numDelays;

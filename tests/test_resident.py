@@ -72,6 +72,49 @@ def test_launches_of_every_length_hand_over_to_the_other_paths(name):
     rt.close()
 
 
+@pytest.mark.parametrize("ctas", [1, 3, 40])
+@pytest.mark.parametrize("zero,synapses", [(0, 90), (1, 90), (2, 37), (64, 150), (65, 150), (150, 150)])
+def test_heads_and_shares_of_runs_match_the_cpu_checker(zero, synapses, ctas):
+    """`zero` synapses of every row have delay 0: no heads, heads of one entry, as many as a run may have, more than that (the
+    whole class in front of the update then), nothing else; rows of more than 128 entries are shared out between warps."""
+    from oracle.oracle import OracleRunner
+    rng = np.random.default_rng(zero + synapses)
+    n = 300
+
+    def model():
+        m = GeNNModel("float", "heads")
+        m.dt = 1.0
+        lif = {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.3, "TauRefrac": 2.0}
+        pops = [m.add_neuron_population(name, n, "LIF", lif, {"V": v0[name], "RefracTime": 0.0}) for name in "ab"]
+        for i, (src, trg) in enumerate(((pops[0], pops[1]), (pops[1], pops[1]))):
+            sg = m.add_synapse_population(f"s{i}", "SPARSE", src, trg, init_weight_update("StaticPulseDendriticDelay", {}, {"g": g[i], "d": d}),
+                                          init_postsynaptic("ExpCurr", {"tau": 3.0}))
+            sg.set_sparse_connections(pre, post[i], presorted=True)
+            sg.max_dendritic_delay_timesteps = 5
+        return m
+
+    v0 = {name: rng.uniform(-65, -49, n).astype(np.float32) for name in "ab"}
+    pre = np.repeat(np.arange(n, dtype=np.uint32), synapses)
+    # (equal targets side by side as well: rows are drawn with replacement)
+    post = [np.sort(rng.integers(0, n, (n, synapses)), axis=1).astype(np.uint32).ravel() for _ in range(2)]
+    d = np.tile(np.where(np.arange(synapses) < zero, 0, 1 + np.arange(synapses) % 4).astype(np.uint8), n)
+    g = [rng.uniform(0, 2e-3, n * synapses).astype(np.float32) for _ in range(2)]
+    net = resolve(model())
+    rt, orc = _runtime(net, 20), OracleRunner(resolve(model()), 20)
+    rt.set_option("resident_ctas", ctas)
+    assert rt.counter("resident") == 1
+    rt.set_option("count_events", 1)
+    for steps in (1, 1, 6, 12):
+        rt.step_time(steps)
+        orc.step(steps)
+        for p in net.pops:
+            assert np.array_equal(np.sort(rt.current_spikes(p.name)), np.sort(orc.current_spikes(p.name))), p.name
+            helpers.assert_close(rt.array(f"{p.name}.V")[0], orc.array(f"{p.name}.V")[0], f"V {p.name}", 1e-5, 2e-6)
+    assert rt.counter("spikes") > 0 and rt.counter("synaptic_events") % synapses == 0
+    rt.close()
+    orc.close()
+
+
 def _mixed():
     """Two populations that all fire at once (more spikes than a message head or the delivery list holds), groups of all
     three connectivities, axonal delays 0, 2 and 5, inputs with and without a ring."""
