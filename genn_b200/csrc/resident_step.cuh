@@ -42,14 +42,21 @@ __device__ __forceinline__ void residentAdd(float *cell, float v)
 }
 
 // ---- time steps ----------------------------------------------------------------------------------
-// The commonest neuron (LIF, one exponential current input, at most one Poisson source) with its constants side by side in
-// shared memory: the operations of neuronCompute in its order, without its choices of a model.
+// The commonest neurons (LIF, one or two exponential inputs, at most one Poisson source; spike sources) without neuronCompute's
+// choices of a model: its operations in its order, constants side by side in shared memory, places of the inputs in registers.
+// An SM with 21 warps of neurons is bound by their instructions, a smaller one by the chain of them: with the choices, a neuron
+// of two conductances took 1100 cycles of a step, one of a current input 500.
 struct ResidentLif
 {
     float vthresh, vreset, vrest, ioffset;
-    float rmembrane, exp_tc, tau_refrac, psm_init;
-    float psm_decay, cs_init, cs_decay, pad;
+    float rmembrane, exp_tc, tau_refrac, cs_init;
+    float cs_decay, pad[3];
+    struct { float level, decay; } input[2];    // EXP_CURR: its factor, EXP_COND: its reversal potential
 };
+
+// What a warp's neurons are (bits).
+constexpr unsigned int RESIDENT_IS_LIF = 1u, RESIDENT_IS_POISSON = 2u, RESIDENT_IS_ARRAY = 4u, RESIDENT_IS_DRAWN = 8u, RESIDENT_IS_SOURCE = 16u,
+                       RESIDENT_HAS_INPUT = 32u, RESIDENT_HAS_TWO = 64u, RESIDENT_COND = 128u, RESIDENT_COND_TWO = 256u;
 
 struct ResidentShared
 {
@@ -74,12 +81,17 @@ struct ResidentShared
 template<bool ONE>
 struct ResidentFronts
 {
-    unsigned int f[ONE ? 1 : RESIDENT_CLASSES];
-    __device__ __forceinline__ unsigned int operator[](unsigned int c) const
-    {
-        if constexpr(ONE) return f[0];
-        else return (c == 0u) ? f[0] : (c == 1u) ? f[1] : (c == 2u) ? f[2] : f[3];
-    }
+    unsigned int f[RESIDENT_CLASSES];
+    __device__ __forceinline__ unsigned int operator[](unsigned int c) const { return (c == 0u) ? f[0] : (c == 1u) ? f[1] : (c == 2u) ? f[2] : f[3]; }
+};
+
+// One ring class: where its front buffer begins, the columns of a buffer, and all of them.
+template<>
+struct ResidentFronts<true>
+{
+    unsigned int at, columns, all;
+    __device__ __forceinline__ void advance() { at = (at + columns == all) ? 0u : at + columns; }
+    __device__ __forceinline__ void back() { at = (at == 0u) ? all - columns : at - columns; }
 };
 
 extern __shared__ __align__(16) unsigned char residentSmem[];
@@ -126,10 +138,18 @@ struct ResidentDeliver
 
     __device__ __forceinline__ void add(unsigned int cls, unsigned int delay, unsigned int col, float v, const Fronts &front)
     {
-        unsigned int slot = front[cls] + delay;
-        const unsigned int D = ONE ? L.depth[0] : sh.depth[cls];
-        if(slot >= D) slot -= D;
-        residentAdd(residentTable<float>(L.at.acc) + (ONE ? 0u : sh.base[cls]) + slot * sh.columns[ONE ? 0u : cls] + col, v);
+        float *const acc = residentTable<float>(L.at.acc);
+        if constexpr(ONE) {
+            unsigned int at = front.at + delay * front.columns;
+            if(at >= front.all) at -= front.all;
+            residentAdd(acc + at + col, v);
+        }
+        else {
+            unsigned int slot = front[cls] + delay;
+            const unsigned int D = sh.depth[cls];
+            if(slot >= D) slot -= D;
+            residentAdd(acc + sh.base[cls] + slot * sh.columns[cls] + col, v);
+        }
         events++;
     }
 
@@ -319,13 +339,19 @@ __device__ __forceinline__ unsigned int residentPoisson(float u, const float *ta
 }
 
 template<int NPSM, int NCS>
-__device__ __forceinline__ bool residentLif(const ResidentLif &q, float dt, NeuronRegs<NPSM, NCS> &r, float in, bool source, unsigned int count)
+__device__ __forceinline__ bool residentLif(const ResidentLif &q, float dt, NeuronRegs<NPSM, NCS> &r, const float (&in)[NPSM], unsigned int what, unsigned int count)
 {
-    float V = __uint_as_float(r.v[0]), R = __uint_as_float(r.v[1]);
-    const float lin = B200_FADD(r.lin[0], in);
-    float Isyn = B200_FADD(0.0f, B200_FMUL(q.psm_init, lin));
-    r.lin[0] = B200_FMUL(lin, q.psm_decay);
-    if(NCS > 0 && source) {
+    float V = __uint_as_float(r.v[0]), R = __uint_as_float(r.v[1]), Isyn = 0.0f;
+    #pragma unroll
+    for(unsigned int p = 0; p < (NPSM < 2 ? NPSM : 2); p++) {
+        if(what & (p ? RESIDENT_HAS_TWO : RESIDENT_HAS_INPUT)) {
+            const float lin = B200_FADD(r.lin[p], in[p]), level = q.input[p].level;
+            const float factor = (what & (p ? RESIDENT_COND_TWO : RESIDENT_COND)) ? B200_FSUB(level, V) : level;
+            Isyn = B200_FADD(Isyn, B200_FMUL(lin, factor));
+            r.lin[p] = B200_FMUL(lin, q.input[p].decay);
+        }
+    }
+    if(NCS > 0 && (what & RESIDENT_IS_DRAWN)) {
         const float current = B200_FADD(r.cs[0], B200_FMUL(q.cs_init, (float)count));
         Isyn = B200_FADD(Isyn, current);
         r.cs[0] = B200_FMUL(current, q.cs_decay);
@@ -391,8 +417,15 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     for(unsigned int i = threadIdx.x; i < L.acc_floats; i += blockDim.x) acc[i] = 0.0f;
     if(threadIdx.x < numGroups) {
         const b200_neuron_group &g = L.neuron.groups[threadIdx.x];
-        sh.lif[threadIdx.x] = ResidentLif{g.params[0], g.params[1], g.params[2], g.params[3], g.params[4], g.params[5], g.params[6],
-                                          g.psm[0].params[0], g.psm[0].params[1], g.cs[0].params[0], g.cs[0].params[1], 0.0f};
+        ResidentLif &q = sh.lif[threadIdx.x];
+        q.vthresh = g.params[0]; q.vreset = g.params[1]; q.vrest = g.params[2]; q.ioffset = g.params[3];
+        q.rmembrane = g.params[4]; q.exp_tc = g.params[5]; q.tau_refrac = g.params[6];
+        q.cs_init = g.cs[0].params[0]; q.cs_decay = g.cs[0].params[1];
+        for(int i = 0; i < 2; i++) {
+            const bool cond = g.psm[i].model == B200_PSM_EXP_COND;
+            q.input[i].level = g.psm[i].params[cond ? 1 : 0];
+            q.input[i].decay = g.psm[i].params[cond ? 0 : 1];
+        }
     }
     __syncthreads();
     const unsigned int no0 = (unsigned int)sh.done;         // (step numbers of messages: 20 bits)
@@ -402,17 +435,25 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         sh.firstWarp[threadIdx.x] = (u <= me) ? 0u : (u - me + G - 1u) / G;
     }
     ResidentFronts<ONE> front;
-    #pragma unroll
-    for(unsigned int c = 0; c < (ONE ? 1u : RESIDENT_CLASSES); c++) front.f[c] = (sh.phase + 1u) % sh.depth[c];
+    if constexpr(ONE) {
+        front.columns = sh.columns[0];
+        front.all = sh.depth[0] * front.columns;
+        front.at = ((sh.phase + 1u) % sh.depth[0]) * front.columns;
+    }
+    else {
+        #pragma unroll
+        for(unsigned int c = 0; c < RESIDENT_CLASSES; c++) front.f[c] = (sh.phase + 1u) % sh.depth[c];
+    }
 
     // this thread's neuron
     const bool mine = warp < RESIDENT_UNITS && warp * G + me < L.num_units;
     unsigned int group = 0, local = 0;
-    bool active = false, isSource = false, lif = false;
+    bool active = false;
+    unsigned int what = 0;          // RESIDENT_IS_... (the same for a whole warp)
+    float nextTime = 0.0f;          // RESIDENT_IS_ARRAY: of the next spike
     NeuronRegs<NPSM, NCS> regs;
     unsigned int myCol[NPSM];       // ring class << 24 | place of buffer 0 of this neuron's input
     ResidentDraws draws;
-    bool drawn = false;             // one Poisson source: its draws come from `draws`
     #pragma unroll
     for(unsigned int p = 0; p < NPSM; p++) myCol[p] = 0u;
     if(mine) {
@@ -420,9 +461,20 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         local = (unitFirst[warp * G + me] & 0xFFFFFFu) + lane;
         const b200_neuron_group &g = groups[group];
         active = local < g.num_update;
-        isSource = (L.source_groups >> group) & 1ull;
-        lif = NPSM == 1 && NCS <= 1 && g.model == B200_NEURON_LIF && g.num_psm == 1u && g.psm[0].model == B200_PSM_EXP_CURR &&
-              (g.num_cs == 0u || (g.cs[0].model == B200_CS_POISSON_EXP && L.poisson));
+        if((L.source_groups >> group) & 1ull) what |= RESIDENT_IS_SOURCE;
+        const bool drawn = NCS == 1 && L.poisson && g.num_cs && g.cs[0].model == B200_CS_POISSON_EXP;
+        if(drawn) what |= RESIDENT_IS_DRAWN;
+        bool plain = g.num_psm <= 2u && (g.num_cs == 0u || drawn);
+        for(unsigned int p = 0; p < min(g.num_psm, 2u); p++) plain = plain && (g.psm[p].model == B200_PSM_EXP_CURR || g.psm[p].model == B200_PSM_EXP_COND);
+        if(g.model == B200_NEURON_LIF && plain) {
+            what |= RESIDENT_IS_LIF;
+            if(g.num_psm > 0u) what |= RESIDENT_HAS_INPUT | (g.psm[0].model == B200_PSM_EXP_COND ? RESIDENT_COND : 0u);
+            if(g.num_psm > 1u) what |= RESIDENT_HAS_TWO | (g.psm[1].model == B200_PSM_EXP_COND ? RESIDENT_COND_TWO : 0u);
+        }
+        if(g.num_psm == 0u && g.num_cs == 0u) {
+            if(g.model == B200_NEURON_POISSON) what |= RESIDENT_IS_POISSON;
+            if(g.model == B200_NEURON_SPIKE_SOURCE_ARRAY) what |= RESIDENT_IS_ARRAY;
+        }
         #pragma unroll
         for(unsigned int p = 0; p < NPSM; p++) {
             const unsigned int col = residentTable<const unsigned int>(L.at.columns)[warp * B200_MAX_PSM + p], c = col >> 16;
@@ -440,10 +492,8 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                     for(unsigned int d = 0; d < sh.depth[c]; d++) cell[d * n] = __ldcg(ring + (size_t)d * g.num_neurons);
                 }
             }
-            if(NCS == 1 && L.poisson && g.num_cs && g.cs[0].model == B200_CS_POISSON_EXP) {
-                drawn = true;
-                draws.start(L.neuron.seed, g.cs[0].rng_stream, local, t0);
-            }
+            if(NCS == 1 && drawn) draws.start(L.neuron.seed, g.cs[0].rng_stream, local, t0);
+            if((what & RESIDENT_IS_ARRAY) && regs.v[0] != regs.v[1]) nextTime = __ldg(&g.egp[regs.v[0]]);
         }
     }
     ResidentDeliver<ONE> deliver{L, sh, 0u};
@@ -494,9 +544,9 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     for(unsigned int step = 0; step < L.num_steps; step++) {
         // this step's random draws, while the messages are on their way
         unsigned int csCount[NCS > 0 ? NCS : 1] = {0};
-        if(mine && active) {
+        if(mine && active && !(what & RESIDENT_IS_ARRAY) && (NCS > 0 || !(what & RESIDENT_IS_LIF))) {
             const b200_neuron_group &g = groups[group];
-            if(NCS == 1 && drawn) {
+            if(NCS == 1 && (what & RESIDENT_IS_DRAWN)) {
                 csCount[0] = residentPoisson(draws.draw(L.neuron.seed, g.cs[0].rng_stream, local, t0 + step), residentTable<const float>(L.at.poisson) + 64u * group);
             }
             else drawCurrentSources<NCS>(L.neuron, g, 0u, local, t0 + step, csCount);
@@ -509,7 +559,6 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         }
 
         // ---------------- the spikes that reach their targets in this step (LATE: in the next) --------------------
-        ResidentHeld held;
         const unsigned int *heldList = nullptr;     // the last class's list, if some of its runs wait for the neuron update
         unsigned int heldCount = 0;
         for(unsigned int a = 0; a < numDelays; a++) {
@@ -537,8 +586,11 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                             // (entries of a LATE class say one step ahead)
                             ResidentFronts<ONE> at = front;
                             if(late && !ahead) {
-                                #pragma unroll
-                                for(unsigned int c = 0; c < (ONE ? 1u : RESIDENT_CLASSES); c++) at.f[c] = (at.f[c] == 0u) ? sh.depth[c] - 1u : at.f[c] - 1u;
+                                if constexpr(ONE) at.back();
+                                else {
+                                    #pragma unroll
+                                    for(unsigned int c = 0; c < RESIDENT_CLASSES; c++) at.f[c] = (at.f[c] == 0u) ? sh.depth[c] - 1u : at.f[c] - 1u;
+                                }
                             }
                             if(kind == RESIDENT_SPLIT) deliver.near(sh.list[turn], a, m, at);
                             deliver.runs(sh.list[turn], a, m, warp, at);
@@ -614,20 +666,27 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                 if(m && !(numDelays > 1u && late && step + 1u == sh.steps)) {
                     // runs of the last class that may wait for the neuron update
                     if(kind != RESIDENT_IMMEDIATE && all <= RESIDENT_LIST && a + 1u == numDelays) {
-                        deliver.fetch(held, list, a, m, warp);
                         heldList = list;
                         heldCount = m;
-                        if(kind == RESIDENT_SPLIT) deliver.near(list, a, m, front);
+                        break;
                     }
-                    else {
-                        if(kind == RESIDENT_SPLIT) deliver.near(list, a, m, front);
-                        deliver.runs(list, a, m, warp, front);
-                        deliver.spans(list, a, m, late, front);
-                    }
+                    if(kind == RESIDENT_SPLIT) deliver.near(list, a, m, front);
+                    deliver.runs(list, a, m, warp, front);
+                    deliver.spans(list, a, m, late, front);
                     // (nothing of a LATE class is for this step's update)
                     if(!late) __syncthreads();
                 }
                 if(all <= RESIDENT_LIST) break;
+            }
+        }
+        // (loaded here and nowhere else, so that no copy between registers waits for the loads)
+        ResidentHeld held;
+        if(heldList) {
+            const unsigned int a = numDelays - 1u;
+            deliver.fetch(held, heldList, a, heldCount, warp);
+            if(L.kind[a] == RESIDENT_SPLIT) {
+                deliver.near(heldList, a, heldCount, front);
+                __syncthreads();
             }
         }
         // ---------------- neuron update -------------------------------------------------------------------
@@ -637,24 +696,38 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
             const b200_neuron_group &g = groups[group];
             bool spiked = false;
             if(active) {
-                float in[NPSM];
-                #pragma unroll
-                for(unsigned int p = 0; p < NPSM; p++) {
-                    in[p] = 0.0f;
-                    if(p < g.num_psm) {
-                        const unsigned int c = ONE ? 0u : myCol[p] >> 24;
-                        float *cell = acc + (ONE ? myCol[p] : myCol[p] & 0xFFFFFFu) + front[c] * sh.columns[c];
-                        const float v = *cell;
-                        *cell = 0.0f;
-                        if(lif || g.psm[p].max_den_delay) in[p] = v;
-                        else regs.lin[p] = B200_FADD(regs.lin[p], v);
+                if(what & (RESIDENT_IS_POISSON | RESIDENT_IS_ARRAY)) {
+                    if(what & RESIDENT_IS_POISSON) {
+                        const float left = B200_FSUB(__uint_as_float(regs.v[0]), 1.0f);
+                        spiked = left <= 0.0f;
+                        regs.v[0] = __float_as_uint(left);
+                    }
+                    else if(regs.v[0] != regs.v[1] && B200_FMUL((float)(t0 + step), L.neuron.dt) >= nextTime) {
+                        spiked = true;
+                        if(++regs.v[0] != regs.v[1]) nextTime = __ldg(&g.egp[regs.v[0]]);
                     }
                 }
-                if(lif) spiked = residentLif(sh.lif[group], L.neuron.dt, regs, in[0], drawn, csCount[0]);
-                else spiked = neuronCompute(L.neuron, g, 0u, local, t0 + step, B200_FMUL((float)(t0 + step), L.neuron.dt), regs, in, csCount, true);
+                else {
+                    float in[NPSM];
+                    #pragma unroll
+                    for(unsigned int p = 0; p < NPSM; p++) {
+                        in[p] = 0.0f;
+                        if((what & RESIDENT_IS_LIF) ? p < 2u && (what & (p ? RESIDENT_HAS_TWO : RESIDENT_HAS_INPUT)) : p < g.num_psm) {
+                            float *cell = acc;
+                            if constexpr(ONE) cell += myCol[p] + front.at;
+                            else cell += (myCol[p] & 0xFFFFFFu) + front[myCol[p] >> 24] * sh.columns[myCol[p] >> 24];
+                            const float v = *cell;
+                            *cell = 0.0f;
+                            if((what & RESIDENT_IS_LIF) || g.psm[p].max_den_delay) in[p] = v;
+                            else regs.lin[p] = B200_FADD(regs.lin[p], v);
+                        }
+                    }
+                    if(what & RESIDENT_IS_LIF) spiked = residentLif(sh.lif[group], L.neuron.dt, regs, in, what, csCount[0]);
+                    else spiked = neuronCompute(L.neuron, g, 0u, local, t0 + step, B200_FMUL((float)(t0 + step), L.neuron.dt), regs, in, csCount, true);
+                }
             }
             ballot = __ballot_sync(0xFFFFFFFFu, spiked);
-            if(ballot && isSource) {
+            if(ballot && (what & RESIDENT_IS_SOURCE)) {
                 unsigned int at = 0;
                 if(lane == 0) at = atomicAdd(&sh.sent[par], __popc(ballot));
                 at = __shfl_sync(0xFFFFFFFFu, at, 0);
@@ -715,9 +788,12 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
             deliver.runs(heldList, a, heldCount, warp + warps, front);
             if(L.kind[a] == RESIDENT_LATE) deliver.spans(heldList, a, heldCount, 1u, front);
         }
-        #pragma unroll
-        for(unsigned int c = 0; c < (ONE ? 1u : RESIDENT_CLASSES); c++) {
-            if(c < L.num_depths) front.f[c] = (front.f[c] + 1u == L.depth[c]) ? 0u : front.f[c] + 1u;
+        if constexpr(ONE) front.advance();
+        else {
+            #pragma unroll
+            for(unsigned int c = 0; c < RESIDENT_CLASSES; c++) {
+                if(c < L.num_depths) front.f[c] = (front.f[c] + 1u == L.depth[c]) ? 0u : front.f[c] + 1u;
+            }
         }
         buf = (buf + 1u == L.buffers) ? 0u : buf + 1u;
         histAt = (histAt + 1u == L.history) ? 0u : histAt + 1u;

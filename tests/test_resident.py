@@ -115,6 +115,52 @@ def test_heads_and_shares_of_runs_match_the_cpu_checker(zero, synapses, ctas):
     orc.close()
 
 
+@pytest.mark.parametrize("kinds", [("ExpCurr", "ExpCond"), ("ExpCond", "ExpCurr"), ("ExpCond", "DeltaCurr"), ("ExpCurr", "ExpCurr", "ExpCond"), ()])
+def test_inputs_of_every_kind_match_the_cpu_checker(kinds):
+    """LIF neurons with one, two or three unfused inputs (none of them, and the spike sources, have a neuron update of their own),
+    spike sources whose trains end, begin late or hold several spikes of one step."""
+    from oracle.oracle import OracleRunner
+    rng = np.random.default_rng(len(kinds))
+    n, k = 100, 40
+    trains = [np.sort(rng.integers(0, 30, c)).astype(np.float32) for c in np.arange(n) % 5]
+    v0 = rng.uniform(-65, -51, n).astype(np.float32)
+    pre, posts = np.repeat(np.arange(n, dtype=np.uint32), k), [rng.integers(0, n, n * k).astype(np.uint32) for _ in kinds]
+    weights = [rng.uniform(0, 0.05, n * k).astype(np.float32) for _ in kinds]
+
+    def model():
+        m = GeNNModel("float", "inputs")
+        m.dt = 1.0
+        ends = np.cumsum([len(t) for t in trains]).astype(np.uint32)
+        src = m.add_neuron_population("src", n, "SpikeSourceArray", {}, {"startSpike": np.concatenate([[0], ends[:-1]]).astype(np.uint32), "endSpike": ends})
+        src.set_extra_global_param("spikeTimes", np.concatenate(trains))
+        trg = m.add_neuron_population("trg", n, "LIF", {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.4,
+                                                        "TauRefrac": 2.0}, {"V": v0, "RefracTime": 0.0})
+        for i, kind in enumerate(kinds):
+            params = {"ExpCurr": {"tau": 3.0 + i}, "ExpCond": {"tau": 5.0 + i, "E": 0.0}, "DeltaCurr": {}}[kind]
+            g = weights[i] * (0.02 if kind == "ExpCond" else 1.0)
+            sg = m.add_synapse_population(f"s{i}", "SPARSE", src, trg, init_weight_update("StaticPulse", {}, {"g": g.astype(np.float32)}), init_postsynaptic(kind, params))
+            sg.set_sparse_connections(pre, posts[i])
+        if not kinds:       # (a model needs synapses: from the neurons without an input, onto sources that keep none of it)
+            sg = m.add_synapse_population("back", "SPARSE", trg, src, init_weight_update("StaticPulse", {}, {"g": np.ones(n * k, np.float32)}), init_postsynaptic("ExpCurr", {"tau": 3.0}))
+            sg.set_sparse_connections(pre, rng.integers(0, n, n * k).astype(np.uint32))
+        return m
+
+    state = rng.bit_generator.state
+    net = resolve(model())
+    rng.bit_generator.state = state
+    rt, orc = _runtime(net, 40), OracleRunner(resolve(model()), 40)
+    assert rt.counter("resident") == 1
+    for steps in (1, 2, 7, 30):
+        rt.step_time(steps)
+        orc.step(steps)
+        for p in net.pops:
+            assert np.array_equal(np.sort(rt.current_spikes(p.name)), np.sort(orc.current_spikes(p.name))), p.name
+        helpers.assert_close(rt.array("trg.V")[0], orc.array("trg.V")[0], "V", 1e-5, 2e-6)
+        assert np.array_equal(rt.array("src.startSpike"), orc.array("src.startSpike"))
+    rt.close()
+    orc.close()
+
+
 def _mixed():
     """Two populations that all fire at once (more spikes than a message head or the delivery list holds), groups of all
     three connectivities, axonal delays 0, 2 and 5, inputs with and without a ring."""
