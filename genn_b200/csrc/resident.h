@@ -168,7 +168,40 @@ struct ResidentBuild
     unsigned int runs_stride;           // distance between the pair's runs of two CTAs
 };
 
-// kernels: resident.cu
+// ---- windows of steps (resident_window.cuh) ----------------------------------------------------------
+// Where no spike of a window of steps reaches anybody in that window, CTAs exchange once a window.
+constexpr unsigned int RESIDENT_WINDOW_MOST = 16;       // most steps of a window
+constexpr unsigned int RESIDENT_WINDOW_LEAST = 4;       // fewest
+constexpr unsigned int RESIDENT_HEADS = RESIDENT_MAX_CTAS + RESIDENT_UNITS;     // (those of a reading warp lie side by side, the last of each short)
+constexpr unsigned int RESIDENT_WINDOW_LIST = 40960;    // spikes of a window that the list has room for (160 KB)
+
+constexpr unsigned int RESIDENT_WINDOW_SPARE = 5500;    // ns that a step without spikes costs less than on the kernel with a grid barrier
+
+struct ResidentWindow
+{
+    unsigned int steps;                 // of a window
+    unsigned int feed;                  // 1: the spikes come from populations without inputs, which are a window ahead of the others
+    unsigned int lag;                   // else: windows between a spike's and the one it arrives in
+    unsigned int cap;                   // spikes of one step that the list has room for
+    unsigned int ring;                  // steps whose ballots are kept
+    unsigned int buffers;               // of messages
+    unsigned int body;                  // most spikes of a message
+    unsigned int run_groups;            // groups of 32 entries of the longest run (0: no runs)
+    unsigned int list_at, words_at, acc_at;     // in dynamic shared memory, behind the tables of ResidentLayout
+    unsigned int epoch;                 // of the launch
+    unsigned long long free_groups;     // populations without inputs (FEED)
+    unsigned long long *heads;          // [buffers][copies][RESIDENT_HEADS] tag << 20 | spikes
+    unsigned short *bodies;             // [buffers][grid][body] step of the window << 10 | unit of the CTA << 5 | neuron
+};
+
+struct ResidentWindowLaunch
+{
+    ResidentLaunch L;
+    ResidentWindow W;
+};
+
+// kernels: resident.cu, resident_window.cu
+const void *residentWindowKernelFor(int npsm, int ncs);
 const void *residentKernelFor(int npsm, int ncs, bool one_class, unsigned int threads);
 cudaError_t residentBuild(const ResidentBuild &B, int pass, unsigned int *longest, const ResidentRun *runs, uint2 *entries, StepState *state,
                           unsigned int blocks, cudaStream_t stream);

@@ -338,6 +338,56 @@ __device__ __forceinline__ unsigned int residentPoisson(float u, const float *ta
     return n;
 }
 
+__device__ __forceinline__ void residentLifTable(ResidentLif &q, const b200_neuron_group &g)
+{
+    q.vthresh = g.params[0]; q.vreset = g.params[1]; q.vrest = g.params[2]; q.ioffset = g.params[3];
+    q.rmembrane = g.params[4]; q.exp_tc = g.params[5]; q.tau_refrac = g.params[6];
+    q.cs_init = g.cs[0].params[0]; q.cs_decay = g.cs[0].params[1];
+    for(int i = 0; i < 2; i++) {
+        const bool cond = g.psm[i].model == B200_PSM_EXP_COND;
+        q.input[i].level = g.psm[i].params[cond ? 1 : 0];
+        q.input[i].decay = g.psm[i].params[cond ? 0 : 1];
+    }
+}
+
+// `table`: Poisson sources have their counts looked up (residentPoisson).
+template<int NCS>
+__device__ __forceinline__ unsigned int residentWhat(const b200_neuron_group &g, bool source, bool table)
+{
+    unsigned int what = source ? RESIDENT_IS_SOURCE : 0u;
+    const bool drawn = NCS == 1 && table && g.num_cs && g.cs[0].model == B200_CS_POISSON_EXP;
+    if(drawn) what |= RESIDENT_IS_DRAWN;
+    bool plain = g.num_psm <= 2u && (g.num_cs == 0u || drawn);
+    for(unsigned int p = 0; p < min(g.num_psm, 2u); p++) plain = plain && (g.psm[p].model == B200_PSM_EXP_CURR || g.psm[p].model == B200_PSM_EXP_COND);
+    if(g.model == B200_NEURON_LIF && plain) {
+        what |= RESIDENT_IS_LIF;
+        if(g.num_psm > 0u) what |= RESIDENT_HAS_INPUT | (g.psm[0].model == B200_PSM_EXP_COND ? RESIDENT_COND : 0u);
+        if(g.num_psm > 1u) what |= RESIDENT_HAS_TWO | (g.psm[1].model == B200_PSM_EXP_COND ? RESIDENT_COND_TWO : 0u);
+    }
+    if(g.num_psm == 0u && g.num_cs == 0u) {
+        if(g.model == B200_NEURON_POISSON) what |= RESIDENT_IS_POISSON;
+        if(g.model == B200_NEURON_SPIKE_SOURCE_ARRAY) what |= RESIDENT_IS_ARRAY;
+    }
+    return what;
+}
+
+// What a launch leaves behind of its account: `debt` at its end, `done` steps by then.
+__device__ __forceinline__ void residentSettle(const ResidentLaunch &L, StepState &state, int debt, unsigned int step, unsigned long long done)
+{
+    if(step < L.num_steps || (unsigned int)debt > L.patience) {
+        const unsigned int rest = min(max(2u * state.resident_rest, RESIDENT_REST), RESIDENT_MOST_REST);
+        state.resident_rest = rest;
+        state.resident_hold = done + rest;
+        state.resident_debt = min((unsigned int)debt, L.patience - L.patience / 4u);       // (the next time it is seen sooner)
+        *reinterpret_cast<volatile unsigned long long*>(L.hold) = done + rest;
+    }
+    else {
+        // (as many steps without that make up for one time)
+        state.resident_rest -= min(state.resident_rest, step);
+        state.resident_debt = (unsigned int)debt;
+    }
+}
+
 template<int NPSM, int NCS>
 __device__ __forceinline__ bool residentLif(const ResidentLif &q, float dt, NeuronRegs<NPSM, NCS> &r, const float (&in)[NPSM], unsigned int what, unsigned int count)
 {
@@ -416,16 +466,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     }
     for(unsigned int i = threadIdx.x; i < L.acc_floats; i += blockDim.x) acc[i] = 0.0f;
     if(threadIdx.x < numGroups) {
-        const b200_neuron_group &g = L.neuron.groups[threadIdx.x];
-        ResidentLif &q = sh.lif[threadIdx.x];
-        q.vthresh = g.params[0]; q.vreset = g.params[1]; q.vrest = g.params[2]; q.ioffset = g.params[3];
-        q.rmembrane = g.params[4]; q.exp_tc = g.params[5]; q.tau_refrac = g.params[6];
-        q.cs_init = g.cs[0].params[0]; q.cs_decay = g.cs[0].params[1];
-        for(int i = 0; i < 2; i++) {
-            const bool cond = g.psm[i].model == B200_PSM_EXP_COND;
-            q.input[i].level = g.psm[i].params[cond ? 1 : 0];
-            q.input[i].decay = g.psm[i].params[cond ? 0 : 1];
-        }
+        residentLifTable(sh.lif[threadIdx.x], L.neuron.groups[threadIdx.x]);
     }
     __syncthreads();
     const unsigned int no0 = (unsigned int)sh.done;         // (step numbers of messages: 20 bits)
@@ -461,20 +502,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         local = (unitFirst[warp * G + me] & 0xFFFFFFu) + lane;
         const b200_neuron_group &g = groups[group];
         active = local < g.num_update;
-        if((L.source_groups >> group) & 1ull) what |= RESIDENT_IS_SOURCE;
-        const bool drawn = NCS == 1 && L.poisson && g.num_cs && g.cs[0].model == B200_CS_POISSON_EXP;
-        if(drawn) what |= RESIDENT_IS_DRAWN;
-        bool plain = g.num_psm <= 2u && (g.num_cs == 0u || drawn);
-        for(unsigned int p = 0; p < min(g.num_psm, 2u); p++) plain = plain && (g.psm[p].model == B200_PSM_EXP_CURR || g.psm[p].model == B200_PSM_EXP_COND);
-        if(g.model == B200_NEURON_LIF && plain) {
-            what |= RESIDENT_IS_LIF;
-            if(g.num_psm > 0u) what |= RESIDENT_HAS_INPUT | (g.psm[0].model == B200_PSM_EXP_COND ? RESIDENT_COND : 0u);
-            if(g.num_psm > 1u) what |= RESIDENT_HAS_TWO | (g.psm[1].model == B200_PSM_EXP_COND ? RESIDENT_COND_TWO : 0u);
-        }
-        if(g.num_psm == 0u && g.num_cs == 0u) {
-            if(g.model == B200_NEURON_POISSON) what |= RESIDENT_IS_POISSON;
-            if(g.model == B200_NEURON_SPIKE_SOURCE_ARRAY) what |= RESIDENT_IS_ARRAY;
-        }
+        what = residentWhat<NCS>(g, (L.source_groups >> group) & 1ull, L.poisson != nullptr);
         #pragma unroll
         for(unsigned int p = 0; p < NPSM; p++) {
             const unsigned int col = residentTable<const unsigned int>(L.at.columns)[warp * B200_MAX_PSM + p], c = col >> 16;
@@ -492,7 +520,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
                     for(unsigned int d = 0; d < sh.depth[c]; d++) cell[d * n] = __ldcg(ring + (size_t)d * g.num_neurons);
                 }
             }
-            if(NCS == 1 && drawn) draws.start(L.neuron.seed, g.cs[0].rng_stream, local, t0);
+            if(what & RESIDENT_IS_DRAWN) draws.start(L.neuron.seed, g.cs[0].rng_stream, local, t0);
             if((what & RESIDENT_IS_ARRAY) && regs.v[0] != regs.v[1]) nextTime = __ldg(&g.egp[regs.v[0]]);
         }
     }
@@ -878,19 +906,7 @@ ended: __attribute__((unused));
         state->steps_done = doneNow;
         state->phase = k;
         const unsigned int quiet = (step > sh.accounted) ? min(step - sh.accounted, 1u << 14) : 0u;
-        const unsigned int debt = (unsigned int)max(sh.debt - (int)(quiet * (L.spare / 2u)), 0);
-        if(step < L.num_steps || debt > L.patience) {
-            const unsigned int rest = min(max(2u * state->resident_rest, RESIDENT_REST), RESIDENT_MOST_REST);
-            state->resident_rest = rest;
-            state->resident_hold = doneNow + rest;
-            state->resident_debt = min(debt, L.patience - L.patience / 4u);       // (the next time it is seen sooner)
-            *reinterpret_cast<volatile unsigned long long*>(L.hold) = doneNow + rest;
-        }
-        else {
-            // (as many steps without that make up for one time)
-            state->resident_rest -= min(state->resident_rest, step);
-            state->resident_debt = debt;
-        }
+        residentSettle(L, *state, max(sh.debt - (int)(quiet * (L.spare / 2u)), 0), step, doneNow);
     }
 }
 

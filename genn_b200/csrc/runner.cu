@@ -70,6 +70,7 @@ constexpr uint64_t FIRST_BLOCK = 64;         // steps of the first launch of the
 constexpr uint64_t QUIET_BLOCK = 2048;       // a network that was busy at first is soon tried again; once a call has passed quietly
 constexpr uint64_t LONG_CALL = 10000;        // steps of a first call in the middle of which the host looks whether the other kernel has taken over
 constexpr uint64_t LONG_HOLD = 512;          // steps of that kernel's turn from which its own tables are made (with rings: 2 - 20 ms)
+constexpr uint64_t WINDOW_STEPS = 4;         // steps of a launch from which they are done in windows where they can be
 constexpr double MOST_LOSS = 1.0e6;          // ns that a call of the target-resident kernel may lose with no launch behind it, for each of the
 constexpr unsigned int MOST_QUIET = 50;      // quiet calls before it, up to this many (a launch for nothing: 4 us, a tenth of a short call)
 constexpr size_t ARRAY_TAIL_PAD = 256;     // vector loads may read up to 15 bytes past the last element
@@ -341,6 +342,12 @@ struct b200_runner
     size_t residentMailBytes = 0;
     const void *residentKernel = nullptr;
     ResidentLaunch resident{};
+    bool useWindow = true, windowReady = false;             // windows of steps (resident_window.cuh)
+    ResidentWindow window{};
+    const void *windowKernel = nullptr;
+    size_t windowSmem = 0;
+    unsigned int windowBlock = 0;
+    bool windowMayOverflow = false;                         // a step may have more spikes than its list holds: a launch has to follow
     std::vector<void*> residentBuffers;
     // busy networks (resident.h): the kernel with a grid barrier takes over
     volatile unsigned long long *residentHold = nullptr;    // page-locked: until which step it goes on
@@ -357,7 +364,7 @@ struct b200_runner
     {
         for(void *p : residentBuffers) poolFree(p, stream);
         residentBuffers.clear();
-        residentReady = false;
+        residentReady = windowReady = false;
         residentCleared = ~0ull;
     }
 
@@ -1582,6 +1589,39 @@ int buildResident(b200_runner *r)
         return (unsigned int)(std::find(depths.begin(), depths.end(), d) - depths.begin());
     };
 
+    // ---- windows of steps (resident_window.cuh) ----------------------------------------------------------------
+    ResidentWindow &win = r->window;
+    win = ResidentWindow{};
+    bool windowed = r->useWindow && numDelays == 1 && depths.size() == 1;
+    unsigned long long sourceGroups = 0, freeGroups = 0, sourceNeurons = 0;
+    for(const auto &l : links) sourceGroups |= 1ull << l.src;
+    for(size_t ni = 0; ni < numGroups; ni++) {
+        const auto &g = r->neuronGroups[ni];
+        for(unsigned int p = 0; p < g.num_psm; p++) windowed = windowed && !g.psm[p].max_den_delay;
+        if(!((sourceGroups >> ni) & 1ull)) continue;
+        sourceNeurons += g.num_neurons;
+        if((g.model == B200_NEURON_POISSON || g.model == B200_NEURON_SPIKE_SOURCE_ARRAY) && !g.num_psm && !g.num_cs) freeGroups |= 1ull << ni;
+    }
+    if(windowed) {
+        const unsigned int after = delays[0] + 1u;
+        if(freeGroups == sourceGroups) {
+            // (a list that holds every source: a launch cannot stop short of where the sources have got to)
+            win.feed = 1u;
+            win.free_groups = freeGroups;
+            win.steps = (unsigned int)std::min<unsigned long long>(RESIDENT_WINDOW_MOST, RESIDENT_WINDOW_LIST / std::max(1ull, sourceNeurons));
+            win.cap = (unsigned int)std::min<unsigned long long>(sourceNeurons, RESIDENT_WINDOW_LIST);
+            win.buffers = 4u;
+        }
+        else {
+            for(win.lag = 1; after % win.lag || after / win.lag > RESIDENT_WINDOW_MOST; win.lag++) {}
+            win.steps = after / win.lag;
+            win.cap = (unsigned int)std::min<unsigned long long>(sourceNeurons, RESIDENT_LIST);
+            win.buffers = 2u * win.lag + 2u;
+            windowed = win.cap >= sourceNeurons || r->residentHandsOver;
+        }
+        windowed = windowed && win.steps >= RESIDENT_WINDOW_LEAST;
+    }
+
     // ---- how many CTAs, how many warps ----------------------------------------------------------------------
     const NeuronShape shape = neuronShape(r);
     cudaFuncAttributes attr{};
@@ -1621,6 +1661,12 @@ int buildResident(b200_runner *r)
     int optin = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, r->device));
     const size_t room = (size_t)optin - attr.sharedSizeBytes;
+    size_t windowRoom = 0;
+    if(windowed) {
+        CUDA_TRY(cudaFuncGetAttributes(&attr, residentWindowKernelFor(shape.npsm, shape.ncs)));
+        windowRoom = (size_t)optin - attr.sharedSizeBytes;
+        win.ring = std::max(history, win.steps);
+    }
     auto groupOf = [&](unsigned int u) { return (unsigned int)(std::upper_bound(unitStart.begin(), unitStart.end(), u) - unitStart.begin()) - 1u; };
     std::vector<unsigned int> columns, ctaColumns;
     unsigned int grid = 0;
@@ -1645,7 +1691,25 @@ int buildResident(b200_runner *r)
         }
     };
     const unsigned int most = std::min<unsigned int>((unsigned int)sms, RESIDENT_MAX_CTAS);
-    {
+    // the list and the ballots lie where the other kernel's input buffers begin, the buffers of a window behind them
+    auto windowBytes = [&] {
+        win.list_at = L.at.history;
+        win.words_at = win.list_at + (unsigned int)align16(sizeof(unsigned int) * win.steps * win.cap);
+        win.acc_at = win.words_at + (unsigned int)align16(sizeof(unsigned int) * win.ring * RESIDENT_UNITS);
+        return win.acc_at + accFloats / depths[0] * win.steps * sizeof(float);
+    };
+    if(windowed) {
+        // (a window's messages cost little, and its deliveries and updates are shared by all SMs.  us a step on 48 / 100 / 148 CTAs: 1000 ->
+        // 10 000 neurons 0.33 / 0.32 / 0.32, BITMASK 2003 x 5009 0.93 / 0.88 / 0.82, DENSE 4096 x 4096 2.14 / 1.77 / 1.41)
+        const unsigned int G = std::min(std::max(r->residentCtas ? r->residentCtas : most, (units + RESIDENT_UNITS - 1u) / RESIDENT_UNITS), std::min(most, units));
+        if((units + G - 1u) / G <= RESIDENT_UNITS) {
+            layOut(G);
+            r->windowSmem = windowBytes();
+            if(tables + accFloats * sizeof(float) <= room && r->windowSmem <= windowRoom) grid = G;
+        }
+        windowed = grid != 0u;
+    }
+    if(!windowed) {
         // Units of 32 neurons for a CTA.  More CTAs share the work of a step but lengthen the exchange.  us a step, this rule / the
         // best of seven grids from 16 to 148 CTAs (at which): SPARSE 1000 + 1000 3.0 / 2.9 (64), 3000 3.5 / 3.5, 5000 4.2 / 4.2,
         // 10 000 4.4 / 3.8 (32), 20 000 6.3 / 5.3 (64), 50 000 6.8 / 6.7; with rings 1000 2.6 / 2.5, 3000 3.4 / 3.1 (16), 8000 5.9
@@ -1671,6 +1735,7 @@ int buildResident(b200_runner *r)
     unsigned int warps = r->residentWarps ? r->residentWarps : std::max(numSpans ? 16u : 8u, neuronWarps + (grid + 31u) / 32u);
     if(neuronWarps <= RESIDENT_FEW / 32u && !r->residentWarps) warps = std::min(warps, RESIDENT_FEW / 32u);
     warps = std::min(std::max(warps, std::max(neuronWarps, (grid + 31u) / 32u)), RESIDENT_UNITS);
+    r->windowBlock = 32u * (r->residentWarps ? warps : RESIDENT_UNITS);
     r->residentKernel = residentKernelFor(shape.npsm, shape.ncs, oneClass, warps * 32u);
 
     auto device = [&](size_t bytes, void **out) -> int {
@@ -1762,6 +1827,7 @@ int buildResident(b200_runner *r)
                 run.length = ((near + longestHost[c * runsPerCta + pair] + 3u) & ~3u) - near;
                 row += near + run.length;
                 L.chunks[a] = std::max(L.chunks[a], (run.length + RESIDENT_CHUNK - 1u) / RESIDENT_CHUNK);
+                win.run_groups = std::max(win.run_groups, (run.length + 31u) / 32u);
             }
             rowStarts[pair] = cells;
             cells += (unsigned long long)row * r->neuronGroups[pair % numGroups].num_neurons;
@@ -1861,8 +1927,24 @@ int buildResident(b200_runner *r)
         *r->residentHold = 0ull;
     }
     L.hold = const_cast<unsigned long long*>(r->residentHold);
+    if(windowed) {
+        win.body = neuronWarps * 32u * win.steps;
+        if(const int err = device(sizeof(unsigned long long) * win.buffers * L.copies * RESIDENT_HEADS, (void**)&win.heads)) return err;
+        if(const int err = device(sizeof(unsigned short) * win.buffers * grid * win.body, (void**)&win.bodies)) return err;
+        CUDA_TRY(cudaMemsetAsync(win.heads, 0, sizeof(unsigned long long) * win.buffers * L.copies * RESIDENT_HEADS, r->stream));
+        r->windowKernel = residentWindowKernelFor(shape.npsm, shape.ncs);
+        CUDA_TRY(cudaFuncSetAttribute(r->windowKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)windowRoom));
+        r->windowMayOverflow = win.cap < sourceNeurons;
+        r->windowReady = true;
+    }
     r->residentReady = true;
     return B200_OK;
+}
+
+// Whether a launch of so many steps goes through them in windows.
+bool useWindows(const b200_runner *r, unsigned long long numSteps)
+{
+    return r->windowReady && numSteps >= WINDOW_STEPS;
 }
 
 // `done`: steps done when the launch begins; `leave`: a launch of the kernel with a grid barrier follows for what it leaves.
@@ -1884,6 +1966,21 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
     L.may_leave = leave ? 1u : 0u;
     L.patience = (unsigned int)std::min(1000.0 * r->residentPatience, (double)RESIDENT_MOST_DEBT - 1.0);
     L.barrier = r->fusedBarrier;
+    if(useWindows(r, numSteps)) {
+        // (a head is known by its launch's number: before it repeats, no old head may be left)
+        r->window.epoch = (r->window.epoch + 1u) & 0xFFFFFu;
+        if(r->window.epoch == 0u) {
+            CUDA_TRY(cudaMemsetAsync(r->window.heads, 0, sizeof(unsigned long long) * r->window.buffers * L.copies * RESIDENT_HEADS, r->stream));
+            r->window.epoch = 1u;
+        }
+        ResidentWindowLaunch A{L, r->window};
+        if(r->residentHandsOver) A.L.spare = RESIDENT_WINDOW_SPARE;
+        void *args[] = {&A};
+        CUDA_TRY(cudaLaunchCooperativeKernel(r->windowKernel, dim3(r->residentGrid), dim3(r->windowBlock), args, r->windowSmem, r->stream));
+        r->launches++;
+        r->fusedLaunches++;
+        return B200_OK;
+    }
     // a message word is known by the last 20 bits of its step: before they repeat, no old word may be left.  (Steps on other
     // paths count too: they leave the words of earlier steps where they are.)
     if(r->residentCleared == ~0ull || done + numSteps - r->residentCleared >= RESIDENT_TAG_STEPS - 1ull) {
@@ -2725,6 +2822,7 @@ int b200_set_option(b200_runner *r, const char *name, double value)
             r->residentRent = 0;
         }
     }
+    else if(n == "use_windows") { r->useWindow = (value != 0.0); r->residentStale = true; r->residentRent = 0; }
     else if(n == "resident_ctas") { r->residentCtas = (unsigned int)std::max(0.0, value); r->residentStale = true; r->residentRent = 0; }
     else if(n == "resident_warps") { r->residentWarps = (unsigned int)std::max(0.0, value); r->residentStale = true; r->residentRent = 0; }
     else if(n == "resident_patience") {
@@ -2969,7 +3067,7 @@ int b200_step_time(b200_runner *r, uint64_t num_steps, uint64_t num_recording_ti
                 continue;
             }
             const uint64_t n = std::min<uint64_t>(left, std::min<uint64_t>(block, RESIDENT_TAG_STEPS / 2));
-            const bool leave = r->residentHandsOver && (r->residentPatienceChosen || (double)n * r->residentWorst > MOST_LOSS * (1u + std::min(r->residentQuiet, MOST_QUIET)));
+            const bool leave = r->residentHandsOver && (r->residentPatienceChosen || (r->windowMayOverflow && useWindows(r, n)) || (double)n * r->residentWorst > MOST_LOSS * (1u + std::min(r->residentQuiet, MOST_QUIET)));
             e = launchResident(r, n, num_recording_timesteps, done, leave);
             if(e == B200_OK && leave) e = launchFused(r, n, num_recording_timesteps, done + n);
             if(e) return e;
@@ -3205,6 +3303,15 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
     if(n == "resident_builds") {
         // how often the copy has been made (not: filled again with other weights)
         *value = r->residentBuilds;
+        return B200_OK;
+    }
+    if(n == "window_steps") {
+        // steps of a window (resident_window.cuh), 0 where that kernel does not apply
+        int e = prepare(r);
+        bool yes = false;
+        if(!e) e = chooseResident(r, &yes);
+        if(e) return e;
+        *value = yes && r->windowReady ? r->window.steps : 0u;
         return B200_OK;
     }
     if(n == "resident_hold") {

@@ -393,6 +393,8 @@ int  b200_get_counter(b200_runner *r, const char *name, uint64_t *value);
  * "resident_warps" (its grid and block; 0: chosen by size), "resident_patience" (microseconds that it may lose to the kernel with a
  * grid barrier, which is faster from some 100 spikes a step on, before that one takes over for a while; default 200; counter
  * "resident_hold": the step until which; "resident_builds": how often the copy was made),
+ * "use_windows" (default 1: where no spike of several steps reaches anybody within them, that kernel goes through them a window at a
+ * time; counter "window_steps": how many, 0 where that does not apply),
  * "scatter_min_spikes" (batched networks: spikes of a copy and step, by the largest count of the steps before, from which SPARSE
  * groups whose target buffer fits an SM's shared memory are summed there, default 64; 0: always; counter "scatter_armed"),
  * "barrier_spin_limit" / "exchange_spin_limit" (polls) and "stream_wait_cycles" (SM cycles): how long a wait
