@@ -141,5 +141,21 @@ __device__ __forceinline__ void stageWords(void *dst, const void *src, size_t by
     for(size_t w = threadIdx.x; w < bytes / 4; w += blockDim.x) d[w] = __ldg(&s[w]);
 }
 
+// The same without waiting: several tables take one round trip to memory, not one each.  stagedWords() and a barrier of the CTA
+// end it.
+__device__ __forceinline__ void stageWordsAsync(void *dst, const void *src, size_t bytes)
+{
+    const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+    const unsigned int *s = static_cast<const unsigned int*>(src);
+    for(unsigned int w = threadIdx.x; w < (unsigned int)(bytes / 4); w += blockDim.x) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(d + 4u * w), "l"(__cvta_generic_to_global(s + w)) : "memory");
+    }
+}
+
+__device__ __forceinline__ void stagedWords()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 }   // namespace b200

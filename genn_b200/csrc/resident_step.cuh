@@ -431,19 +431,22 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     const unsigned int *const unitFirst = residentTable<const unsigned int>(L.at.unit_first);
     float *const acc = residentTable<float>(L.at.acc);
     // tables into shared memory
-    stageWords(residentSmem + L.at.groups, L.neuron.groups, sizeof(b200_neuron_group) * numGroups);
-    stageWords(residentSmem + L.at.unit_start, L.unit_start, sizeof(unsigned int) * (numGroups + 1));
-    stageWords(residentSmem + L.at.unit_first, L.unit_first, sizeof(unsigned int) * L.num_units);
-    stageWords(residentSmem + L.at.columns, L.columns + (size_t)me * RESIDENT_UNITS * B200_MAX_PSM, sizeof(unsigned int) * RESIDENT_UNITS * B200_MAX_PSM);
-    stageWords(residentSmem + L.at.runs, L.runs + (size_t)me * numDelays * numGroups, sizeof(ResidentRun) * numDelays * numGroups);
-    stageWords(residentSmem + L.at.rows, L.rows, sizeof(unsigned long long) * numDelays * numGroups);
-    stageWords(residentSmem + L.at.spans, L.spans, sizeof(ResidentSpan) * L.num_spans);
-    if(L.poisson) stageWords(residentSmem + L.at.poisson, L.poisson, sizeof(float) * 64u * numGroups);
+    stageWordsAsync(residentSmem + L.at.groups, L.neuron.groups, sizeof(b200_neuron_group) * numGroups);
+    stageWordsAsync(residentSmem + L.at.unit_start, L.unit_start, sizeof(unsigned int) * (numGroups + 1));
+    stageWordsAsync(residentSmem + L.at.unit_first, L.unit_first, sizeof(unsigned int) * L.num_units);
+    stageWordsAsync(residentSmem + L.at.columns, L.columns + (size_t)me * RESIDENT_UNITS * B200_MAX_PSM, sizeof(unsigned int) * RESIDENT_UNITS * B200_MAX_PSM);
+    stageWordsAsync(residentSmem + L.at.runs, L.runs + (size_t)me * numDelays * numGroups, sizeof(ResidentRun) * numDelays * numGroups);
+    stageWordsAsync(residentSmem + L.at.rows, L.rows, sizeof(unsigned long long) * numDelays * numGroups);
+    stageWordsAsync(residentSmem + L.at.spans, L.spans, sizeof(ResidentSpan) * L.num_spans);
+    if(L.poisson) stageWordsAsync(residentSmem + L.at.poisson, L.poisson, sizeof(float) * 64u * numGroups);
     StepState *const state = L.neuron.state;
     const unsigned long long t0 = state->timestep;
     if(L.may_leave) {
         if(me == 0 && threadIdx.x == 0) *L.barrier = 0ull;
-        if(state->steps_done < state->resident_hold) return;        // (the same for every CTA: both change at the end of a launch)
+        if(state->steps_done < state->resident_hold) {              // (the same for every CTA: both change at the end of a launch)
+            stagedWords();
+            return;
+        }
     }
     if(threadIdx.x == 0) {
         sh.debt = (int)state->resident_debt;
@@ -468,6 +471,7 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
     if(threadIdx.x < numGroups) {
         residentLifTable(sh.lif[threadIdx.x], L.neuron.groups[threadIdx.x]);
     }
+    stagedWords();
     __syncthreads();
     const unsigned int no0 = (unsigned int)sh.done;         // (step numbers of messages: 20 bits)
     if(threadIdx.x <= numGroups) {

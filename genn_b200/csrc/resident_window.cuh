@@ -111,18 +111,21 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
     unsigned int *const list = residentTable<unsigned int>(W.list_at);
     unsigned int *const words = residentTable<unsigned int>(W.words_at);
     float *const acc = residentTable<float>(W.acc_at);
-    stageWords(residentSmem + L.at.groups, L.neuron.groups, sizeof(b200_neuron_group) * numGroups);
-    stageWords(residentSmem + L.at.unit_start, L.unit_start, sizeof(unsigned int) * (numGroups + 1));
-    stageWords(residentSmem + L.at.unit_first, L.unit_first, sizeof(unsigned int) * L.num_units);
-    stageWords(residentSmem + L.at.columns, L.columns + (size_t)me * RESIDENT_UNITS * B200_MAX_PSM, sizeof(unsigned int) * RESIDENT_UNITS * B200_MAX_PSM);
-    stageWords(residentSmem + L.at.runs, L.runs + (size_t)me * numGroups, sizeof(ResidentRun) * numGroups);
-    stageWords(residentSmem + L.at.rows, L.rows, sizeof(unsigned long long) * numGroups);
-    stageWords(residentSmem + L.at.spans, L.spans, sizeof(ResidentSpan) * L.num_spans);
+    stageWordsAsync(residentSmem + L.at.groups, L.neuron.groups, sizeof(b200_neuron_group) * numGroups);
+    stageWordsAsync(residentSmem + L.at.unit_start, L.unit_start, sizeof(unsigned int) * (numGroups + 1));
+    stageWordsAsync(residentSmem + L.at.unit_first, L.unit_first, sizeof(unsigned int) * L.num_units);
+    stageWordsAsync(residentSmem + L.at.columns, L.columns + (size_t)me * RESIDENT_UNITS * B200_MAX_PSM, sizeof(unsigned int) * RESIDENT_UNITS * B200_MAX_PSM);
+    stageWordsAsync(residentSmem + L.at.runs, L.runs + (size_t)me * numGroups, sizeof(ResidentRun) * numGroups);
+    stageWordsAsync(residentSmem + L.at.rows, L.rows, sizeof(unsigned long long) * numGroups);
+    stageWordsAsync(residentSmem + L.at.spans, L.spans, sizeof(ResidentSpan) * L.num_spans);
     StepState *const state = L.neuron.state;
     const unsigned long long t0 = state->timestep;
     if(L.may_leave) {
         if(me == 0 && threadIdx.x == 0) *L.barrier = 0ull;
-        if(state->steps_done < state->resident_hold) return;        // (the same for every CTA: both change at the end of a launch)
+        if(state->steps_done < state->resident_hold) {              // (the same for every CTA: both change at the end of a launch)
+            stagedWords();
+            return;
+        }
     }
     const unsigned int K = W.steps, delay = L.delay[0], columns = L.cta_columns[me * RESIDENT_CLASSES];
     if(threadIdx.x == 0) {
@@ -138,6 +141,7 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
     if(threadIdx.x < 32u) sh.count[0][threadIdx.x] = sh.count[1][threadIdx.x] = 0u;
     for(unsigned int i = threadIdx.x; i < K * columns; i += blockDim.x) acc[i] = 0.0f;
     if(threadIdx.x < numGroups) residentLifTable(sh.lif[threadIdx.x], L.neuron.groups[threadIdx.x]);
+    stagedWords();
     __syncthreads();
     if(threadIdx.x <= numGroups) {
         // first warp whose unit (warp * G + me) is not before the group
