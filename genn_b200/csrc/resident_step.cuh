@@ -845,13 +845,16 @@ ended: __attribute__((unused));
     const unsigned long long doneNow = sh.done + step;
     const unsigned int k = (sh.phase + step) % sh.period, period = sh.period;
     __syncthreads();
-    if(asked < G) awaitCell(buf == 0u ? L.buffers - 1u : buf - 1u, no0 + step, &sh.stop[turn]);
+    // (A launch of one step fills one list, which the step before it has emptied: only the counters wait for the other CTAs.  The
+    // hand-shake took 1 us of such a launch.)
+    const bool single = step == 1u;
+    if(asked < G && (!single || me == 0)) awaitCell(buf == 0u ? L.buffers - 1u : buf - 1u, no0 + step, &sh.stop[turn]);
     __syncthreads();
     if(sh.stop[turn] & 1u) return;
     // lists of the last steps: emptied by the first CTA (and the one the next step writes), filled by all
     const unsigned int lists = min(L.history, step);
     if(me == 0) {
-        for(unsigned int i = threadIdx.x; i < numGroups * (lists + 1u); i += blockDim.x) {
+        for(unsigned int i = threadIdx.x; i < numGroups * (single ? 1u : lists + 1u); i += blockDim.x) {
             const b200_neuron_group &g = groups[i % numGroups];
             const unsigned int t = i / numGroups;      // 0: the next step, t: t - 1 steps ago
             if(t < g.num_delay_slots) g.spk_cnt[ringSlot(k + 1u + g.num_delay_slots - t, g.num_delay_slots)] = 0u;
@@ -860,7 +863,7 @@ ended: __attribute__((unused));
         __syncthreads();
         if(threadIdx.x == 0) storeRelaxedGpu(L.leave, doneNow);
     }
-    else {
+    else if(!single) {
         if(threadIdx.x == 0) {
             unsigned int polls = 0;
             while(loadRelaxedGpu(L.leave) != doneNow && !gaveUp(polls, &sh.stop[turn])) {}
