@@ -41,21 +41,27 @@ __device__ __forceinline__ unsigned long long loadAcquireGpu(const unsigned long
     return v;
 }
 
-// Spikes of one step through a DENSE or BITMASK group onto 32 targets: a lane's sum.  (The whole warp calls.)
-__device__ __forceinline__ float windowSpan(const ResidentSpan &S, const unsigned int *list, unsigned int from, unsigned int to, unsigned int unit, unsigned int &events)
+// Spikes [from, to) of a step's list through a DENSE or BITMASK group onto 32 targets: a lane's sum.  (The whole warp calls; `from`
+// and the list are multiples of four entries.)  `mixed`: the list has spikes of other populations too.  A row's part is 128 bytes out
+// of L2 and an addition, so instructions count: with every choice made for every spike there were 49 for one, and DENSE 4096 x 4096 with
+// 100 spikes a step took 1.12 us a step; SPAN_FIGURES.
+__device__ __forceinline__ float windowSpan(const ResidentSpan &S, const unsigned int *list, unsigned int from, unsigned int to, unsigned int unit, bool mixed, unsigned int &events)
 {
     const unsigned int lane = threadIdx.x & 31u, post = unit * 32u + lane, src = S.src_group, numTrg = S.num_trg;
+    const float weight = S.weight;
+    const bool valid = post < numTrg;
     float sum = 0.0f;
-    if(S.gp) {
+    unsigned int n = 0;
+    if(const unsigned int *const gp = S.gp) {
         constexpr unsigned int SIDE = 4;            // words of a lane in flight
-        unsigned int n = 0;
+        const unsigned int rowWords = S.row_stride / 32u;
         for(; from < to; from += 32u * SIDE) {
             unsigned int word[SIDE];
             #pragma unroll
             for(unsigned int u = 0; u < SIDE; u++) {
                 const unsigned int at = from + u * 32u + lane, spike = (at < to) ? list[at] : 0xFFFFFFFFu;
                 word[u] = 0u;
-                if((spike >> 24) == src) word[u] = __ldg(&S.gp[(((unsigned long long)(spike & 0xFFFFFFu) * S.row_stride) >> 5) + unit]);
+                if((spike >> 24) == src) word[u] = __ldg(gp + (unsigned long long)(spike & 0xFFFFFFu) * rowWords + unit);
             }
             #pragma unroll
             for(unsigned int u = 0; u < SIDE; u++) {
@@ -71,28 +77,60 @@ __device__ __forceinline__ float windowSpan(const ResidentSpan &S, const unsigne
                 n += __popc(c);
             }
         }
-        if(post < numTrg) {
+        if(valid) {
             events += n;
-            sum = (float)n * S.weight;
+            sum = (float)n * weight;
+        }
+        return sum;
+    }
+    const float *const g = S.g;
+    if(g && !mixed) {
+        // (lanes beyond the targets read the last one's weights)
+        constexpr unsigned int LOADS = 16;
+        const char *const base = reinterpret_cast<const char*>(g + min(post, numTrg - 1u));
+        const unsigned int rowBytes = numTrg * (unsigned int)sizeof(float);
+        n = to - from;
+        for(; from + LOADS <= to; from += LOADS) {
+            float w[LOADS];
+            #pragma unroll
+            for(unsigned int u = 0; u < LOADS; u += 4u) {
+                const uint4 s4 = *reinterpret_cast<const uint4*>(list + from + u);
+                w[u] = __ldg(reinterpret_cast<const float*>(base + (unsigned long long)(s4.x & 0xFFFFFFu) * rowBytes));
+                w[u + 1u] = __ldg(reinterpret_cast<const float*>(base + (unsigned long long)(s4.y & 0xFFFFFFu) * rowBytes));
+                w[u + 2u] = __ldg(reinterpret_cast<const float*>(base + (unsigned long long)(s4.z & 0xFFFFFFu) * rowBytes));
+                w[u + 3u] = __ldg(reinterpret_cast<const float*>(base + (unsigned long long)(s4.w & 0xFFFFFFu) * rowBytes));
+            }
+            #pragma unroll
+            for(unsigned int u = 0; u < LOADS; u++) sum += w[u];
+        }
+        for(; from < to; from += 4u) {
+            float w[4];
+            #pragma unroll
+            for(unsigned int u = 0; u < 4u; u++) {
+                w[u] = 0.0f;
+                if(from + u < to) w[u] = __ldg(reinterpret_cast<const float*>(base + (unsigned long long)(list[from + u] & 0xFFFFFFu) * rowBytes));
+            }
+            sum += (w[0] + w[1]) + (w[2] + w[3]);
         }
     }
     else {
-        constexpr unsigned int LOADS = 2u * RESIDENT_DENSE_SPIKES;
-        const float *const g = S.g;
+        constexpr unsigned int LOADS = RESIDENT_DENSE_SPIKES;
         for(; from < to; from += LOADS) {
             float w[LOADS];
             #pragma unroll
             for(unsigned int u = 0; u < LOADS; u++) {
                 const unsigned int spike = (from + u < to) ? list[from + u] : 0xFFFFFFFFu;
-                const bool take = (spike >> 24) == src && post < numTrg;
-                w[u] = (take && !g) ? S.weight : 0.0f;
+                const bool take = (spike >> 24) == src && valid;
+                w[u] = (take && !g) ? weight : 0.0f;
                 if(take && g) w[u] = __ldg(&g[(unsigned long long)(spike & 0xFFFFFFu) * numTrg + post]);
-                events += take ? 1u : 0u;
+                n += take ? 1u : 0u;
             }
             #pragma unroll
             for(unsigned int u = 0; u < LOADS; u++) sum += w[u];
         }
     }
+    if(!valid) return 0.0f;
+    events += n;
     return sum;
 }
 
@@ -172,8 +210,10 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
             if((what & RESIDENT_IS_ARRAY) && regs.v[0] != regs.v[1]) nextTime = __ldg(&g.egp[regs.v[0]]);
         }
     }
-    // FEED: the warps without neurons read the messages, while the others update theirs
-    const unsigned int neuronWarps = (L.num_units + G - 1u) / G, firstReader = (W.feed && 2u * neuronWarps <= warps && (warps - neuronWarps) * 32u >= G) ? neuronWarps : 0u;
+    // FEED: the warps without neurons read the messages, while the others update theirs.  LATE: as few as it takes, for nobody has
+    // anything else to do, and the more ask for the heads, the longer each waits (24 warps of each CTA: LATE_FIGURES)
+    const unsigned int neuronWarps = (L.num_units + G - 1u) / G;
+    const unsigned int firstReader = !W.feed ? warps - (G + 31u) / 32u : (2u * neuronWarps <= warps && (warps - neuronWarps) * 32u >= G) ? neuronWarps : 0u;
     const unsigned int readers = warps - firstReader, perReader = (G + readers - 1u) / readers;
     const unsigned int recAt = L.neuron.num_recording_timesteps ? (unsigned int)(t0 % L.neuron.num_recording_timesteps) : 0u;
     unsigned int spikes = 0, events = 0;
@@ -496,18 +536,19 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
                 }
             }
         }
+        const bool mixed = (L.sources[0] & (L.sources[0] - 1ull)) != 0ull;
         for(unsigned int q = 0; q < L.num_spans && all; q++) {
             const ResidentSpan &S = residentTable<const ResidentSpan>(L.at.spans)[q];
             const unsigned int w0 = sh.firstWarp[S.trg_group], targets = sh.firstWarp[S.trg_group + 1] - w0;
             if(!targets) continue;
             // (few units and steps: several warps share a step's spikes)
-            const unsigned int parts = (2u * warps - 1u) / (targets * n) + 1u, least = S.gp ? 32u : 2u * RESIDENT_DENSE_SPIKES;
+            const unsigned int parts = (2u * warps - 1u) / (targets * n) + 1u, least = S.gp ? 32u : 16u;
             for(unsigned int it = warp; it < targets * n * parts; it += warps) {
                 const unsigned int j = it % n, rest = it / n, part = rest / targets, unitWarp = w0 + rest % targets;
                 const unsigned int m = __shfl_sync(0xFFFFFFFFu, mineCount, j), per = ((m + parts - 1u) / parts + least - 1u) / least * least;
                 if(part * per >= m) continue;
                 const unsigned int unit = unitWarp * G + me - residentTable<const unsigned int>(L.at.unit_start)[S.trg_group];
-                const float sum = windowSpan(S, list + j * W.cap, part * per, min(m, (part + 1u) * per), unit, events);
+                const float sum = windowSpan(S, list + j * W.cap, part * per, min(m, (part + 1u) * per), unit, mixed, events);
                 const unsigned int col = residentTable<const unsigned int>(L.at.columns)[unitWarp * B200_MAX_PSM + S.psm] & 0xFFFFu;
                 if(sum != 0.0f) residentAdd(acc + j * columns + col + lane, sum);
             }

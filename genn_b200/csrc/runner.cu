@@ -1617,8 +1617,9 @@ int buildResident(b200_runner *r)
             win.steps = after / win.lag;
             win.cap = (unsigned int)std::min<unsigned long long>(sourceNeurons, RESIDENT_LIST);
             win.buffers = 2u * win.lag + 2u;
-            windowed = win.cap >= sourceNeurons || r->residentHandsOver;
+            windowed = win.cap >= sourceNeurons || r->residentHandsOver;      // (before it is rounded up)
         }
+        win.cap = (win.cap + 3u) & ~3u;         // (entries are read four at a time)
         windowed = windowed && win.steps >= RESIDENT_WINDOW_LEAST;
     }
 
