@@ -59,7 +59,8 @@ denseBatchKernel(const DenseLaunch L)
     __shared__ unsigned int listed;
     __shared__ __align__(8) unsigned long long arrived[DENSE_STAGES], released[DENSE_STAGES];
     const uint4 part = __ldg(&L.parts[blockIdx.x]);
-    const b200_synapse_group &g = L.S.groups[part.x];
+    __shared__ __align__(16) b200_synapse_group g;
+    stageGroup(g, L.S.groups[part.x]);
     const unsigned int firstCopy = blockIdx.z * DENSE_COPIES, copies = min(DENSE_COPIES, L.S.batch - firstCopy);
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const unsigned int rowStride = g.num_trg, cols = min(DENSE_COLS, rowStride - part.y);

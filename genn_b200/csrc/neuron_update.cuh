@@ -27,6 +27,7 @@ namespace b200
 {
 constexpr int NEURON_BLOCK = 128;
 constexpr unsigned int NEURON_BLOCKS_PER_SM = 16;
+constexpr unsigned int NEURON_STAGED = 8;           // groups whose tables a block takes into shared memory (5 KB of 16 blocks an SM)
 // Warps of an SM before a warp takes four words of neurons.  us a step of a network of 80 000 / 150 000 / 200 000 / 300 000 / 1 200 000
 // neurons with one word a warp 4.4 / 4.7 / 6.7 / 7.4 / 15.1, with four 5.3 / 5.6 / 5.5 / 5.5 / 11.9; with a Poisson source each 5.3 / 5.6 /
 // 8.0 / 9.0 / 21.7 and 7.2 / 8.1 / 8.2 / 7.9 / 21.8: the line, 152 000 neurons, is where the second wave of blocks begins.
@@ -528,15 +529,26 @@ __global__ void __launch_bounds__(NEURON_BLOCK)
 neuronUpdateKernel(const NeuronLaunch L)
 {
     constexpr unsigned int PARTS = NEURON_BLOCK / (32 * WORDS);         // warps of a padded block
-    const unsigned int blocks = __ldg(&L.block_start[L.num_groups]), launched = gridDim.x * gridDim.y;
+    // (common.cuh: stageGroup)
+    __shared__ __align__(16) b200_neuron_group stagedGroups[NEURON_STAGED];
+    __shared__ unsigned int stagedStarts[NEURON_STAGED + 1];
+    const bool staged = L.num_groups <= NEURON_STAGED;
+    if(staged) {
+        stageWords(stagedGroups, L.groups, sizeof(b200_neuron_group) * L.num_groups);
+        stageWords(stagedStarts, L.block_start, sizeof(unsigned int) * (L.num_groups + 1u));
+        __syncthreads();
+    }
+    const b200_neuron_group *const groups = staged ? stagedGroups : L.groups;
+    const unsigned int *const blockStart = staged ? stagedStarts : L.block_start;
+    const unsigned int blocks = blockStart[L.num_groups], launched = gridDim.x * gridDim.y;
     const unsigned int rank = blockIdx.y * gridDim.x + blockIdx.x;
     chainWait();
     const unsigned int k = chainPhase(L.state, L.ahead);
     const unsigned long long timestep = L.state->timestep + L.ahead;
     for(unsigned int unit = rank * (NEURON_BLOCK / 32) + (threadIdx.x >> 5); unit < blocks * L.batch * PARTS; unit += launched * (NEURON_BLOCK / 32)) {
         const unsigned int item = unit / PARTS, b = item / blocks, block = item - b * blocks;
-        const unsigned int gi = findGroup(L.block_start, L.num_groups, block);
-        neuronWords<NPSM, NCS, WORDS>(L, L.groups[gi], b, (block - __ldg(&L.block_start[gi])) * NEURON_BLOCK + (unit % PARTS) * 32u * WORDS, k, timestep);
+        const unsigned int gi = findGroup(blockStart, L.num_groups, block);
+        neuronWords<NPSM, NCS, WORDS>(L, groups[gi], b, (block - blockStart[gi]) * NEURON_BLOCK + (unit % PARTS) * 32u * WORDS, k, timestep);
     }
 
     // ---- queue update for the next step: its slot was last read three steps ago at the latest -------
@@ -545,7 +557,7 @@ neuronUpdateKernel(const NeuronLaunch L)
         if(threadIdx.x == 0) stepSpikes = 0u;
         __syncthreads();
         for(unsigned int q = threadIdx.x; q < L.num_groups * L.batch; q += blockDim.x) {
-            const b200_neuron_group &o = L.groups[q / L.batch];
+            const b200_neuron_group &o = groups[q / L.batch];
             const unsigned int ob = q % L.batch;
             // (the spikes of the step before: this one's are not all there yet)
             if(q / L.batch >= 64u || ((L.peak_groups >> (q / L.batch)) & 1ull)) {

@@ -31,6 +31,7 @@ constexpr unsigned int SCATTER_ALIGN = 16;                              // synap
 constexpr unsigned int SCATTER_MOST_DEPTH = 4;                          // pieces in a warp's ring
 constexpr unsigned int SCATTER_SMEM = 225 * 1024;
 constexpr unsigned int SCATTER_MOST_SOURCES = 64;                       // groups onto one buffer
+constexpr unsigned int SCATTER_STAGED = 2;                              // of these in shared memory (with the rest of it, all an SM has)
 // An event costs 0.19 ns of an SM's shared memory and 0.78 ns of its share of the L2's reductions; clearing and flushing
 // the sums about 2.5 us.
 constexpr unsigned int SCATTER_FEW = 4096;
@@ -255,18 +256,28 @@ sparseBatchKernel(const ScatterLaunch L)
     extern __shared__ __align__(16) float scatterSums[];
     __shared__ __align__(8) unsigned long long scatterBars[SCATTER_WARPS][SCATTER_MOST_DEPTH];
     __shared__ unsigned int firstSpike[SCATTER_MOST_SOURCES], spikes[SCATTER_MOST_SOURCES];
-    __shared__ unsigned long long line[SCATTER_MOST_SOURCES];
+    unsigned long long *const line = reinterpret_cast<unsigned long long*>(scatterSums + ((L.cells + 31u) & ~31u));     // (until pieces come into the rings)
     const ScatterPart part = L.parts[blockIdx.x];
     const ScatterTarget T = L.targets[part.target];
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    // (common.cuh: stageGroup; the groups of a buffer, where they are few)
+    __shared__ __align__(16) b200_synapse_group stagedGroups[SCATTER_STAGED];
+    const bool staged = T.num_groups <= SCATTER_STAGED;
+    if(staged) stageWords(stagedGroups, L.S.groups + T.first_group, sizeof(b200_synapse_group) * T.num_groups);
+    const b200_synapse_group *const groups = staged ? stagedGroups : L.S.groups + T.first_group;
     if(lane < L.depth) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(scatterShare(&scatterBars[warp][lane])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // (the sums are cleared while the kernel before this one ends, whether they will be needed or not)
+    for(unsigned int i = threadIdx.x; i < (T.num_cells + 3u) / 4u; i += SCATTER_BLOCK) {
+        reinterpret_cast<float4*>(scatterSums)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    __syncthreads();
     chainWait();
     const unsigned int k = chainPhase(L.S.state, L.S.ahead), polls = L.S.state->copy_wait_limit;
     // ---- this CTA's stretch of the line of spikes
     if(threadIdx.x < T.num_groups) {
-        const b200_synapse_group &g = L.S.groups[T.first_group + threadIdx.x];
+        const b200_synapse_group &g = groups[threadIdx.x];
         const unsigned int slots = g.src_delay_slots, slot = ringSlot(k + slots - g.axonal_delay, slots);
         spikes[threadIdx.x] = min(g.src_spk_cnt[part.copy * slots + slot], g.num_src);
         line[threadIdx.x] = (unsigned long long)spikes[threadIdx.x] * g.row_stride;
@@ -283,7 +294,7 @@ sparseBatchKernel(const ScatterLaunch L)
     __syncthreads();
     if(threadIdx.x < T.num_groups) {
         // spike i of a group stands at `before` + i * row_stride
-        const unsigned int stride = max(1u, L.S.groups[T.first_group + threadIdx.x].row_stride);
+        const unsigned int stride = max(1u, groups[threadIdx.x].row_stride);
         auto from = [&](unsigned long long at) {
             return at <= before ? 0u : (unsigned int)min((unsigned long long)spikes[threadIdx.x], (at - before + stride - 1u) / stride);
         };
@@ -291,18 +302,13 @@ sparseBatchKernel(const ScatterLaunch L)
         firstSpike[threadIdx.x] = first;
         spikes[threadIdx.x] = from(high) - first;
     }
-    if(!few) {
-        for(unsigned int i = threadIdx.x; i < (T.num_cells + 3u) / 4u; i += SCATTER_BLOCK) {
-            reinterpret_cast<float4*>(scatterSums)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-    }
     __syncthreads();
     float *const cells = T.cells + (unsigned long long)part.copy * T.num_cells;
     ScatterRing ring{reinterpret_cast<unsigned char*>(scatterSums + ((L.cells + 31u) & ~31u)) + (size_t)warp * L.depth * L.piece_bytes,
                      scatterBars[warp], L.depth, L.piece_bytes, 0u, 0u, 0u, polls, false};
     unsigned int item = warp;
     for(unsigned int gi = 0; gi < T.num_groups && !ring.failed; gi++) {
-        const b200_synapse_group &g = L.S.groups[T.first_group + gi];
+        const b200_synapse_group &g = groups[gi];
         const unsigned int slots = g.src_delay_slots, slot = ringSlot(k + slots - g.axonal_delay, slots);
         const unsigned int *const spk = g.src_spk + ((unsigned long long)part.copy * slots + slot) * g.num_src + firstSpike[gi];
         const unsigned int front = g.max_den_delay ? ringSlot(k + 1u, g.max_den_delay) : 0u;
