@@ -156,6 +156,64 @@ inline uint64_t countBits(const uint32_t *words, uint64_t n)
     return bits;
 }
 
+// Pairs [from, to) of a list, all from one turn of the ring.  The list is in index order, so the row and the batch entry of a pair are
+// those of the one before or come soon after (divisions took half of the time).
+struct RecordPairs
+{
+    const uint32_t *pairs;
+    uint32_t base, rows, batch, words_per_row, first_row, first_id, lastMask;
+    double start, dt;
+    uint64_t *counts;
+    double *const *times;
+    uint32_t *const *ids;
+};
+
+__attribute__((always_inline)) inline void decodePairsAs(const RecordPairs &R, uint64_t from, uint64_t to)
+{
+    if(from >= to) return;
+    const uint32_t words = R.words_per_row, first = R.pairs[2 * from] - R.base;
+    // section: one batch entry of one row
+    uint64_t section = first / words, sectionEnd = (section + 1u) * words;
+    uint32_t row = (uint32_t)(section / R.batch), b = (uint32_t)(section - (uint64_t)row * R.batch);
+    auto timeOf = [&] { return R.start + (double)(row >= R.first_row ? row - R.first_row : row + R.rows - R.first_row) * R.dt; };
+    double t = timeOf();
+    uint64_t at = R.counts[b];
+    double *times = R.ids ? R.times[b] : nullptr;
+    uint32_t *ids = R.ids ? R.ids[b] : nullptr;
+    for(uint64_t i = from; i < to; i++) {
+        const uint32_t index = R.pairs[2 * i] - R.base;
+        uint32_t word = R.pairs[2 * i + 1];
+        if(index >= sectionEnd) {
+            R.counts[b] = at;
+            do {
+                sectionEnd += words;
+                if(++b == R.batch) {
+                    b = 0;
+                    row++;
+                }
+            } while(index >= sectionEnd);
+            t = timeOf();
+            at = R.counts[b];
+            if(ids) {
+                times = R.times[b];
+                ids = R.ids[b];
+            }
+        }
+        if(index + 1u == sectionEnd) word &= R.lastMask;
+        if(!ids) {
+            at += (uint64_t)__builtin_popcount(word);
+            continue;
+        }
+        const uint32_t id = R.first_id + (uint32_t)(index - (sectionEnd - words)) * 32u;
+        for(; word; word &= word - 1u, at++) {
+            times[at] = t;
+            ids[at] = id + (uint32_t)__builtin_ctz(word);
+        }
+    }
+    R.counts[b] = at;
+}
+__attribute__((target("popcnt,bmi"))) inline void decodePairsNative(const RecordPairs &R, uint64_t from, uint64_t to) { decodePairsAs(R, from, to); }
+
 // Host side.  The spikes in a recording of one population: bits of `words` ([rows][batch][words_per_row], the whole
 // array) or, if `words` is NULL, of the (index, word) pairs of a list in index order in which the array begins at
 // index `base`.  Row `first_row` is the oldest (the recording is a ring over the steps).  Without `ids`, counts them per
@@ -216,13 +274,12 @@ inline void decodeRecording(const uint32_t *words, const uint32_t *pairs, uint64
     };
     const uint64_t begin = find(base), split = find((uint64_t)base + (uint64_t)first_row * perRow);
     const uint64_t end = find((uint64_t)base + (uint64_t)rows * perRow);
+    const RecordPairs R{pairs, base, rows, batch, words_per_row, first_row, first_id, lastMask, start, dt, counts, times, ids};
+    static const bool native = __builtin_cpu_supports("popcnt") && __builtin_cpu_supports("bmi");
     const uint64_t part[2][2] = {{split, end}, {begin, split}};
     for(const auto &p : part) {
-        for(uint64_t i = p[0]; i < p[1]; i++) {
-            const uint32_t index = pairs[2 * i] - base;
-            const uint32_t row = index / perRow, in = index - row * perRow, b = in / words_per_row;
-            take(row, b, in - b * words_per_row, pairs[2 * i + 1]);
-        }
+        if(native) decodePairsNative(R, p[0], p[1]);
+        else decodePairsAs(R, p[0], p[1]);
     }
 }
 }   // namespace b200

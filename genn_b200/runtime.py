@@ -544,8 +544,9 @@ class Runtime:
         sizes = [int(np.prod(a.shape, dtype=np.int64)) for _, a in recs]
         total = sum(sizes)
         if recs and total < (1 << 32):
-            # room for one non-zero word in sixteen unless the caller chose
-            cap = int(self.recording_pairs_capacity or max(1024, total // 16))
+            # room for one non-zero word in eight unless the caller chose (313 000 words of which 7 % are not zero: pulled and
+            # decoded in 150 us; as a whole array, 560)
+            cap = int(self.recording_pairs_capacity or max(1024, total // 8))
             pairs, count = C.c_void_p(), C.c_uint64()
             check(self.lib.b200_pull_recording(self.handle, len(recs), (C.c_void_p * len(recs))(*[a.ptr for _, a in recs]),
                                                (C.c_uint64 * len(recs))(*sizes), cap, C.byref(pairs), C.byref(count)))

@@ -18,7 +18,7 @@ def _numpy_decode(words, num_neurons, first_row, first_id, start, dt):
 
 
 @pytest.mark.parametrize("rows,batch,num_neurons,first_row,density", [(1, 1, 1, 0, 1.0), (7, 1, 32, 3, 0.3), (5, 3, 33, 4, 0.2), (20, 2, 95, 0, 0.02),
-                                                                      (4, 1, 64, 2, 0.0)])
+                                                                      (4, 1, 64, 2, 0.0), (50, 3, 70, 20, 0.03)])
 @pytest.mark.parametrize("whole", [False, True])
 def test_decoded_spikes_equal_the_unpacked_bits(rows, batch, num_neurons, first_row, density, whole):
     lib = abi.load_library()
