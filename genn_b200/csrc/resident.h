@@ -172,6 +172,7 @@ struct ResidentBuild
 // Where no spike of a window of steps reaches anybody in that window, CTAs exchange once a window.
 constexpr unsigned int RESIDENT_WINDOW_MOST = 16;       // most steps of a window
 constexpr unsigned int RESIDENT_WINDOW_LEAST = 4;       // fewest
+constexpr unsigned int RESIDENT_WINDOW_INLINE = 3;      // entries that travel with the head
 constexpr unsigned int RESIDENT_HEADS = RESIDENT_MAX_CTAS + RESIDENT_UNITS;     // (those of a reading warp lie side by side, the last of each short)
 constexpr unsigned int RESIDENT_WINDOW_LIST = 40960;    // spikes of a window that the list has room for (160 KB)
 
@@ -190,7 +191,7 @@ struct ResidentWindow
     unsigned int list_at, words_at, acc_at;     // in dynamic shared memory, behind the tables of ResidentLayout
     unsigned int epoch;                 // of the launch
     unsigned long long free_groups;     // populations without inputs (FEED)
-    unsigned long long *heads;          // [buffers][copies][RESIDENT_HEADS] tag << 20 | spikes
+    ulonglong2 *heads;                  // [buffers][copies][RESIDENT_HEADS] tag << 20 | spikes, tag << 48 | the first three entries
     unsigned short *bodies;             // [buffers][grid][body] step of the window << 10 | unit of the CTA << 5 | neuron
 };
 

@@ -13,8 +13,9 @@
 // takes its 32 neurons through all steps on its own.  Two or three barriers of a CTA a window instead of a step, loads of a
 // window's runs side by side instead of a step's, and the wait for the messages once (FEED: hidden behind a window).
 //
-// us a step, step by step / in windows: 1000 sources -> 10 000 neurons, p = 0.1, 2 spikes a step 2.15 / 0.32; BITMASK 2003 -> 5009, 80
-// spikes 4.0 / 0.82; DENSE 4096 x 4096, 100 spikes 4.3 / 1.41; 100 000 neurons with conductances, 8 spikes, delay 10 2.7 / 1.44.
+// us a step, step by step / in windows: 1000 sources -> 10 000 neurons, p = 0.1, 2 spikes a step 2.15 / 0.28; BITMASK 2003 -> 5009, 80
+// spikes 4.0 / 0.82; DENSE 4096 x 4096, 100 spikes 4.3 / 1.16; 100 000 neurons with conductances, 8 spikes, delay 10 2.7 / 1.13.
+// Cycles of a window of the last two: deliveries 7400 and 3500, updates 1000 and 5000, messages 4800 - 8500 and 9800.
 #pragma once
 
 #include "resident_step.cuh"
@@ -25,6 +26,7 @@ struct WindowShared
 {
     unsigned int count[2][32];          // spikes of each step of the window (counts on beyond the list's end): of even and odd windows
     unsigned int sent[2];               // entries of the message that is being made, of even and odd ones
+    unsigned short first[2][4];         // and the first of them
     unsigned int stop;                  // 1: a wait ran out, 4: more spikes than the list holds
     unsigned int steps;                 // of this launch
     int debt;
@@ -34,17 +36,12 @@ struct WindowShared
     __align__(16) ResidentLif lif[RESIDENT_MAX_GROUPS];
 };
 
-__device__ __forceinline__ unsigned long long loadAcquireGpu(const unsigned long long *p)
-{
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
+__device__ __forceinline__ void fenceGpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 // Spikes [from, to) of a step's list through a DENSE or BITMASK group onto 32 targets: a lane's sum.  (The whole warp calls; `from`
 // and the list are multiples of four entries.)  `mixed`: the list has spikes of other populations too.  A row's part is 128 bytes out
 // of L2 and an addition, so instructions count: with every choice made for every spike there were 49 for one, and DENSE 4096 x 4096 with
-// 100 spikes a step took 1.12 us a step; SPAN_FIGURES.
+// 100 spikes a step took 1.41 us a step in all; now 1.14.
 __device__ __forceinline__ float windowSpan(const ResidentSpan &S, const unsigned int *list, unsigned int from, unsigned int to, unsigned int unit, bool mixed, unsigned int &events)
 {
     const unsigned int lane = threadIdx.x & 31u, post = unit * 32u + lane, src = S.src_group, numTrg = S.num_trg;
@@ -169,6 +166,7 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
     if(threadIdx.x == 0) {
         sh.debt = (int)state->resident_debt;
         sh.sent[0] = sh.sent[1] = 0u;
+        for(int i = 0; i < 8; i++) sh.first[i / 4][i % 4] = 0u;
         sh.stop = 0u;
         sh.steps = L.num_steps;
         sh.done = state->steps_done;
@@ -211,7 +209,7 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         }
     }
     // FEED: the warps without neurons read the messages, while the others update theirs.  LATE: as few as it takes, for nobody has
-    // anything else to do, and the more ask for the heads, the longer each waits (24 warps of each CTA: LATE_FIGURES)
+    // anything else to do, and the more ask for the heads, the longer each waits (100 000 neurons on 148 CTAs, five warps instead of 24: 1.44 -> 1.38 us a step)
     const unsigned int neuronWarps = (L.num_units + G - 1u) / G;
     const unsigned int firstReader = !W.feed ? warps - (G + 31u) / 32u : (2u * neuronWarps <= warps && (warps - neuronWarps) * 32u >= G) ? neuronWarps : 0u;
     const unsigned int readers = warps - firstReader, perReader = (G + readers - 1u) / readers;
@@ -352,29 +350,35 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         unsigned int base = 0;
         if(lane == 31u) base = atomicAdd(&sh.sent[message & 1u], upTo);
         base = __shfl_sync(0xFFFFFFFFu, base, 31);
-        unsigned short *to = W.bodies + ((size_t)(message % W.buffers) * G + me) * W.body + base + (upTo - mineCount);
+        unsigned short *const body = W.bodies + ((size_t)(message % W.buffers) * G + me) * W.body;
+        unsigned int at = base + (upTo - mineCount);
         if(lane < n) {
             const unsigned int row = runTable[group].row;
-            for(unsigned int left = word; left; left &= left - 1u) {
+            for(unsigned int left = word; left; left &= left - 1u, at++) {
                 const unsigned int who = __ffs(left) - 1u;
-                *to++ = (unsigned short)(((entry + lane) << 10) | (warp << 5) | who);
+                const unsigned short e = (unsigned short)(((entry + lane) << 10) | (warp << 5) | who);
+                if(at < RESIDENT_WINDOW_INLINE) sh.first[message & 1u][at] = e;
+                body[at] = e;
                 // its runs, while the message is on its way (lengths are multiples of four entries)
                 if(L.prefetch) prefetchL2(L.entries + residentTable<const unsigned long long>(L.at.rows)[group] + (size_t)(local - lane + who) * row, row * (unsigned int)sizeof(uint2));
             }
         }
     };
-    // the CTA's message, behind a barrier behind its entries
+    // the CTA's message, by its last warp, behind a barrier behind the entries: a copy for every RESIDENT_READERS readers (resident.h).
+    // Few entries travel with the head, which says of itself when it is there; more lie in the body, behind a fence (all in the body:
+    // 1000 -> 10 000 neurons 0.32 instead of 0.28 us a step, 100 000 neurons 1.38 instead of 1.13).
     auto send = [&](unsigned int message) {
-        if(threadIdx.x == blockDim.x - 32u) {
-            const unsigned int n = sh.sent[message & 1u];
-            sh.sent[message & 1u] = 0u;
-            __threadfence();
-            // (a copy for every RESIDENT_READERS readers: resident.h)
-            const unsigned int at = (me % readers) * perReader + me / readers;
-            for(unsigned int c = 0; c < L.copies; c++) {
-                storeRelaxedGpu(W.heads + ((size_t)(message % W.buffers) * L.copies + c) * RESIDENT_HEADS + at, (tagOf(message) << 20) | n);
-            }
+        if(warp != warps - 1u) return;
+        const unsigned int n = sh.sent[message & 1u], at = (me % readers) * perReader + me / readers;
+        const unsigned short *const e = sh.first[message & 1u];
+        const unsigned long long tag = tagOf(message);
+        if(n > RESIDENT_WINDOW_INLINE) fenceGpu();
+        if(lane < L.copies) {
+            storeRelaxedGpu(W.heads + ((size_t)(message % W.buffers) * L.copies + lane) * RESIDENT_HEADS + at, (tag << 20) | n,
+                            (tag << 48) | ((unsigned long long)e[2] << 32) | ((unsigned long long)e[1] << 16) | e[0]);
         }
+        __syncwarp();
+        if(lane == 0u) sh.sent[message & 1u] = 0u;
     };
     auto append = [&](unsigned int w, unsigned int j, unsigned int spike) {
         const unsigned int at = atomicAdd(&sh.count[w & 1u][j], 1u);
@@ -388,23 +392,32 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         if(warp < firstReader) return;
         const unsigned int reader = warp - firstReader, sender = lane * readers + reader;
         unsigned int total = 0;
+        unsigned long long first = 0;
         if(lane < perReader && sender < G) {
-            const unsigned long long *p = W.heads + ((size_t)(message % W.buffers) * L.copies + me % L.copies) * RESIDENT_HEADS + reader * perReader + lane;
+            const ulonglong2 *p = W.heads + ((size_t)(message % W.buffers) * L.copies + me % L.copies) * RESIDENT_HEADS + reader * perReader + lane;
             const unsigned long long tag = tagOf(message);
             unsigned int polls = 0;
             for(;;) {
-                const unsigned long long v = loadAcquireGpu(p);
-                if((v >> 20) == tag) {
-                    total = min((unsigned int)(v & 0xFFFFFull), W.body);
+                const ulonglong2 v = loadRelaxedGpu(p);
+                if((v.x >> 20) == tag && (v.y >> 48) == (tag & 0xFFFFull)) {
+                    total = min((unsigned int)(v.x & 0xFFFFFull), W.body);
+                    first = v.y;
                     break;
                 }
                 if(gaveUp(polls)) break;
             }
         }
-        __syncwarp();
+        if(__any_sync(0xFFFFFFFFu, total > RESIDENT_WINDOW_INLINE)) fenceGpu();
         if(steps == 0u) return;
+        auto spikeOf = [&](unsigned int e, unsigned int from) { return unitFirst[min(((e >> 5) & 31u) * G + from, L.num_units - 1u)] + (e & 31u); };
+        // entries that came with the heads: a lane its sender's
+        #pragma unroll
+        for(unsigned int u = 0; u < RESIDENT_WINDOW_INLINE; u++) {
+            const unsigned int e = (unsigned int)(first >> (16u * u)) & 0xFFFFu;
+            if(u < total && total <= RESIDENT_WINDOW_INLINE && (e >> 10) < steps) append(to, e >> 10, spikeOf(e, sender));
+        }
         const unsigned short *const bodies = W.bodies + (size_t)(message % W.buffers) * G * W.body;
-        for(unsigned int left = __ballot_sync(0xFFFFFFFFu, total > 0u); left;) {
+        for(unsigned int left = __ballot_sync(0xFFFFFFFFu, total > RESIDENT_WINDOW_INLINE); left;) {
             // (loads, places and stores of several senders side by side: one after another each takes its latency)
             constexpr unsigned int SIDE = 4;
             unsigned int from[SIDE], n[SIDE], e[SIDE], at[SIDE];
@@ -421,15 +434,14 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
             #pragma unroll
             for(unsigned int u = 0; u < SIDE; u++) {
                 if((e[u] >> 10) >= steps) continue;
-                const unsigned int spike = unitFirst[min(((e[u] >> 5) & 31u) * G + from[u], L.num_units - 1u)] + (e[u] & 31u);
-                if(at[u] < W.cap) list[(e[u] >> 10) * W.cap + at[u]] = spike;
+                if(at[u] < W.cap) list[(e[u] >> 10) * W.cap + at[u]] = spikeOf(e[u], from[u]);
                 else atomicOr(&sh.stop, 4u);
             }
             #pragma unroll
             for(unsigned int u = 0; u < SIDE; u++) {
                 for(unsigned int i = lane + 32u; i < n[u]; i += 32u) {
                     const unsigned int entry = __ldcg(bodies + (size_t)from[u] * W.body + i);
-                    if((entry >> 10) < steps) append(to, entry >> 10, unitFirst[min(((entry >> 5) & 31u) * G + from[u], L.num_units - 1u)] + (entry & 31u));
+                    if((entry >> 10) < steps) append(to, entry >> 10, spikeOf(entry, from[u]));
                 }
             }
             __syncwarp();

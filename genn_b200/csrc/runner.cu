@@ -1930,9 +1930,9 @@ int buildResident(b200_runner *r)
     L.hold = const_cast<unsigned long long*>(r->residentHold);
     if(windowed) {
         win.body = neuronWarps * 32u * win.steps;
-        if(const int err = device(sizeof(unsigned long long) * win.buffers * L.copies * RESIDENT_HEADS, (void**)&win.heads)) return err;
+        if(const int err = device(sizeof(ulonglong2) * win.buffers * L.copies * RESIDENT_HEADS, (void**)&win.heads)) return err;
         if(const int err = device(sizeof(unsigned short) * win.buffers * grid * win.body, (void**)&win.bodies)) return err;
-        CUDA_TRY(cudaMemsetAsync(win.heads, 0, sizeof(unsigned long long) * win.buffers * L.copies * RESIDENT_HEADS, r->stream));
+        CUDA_TRY(cudaMemsetAsync(win.heads, 0, sizeof(ulonglong2) * win.buffers * L.copies * RESIDENT_HEADS, r->stream));
         r->windowKernel = residentWindowKernelFor(shape.npsm, shape.ncs);
         CUDA_TRY(cudaFuncSetAttribute(r->windowKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)windowRoom));
         r->windowMayOverflow = win.cap < sourceNeurons;
@@ -1971,7 +1971,7 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
         // (a head is known by its launch's number: before it repeats, no old head may be left)
         r->window.epoch = (r->window.epoch + 1u) & 0xFFFFFu;
         if(r->window.epoch == 0u) {
-            CUDA_TRY(cudaMemsetAsync(r->window.heads, 0, sizeof(unsigned long long) * r->window.buffers * L.copies * RESIDENT_HEADS, r->stream));
+            CUDA_TRY(cudaMemsetAsync(r->window.heads, 0, sizeof(ulonglong2) * r->window.buffers * L.copies * RESIDENT_HEADS, r->stream));
             r->window.epoch = 1u;
         }
         ResidentWindowLaunch A{L, r->window};
