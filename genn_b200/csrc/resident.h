@@ -17,7 +17,8 @@
 //     first seven ids); further ids wait at the sender.  Every word carries its step number, so readers poll the
 //     cells themselves: the all-gather IS the barrier, with no fence, no counter and no list.  A message is stored
 //     once for every RESIDENT_READERS CTAs: with one copy for all, polling it grew from 1.8 k cycles at 32 CTAs to
-//     8 k at 148, and with a copy for each the sender's stores took 10 cycles apiece, 1.6 k at 148.  A cell is
+//     8 k at 148, and with a copy for each the sender's stores took 10 cycles apiece, 1.6 k at 148.  (A step of 77 169 neurons
+//     on 148 CTAs with 20 / 12 / 8 / 5 readers a copy: 4.17 / 4.15 / 4.07 / 4.04 us.)  A cell is
 //     written again `buffers` steps later; its sender has by then received messages that every reader sent after it had
 //     read this one.
 //
@@ -63,7 +64,7 @@ constexpr unsigned int RESIDENT_MAX_CTAS = 256;
 constexpr unsigned int RESIDENT_MAX_GROUPS = 64;        // neuron groups (a bit mask says which are sources)
 constexpr unsigned int RESIDENT_CLASSES = 4;            // distinct ring depths / distinct axonal delays
 constexpr unsigned int RESIDENT_LIST = 2048;            // spikes delivered between two barriers of a CTA
-constexpr unsigned int RESIDENT_READERS = 12;           // CTAs that poll one copy of the messages
+constexpr unsigned int RESIDENT_READERS = 5;            // CTAs that poll one copy of the messages (a lane stores each: at most 32 copies)
 constexpr unsigned int RESIDENT_LOADS = 4;              // loads of a run that a lane has in flight
 constexpr unsigned int RESIDENT_CHUNK = 32 * RESIDENT_LOADS;    // entries of a run that one warp takes
 constexpr unsigned int RESIDENT_NEAR_LOADS = 4;         // entries of the runs' heads that a lane has in flight

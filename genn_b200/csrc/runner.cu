@@ -1901,7 +1901,7 @@ int buildResident(b200_runner *r)
     L.history = history;
     const unsigned int mostIds = neuronWarps * 32u;
     L.more_words = (mostIds - RESIDENT_CELL_IDS + RESIDENT_MORE_IDS - 1u) / RESIDENT_MORE_IDS;
-    L.copies = (grid + RESIDENT_READERS - 1u) / RESIDENT_READERS;
+    L.copies = std::min(32u, (grid + RESIDENT_READERS - 1u) / RESIDENT_READERS);
     const size_t headWords = (size_t)L.buffers * L.copies * grid * 2u, moreWords = (size_t)L.buffers * grid * L.more_words;
     void *mail = nullptr;
     r->residentMailBytes = sizeof(unsigned long long) * (headWords + moreWords + 1u);
