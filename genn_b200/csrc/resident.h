@@ -178,6 +178,10 @@ constexpr unsigned int RESIDENT_HEADS = RESIDENT_MAX_CTAS + RESIDENT_UNITS;     
 constexpr unsigned int RESIDENT_WINDOW_LIST = 40960;    // spikes of a window that the list has room for (160 KB)
 
 constexpr unsigned int RESIDENT_WINDOW_SPARE = 5500;    // ns that a step without spikes costs less than on the kernel with a grid barrier
+// ns of a warp for 32 entries of a run.  us a step at 10 / 100 / 300 / 1000 / 3000 spikes, in windows and with a grid barrier: 10 000 -> 10 000
+// neurons, 1000 synapses 1.0 / 3.1 / 7.0 / 20 / 56 and 6.8 / 7.9 / 11.4 / 24 / 61, 8000 -> 80 000, 500 synapses 1.0 / 2.8 / 5.8 / 17 / 47
+// and 6.6 / 7.0 / 7.2 / 10.3 / 19.
+constexpr float RESIDENT_WINDOW_COST = 430.0f;
 
 struct ResidentWindow
 {

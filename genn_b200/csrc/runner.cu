@@ -346,7 +346,7 @@ struct b200_runner
     ResidentWindow window{};
     const void *windowKernel = nullptr;
     size_t windowSmem = 0;
-    unsigned int windowBlock = 0;
+    unsigned int windowBlock = 0, windowWeight = 0;
     bool windowMayOverflow = false;                         // a step may have more spikes than its list holds: a launch has to follow
     std::vector<void*> residentBuffers;
     // busy networks (resident.h): the kernel with a grid barrier takes over
@@ -1851,6 +1851,10 @@ int buildResident(b200_runner *r)
             // spike, and the tiled kernels, whose launches and flush take some 35 us)
             const double there = !r->residentHandsOver ? 0.0 : (L.kind[a] == RESIDENT_SPLIT ? 0.02 : 0.0085) * all / std::max(1.0, sources);
             L.weight[a] = (unsigned int)std::min(std::max(0.0, here - there) + 0.5, (double)RESIDENT_MOST_WEIGHT);
+            if(windowed) {
+                const double inWindows = RESIDENT_WINDOW_COST * win.run_groups * 32.0 / r->windowBlock;
+                r->windowWeight = (unsigned int)std::min(std::max(0.0, inWindows - there) + 0.5, (double)RESIDENT_MOST_WEIGHT);
+            }
             r->residentSources += sources;
             r->residentSteeper = r->residentSteeper || (L.kind[a] == RESIDENT_SPLIT && L.weight[a]);
             r->residentWorst += sources * L.weight[a] + std::max(0.0, sources / RESIDENT_LIST - 1.0) * RESIDENT_PIECE_COST;
@@ -1975,7 +1979,10 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
             r->window.epoch = 1u;
         }
         ResidentWindowLaunch A{L, r->window};
-        if(r->residentHandsOver) A.L.spare = RESIDENT_WINDOW_SPARE;
+        if(r->residentHandsOver) {
+            A.L.spare = RESIDENT_WINDOW_SPARE;
+            A.L.weight[0] = r->windowWeight;
+        }
         void *args[] = {&A};
         CUDA_TRY(cudaLaunchCooperativeKernel(r->windowKernel, dim3(r->residentGrid), dim3(r->windowBlock), args, r->windowSmem, r->stream));
         r->launches++;
