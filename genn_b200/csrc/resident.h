@@ -47,6 +47,9 @@
 // the other kernel at once (models with one delay, up to 20 units a CTA): the messages' further ids are fetched by one lane per
 // sender, 0.3 ms for every 2048 of them.
 //
+// Networks whose spikes need several steps, or come from populations without inputs, go through windows of steps instead
+// (resident_window.cuh); there a spike costs the less and the account is kept window by window.
+//
 // Memory between launches is what every other path leaves: the first steps of a launch take the spikes of the steps
 // before it from the spike lists, the last ones write them.
 #pragma once
@@ -162,7 +165,7 @@ struct ResidentBuild
     const unsigned int *unit_start, *columns;
     const unsigned int *depth;          // buffers per input, by ring class
     unsigned int late;                  // 1: LATE class: every synapse arrives one step after its delivery
-    unsigned int split;                 // 1: SPLIT class: delay-0 synapses go into the rows
+    unsigned int split;                 // 1: SPLIT class: delay-0 synapses stand at the head of a run
     unsigned int *near_longest;         // longest head of a run
     unsigned long long *synapses;       // all of the pair
     unsigned int grid;
@@ -196,7 +199,7 @@ struct ResidentWindow
     unsigned int list_at, words_at, acc_at;     // in dynamic shared memory, behind the tables of ResidentLayout
     unsigned int epoch;                 // of the launch
     unsigned long long free_groups;     // populations without inputs (FEED)
-    ulonglong2 *heads;                  // [buffers][copies][RESIDENT_HEADS] tag << 20 | spikes, tag << 48 | the first three entries
+    ulonglong2 *heads;                  // [buffers][copies][RESIDENT_HEADS] tag << 20 | spikes, short tag << 48 | the first three entries
     unsigned short *bodies;             // [buffers][grid][body] step of the window << 10 | unit of the CTA << 5 | neuron
 };
 

@@ -209,7 +209,8 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         }
     }
     // FEED: the warps without neurons read the messages, while the others update theirs.  LATE: as few as it takes, for nobody has
-    // anything else to do, and the more ask for the heads, the longer each waits (100 000 neurons on 148 CTAs, five warps instead of 24: 1.44 -> 1.38 us a step)
+    // anything else to do, and the more ask for the heads, the longer each waits (100 000 neurons on 148 CTAs, five warps instead of
+    // 24: 1.44 -> 1.38 us a step)
     const unsigned int neuronWarps = (L.num_units + G - 1u) / G;
     const unsigned int firstReader = !W.feed ? warps - (G + 31u) / 32u : (2u * neuronWarps <= warps && (warps - neuronWarps) * 32u >= G) ? neuronWarps : 0u;
     const unsigned int readers = warps - firstReader, perReader = (G + readers - 1u) / readers;
@@ -222,6 +223,8 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         return true;
     };
     auto tagOf = [&](unsigned int message) { return ((unsigned long long)W.epoch << 24) | (message & 0xFFFFFFu); };
+    // (the second word's: the word that lay there before it was of another message of this launch, or of another launch)
+    auto shortTagOf = [&](unsigned int message) { return ((W.epoch & 0xFFu) << 8) | (message & 0xFFu); };
 
     // ---- the neurons of this warp through steps [first, first + n) of the launch; lane j gets the ballot of the j-th.
     // Populations without inputs: nothing to add up, and a Poisson neuron goes from spike to spike.
@@ -375,7 +378,7 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         if(n > RESIDENT_WINDOW_INLINE) fenceGpu();
         if(lane < L.copies) {
             storeRelaxedGpu(W.heads + ((size_t)(message % W.buffers) * L.copies + lane) * RESIDENT_HEADS + at, (tag << 20) | n,
-                            (tag << 48) | ((unsigned long long)e[2] << 32) | ((unsigned long long)e[1] << 16) | e[0]);
+                            ((unsigned long long)shortTagOf(message) << 48) | ((unsigned long long)e[2] << 32) | ((unsigned long long)e[1] << 16) | e[0]);
         }
         __syncwarp();
         if(lane == 0u) sh.sent[message & 1u] = 0u;
@@ -399,7 +402,7 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
             unsigned int polls = 0;
             for(;;) {
                 const ulonglong2 v = loadRelaxedGpu(p);
-                if((v.x >> 20) == tag && (v.y >> 48) == (tag & 0xFFFFull)) {
+                if((v.x >> 20) == tag && (v.y >> 48) == shortTagOf(message)) {
                     total = min((unsigned int)(v.x & 0xFFFFFull), W.body);
                     first = v.y;
                     break;
