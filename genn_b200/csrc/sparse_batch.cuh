@@ -302,6 +302,8 @@ sparseBatchKernel(const ScatterLaunch L)
         firstSpike[threadIdx.x] = first;
         spikes[threadIdx.x] = from(high) - first;
     }
+    // (`line` lies where bulk copies are about to write)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     float *const cells = T.cells + (unsigned long long)part.copy * T.num_cells;
     ScatterRing ring{reinterpret_cast<unsigned char*>(scatterSums + ((L.cells + 31u) & ~31u)) + (size_t)warp * L.depth * L.piece_bytes,
