@@ -144,7 +144,8 @@ struct ResidentLaunch
     unsigned int copies;
     unsigned int prefetch;              // 1: the runs do not stay in L2: a spiking neuron's are fetched ahead of its message
     unsigned long long *more;           // [buffers][sender][more_words]
-    unsigned long long *leave;          // steps done when the spike lists may be written at the end of a launch
+    unsigned long long *leave;          // number of the launch at whose end the spike lists may be written
+    unsigned long long launch;          // number of this launch: no other of the runner has it, and none is 0
     unsigned int num_steps;
     unsigned int count_events;
     unsigned int weight[RESIDENT_CLASSES];  // ns that a spike of that delay costs above what it costs the other kernel

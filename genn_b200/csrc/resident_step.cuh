@@ -861,12 +861,12 @@ ended: __attribute__((unused));
         }
         __threadfence();
         __syncthreads();
-        if(threadIdx.x == 0) storeRelaxedGpu(L.leave, doneNow);
+        if(threadIdx.x == 0) storeRelaxedGpu(L.leave, L.launch);
     }
     else if(!single) {
         if(threadIdx.x == 0) {
             unsigned int polls = 0;
-            while(loadRelaxedGpu(L.leave) != doneNow && !gaveUp(polls, &sh.stop[turn])) {}
+            while(loadRelaxedGpu(L.leave) != L.launch && !gaveUp(polls, &sh.stop[turn])) {}
             __threadfence();
         }
         __syncthreads();

@@ -618,12 +618,12 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         }
         __threadfence();
         __syncthreads();
-        if(threadIdx.x == 0) storeRelaxedGpu(L.leave, doneNow);
+        if(threadIdx.x == 0) storeRelaxedGpu(L.leave, L.launch);
     }
     else {
         if(threadIdx.x == 0) {
             unsigned int polls = 0;
-            while(loadRelaxedGpu(L.leave) != doneNow && !gaveUp(polls)) {}
+            while(loadRelaxedGpu(L.leave) != L.launch && !gaveUp(polls)) {}
             __threadfence();
         }
         __syncthreads();

@@ -329,7 +329,7 @@ struct b200_runner
     // the model's other path, which reads the arrays, have cost as much as that
     unsigned long long residentRent = 0;    // steps left to do there
     double residentCells = 0.0;             // entries of the copy, millions
-    unsigned long long residentBuilds = 0;
+    unsigned long long residentBuilds = 0, residentLaunches = 0;
     struct ResidentPair { unsigned int delay_class, src, first, count; };
     std::vector<ResidentPair> residentPairs;            // what the copy is filled from
     const b200_synapse_group *residentGroups = nullptr; // (device)
@@ -1913,6 +1913,8 @@ int buildResident(b200_runner *r)
     L.inbox = static_cast<ulonglong2*>(mail);
     L.more = static_cast<unsigned long long*>(mail) + headWords;
     L.leave = L.more + moreWords;
+    // (memory of the pool: the word that another model, or this one before, left there could be the one that is waited for)
+    CUDA_TRY(cudaMemsetAsync(L.leave, 0, sizeof(unsigned long long), r->stream));
 
     L.unit_start = dUnitStart; L.unit_first = dUnitFirst; L.columns = dColumns; L.cta_columns = dCtaColumns; L.runs = dRuns; L.entries = dEntries;
     L.num_spans = numSpans; L.num_units = units;
@@ -1971,6 +1973,7 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
     L.may_leave = leave ? 1u : 0u;
     L.patience = (unsigned int)std::min(1000.0 * r->residentPatience, (double)RESIDENT_MOST_DEBT - 1.0);
     L.barrier = r->fusedBarrier;
+    L.launch = ++r->residentLaunches;
     if(useWindows(r, numSteps)) {
         // (a head is known by its launch's number: before it repeats, no old head may be left)
         r->window.epoch = (r->window.epoch + 1u) & 0xFFFFFu;

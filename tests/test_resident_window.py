@@ -186,3 +186,26 @@ def test_windows_and_single_steps_hand_over_to_each_other():
         helpers.assert_close(rt.array("a.V")[0], orc.array("a.V")[0], "V", 1e-5, 5e-6)
     rt.close()
     orc.close()
+
+
+@pytest.mark.parametrize("build", [lambda: _late(7), lambda: _feed("SPARSE", "Poisson", 500, 2000, 2)], ids=["late", "feed"])
+def test_a_model_built_where_another_of_its_kind_ended(build):
+    """Models built and closed one after another get the same memory, and their calls end at the same steps: what an earlier one left
+    there is not taken for a word of this one.  (The lists of spikes a call leaves are emptied by one CTA before all fill them.)"""
+    from oracle.oracle import OracleRunner
+    calls, want = (24, 9, 33), []
+    orc = OracleRunner(resolve(build()), sum(calls))
+    for n in calls:
+        orc.step(n)
+        want.append({p.name: np.sort(orc.current_spikes(p.name)) for p in orc.net.pops})
+    assert sum(len(v) for v in want[0].values()) > 0
+    for _ in range(30):
+        rt = _runtime(resolve(build()), sum(calls))
+        rt.set_option("resident_ctas", 148)
+        assert rt.counter("window_steps") > 0
+        for n, spikes in zip(calls, want):
+            rt.step_time(n)
+            for name, ids in spikes.items():
+                assert np.array_equal(np.sort(rt.current_spikes(name)), ids), name
+        rt.close()
+    orc.close()
