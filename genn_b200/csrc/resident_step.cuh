@@ -468,16 +468,15 @@ residentStepKernel(const __grid_constant__ ResidentLaunch L)
         sh.limit = (unsigned int)min(state->barrier_spin_limit, 0xFFFFFFFFull);
     }
     for(unsigned int i = threadIdx.x; i < L.acc_floats; i += blockDim.x) acc[i] = 0.0f;
-    if(threadIdx.x < numGroups) {
-        residentLifTable(sh.lif[threadIdx.x], L.neuron.groups[threadIdx.x]);
-    }
+    for(unsigned int i = threadIdx.x; i < numGroups; i += blockDim.x) residentLifTable(sh.lif[i], L.neuron.groups[i]);
     stagedWords();
     __syncthreads();
     const unsigned int no0 = (unsigned int)sh.done;         // (step numbers of messages: 20 bits)
-    if(threadIdx.x <= numGroups) {
+    // (up to 65 entries; the option "resident_warps" allows blocks of 32 threads)
+    for(unsigned int i = threadIdx.x; i <= numGroups; i += blockDim.x) {
         // first warp whose unit (warp * G + me) is not before the group
-        const unsigned int u = residentTable<const unsigned int>(L.at.unit_start)[threadIdx.x];
-        sh.firstWarp[threadIdx.x] = (u <= me) ? 0u : (u - me + G - 1u) / G;
+        const unsigned int u = residentTable<const unsigned int>(L.at.unit_start)[i];
+        sh.firstWarp[i] = (u <= me) ? 0u : (u - me + G - 1u) / G;
     }
     ResidentFronts<ONE> front;
     if constexpr(ONE) {

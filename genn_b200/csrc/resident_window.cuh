@@ -176,13 +176,14 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
     }
     if(threadIdx.x < 32u) sh.count[0][threadIdx.x] = sh.count[1][threadIdx.x] = 0u;
     for(unsigned int i = threadIdx.x; i < K * columns; i += blockDim.x) acc[i] = 0.0f;
-    if(threadIdx.x < numGroups) residentLifTable(sh.lif[threadIdx.x], L.neuron.groups[threadIdx.x]);
+    for(unsigned int i = threadIdx.x; i < numGroups; i += blockDim.x) residentLifTable(sh.lif[i], L.neuron.groups[i]);
     stagedWords();
     __syncthreads();
-    if(threadIdx.x <= numGroups) {
+    // (up to 65 entries; the option "resident_warps" allows blocks of 32 threads)
+    for(unsigned int i = threadIdx.x; i <= numGroups; i += blockDim.x) {
         // first warp whose unit (warp * G + me) is not before the group
-        const unsigned int u = residentTable<const unsigned int>(L.at.unit_start)[threadIdx.x];
-        sh.firstWarp[threadIdx.x] = (u <= me) ? 0u : (u - me + G - 1u) / G;
+        const unsigned int u = residentTable<const unsigned int>(L.at.unit_start)[i];
+        sh.firstWarp[i] = (u <= me) ? 0u : (u - me + G - 1u) / G;
     }
 
     // this thread's neuron

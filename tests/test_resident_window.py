@@ -87,13 +87,14 @@ def _several(delay):
     return m
 
 
-def _check(build, window, ctas=0, calls=CALLS, warps=0):
+def _check(build, window, ctas=0, calls=CALLS, warps=0, windows=True):
     from oracle.oracle import OracleRunner
     net, total = resolve(build()), sum(calls)
     rt, orc, other = _runtime(net, total), OracleRunner(resolve(build()), total), _runtime(resolve(build()), total)
     other.set_option("use_fused", 0)                # (counts the same spikes and events)
     rt.set_option("resident_ctas", ctas)
     rt.set_option("resident_warps", warps)
+    rt.set_option("use_windows", windows)
     assert rt.counter("window_steps") == window
     for r in (rt, other):
         r.set_option("count_events", 1)
@@ -209,3 +210,20 @@ def test_a_model_built_where_another_of_its_kind_ended(build):
                 assert np.array_equal(np.sort(rt.current_spikes(name)), ids), name
         rt.close()
     orc.close()
+
+
+@pytest.mark.parametrize("windows", [True, False])
+@pytest.mark.parametrize("groups,warps", [(64, 2), (32, 1), (63, 2)])
+def test_as_many_populations_as_a_block_has_threads(groups, warps, windows):
+    """The table of a CTA's warps has an entry more than there are populations; groups without a run of entries onto the last one use it."""
+    def build():
+        rng = np.random.default_rng(groups)
+        m = GeNNModel("float", "many")
+        m.dt, m.seed = 1.0, 3
+        src = _sources(m, "src", "Poisson", 30, rng, 200.0)
+        pops = [m.add_neuron_population(f"p{i}", 1 + (i * 7) % 32, "LIF", LIF, {"V": -56.0, "RefracTime": 0.0}) for i in range(groups - 1)]
+        for i, trg in ((0, pops[0]), (1, pops[-2]), (2, pops[-1])):
+            _connect(m, f"d{i}", "DENSE", src, trg, rng, 1)
+            _connect(m, f"b{i}", "BITMASK", src, trg, rng, 1, k=1)
+        return m
+    _check(build, 16 if windows else 0, groups, (5, 1, 17, 2), warps, windows)
