@@ -411,6 +411,9 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
                 if(gaveUp(polls)) break;
             }
         }
+        // (entries that did not fit a head are read by other lanes than the one that saw it: __syncwarp() orders the lanes' memory
+        // accesses, the vote alone is not said to)
+        __syncwarp();
         if(__any_sync(0xFFFFFFFFu, total > RESIDENT_WINDOW_INLINE)) fenceGpu();
         if(steps == 0u) return;
         auto spikeOf = [&](unsigned int e, unsigned int from) { return unitFirst[min(((e >> 5) & 31u) * G + from, L.num_units - 1u)] + (e & 31u); };
