@@ -57,6 +57,7 @@
 #include <cuda_runtime.h>
 
 #include "neuron_update.cuh"
+#include "window_tags.h"
 
 namespace b200
 {
@@ -198,7 +199,7 @@ struct ResidentWindow
     unsigned int body;                  // most spikes of a message
     unsigned int run_groups;            // groups of 32 entries of the longest run (0: no runs)
     unsigned int list_at, words_at, acc_at;     // in dynamic shared memory, behind the tables of ResidentLayout
-    unsigned int epoch;                 // of the launch
+    unsigned int epoch;                 // of the launch (window_tags.h)
     unsigned long long free_groups;     // populations without inputs (FEED)
     ulonglong2 *heads;                  // [buffers][copies][RESIDENT_HEADS] tag << 20 | spikes, short tag << 48 | the first three entries
     unsigned short *bodies;             // [buffers][grid][body] step of the window << 10 | unit of the CTA << 5 | neuron

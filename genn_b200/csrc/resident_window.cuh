@@ -223,9 +223,8 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         atomicOr(&sh.stop, 1u);
         return true;
     };
-    auto tagOf = [&](unsigned int message) { return ((unsigned long long)W.epoch << 24) | (message & 0xFFFFFFu); };
-    // (the second word's: the word that lay there before it was of another message of this launch, or of another launch)
-    auto shortTagOf = [&](unsigned int message) { return ((W.epoch & 0xFFu) << 8) | (message & 0xFFu); };
+    auto tagOf = [&](unsigned int message) { return windowTag(W.epoch, message); };
+    auto shortTagOf = [&](unsigned int message) { return windowShortTag(W.epoch, message); };
 
     // ---- the neurons of this warp through steps [first, first + n) of the launch; lane j gets the ballot of the j-th.
     // Populations without inputs: nothing to add up, and a Poisson neuron goes from spike to spike.

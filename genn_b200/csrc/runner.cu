@@ -1616,7 +1616,7 @@ int buildResident(b200_runner *r)
             for(win.lag = 1; after % win.lag || after / win.lag > RESIDENT_WINDOW_MOST; win.lag++) {}
             win.steps = after / win.lag;
             win.cap = (unsigned int)std::min<unsigned long long>(sourceNeurons, RESIDENT_LIST);
-            win.buffers = 2u * win.lag + 2u;
+            win.buffers = windowBuffers(2u * win.lag + 2u);
             windowed = win.cap >= sourceNeurons || r->residentHandsOver;      // (before it is rounded up)
         }
         win.cap = (win.cap + 3u) & ~3u;         // (entries are read four at a time)
@@ -1975,12 +1975,9 @@ int launchResident(b200_runner *r, unsigned long long numSteps, unsigned long lo
     L.barrier = r->fusedBarrier;
     L.launch = ++r->residentLaunches;
     if(useWindows(r, numSteps)) {
-        // (a head is known by its launch's number: before it repeats, no old head may be left)
-        r->window.epoch = (r->window.epoch + 1u) & 0xFFFFFu;
-        if(r->window.epoch == 0u) {
-            CUDA_TRY(cudaMemsetAsync(r->window.heads, 0, sizeof(ulonglong2) * r->window.buffers * L.copies * RESIDENT_HEADS, r->stream));
-            r->window.epoch = 1u;
-        }
+        bool clear = false;
+        r->window.epoch = windowNextEpoch(r->window.epoch, &clear);
+        if(clear) CUDA_TRY(cudaMemsetAsync(r->window.heads, 0, sizeof(ulonglong2) * r->window.buffers * L.copies * RESIDENT_HEADS, r->stream));
         ResidentWindowLaunch A{L, r->window};
         if(r->residentHandsOver) {
             A.L.spare = RESIDENT_WINDOW_SPARE;
