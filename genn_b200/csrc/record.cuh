@@ -178,8 +178,10 @@ __attribute__((always_inline)) inline void decodePairsAs(const RecordPairs &R, u
     auto timeOf = [&] { return R.start + (double)(row >= R.first_row ? row - R.first_row : row + R.rows - R.first_row) * R.dt; };
     double t = timeOf();
     uint64_t at = R.counts[b];
-    double *times = R.ids ? R.times[b] : nullptr;
-    uint32_t *ids = R.ids ? R.ids[b] : nullptr;
+    // (an entry that has nothing but padding may come without arrays)
+    const bool store = R.ids != nullptr;
+    double *times = store ? R.times[b] : nullptr;
+    uint32_t *ids = store ? R.ids[b] : nullptr;
     for(uint64_t i = from; i < to; i++) {
         const uint32_t index = R.pairs[2 * i] - R.base;
         uint32_t word = R.pairs[2 * i + 1];
@@ -194,13 +196,13 @@ __attribute__((always_inline)) inline void decodePairsAs(const RecordPairs &R, u
             } while(index >= sectionEnd);
             t = timeOf();
             at = R.counts[b];
-            if(ids) {
+            if(store) {
                 times = R.times[b];
                 ids = R.ids[b];
             }
         }
         if(index + 1u == sectionEnd) word &= R.lastMask;
-        if(!ids) {
+        if(!store) {
             at += (uint64_t)__builtin_popcount(word);
             continue;
         }

@@ -40,6 +40,25 @@ def test_decoded_spikes_equal_the_unpacked_bits(rows, batch, num_neurons, first_
         assert np.array_equal(t, wt) and np.array_equal(i, wi)
 
 
+@pytest.mark.parametrize("whole", [False, True])
+def test_a_batch_entry_without_spikes_needs_no_room(whole):
+    """Bits beyond the neurons are no spikes: an entry that has nothing else may come without arrays, and those behind it are decoded."""
+    lib = abi.load_library()
+    words = np.zeros((3, 2, 2), np.uint32)
+    words[:, 0, 1] = 1 << 20            # (beyond neuron 39)
+    words[:, 1] = 5, 1 << 6
+    index = np.flatnonzero(words)
+    pairs = np.ascontiguousarray(np.stack([index, words.reshape(-1)[index]], axis=1).astype(np.uint32))
+    source = (words.ctypes.data, None, 0) if whole else (None, pairs.ctypes.data, len(pairs))
+    counts = (C.c_uint64 * 2)()
+    args = (*source, 0, 3, 2, 2, 1, 40, 0, 0.0, 1.0, counts)
+    abi.check(lib.b200_decode_recording(*args, None, None))
+    assert list(counts) == [0, 9]
+    times, ids = np.full(9, -1.0), np.full(9, 99, np.uint32)
+    abi.check(lib.b200_decode_recording(*args, (C.c_void_p * 2)(None, times.ctypes.data), (C.c_void_p * 2)(None, ids.ctypes.data)))
+    assert np.array_equal(times, np.repeat([0.0, 1.0, 2.0], 3)) and np.array_equal(ids, np.tile([0, 2, 38], 3)) and list(counts) == [0, 9]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("sizes,density", [([1], 1.0), ([4095, 4096, 4097], 0.05), ([16] * 60, 0.5), ([100003], 0.01), ([5000, 0, 37], 0.0)])
 def test_the_list_holds_the_non_zero_words_in_order(sizes, density):
