@@ -339,7 +339,7 @@ struct b200_runner
     unsigned int residentGrid = 0, residentBlock = 0;
     size_t residentSmem = 0;
     unsigned long long residentCleared = ~0ull;             // steps done when the message buffers were last cleared (~0: they are not)
-    size_t residentMailBytes = 0;
+    size_t residentMailBytes = 0, windowMailBytes = 0;
     const void *residentKernel = nullptr;
     ResidentLaunch resident{};
     bool useWindow = true, windowReady = false;             // windows of steps (resident_window.cuh)
@@ -1692,6 +1692,7 @@ int buildResident(b200_runner *r)
         }
     };
     const unsigned int most = std::min<unsigned int>((unsigned int)sms, RESIDENT_MAX_CTAS);
+    auto copiesFor = [](unsigned int G) { return std::min(32u, (G + RESIDENT_READERS - 1u) / RESIDENT_READERS); };
     // the list and the ballots lie where the other kernel's input buffers begin, the buffers of a window behind them
     auto windowBytes = [&] {
         win.list_at = L.at.history;
@@ -1703,7 +1704,15 @@ int buildResident(b200_runner *r)
         // (a window's messages cost little, and its deliveries and updates are shared by all SMs.  us a step on 48 / 100 / 148 CTAs: 1000 ->
         // 10 000 neurons 0.33 / 0.32 / 0.32, BITMASK 2003 x 5009 0.93 / 0.88 / 0.82, DENSE 4096 x 4096 2.14 / 1.77 / 1.41)
         const unsigned int G = std::min(std::max(r->residentCtas ? r->residentCtas : most, (units + RESIDENT_UNITS - 1u) / RESIDENT_UNITS), std::min(most, units));
-        if((units + G - 1u) / G <= RESIDENT_UNITS) {
+        // Messages: room for every neuron in every step of `buffers` windows, about as much as a spike queue of that delay (100 000 neurons, 199
+        // steps: 84 MB beside 81).  No more than a quarter of the free memory (what the pool may keep needs no asking).
+        const unsigned int perCta = (units + G - 1u) / G;
+        win.body = perCta * 32u * win.steps;
+        const size_t headBytes = sizeof(ulonglong2) * win.buffers * copiesFor(G) * RESIDENT_HEADS;
+        r->windowMailBytes = headBytes + sizeof(unsigned short) * win.buffers * G * win.body;
+        size_t freeBytes = POOL_KEEP * 4, totalBytes = 0;
+        if(r->windowMailBytes > freeBytes / 4) CUDA_TRY(cudaMemGetInfo(&freeBytes, &totalBytes));
+        if(perCta <= RESIDENT_UNITS && r->windowMailBytes <= freeBytes / 4) {
             layOut(G);
             r->windowSmem = windowBytes();
             if(tables + accFloats * sizeof(float) <= room && r->windowSmem <= windowRoom) grid = G;
@@ -1905,7 +1914,7 @@ int buildResident(b200_runner *r)
     L.history = history;
     const unsigned int mostIds = neuronWarps * 32u;
     L.more_words = (mostIds - RESIDENT_CELL_IDS + RESIDENT_MORE_IDS - 1u) / RESIDENT_MORE_IDS;
-    L.copies = std::min(32u, (grid + RESIDENT_READERS - 1u) / RESIDENT_READERS);
+    L.copies = copiesFor(grid);
     const size_t headWords = (size_t)L.buffers * L.copies * grid * 2u, moreWords = (size_t)L.buffers * grid * L.more_words;
     void *mail = nullptr;
     r->residentMailBytes = sizeof(unsigned long long) * (headWords + moreWords + 1u);
@@ -1935,7 +1944,6 @@ int buildResident(b200_runner *r)
     }
     L.hold = const_cast<unsigned long long*>(r->residentHold);
     if(windowed) {
-        win.body = neuronWarps * 32u * win.steps;
         if(const int err = device(sizeof(ulonglong2) * win.buffers * L.copies * RESIDENT_HEADS, (void**)&win.heads)) return err;
         if(const int err = device(sizeof(unsigned short) * win.buffers * grid * win.body, (void**)&win.bodies)) return err;
         CUDA_TRY(cudaMemsetAsync(win.heads, 0, sizeof(ulonglong2) * win.buffers * L.copies * RESIDENT_HEADS, r->stream));
@@ -3306,6 +3314,10 @@ int b200_get_counter(b200_runner *r, const char *name, uint64_t *value)
     }
     if(n == "resident_bytes") {
         *value = r->residentReady ? (uint64_t)(r->residentCells * 1e6 * sizeof(uint2) + 0.5) : 0u;
+        return B200_OK;
+    }
+    if(n == "resident_message_bytes") {
+        *value = r->residentReady ? r->residentMailBytes + (r->windowReady ? r->windowMailBytes : 0u) : 0u;
         return B200_OK;
     }
     if(n == "resident_builds") {

@@ -389,7 +389,9 @@ int  b200_get_counter(b200_runner *r, const char *name, uint64_t *value);
  * its fixed cost in synaptic events when a step's work is cut into equal stretches per CTA, default 256),
  * "use_resident" (default 1: batch-1 networks without learning and PROCEDURAL groups run on the target-resident kernel, which
  * works on a private copy of the SPARSE groups, 8 bytes an entry, padded per block of targets: 12 to 26 bytes a synapse,
- * measured; 0 gives it back.  Counter "resident": whether the next steps run on it, "resident_bytes": the copy's size), "resident_ctas" /
+ * measured; 0 gives it back.  Counter "resident": whether the next steps run on it, "resident_bytes": the copy's size,
+ * "resident_message_bytes": that of the buffers of its messages, about two
+ * spike queues of the longest axonal delay and 0.2 MB for each step of it), "resident_ctas" /
  * "resident_warps" (its grid and block; 0: chosen by size), "resident_patience" (microseconds that it may lose to the kernel with a
  * grid barrier, which is faster from some 100 spikes a step on, before that one takes over for a while; default 200; counter
  * "resident_hold": the step until which; "resident_builds": how often the copy was made),

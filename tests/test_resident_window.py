@@ -212,6 +212,30 @@ def test_a_model_built_where_another_of_its_kind_ended(build):
     orc.close()
 
 
+def test_messages_take_no_more_than_some_spike_queues():
+    """They have room for every neuron in every step of a delay, as the queues have, and go back with the rest."""
+    n, delay = 20000, 199
+    rng = np.random.default_rng(6)
+    m = GeNNModel("float", "messages")
+    m.dt, m.seed = 1.0, 7
+    a = m.add_neuron_population("a", n, "LIF", LIF, {"V": -60.0, "RefracTime": 0.0})
+    _connect(m, "aa", "SPARSE", a, a, rng, delay, k=2)
+    rt = _runtime(resolve(m), 10)
+    assert rt.counter("window_steps") == 10
+    queue, size = 4 * n * (delay + 4), rt.counter("resident_message_bytes")
+    assert queue < size < 2.5 * queue + 0.25e6 * delay
+    rt.step_time(30)
+    rt.set_option("use_windows", 0)
+    assert rt.counter("resident") == 1 and rt.counter("resident_message_bytes") < size
+    rt.set_option("use_resident", 0)
+    rt.step_time(5)
+    assert rt.counter("resident_message_bytes") == 0
+    rt.set_option("use_resident", 1)
+    rt.set_option("use_windows", 1)
+    assert rt.counter("resident") == 1 and rt.counter("resident_message_bytes") == size
+    rt.close()
+
+
 @pytest.mark.parametrize("windows", [True, False])
 @pytest.mark.parametrize("groups,warps", [(64, 2), (32, 1), (63, 2)])
 def test_as_many_populations_as_a_block_has_threads(groups, warps, windows):
