@@ -87,7 +87,7 @@ def _several(delay):
     return m
 
 
-def _check(build, window, ctas=0, calls=CALLS, warps=0, windows=True):
+def _check(build, window, ctas=0, calls=CALLS, warps=0, windows=True, patience=None):
     from oracle.oracle import OracleRunner
     net, total = resolve(build()), sum(calls)
     rt, orc, other = _runtime(net, total), OracleRunner(resolve(build()), total), _runtime(resolve(build()), total)
@@ -95,13 +95,17 @@ def _check(build, window, ctas=0, calls=CALLS, warps=0, windows=True):
     rt.set_option("resident_ctas", ctas)
     rt.set_option("resident_warps", warps)
     rt.set_option("use_windows", windows)
+    if patience is not None:
+        rt.set_option("resident_patience", patience)
     assert rt.counter("window_steps") == window
+    holds = set()
     for r in (rt, other):
         r.set_option("count_events", 1)
     done, seen = 0, {p.name: [] for p in net.pops}
     for n in calls:
         rt.step_time(n)
         other.step_time(n)
+        holds.add(rt.counter("resident_hold"))
         for _ in range(n):
             orc.step(1)
             done += 1
@@ -124,6 +128,7 @@ def _check(build, window, ctas=0, calls=CALLS, warps=0, windows=True):
             assert np.array_equal(got, helpers.sorted_pairs(seen[p.name])), f"recorded spikes of {p.name}"
     for r in (rt, other, orc):
         r.close()
+    return holds
 
 
 @pytest.mark.parametrize("delay", [0, 3, 15, 20])
@@ -210,6 +215,29 @@ def test_a_model_built_where_another_of_its_kind_ended(build):
                 assert np.array_equal(np.sort(rt.current_spikes(name)), ids), name
         rt.close()
     orc.close()
+
+
+def _busy(kind, delay):
+    """Sources of half a spike a step, alone (feed), with a recurrent population (late), or with one that fires as a whole (burst)."""
+    rng = np.random.default_rng(delay)
+    n = 3000 if kind == "burst" else 200
+    m = GeNNModel("float", "busy")
+    m.dt, m.seed = 1.0, 23
+    src = _sources(m, "in", "Poisson", 300, rng, 600.0)
+    trg = m.add_neuron_population("out", n, "LIF", dict(LIF, Ioffset=0.3), {"V": -65.0 if kind == "burst" else rng.uniform(-65, -50, n).astype(np.float32), "RefracTime": 0.0})
+    src.spike_recording_enabled = trg.spike_recording_enabled = True
+    _connect(m, "syn", "SPARSE", src, trg, rng, delay, scale=1e-4, k=10)
+    if kind != "feed":
+        _connect(m, "rec", "SPARSE", trg, trg, rng, delay, scale=1e-4, k=10)
+    return m
+
+
+@pytest.mark.parametrize("kind,delay,window", [("feed", 0, 16), ("feed", 5, 16), ("feed", 21, 16), ("late", 15, 16), ("late", 19, 10), ("late", 44, 15), ("burst", 19, 10)])
+def test_a_busy_network_leaves_in_the_middle_of_a_call(kind, delay, window):
+    """Launches that end early behind a window, the sources of some a window ahead by then, others with spikes that are still on their way
+    in messages of one to three windows; the other kernel's share of the call, and this kernel again."""
+    holds = _check(lambda: _busy(kind, delay), window, calls=(1, 2, 3, 5, 60, 1, 1, 40, 87), warps=4, patience=1e6 if kind == "burst" else 0)
+    assert len(holds) >= 3, holds       # (left more than once)
 
 
 def test_messages_take_no_more_than_some_spike_queues():
