@@ -336,7 +336,8 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
         if(lane < n) {
             words[((first + lane) % W.ring) * RESIDENT_UNITS + warp] = word;
             const b200_neuron_group &g = groups[group];
-            if(L.neuron.num_recording_timesteps && g.record_spk) {
+            // (a recording of fewer steps than these keeps the last ones: no two lanes write the same word)
+            if(lane + L.neuron.num_recording_timesteps >= n && L.neuron.num_recording_timesteps && g.record_spk) {
                 const unsigned int at = (unsigned int)(((unsigned long long)recAt + first + lane) % L.neuron.num_recording_timesteps);
                 g.record_spk[(size_t)at * ((g.num_update + 31u) / 32u) + (local - lane) / 32u] = word;
             }

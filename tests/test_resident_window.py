@@ -217,6 +217,34 @@ def test_a_model_built_where_another_of_its_kind_ended(build):
     orc.close()
 
 
+@pytest.mark.parametrize("rows", [1, 3, 7, 15, 16, 17])
+@pytest.mark.parametrize("build", [lambda: _feed("SPARSE", "Poisson", 131, 300, 2), lambda: _late(15)], ids=["feed", "late"])
+def test_recordings_of_fewer_steps_than_a_window(build, rows):
+    """A recording holds the last steps of a call, however few: the rows of the steps before, of the same window too, are written over."""
+    from oracle.oracle import OracleRunner
+    net = resolve(build())
+    rt, orc = _runtime(net, rows), OracleRunner(resolve(build()), rows)
+    assert rt.counter("window_steps") == 16
+    done, seen = 0, {p.name: [] for p in net.pops}
+    for n in (21, 16, 37, 64):
+        rt.step_time(n)
+        for _ in range(n):
+            orc.step(1)
+            done += 1
+            for p in net.pops:
+                seen[p.name] += [(done - 1, int(i)) for i in orc.current_spikes(p.name)]
+        rt.synchronize()
+        rt.pull_recording_buffers()
+        for p in net.pops:
+            want = [s for s in seen[p.name] if s[0] >= done - rows]
+            times, ids = rt.recorded_spikes(p.name)[0]
+            got = np.stack([np.rint(times / net.dt).astype(np.uint32), ids], axis=1)
+            assert np.array_equal(helpers.sorted_pairs(got), helpers.sorted_pairs(np.array(want, np.int64).reshape(-1, 2))), f"{p.name} after {done} steps"
+    assert sum(map(len, seen.values())) > 1000
+    rt.close()
+    orc.close()
+
+
 def _busy(kind, delay):
     """Sources of half a spike a step, alone (feed), with a recurrent population (late), or with one that fires as a whole (burst)."""
     rng = np.random.default_rng(delay)
