@@ -70,6 +70,13 @@ def lock_view(view: np.ndarray):
             _view_bytes -= nbytes
 
 
+def pairs_room(words: int) -> int:
+    """Room in the list of a recording's non-zero words at first: one in sixteen, one in eight of short recordings.  The list lies in
+    page-locked memory, which costs 0.2 to 0.45 ms a MB when it is first asked for: the first pull of 250 M words took 54 - 89 ms with one in
+    sixteen and 112 - 155 with one in eight."""
+    return max(1024, words // 16, min(words // 8, 1 << 16))
+
+
 class DeviceArray:
     def __init__(self, rt: "DeviceFactory", nbytes: int):
         self._rt = rt
@@ -177,7 +184,8 @@ class Runtime:
         self.factory = DeviceFactory(self.lib, self.handle)
         self._pinned = []
         self._rec_host = {}
-        self.recording_pairs_capacity = None        # (index, word) pairs a recording pull has room for; None: 1/16 of the words
+        self.recording_pairs_capacity = None        # (index, word) pairs a recording pull has room for; None: pairs_room, up to 1/8 of the words
+        self._rec_room = 0
         self._rec_pairs, self._rec_layout = None, {}
         self._rec_timestep = 0
         self.shard = shard
@@ -544,12 +552,17 @@ class Runtime:
         sizes = [int(np.prod(a.shape, dtype=np.int64)) for _, a in recs]
         total = sum(sizes)
         if recs and total < (1 << 32):
-            # room for one non-zero word in eight unless the caller chose (313 000 words of which 7 % are not zero: pulled and
-            # decoded in 150 us; as a whole array, 560)
-            cap = int(self.recording_pairs_capacity or max(1024, total // 8))
             pairs, count = C.c_void_p(), C.c_uint64()
-            check(self.lib.b200_pull_recording(self.handle, len(recs), (C.c_void_p * len(recs))(*[a.ptr for _, a in recs]),
-                                               (C.c_uint64 * len(recs))(*sizes), cap, C.byref(pairs), C.byref(count)))
+
+            def pull(capacity):
+                check(self.lib.b200_pull_recording(self.handle, len(recs), (C.c_void_p * len(recs))(*[a.ptr for _, a in recs]),
+                                                   (C.c_uint64 * len(recs))(*sizes), capacity, C.byref(pairs), C.byref(count)))
+            pull(int(self.recording_pairs_capacity or max(self._rec_room, pairs_room(total))))
+            # room for one word in eight where that many are not zero, unless the caller chose (313 000 words of which 7 % are not
+            # zero: pulled and decoded in 150 us; as a whole array, 560)
+            if not pairs.value and not self.recording_pairs_capacity and count.value <= total // 8:
+                self._rec_room = total // 8
+                pull(self._rec_room)
             base = 0
             for (name, arr), n in zip(recs, sizes):
                 self._rec_layout[name] = (base, arr.shape)

@@ -40,6 +40,15 @@ def test_decoded_spikes_equal_the_unpacked_bits(rows, batch, num_neurons, first_
         assert np.array_equal(t, wt) and np.array_equal(i, wi)
 
 
+def test_room_for_the_non_zero_words():
+    """One in eight of short recordings; a long one asks for no more page-locked memory at first than one in sixteen; never less for
+    more words."""
+    from genn_b200.runtime import pairs_room
+    assert [pairs_room(n) for n in (0, 100, 8192, 313000, 8 << 20, 16 << 20, 250000000)] == [1024, 1024, 1024, 39125, 1 << 19, 1 << 20, 15625000]
+    rooms = [pairs_room(n) for n in range(0, 40 << 20, 99991)]
+    assert rooms == sorted(rooms)
+
+
 @pytest.mark.parametrize("whole", [False, True])
 def test_a_batch_entry_without_spikes_needs_no_room(whole):
     """Bits beyond the neurons are no spikes: an entry that has nothing else may come without arrays, and those behind it are decoded."""
@@ -87,3 +96,35 @@ def test_the_list_holds_the_non_zero_words_in_order(sizes, density):
             got = np.ctypeslib.as_array((C.c_uint32 * (2 * len(index))).from_address(pairs.value)).reshape(-1, 2)
             assert np.array_equal(got[:, 0], index) and np.array_equal(got[:, 1], flat[index])
     lib.b200_runner_destroy(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rate", [1.0, 2.4, 3.4, 5.0])
+def test_long_recordings_come_as_pairs_up_to_one_word_in_eight(rate):
+    """1.25 M words, of which 3, 7, 10 and 15 % are not zero: fewer than the list has room for at first, more, and too many."""
+    from genn_b200 import GeNNModel, init_postsynaptic, init_weight_update
+    n, steps = 40000, 1000
+    m = GeNNModel("float", "recording")
+    m.dt, m.seed = 1.0, 3
+    src = m.add_neuron_population("src", n, "Poisson", {"rate": rate}, {"timeStepToSpike": 0.0})
+    trg = m.add_neuron_population("trg", 32, "LIF", {"C": 0.25, "TauM": 20.0, "Vrest": -65.0, "Vreset": -70.0, "Vthresh": -50.0, "Ioffset": 0.0, "TauRefrac": 2.0},
+                                  {"V": -65.0, "RefracTime": 0.0})
+    src.spike_recording_enabled = True
+    sg = m.add_synapse_population("syn", "SPARSE", src, trg, init_weight_update("StaticPulseConstantWeight", {"g": 0.0}), init_postsynaptic("DeltaCurr", {}))
+    sg.set_sparse_connections(np.arange(n, dtype=np.uint32), np.arange(n, dtype=np.uint32) % 32, presorted=True)
+    m.build()
+    m.load(num_recording_timesteps=steps)
+    rt = m._runtime
+    for _ in range(2):
+        m.step_time(steps)
+        rt.recording_pairs_capacity = None
+        m.pull_recording_buffers_from_device()
+        times, ids = rt.recorded_spikes("src")[0]
+        share = len(rt._rec_pairs) / (steps * n / 32) if rt._rec_pairs is not None else 1.0
+        assert (rt._rec_pairs is None) == (rate == 5.0) and (share > 1 / 16) == (rate > 2.0)
+        rt.recording_pairs_capacity = 1
+        m.pull_recording_buffers_from_device()
+        assert rt._rec_pairs is None
+        whole = rt.recorded_spikes("src")[0]
+        assert np.array_equal(times, whole[0]) and np.array_equal(ids, whole[1]) and len(ids) > 0.8 * n * rate * steps * 1e-3
+    m.unload()
