@@ -60,8 +60,7 @@ def test_wait_limits_are_options():
     rt.close()
 
 
-@pytest.mark.parametrize("windows", [1, 0], ids=["in windows", "step by step"])
-def test_a_missing_message_of_the_target_resident_kernel_runs_into_the_wait_limit(windows):
+def test_a_missing_message_of_the_target_resident_kernel_runs_into_the_wait_limit():
     """Two polls are fewer than a message needs from one CTA to the next."""
     from genn_b200.runtime import Runtime
     from tests import helpers
@@ -69,8 +68,6 @@ def test_a_missing_message_of_the_target_resident_kernel_runs_into_the_wait_limi
     rt = Runtime(None, 10, net=resolve(CASES["c1_full"]()[0]))
     assert rt.counter("resident") == 1
     rt.set_option("resident_ctas", 148)
-    rt.set_option("use_windows", windows)
-    assert (rt.counter("window_steps") > 0) == bool(windows)
     rt.set_option("barrier_spin_limit", 1)
     rt.step_time(200)
     with pytest.raises(abi.B200Error, match="timed out"):

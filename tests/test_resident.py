@@ -14,25 +14,20 @@ pytestmark = pytest.mark.gpu
 NAMES = ["ff_sparse", "ff_sparse_narrow", "ff_bitmask", "ff_dense", "potjans_mini", "potjans_mini_d1", "cond_delay", "izhikevich", "c1_full"]
 
 
-WINDOWED = ["ff_sparse", "ff_sparse_narrow", "ff_bitmask", "ff_dense", "cond_delay", "c1_full"]       # (with the option "use_windows", the default)
-
-
-def _resident(name, ctas=0, warps=0, windows=1):
+def _resident(name, ctas=0, warps=0):
     model, steps, dump_every = CASES[name]()
     net = resolve(model)
     rt = _runtime(net, steps)
     rt.set_option("resident_ctas", ctas)
     rt.set_option("resident_warps", warps)
-    rt.set_option("use_windows", windows)
     assert rt.counter("resident") == 1
-    assert (rt.counter("window_steps") > 0) == (bool(windows) and name in WINDOWED)
     return net, rt, steps, dump_every
 
 
 @pytest.mark.parametrize("ctas,warps", [(0, 0), (1, 24), (7, 4), (148, 24)])
-@pytest.mark.parametrize("name,windows", [(name, 1) for name in NAMES] + [(name, 0) for name in WINDOWED])
-def test_all_steps_in_one_launch_match_the_reference(name, windows, ctas, warps):
-    net, rt, steps, _ = _resident(name, ctas, warps, windows)
+@pytest.mark.parametrize("name", NAMES)
+def test_all_steps_in_one_launch_match_the_reference(name, ctas, warps):
+    net, rt, steps, _ = _resident(name, ctas, warps)
     rt.set_option("count_events", 1)
     before = rt.kernel_launches
     rt.step_time(steps)
@@ -51,11 +46,11 @@ def test_all_steps_in_one_launch_match_the_reference(name, windows, ctas, warps)
     rt.close()
 
 
-@pytest.mark.parametrize("name,windows", [("ff_sparse", 1), ("ff_bitmask", 1), ("potjans_mini", 1), ("cond_delay", 1), ("izhikevich", 1), ("ff_sparse", 0), ("ff_bitmask", 0), ("cond_delay", 0)])
-def test_launches_of_every_length_hand_over_to_the_other_paths(name, windows):
+@pytest.mark.parametrize("name", ["ff_sparse", "ff_bitmask", "potjans_mini", "cond_delay", "izhikevich"])
+def test_launches_of_every_length_hand_over_to_the_other_paths(name):
     """Steps on this path alternate with steps on the one-launch-per-kernel path: spike lists, rings and state between
     launches must be what that path expects, and the current spikes those of the reference."""
-    net, rt, steps, dump_every = _resident(name, windows=windows)
+    net, rt, steps, dump_every = _resident(name)
     chunk = [1, 2, 1, 5, 3, 17, 1, 1, 40]
     spikes = {p.name: [] for p in net.pops}
     done = i = 0
@@ -401,8 +396,8 @@ def _busy(kind, synchronous):
 
 
 @pytest.mark.parametrize("synchronous", [False, True], ids=["patience 0", "more than the list holds"])
-@pytest.mark.parametrize("kind,windows", [("immediate", 1), ("late", 1), ("late", 0), ("rings", 1), ("two delays", 1), ("bit mask", 1)])
-def test_a_busy_network_is_handed_over_and_taken_back(kind, windows, synchronous):
+@pytest.mark.parametrize("kind", ["immediate", "late", "rings", "two delays", "bit mask"])
+def test_a_busy_network_is_handed_over_and_taken_back(kind, synchronous):
     """Launches that end early, the other kernel's share of their steps, and this kernel again: spikes and state of the CPU
     checker at every end of a call, also where a step that had begun is left to the other kernel."""
     from oracle.oracle import OracleRunner
@@ -413,8 +408,7 @@ def test_a_busy_network_is_handed_over_and_taken_back(kind, windows, synchronous
     for r in (rt, other):
         r.set_option("count_events", 1)
     rt.set_option("resident_warps", 4)          # (few warps: a spike costs the more)
-    rt.set_option("use_windows", windows)
-    assert rt.counter("resident") == 1 and (rt.counter("window_steps") > 0) == (kind == "late" and windows == 1)
+    assert rt.counter("resident") == 1
     rt.set_option("resident_patience", 1e6 if synchronous and kind != "bit mask" else 0)
     holds, done = set(), 0
     for n in (1, 2, 3, 5, 60, 1, 1, 40, 87):
