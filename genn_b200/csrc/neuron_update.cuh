@@ -27,7 +27,8 @@ namespace b200
 {
 constexpr int NEURON_BLOCK = 128;
 constexpr unsigned int NEURON_BLOCKS_PER_SM = 16;
-constexpr unsigned int NEURON_STAGED = 8;           // groups whose tables a block takes into shared memory (5 KB of 16 blocks an SM)
+constexpr unsigned int NEURON_STAGED = 8;           // most groups whose tables a block takes into shared memory
+constexpr unsigned int NEURON_STAGED_ANY = 4;       // as many however large the launch and whatever kernel runs before it
 // Warps of an SM before a warp takes four words of neurons.  us a step of a network of 80 000 / 150 000 / 200 000 / 300 000 / 1 200 000
 // neurons with one word a warp 4.4 / 4.7 / 6.7 / 7.4 / 15.1, with four 5.3 / 5.6 / 5.5 / 5.5 / 11.9; with a Poisson source each 5.3 / 5.6 /
 // 8.0 / 9.0 / 21.7 and 7.2 / 8.1 / 8.2 / 7.9 / 21.8: the line, 152 000 neurons, is where the second wave of blocks begins.
@@ -524,22 +525,41 @@ __device__ __forceinline__ void neuronWords(const NeuronLaunch &L, const b200_ne
 
 // WORDS = 4: a warp takes the 128 neurons of a padded block, a quarter of the instructions for each, as long as that leaves
 // every SM its warps; WORDS = 1: a warp takes 32, for small networks, where the chain of one neuron is all there is.
-template<int NPSM, int NCS, int WORDS>
+// Whether the blocks of a launch take the tables of their groups (0.6 KB each) into shared memory ahead of chainWait().  The kernels before
+// and behind use next to none of it, and where they and this one split an SM's memory differently, blocks of one are not placed beside
+// those of the other: with room for eight groups in every block (5 KB) a step of two populations of 400 and 500 neurons with 32 copies took
+// 7.6 us (DENSE) and 11.1 (STDP), without 7.2 and 10.7, with room for its own two 6.3 and 10.2.  us a step without / with, by groups and
+// blocks: 2 to 4 groups, 10 to 2048 blocks: 6.1 / 5.2 to 11.1 / 10.3, at worst 11.3 / 11.4.  5 to 8 groups, DENSE: 25 blocks 6.5 / 5.5,
+// 120 6.6 / 5.7, 200 7.0 / 7.0, 512 7.7 / 8.0, 728 7.8 / 8.4, 896 8.6 / 8.3, 1248 9.4 / 8.4, 4608 19.1 / 17.5; SPARSE: 25 blocks 6.7 / 5.6,
+// 400 8.8 / 8.1, 512 6.8 / 7.1, 728 7.1 / 6.8, 1248 9.1 / 8.3; STDP 10.7 / 10.1, 12.0 / 11.7, 10.9 / 10.7, 11.1 / 11.0, 12.5 / 12.0.
+// `blocks`: of 128 neurons, of all copies.  `dense`: the kernel before is one of a DENSE or BITMASK group.
+inline bool neuronStaged(unsigned int groups, unsigned long long blocks, unsigned int sms, bool dense)
+{
+    if(groups <= NEURON_STAGED_ANY) return true;
+    return groups <= NEURON_STAGED && (!dense || blocks <= sms || blocks >= 7u * sms);
+}
+
+inline size_t neuronTableBytes(unsigned int groups) { return sizeof(b200_neuron_group) * groups + sizeof(unsigned int) * (groups + 1u); }
+
+template<int NPSM, int NCS, int WORDS, bool STAGED>
 __global__ void __launch_bounds__(NEURON_BLOCK)
 neuronUpdateKernel(const NeuronLaunch L)
 {
     constexpr unsigned int PARTS = NEURON_BLOCK / (32 * WORDS);         // warps of a padded block
-    // (common.cuh: stageGroup)
-    __shared__ __align__(16) b200_neuron_group stagedGroups[NEURON_STAGED];
-    __shared__ unsigned int stagedStarts[NEURON_STAGED + 1];
-    const bool staged = L.num_groups <= NEURON_STAGED;
-    if(staged) {
-        stageWords(stagedGroups, L.groups, sizeof(b200_neuron_group) * L.num_groups);
-        stageWords(stagedStarts, L.block_start, sizeof(unsigned int) * (L.num_groups + 1u));
+    const b200_neuron_group *groups = L.groups;
+    const unsigned int *blockStart = L.block_start;
+    if constexpr(STAGED) {
+        // (common.cuh: stageGroup)
+        extern __shared__ __align__(16) unsigned char neuronTables[];
+        b200_neuron_group *const table = reinterpret_cast<b200_neuron_group*>(neuronTables);
+        unsigned int *const starts = reinterpret_cast<unsigned int*>(table + L.num_groups);
+        stageWordsAsync(table, L.groups, sizeof(b200_neuron_group) * L.num_groups);
+        stageWordsAsync(starts, L.block_start, sizeof(unsigned int) * (L.num_groups + 1u));
+        stagedWords();
         __syncthreads();
+        groups = table;
+        blockStart = starts;
     }
-    const b200_neuron_group *const groups = staged ? stagedGroups : L.groups;
-    const unsigned int *const blockStart = staged ? stagedStarts : L.block_start;
     const unsigned int blocks = blockStart[L.num_groups], launched = gridDim.x * gridDim.y;
     const unsigned int rank = blockIdx.y * gridDim.x + blockIdx.x;
     chainWait();

@@ -120,7 +120,7 @@ unsigned long long foldPeriod(unsigned long long period, unsigned int n)
 template<int P, int C>
 void launch(const NeuronLaunch &L, dim3 grid, cudaStream_t stream)
 {
-    neuronUpdateKernel<P, C, 1><<<grid, NEURON_BLOCK, 0, stream>>>(L);
+    neuronUpdateKernel<P, C, 1, false><<<grid, NEURON_BLOCK, 0, stream>>>(L);
 }
 }   // anonymous namespace
 

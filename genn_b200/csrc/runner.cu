@@ -2186,16 +2186,20 @@ int enqueueNeurons(b200_runner *r, unsigned long long numRec, bool capturing)
     const bool four = items >= (unsigned long long)sms * NEURON_WARPS_WANTED;
     const dim3 grid((unsigned int)std::min<unsigned long long>(four ? (items + 3u) / 4u : items, (unsigned long long)sms * NEURON_BLOCKS_PER_SM));
     int e = withNeuronShape(r, [&](auto P, auto C) -> int {
-        // (with many inputs or sources four words would not fit the registers)
-        if constexpr(decltype(P)::value + decltype(C)::value <= 4) {
-            if(four) {
-                CUDA_TRY(chain(r, neuronUpdateKernel<decltype(P)::value, decltype(C)::value, 4>, grid, NEURON_BLOCK, 0, L));
-                return B200_OK;
+        constexpr int NPSM = decltype(P)::value, NCS = decltype(C)::value;
+        auto launch = [&](dim3 blocks, auto *staged, auto *direct) -> int {
+            if(neuronStaged(L.num_groups, items, (unsigned int)sms, r->postSpanTable.num || r->denseTable.num)) {
+                CUDA_TRY(chain(r, staged, blocks, NEURON_BLOCK, neuronTableBytes(L.num_groups), L));
             }
+            else CUDA_TRY(chain(r, direct, blocks, NEURON_BLOCK, 0, L));
+            return B200_OK;
+        };
+        // (with many inputs or sources four words would not fit the registers)
+        if constexpr(NPSM + NCS <= 4) {
+            if(four) return launch(grid, neuronUpdateKernel<NPSM, NCS, 4, true>, neuronUpdateKernel<NPSM, NCS, 4, false>);
         }
-        const dim3 all((unsigned int)std::min<unsigned long long>(items, (unsigned long long)sms * NEURON_BLOCKS_PER_SM));
-        CUDA_TRY(chain(r, neuronUpdateKernel<decltype(P)::value, decltype(C)::value, 1>, all, NEURON_BLOCK, 0, L));
-        return B200_OK;
+        return launch(dim3((unsigned int)std::min<unsigned long long>(items, (unsigned long long)sms * NEURON_BLOCKS_PER_SM)),
+                      neuronUpdateKernel<NPSM, NCS, 1, true>, neuronUpdateKernel<NPSM, NCS, 1, false>);
     });
     if(e) return e;
     r->launches++;
