@@ -143,7 +143,7 @@ __device__ __forceinline__ void stageWords(void *dst, const void *src, size_t by
 
 // What a kernel needs of its group, into shared memory ahead of chainWait(): nothing writes a group's table while kernels run, and read
 // behind the wait every field that leads to an address cost another round trip to memory.  A step of DENSE 1200 x 1200 with 8 copies:
-// 8.25 -> 7.17 us (the DENSE kernel and the neuron update), of 5000 + 5000 neurons with 3 copies 9.18 -> 8.81.  (Shared memory is
+// 8.25 -> 7.00 us (the DENSE kernel and the neuron update), of 5000 + 5000 neurons with 3 copies 9.18 -> 8.81.  (Shared memory is
 // not free in kernels that use little else of it: neuronStaged.)
 template<typename T>
 __device__ __forceinline__ void stageGroup(T &shared, const T &group)

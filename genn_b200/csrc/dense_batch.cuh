@@ -12,7 +12,8 @@
 // memory, the masks' bits walked row by row, took 55 us at the size below, stages of half the columns brought in by all
 // threads 42, eight adding warps 33; now DRAM stands at two thirds of a copy's rate and the issue slots at 43 %.
 //
-// 8192 x 8192, 32 copies, 25 Hz at 1 ms (149 MB of rows a step): 107 us with presynapticPostSpanKernel, 31 here.
+// 8192 x 8192, 32 copies, 25 Hz at 1 ms (149 MB of rows a step): 107 us with presynapticPostSpanKernel, 31 here (a step with the neuron
+// update 36.5).
 #pragma once
 
 #include "common.cuh"
@@ -138,7 +139,7 @@ denseBatchKernel(const DenseLaunch L)
     if(warp == DENSE_WARPS) {
         unsigned int stage = 0;
         // Rows leave L2 before anything else does: the neurons' state, which the next kernel reads, stays there (8192 x 8192, 32
-        // copies: 39.1 -> 37.3 us a step; keeping an eighth, a quarter, half or all of the rows instead 37.0, 37.1, 37.9, 39.2)
+        // copies: a step with the neuron update 39.1 -> 37.3 us; keeping an eighth, a quarter, half or all of the rows instead 37.0, 37.1, 37.9, 39.2)
         unsigned long long soon;
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(soon));
         for(; stage < numStages; stage++) {

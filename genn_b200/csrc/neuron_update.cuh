@@ -553,8 +553,8 @@ neuronUpdateKernel(const NeuronLaunch L)
         extern __shared__ __align__(16) unsigned char neuronTables[];
         b200_neuron_group *const table = reinterpret_cast<b200_neuron_group*>(neuronTables);
         unsigned int *const starts = reinterpret_cast<unsigned int*>(table + L.num_groups);
-        // (small launches wait for the tables: one round trip.  Large ones, a step with loads / asynchronous copies: batched SPARSE 20 000 +
-        // 20 000 with 8 copies 39.2 / 39.8 us, DENSE 6556 x 5007 with 16 40.3 / 40.8, 8192 x 8192 with 32 39.8 / 38.9)
+        // (small launches wait for the tables: one round trip.  Large ones, a pass of 20 steps and its fetches with loads / asynchronous
+        // copies: batched SPARSE 20 000 + 20 000 with 8 copies 783 / 795 us, DENSE 6556 x 5007 with 16 765 / 775, 8192 x 8192 with 32 796 / 778)
         if constexpr(WORDS == 1) {
             stageWordsAsync(table, L.groups, sizeof(b200_neuron_group) * L.num_groups);
             stageWordsAsync(starts, L.block_start, sizeof(unsigned int) * (L.num_groups + 1u));

@@ -13,8 +13,8 @@
 // takes its 32 neurons through all steps on its own.  Two or three barriers of a CTA a window instead of a step, loads of a
 // window's runs side by side instead of a step's, and the wait for the messages once (FEED: hidden behind a window).
 //
-// us a step, step by step / in windows: 1000 sources -> 10 000 neurons, p = 0.1, 2 spikes a step 2.15 / 0.28; BITMASK 2003 -> 5009, 80
-// spikes 4.0 / 0.82; DENSE 4096 x 4096, 100 spikes 4.3 / 1.16; 100 000 neurons with conductances, 8 spikes, delay 10 2.7 / 1.13.
+// us a step of calls of 2000, step by step / in windows: 1000 sources -> 10 000 neurons, p = 0.1, 2 spikes a step 2.19 / 0.26; BITMASK
+// 2003 -> 5009, 80 spikes 3.75 / 0.49; DENSE 4096 x 4096, 100 spikes 3.88 / 0.85; 100 000 neurons with conductances, delay 10 2.67 / 1.32.
 // Cycles of a window of the last two: deliveries 7400 and 3500, updates 1000 and 5000, messages 4800 - 8500 and 9800.
 #pragma once
 
@@ -40,8 +40,8 @@ __device__ __forceinline__ void fenceGpu() { asm volatile("fence.acq_rel.gpu;" :
 
 // Spikes [from, to) of a step's list through a DENSE or BITMASK group onto 32 targets: a lane's sum.  (The whole warp calls; `from`
 // and the list are multiples of four entries.)  `mixed`: the list has spikes of other populations too.  A row's part is 128 bytes out
-// of L2 and an addition, so instructions count: with every choice made for every spike there were 49 for one, and DENSE 4096 x 4096 with
-// 100 spikes a step took 1.41 us a step in all; now 1.14.
+// of L2 and an addition, so instructions count: with every choice made for every spike there were 49 for one, and a step of DENSE
+// 4096 x 4096 with 100 spikes took 0.27 us longer.
 __device__ __forceinline__ float windowSpan(const ResidentSpan &S, const unsigned int *list, unsigned int from, unsigned int to, unsigned int unit, bool mixed, unsigned int &events)
 {
     const unsigned int lane = threadIdx.x & 31u, post = unit * 32u + lane, src = S.src_group, numTrg = S.num_trg;
@@ -370,7 +370,7 @@ residentWindowKernel(const __grid_constant__ ResidentWindowLaunch A)
     };
     // the CTA's message, by its last warp, behind a barrier behind the entries: a copy for every RESIDENT_READERS readers (resident.h).
     // Few entries travel with the head, which says of itself when it is there; more lie in the body, behind a fence (all in the body:
-    // 1000 -> 10 000 neurons 0.32 instead of 0.28 us a step, 100 000 neurons 1.38 instead of 1.13).
+    // 0.04 us a step longer with 1000 -> 10 000 neurons, 0.25 with 100 000).
     auto send = [&](unsigned int message) {
         if(warp != warps - 1u) return;
         const unsigned int n = sh.sent[message & 1u], at = (me % readers) * perReader + me / readers;

@@ -1702,7 +1702,11 @@ int buildResident(b200_runner *r)
     };
     if(windowed) {
         // (a window's messages cost little, and its deliveries and updates are shared by all SMs.  us a step on 48 / 100 / 148 CTAs: 1000 ->
-        // 10 000 neurons 0.33 / 0.32 / 0.32, BITMASK 2003 x 5009 0.93 / 0.88 / 0.82, DENSE 4096 x 4096 2.14 / 1.77 / 1.41)
+        // 10 000 neurons 0.30 / 0.26 / 0.26, BITMASK 2003 x 5009 0.60 / 0.50 / 0.49, DENSE 4096 x 4096 1.11 / 1.04 / 0.85, 100 000 neurons
+        // with conductances 1.35 / 1.36 / 1.32.)  Calls of one to three steps go through them one by one on the same grid, for which
+        // the synapses are laid out: us a call of 1 / 2 / 3 steps, here and on the grid of the rule below: 1000 -> 10 000 10.2 / 12.8 /
+        // 16.0 and 10.0 / 12.4 / 14.4, BITMASK 11.7 / 16.5 / 20.6 and 11.3 / 16.5 / 19.7, 5000 neurons with conductances 10.9 / 14.6 / 17.1 and
+        // 10.7 / 13.9 / 17.0, 100 000 14.3 / 20.8 / 26.2 and 14.5 / 20.7 / 26.2; with a fetch behind each call 30.0 - 50.4 and 30.0 - 50.0.
         const unsigned int G = std::min(std::max(r->residentCtas ? r->residentCtas : most, (units + RESIDENT_UNITS - 1u) / RESIDENT_UNITS), std::min(most, units));
         // Messages: room for every neuron in every step of `buffers` windows, about as much as a spike queue of that delay (100 000 neurons, 199
         // steps: 84 MB beside 81).  No more than a quarter of the free memory (what the pool may keep needs no asking).
